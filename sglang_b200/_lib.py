@@ -105,6 +105,28 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_host = None
+HOST_PATH = os.path.join(_PKG, "lib", "_sglb200_host.so")
+
+
+def host():
+    """The compiled host path (``csrc/torch_ops/host_path.cpp``), loaded on first use.  Raises if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        import torch  # noqa: F401  (the module links against torch's libraries)
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m sglang_b200.build_torch_ops`")
+        import importlib.machinery
+        import importlib.util
+        loader = importlib.machinery.ExtensionFileLoader("_sglb200_host", HOST_PATH)
+        spec = importlib.util.spec_from_file_location("_sglb200_host", HOST_PATH, loader=loader)
+        module = importlib.util.module_from_spec(spec)
+        loader.exec_module(module)
+        _host = module
+    return _host
+
+
 def check(status: int, what: str) -> None:
     if status != 0:
         L = lib()

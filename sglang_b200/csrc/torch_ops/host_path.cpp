@@ -1,0 +1,208 @@
+// Native host path of the layer-level entry points: one call from Python per layer instead of one per op.
+//
+// At decode sizes a linear layer is 8-50 us of GPU work, and the Python route to it (argument checks, three torch
+// allocations, two ctypes calls with ten to nineteen converted arguments each) took 55-60 us, so the host set the rate.
+// Here the same steps are compiled: checks on the tensors, one allocation for everything that does not outlive the
+// call (codes, scales, split-K scratch) and one for the result, then the C-ABI entry points on the current stream.
+//
+// Every function answers None when its arguments are not of the plain form it handles (another dtype, a view that needs
+// a copy, a bad shape, ...); the caller then takes the Python route, which handles or refuses them.  Nothing is launched
+// before all checks have passed.  The temporaries come from torch's caching allocator on the current stream and go back
+// to it when the call returns, which is stream-ordered like any tensor that goes out of scope.
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
+
+#include "../../../include/sglb200.h"
+
+namespace {
+
+// A C-ABI call that failed after the checks here: reported like the Python route does.
+struct LibraryError {
+  int rc;
+  const char* what;
+};
+
+inline void check_rc(int rc, const char* what) {
+  if (rc != 0) throw LibraryError{rc, what};
+}
+
+PyObject* raise(const LibraryError& e) {
+  PyErr_Format(PyExc_RuntimeError, "%s: %s (%s)", e.what, sglb200_status_string(e.rc), sglb200_last_error_detail());
+  return nullptr;
+}
+
+inline const at::Tensor* tensor_or_null(PyObject* o) {
+  return THPVariable_CheckExact(o) || THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
+}
+
+inline int64_t up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
+
+inline bool is16(at::ScalarType t) { return t == at::kBFloat16 || t == at::kHalf; }
+inline int code16(at::ScalarType t) { return t == at::kBFloat16 ? SGLB200_BF16 : SGLB200_F16; }
+
+// eps rounded to the input dtype, as the torch-native quantiser clamps; fp16 keeps the fp32 value where it rounds to 0
+inline float eps_in_dtype(double eps, at::ScalarType t) {
+  if (t == at::kFloat) return (float)eps;
+  const float v = t == at::kBFloat16 ? static_cast<float>(c10::BFloat16((float)eps)) : static_cast<float>(c10::Half((float)eps));
+  return v == 0.f && eps > 0. ? (float)eps : v;
+}
+
+inline at::Tensor empty(at::IntArrayRef sizes, at::ScalarType t, c10::Device dev) {
+  return at::Tensor(at::detail::empty_cuda(sizes, t, dev, c10::nullopt));
+}
+
+// Runs `f`; what it throws becomes the Python exception that torch or the Python route would raise.
+template <typename F>
+PyObject* guarded(F&& f) {
+  HANDLE_TH_ERRORS
+  try {
+    return f();
+  } catch (const LibraryError& e) {
+    return raise(e);
+  }
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------------------------------------- quantiser
+// quant(x, group_size, eps, fp8_min, fp8_max, column_major, tma_aligned, ue8m0, fuse_silu, masked_m) -> (codes, scales)
+PyObject* quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 10) Py_RETURN_NONE;
+  const at::Tensor* xp = tensor_or_null(args[0]);
+  const at::Tensor* mp = args[9] == Py_None ? nullptr : tensor_or_null(args[9]);
+  if (!xp || !PyLong_Check(args[1]) || (args[9] != Py_None && !mp)) Py_RETURN_NONE;
+  const at::Tensor& x = *xp;
+  const int64_t gs = PyLong_AsLong(args[1]);
+  const double eps = PyFloat_AsDouble(args[2]);
+  const double lo = PyFloat_AsDouble(args[3]), hi = PyFloat_AsDouble(args[4]);
+  if (PyErr_Occurred()) return nullptr;
+  const bool col = PyObject_IsTrue(args[5]) == 1, tma = PyObject_IsTrue(args[6]) == 1;
+  const bool ue = PyObject_IsTrue(args[7]) == 1, silu = PyObject_IsTrue(args[8]) == 1;
+  const int64_t dim = x.dim();
+  const at::ScalarType t = x.scalar_type();
+  if (!x.is_cuda() || !(dim == 2 || dim == 3) || !x.is_contiguous() || x.numel() == 0) Py_RETURN_NONE;
+  if (!(is16(t) || (t == at::kFloat && dim == 2)) || (ue && !(col && tma))) Py_RETURN_NONE;
+  const int64_t hidden_in = x.size(dim - 1), hidden = silu ? hidden_in / 2 : hidden_in;
+  if (gs <= 0 || hidden_in % gs != 0 || (silu && hidden_in % 2 != 0) || hidden % gs != 0) Py_RETURN_NONE;
+  const int64_t E = dim == 3 ? x.size(0) : 1, M = x.size(dim - 2), G = hidden / gs;
+  // a 3-D tensor with plain column-major scales keeps the Python route's shape rules
+  if (dim == 3 && col && !tma) Py_RETURN_NONE;
+  const int32_t* mptr = nullptr;
+  if (mp) {
+    if (dim != 3 || !mp->is_cuda() || mp->scalar_type() != at::kInt || !mp->is_contiguous() || mp->numel() != E) Py_RETURN_NONE;
+    mptr = mp->const_data_ptr<int32_t>();
+  }
+  return guarded([&]() -> PyObject* {
+    const c10::Device dev = x.device();
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    const int64_t W = ue ? (G + 3) / 4 : G;                       // scale words per row
+    const int64_t ld = col ? (tma ? up(M, 4) : M) : W;            // stride between word columns (or rows)
+    const at::ScalarType st = ue ? at::kInt : at::kFloat;
+    at::Tensor q, s;
+    if (dim == 2) {
+      q = empty({M, hidden}, at::kFloat8_e4m3fn, dev);
+      s = col ? empty({W, ld}, st, dev) : empty({M, W}, st, dev);
+      if (col) s.unsafeGetTensorImpl()->set_sizes_and_strides(at::IntArrayRef({M, W}), at::IntArrayRef({1, ld}));
+    } else {
+      q = empty({E, M, hidden}, at::kFloat8_e4m3fn, dev);
+      s = col ? empty({E, W, ld}, st, dev) : empty({E, M, W}, st, dev);
+      if (col) s.unsafeGetTensorImpl()->set_sizes_and_strides(at::IntArrayRef({E, M, W}), at::IntArrayRef({W * ld, 1, ld}));
+    }
+    const int code = t == at::kFloat ? SGLB200_F32 : code16(t);
+    const float e = eps_in_dtype(eps, t);
+    if (dim == 3)
+      check_rc(sglb200_group_quant_fp8_batched(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), E, M, hidden,
+                                               (int)gs, e, (float)lo, (float)hi, ue, silu, mptr, s.stride(0), s.stride(1),
+                                               s.stride(2), stream),
+               "sgl_per_token_group_quant_8bit(masked)");
+    else if (silu)
+      check_rc(sglb200_silu_mul_group_quant_fp8(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), nullptr, M,
+                                                hidden, (int)gs, e, (float)lo, (float)hi, ue, s.stride(0), s.stride(1), stream),
+               "sgl_per_token_group_quant_8bit(fuse_silu_and_mul)");
+    else
+      check_rc(sglb200_per_token_group_quant_fp8(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), M, hidden,
+                                                 (int)gs, e, (float)lo, (float)hi, ue, s.stride(0), s.stride(1), stream),
+               "sgl_per_token_group_quant_8bit");
+    PyObject* out = PyTuple_New(2);
+    if (!out) return nullptr;
+    PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(q)));
+    PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(std::move(s)));
+    return out;
+  });
+}
+
+// ---------------------------------------------------------------------------------------------- linear layer
+// block_linear(x, weight, weight_scale, bias, ue8m0) -> out: quantise the activations, multiply, add the bias.
+// weight_scale is fp32 [ceil(N/128), K/128], or with ue8m0 the packed int32 words [ceil(N/128), ceil(K/512)].
+PyObject* block_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 5) Py_RETURN_NONE;
+  const at::Tensor *xp = tensor_or_null(args[0]), *wp = tensor_or_null(args[1]), *sp = tensor_or_null(args[2]);
+  const at::Tensor* bp = args[3] == Py_None ? nullptr : tensor_or_null(args[3]);
+  if (!xp || !wp || !sp || (args[3] != Py_None && !bp)) Py_RETURN_NONE;
+  const at::Tensor &x = *xp, &w = *wp, &ws = *sp;
+  const bool ue = args[4] == Py_True;
+  const at::ScalarType t = x.scalar_type();
+  const int64_t dim = x.dim();
+  if (!x.is_cuda() || !is16(t) || dim < 1 || !x.is_contiguous() || x.numel() == 0) Py_RETURN_NONE;
+  if (w.scalar_type() != at::kFloat8_e4m3fn || w.dim() != 2 || !w.is_contiguous() || w.device() != x.device()) Py_RETURN_NONE;
+  const int64_t N = w.size(0), K = w.size(1), KB = K / 128, NB = (N + 127) / 128, KG = (KB + 3) / 4;
+  if (N == 0 || N % 8 != 0 || K == 0 || K % 128 != 0 || x.size(dim - 1) != K) Py_RETURN_NONE;
+  if (ws.scalar_type() != (ue ? at::kInt : at::kFloat) || ws.dim() != 2 || ws.size(0) != NB || ws.size(1) != (ue ? KG : KB) ||
+      ws.device() != x.device())
+    Py_RETURN_NONE;
+  if (bp && (bp->device() != x.device() || bp->scalar_type() != t || bp->requires_grad())) Py_RETURN_NONE;
+  const int64_t M = x.numel() / K;
+  return guarded([&]() -> PyObject* {
+    const c10::Device dev = x.device();
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    const c10::cuda::CUDAStream cs = c10::cuda::getCurrentCUDAStream(dev.index());
+    void* stream = cs.stream();
+    at::DimVector shape(x.sizes().begin(), x.sizes().end());
+    shape[dim - 1] = N;
+    at::Tensor out = empty(shape, t, dev);
+    // one block: split-K scratch | scales (M-major, rows padded to 4) | codes
+    const int64_t ld = up(M, 4), words = ue ? KG : KB;
+    int64_t ws_bytes = !ue || M <= 64 ? sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) : 0;
+    const int64_t scale_at = up(ws_bytes, 512), code_at = scale_at + up(words * ld * 4, 512);
+    c10::DataPtr block = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)(code_at + M * K));
+    char* base = static_cast<char*>(block.get());
+    void *scratch = ws_bytes > 0 ? base : nullptr, *scales = base + scale_at, *codes = base + code_at;
+    const int code = code16(t);
+    check_rc(sglb200_per_token_group_quant_fp8(x.const_data_ptr(), code, codes, scales, M, K, 128, eps_in_dtype(1e-10, t),
+                                               -448.f, 448.f, ue, 1, ld, stream),
+             "sgl_per_token_group_quant_8bit");
+    if (ue)
+      check_rc(sglb200_fp8_ue8m0_scaled_mm_ws(codes, w.const_data_ptr(), static_cast<const int32_t*>(scales),
+                                              ws.const_data_ptr<int32_t>(), out.mutable_data_ptr(), M, N, K, K, K, N, ld,
+                                              ws.stride(0), ws.stride(1), code, scratch, ws_bytes, stream),
+               "w8a8_block_fp8_matmul_ue8m0");
+    else if (ws_bytes > 0)
+      check_rc(sglb200_fp8_blockwise_scaled_mm_ws(codes, w.const_data_ptr(), static_cast<const float*>(scales),
+                                                  ws.const_data_ptr<float>(), out.mutable_data_ptr(), M, N, K, K, K, N, 1, ld,
+                                                  ws.stride(0), ws.stride(1), code, scratch, ws_bytes, stream),
+               "fp8_blockwise_scaled_mm (split-K)");
+    else
+      check_rc(sglb200_fp8_blockwise_scaled_mm(codes, w.const_data_ptr(), static_cast<const float*>(scales),
+                                               ws.const_data_ptr<float>(), out.mutable_data_ptr(), M, N, K, K, K, N, 1, ld,
+                                               ws.stride(0), ws.stride(1), code, stream),
+               "fp8_blockwise_scaled_mm");
+    if (bp) out.add_(*bp);
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
+PyMethodDef kMethods[] = {
+    {"quant", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(quant)), METH_FASTCALL, nullptr},
+    {"block_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(block_linear)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_sglb200_host", nullptr, -1, kMethods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__sglb200_host() { return PyModule_Create(&kModule); }

@@ -10,7 +10,7 @@ from typing import Any, Dict, List, Optional
 import torch
 from torch.nn import Module, Parameter
 
-from .fp8_utils import dispatch_w8a8_block_fp8_linear
+from .fp8_utils import dispatch_w8a8_block_fp8_linear, w8a8_block_fp8_linear_ue8m0
 
 
 class Fp8Config:
@@ -112,10 +112,14 @@ class Fp8LinearMethod:
 
     def apply(self, layer: Module, x: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``Fp8LinearMethod.apply`` (``fp8.py:453-499``, block-quant branch ``:482-489``)."""
+        # Module.__getattr__ costs about a microsecond per parameter; the parameter table is a plain attribute
+        params = layer._parameters
+        weight = params.get("weight")
+        if weight is None:
+            weight = layer.weight
         packed = getattr(layer, "weight_scale_ue8m0", None)
         if packed is not None:
-            from .fp8_utils import w8a8_block_fp8_linear_ue8m0
-            return w8a8_block_fp8_linear_ue8m0(x, layer.weight, packed, bias)
-        return self.w8a8_block_fp8_linear(input=x, weight=layer.weight,
-                                          block_size=self.quant_config.weight_block_size,
-                                          weight_scale=layer.weight_scale_inv, input_scale=None, bias=bias)
+            return w8a8_block_fp8_linear_ue8m0(x, weight, packed, bias)
+        scale = params.get("weight_scale_inv")
+        return self.w8a8_block_fp8_linear(x, weight, self.quant_config.weight_block_size,
+                                          layer.weight_scale_inv if scale is None else scale, None, bias)

@@ -9,7 +9,7 @@ from typing import List, Optional, Tuple
 import torch
 
 from ...sgl_kernel import fp8_blockwise_scaled_mm, sgl_per_token_group_quant_8bit
-from ..._lib import blockwise_mm, check, dtype_code, lib
+from ..._lib import blockwise_mm, check, dtype_code, host, lib
 
 fp8_dtype = torch.float8_e4m3fn
 fp8_max = torch.finfo(fp8_dtype).max
@@ -58,6 +58,10 @@ def sglang_per_token_group_quant_fp8(
     ``(x_q e4m3, x_s)`` with ``x_s`` in the requested layout.  With a 3-D ``x [E, max_m, K]`` the scales are laid out
     per expert, and ``masked_m [E]`` (int32) limits the work to the first ``masked_m[e]`` rows of every expert; the
     other rows of ``x_q`` / ``x_s`` are left unwritten (``per_token_group_quant_8bit_v2.cu:194-238``)."""
+    done = host().quant(x, group_size, eps, fp8_min, fp8_max, column_major_scales, scale_tma_aligned, scale_ue8m0,
+                        fuse_silu_and_mul, masked_m)
+    if done is not None:
+        return done
     assert x.shape[-1] % group_size == 0, "the last dimension of `x` cannot be divisible by `group_size`"
     assert x.is_contiguous(), "`x` is not contiguous"
     assert x.dim() in (2, 3), "activations must be [M, K] or, for the masked per-expert layout, [E, max_m, K]"

@@ -6,6 +6,7 @@ from typing import List, Optional
 
 import torch
 
+from ..._lib import host
 from .fp8_kernel import sglang_per_token_group_quant_fp8, w8a8_block_fp8_matmul, w8a8_block_fp8_matmul_ue8m0
 
 
@@ -20,6 +21,10 @@ def w8a8_block_fp8_linear(input: torch.Tensor, weight: torch.Tensor, block_size:
     [ceil(N/128), ceil(K/128)]`` fp32.  Activation scales are written M-major so the GEMM's
     per-row scale loads coalesce."""
     assert input_scale is None
+    if block_size[0] == 128 and block_size[1] == 128:
+        done = host().block_linear(input, weight, weight_scale, bias, False)
+        if done is not None:
+            return done
     input_2d = input.view(-1, input.shape[-1])
     if not input_2d.is_contiguous():
         input_2d = input_2d.contiguous()
@@ -51,6 +56,9 @@ def w8a8_block_fp8_linear_ue8m0(input: torch.Tensor, weight: torch.Tensor, weigh
     """The linear for UE8M0 checkpoints, the counterpart of ``deepgemm_w8a8_block_fp8_linear_with_fallback`` on
     Blackwell (``fp8_utils.py:217-255``): activations quantised with power-of-two group scales (packed int32,
     M-major), then the hardware block-scaled GEMM.  ``weight_scale_packed`` comes from ``pack_ue8m0_scales``."""
+    done = host().block_linear(input, weight, weight_scale_packed, bias, True)
+    if done is not None:
+        return done
     input_2d = input.view(-1, input.shape[-1])
     if not input_2d.is_contiguous():
         input_2d = input_2d.contiguous()
