@@ -344,12 +344,14 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   // ---------------------------------------------------------------- roles
   // The per-k-block loops of the producer and the MMA issuer are a serial chain for one warp, so they
   // are kept to a handful of instructions: barrier and tile addresses live in registers as 32-bit
-  // shared-window addresses, every lane waits (no divergence to repair) and lane 0 alone issues.
+  // shared-window addresses, every lane waits (no divergence to repair) and one elected lane issues.
   const uint32_t full0 = ptx::smem_u32(&ctl->full[0]);
   const uint32_t empty0 = ptx::smem_u32(&ctl->empty[0]);
   const uint32_t acc_full0 = ptx::smem_u32(&ctl->acc_full[0]);
   const uint32_t acc_empty0 = ptx::smem_u32(&ctl->acc_empty[0]);
   const uint32_t stage0 = ptx::smem_u32(stage_base);
+
+  const bool leader = ptx::elect_one();  // the lane that issues TMA and tcgen05 instructions
 
   if (is_comm) {
     if constexpr (AR) {
@@ -421,7 +423,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           }
           armed |= 1u << stage;
           armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
-          if (lane == 0) {
+          if (leader) {
             const uint32_t dst = stage0 + stage * kStageBytes;
             ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, kStageBytes);
             ptx::tma_load_2d_a(dst, &map_a, full0 + stage * 8, kb * BK, tl.row0);
@@ -473,7 +475,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             break;
           }
           ptx::tc_fence_after();
-          if (lane == 0) {
+          if (leader) {
             // descriptors differ from stage 0's only in the 16-byte address field
             const uint64_t a_desc = desc0 + (uint64_t)(stage * (kStageBytes >> 4));
             const uint64_t b_desc = a_desc + (kTileABytes >> 4);

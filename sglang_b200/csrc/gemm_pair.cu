@@ -179,6 +179,7 @@ fp8_block_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
       asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
     }
   }
+  const bool leader = ptx::elect_one();  // the lane that issues TMA and tcgen05 instructions
   if (warp < kProducers) {
     uint32_t stage = 0, phase = 0, g = 0;
     uint32_t armed = 0, armed_phase = 0;  // bit i: this warp has armed stage i / the phase bit of its last arming
@@ -196,7 +197,7 @@ fp8_block_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
           }
           armed |= 1u << stage;
           armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
-          if (lane == 0) {
+          if (leader) {
             const uint32_t dst = stage0 + stage * C::kStage;
             if (rank == 0) ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, 2 * C::kStage);  // both CTAs' bytes
             ptx::tma_load_2d_pair(dst, &map_a, lead_full0 + stage * 8, kb * 128, row0);
@@ -245,7 +246,7 @@ fp8_block_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
               break;
             }
             ptx::tc_fence_after();
-            if (lane == 0) {
+            if (leader) {
               const uint64_t a_desc = desc0 + (uint64_t)(stage * (C::kStage >> 4));
               const uint64_t b_desc = a_desc + (C::kTileA >> 4);
               const uint32_t d_tmem = tmem_base + acc * BN;

@@ -273,6 +273,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
 
   if (threadIdx.x == 0) ptx::grid_dep_launch();  // the next kernel of the stream may begin its own set-up
 
+  const bool leader = ptx::elect_one();  // the lane that issues TMA and tcgen05 instructions
   if (warp == 0) {
     // ===== TMA producer.  Pass 0 runs before griddepcontrol.wait: the weight tiles of the first k-blocks (at most one
     // ring of stages, whose barriers are fresh) are requested; pass 1 adds their activation tiles and then continues
@@ -289,7 +290,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
           const uint32_t dst = stage0 + stage * C::kStageBytes;
           if (pass == 0) {
             if (idx >= (uint32_t)C::kStages) { ok = false; break; }
-            if (lane == 0) {
+            if (leader) {
               ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, C::kStageBytes);
               ptx::tma_load_3d_a(dst, &map_w, full0 + stage * 8, kb * BK, nt * BN, 0);
             }
@@ -297,14 +298,14 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
             armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
             pre = idx + 1;
           } else if (idx < pre) {
-            if (lane == 0) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, 0);
+            if (leader) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, 0);
           } else {
             if (!ptx::mbar_wait_a(empty0 + stage * 8, phase ^ 1)) {
               timeout(ctl, 11);
               ok = false;
               break;
             }
-            if (lane == 0) {
+            if (leader) {
               ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, C::kStageBytes);
               ptx::tma_load_3d_a(dst, &map_w, full0 + stage * 8, kb * BK, nt * BN, it.e);
               ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, it.row0);
@@ -347,7 +348,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         if (!ptx::mbar_wait_a(acc_empty0 + acc * 8, acc_phase ^ 1)) { timeout(ctl, 12); ok = false; break; }
         if (!ptx::mbar_wait_a(full0 + stage * 8, phase)) { timeout(ctl, 13); ok = false; break; }
         ptx::tc_fence_after();
-        if (lane == 0) {
+        if (leader) {
           const uint64_t w_desc = desc0 + (uint64_t)(stage * (C::kStageBytes >> 4));
           const uint64_t a_desc = w_desc + (kWBytes >> 4);
           const uint32_t d_tmem = tmem_base + acc * C::kTile;

@@ -248,6 +248,7 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const uint32_t stage0 = ptx::smem_u32(smem);
   const uint32_t sf0 = ptx::smem_u32(sf_smem);
 
+  const bool leader = ptx::elect_one();  // the lane that issues TMA and tcgen05 instructions
   if (warp < 2) {
     // ===== TMA producers
     uint32_t stage = 0, phase = 0, g = 0;
@@ -261,7 +262,7 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             ok = false;
             break;
           }
-          if (lane == 0) {
+          if (leader) {
             const uint32_t dst = stage0 + stage * kStageBytes;
             ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, kStageBytes);
             ptx::tma_load_2d_a(dst, &map_a, full0 + stage * 8, kb * BK, tl.m0);
@@ -299,7 +300,7 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
         ptx::tc_fence_after();
         const uint32_t sf_col = tmem_base + kSfTmemBase + (q & 1) * kSfTmemPerSet;
-        if (lane == 0) {
+        if (leader) {
           const uint32_t src = sf0 + buf * kSfBufBytes;
           ptx::tmem_cp_32x128b_warpx4(sf_col, ptx::make_sf_desc(src));
           ptx::tmem_cp_32x128b_warpx4(sf_col + 4, ptx::make_sf_desc(src + kSfABytes));
@@ -314,7 +315,7 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             break;
           }
           ptx::tc_fence_after();
-          if (lane == 0) {
+          if (leader) {
             const uint64_t a_desc = desc0 + (uint64_t)(stage * (kStageBytes >> 4));
             const uint64_t b_desc = a_desc + (kTileABytes >> 4);
             const uint32_t idesc = ptx::make_idesc_mxf8(BM, BN, (uint32_t)(kb & 3));
@@ -328,7 +329,7 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
       }
       if (!ok || ctl->abort_flag) break;
-      if (lane == 0) ptx::mma_commit_a(acc_full0 + as * 8);  // the tile is complete when everything issued so far is
+      if (leader) ptx::mma_commit_a(acc_full0 + as * 8);  // the tile is complete when everything issued so far is
     }
   } else if (warp == 4) {
     // ===== scale loader
