@@ -3,8 +3,10 @@
 //   out[m, n] = cast( sum_kb ( sum_{k in kb} a[m,k] * b[n,k] ) * sa[m,kb] * sb[n/128,kb] )
 //
 // One CTA per SM, 384 threads, warp-specialised:
-//   warps 0-1  TMA producers (k-blocks alternate between them): A tile [128 rows x 128 B] and B tile [128 rows x 128 B] per k-block into a
+//   warp 0     TMA producer: A tile [128 rows x 128 B] and B tile [128 rows x 128 B] per k-block into a
 //              6-stage ring of 128-byte-swizzled shared memory (32 KiB per stage).
+//   warp 1     scale loader: per group of four k-blocks the 128 x 4 products sa[m, kb] * sb[n/128, kb] into a four-deep
+//              ring of shared memory, one 16-byte vector per tile row.
 //   warps 2-3  MMA issuers (k-blocks alternate): per k-block four tcgen05.mma (128 x 128 x 32, e4m3 -> f32) that OVERWRITE one of
 //              four 128-column TMEM accumulator stages, then tcgen05.commit to free the smem stage and to
 //              publish the TMEM stage.
@@ -12,9 +14,11 @@
 //              columns.  A thread owns one accumulator row: per k-block it pulls its 64 partial sums out
 //              of TMEM (two tcgen05.ld of 32 columns, one wait), multiplies by sa[m,kb] * sb[nb,kb] and
 //              adds into 64 fp32 registers with packed fp32x2 FMAs; after the last k-block it rounds to
-//              bf16/f16 and writes 128 contiguous bytes of the output row.  Scales are fetched four
-//              k-blocks ahead so their latency never sits on the promotion path.  Two warps per quarter
-//              hide each other's TMEM-load latency.
+//              bf16/f16 and writes 128 contiguous bytes of the output row.  The scale of a row comes from the scale
+//              loader's ring with one 16-byte load per four k-blocks: with the promotion warps loading sa and sb
+//              themselves (two global loads with 64-bit addresses per k-block, four k-blocks ahead) a k-block took
+//              580 cycles instead of 427, whatever the latency of the loads.  Two warps per quarter hide each
+//              other's TMEM-load latency.
 // The four TMEM stages let the tensor core run up to four k-blocks ahead of the promotion warps, and the
 // promotion of tile i's tail overlaps the loads and MMAs of tile i+1.
 //
@@ -38,10 +42,12 @@ constexpr int BM = 128, BN = 128, BK = 128;
 constexpr int kStages = 6;
 constexpr int kAccStages = 4;
 constexpr int kThreads = 384;
-constexpr int kIssuers = 2;  // producer warps and MMA warps: each pair splits the k-blocks even/odd
+constexpr int kIssuers = 2;  // MMA warps: they split the k-blocks even/odd
+constexpr int kFirstMmaWarp = 2, kFirstPromoWarp = 4;
 constexpr int kEpiWarps = 8;
 constexpr int kEpiCols = BN / (kEpiWarps / 4);  // columns per promotion warp (64)
-constexpr int kScaleAhead = 4;                 // k-blocks of scale prefetch
+constexpr int kScaleGroup = 4;    // k-blocks per scale vector
+constexpr int kScaleStages = 4;   // scale vectors in flight per tile row
 constexpr uint32_t kTileABytes = BM * BK;
 constexpr uint32_t kTileBBytes = BN * BK;
 constexpr uint32_t kStageBytes = kTileABytes + kTileBBytes;
@@ -51,8 +57,8 @@ constexpr int kGroupM = 16;  // m-tiles per raster group (dense)
 constexpr int kGroupMAr = 16;  // the same in the GEMM with the fused all-reduce: a raster group is the unit that is
                                // reduced over the ranks, and the reduction of the LAST group is not hidden (8 measured
                                // 2-3 % slower at eight ranks: twice the barriers for half the exposed tail)
-constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + (size_t)kStages * kStageBytes + 256 /*barriers*/ +
-                              (kMaxExperts + 1) * sizeof(int32_t);
+constexpr size_t kScaleOffset = (((size_t)kStages * kStageBytes + 256 /*barriers*/ + (kMaxExperts + 1) * sizeof(int32_t)) + 15) / 16 * 16;
+constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + kScaleOffset + (size_t)kScaleStages * BM * sizeof(float4);
 
 // Push epilogue (dense, one tile per (m, n)): instead of writing `out`, every output tile is stored into the receive
 // buffer of every rank, in the slot of this rank, and flagged there.  Receive buffer of a rank:
@@ -77,7 +83,7 @@ struct PushParams {
 // through a private [32 rows][kStageWords] patch of shared memory, 16 payload words per row and pass.
 constexpr int kStageWords = 20;  // 80-byte row stride: 16-byte aligned, conflict-free for the per-lane uint4 writes
 constexpr size_t kStagingBytes = (size_t)kEpiWarps * 32 * kStageWords * sizeof(uint32_t);
-constexpr size_t kStagingOffset = (((size_t)kStages * kStageBytes + 256 + (kMaxExperts + 1) * sizeof(int32_t)) + 15) / 16 * 16;
+constexpr size_t kStagingOffset = kScaleOffset + (size_t)kScaleStages * BM * sizeof(float4);
 constexpr size_t kSmemBytesPush = 1024 + kStagingOffset + kStagingBytes;
 
 struct GemmParams {
@@ -141,10 +147,13 @@ struct SharedCtl {
   uint64_t empty[kStages];
   uint64_t acc_full[kAccStages];
   uint64_t acc_empty[kAccStages];
+  uint64_t sc_full[kScaleStages];
+  uint64_t sc_empty[kScaleStages];
   uint32_t tmem_base;
   volatile int32_t abort_flag;
   int32_t total_tiles;
 };
+static_assert(sizeof(SharedCtl) <= 256, "control block");
 
 // bounded wait; fully inlined where the register limit of the warp was changed (no call allowed there)
 template <bool INLINE>
@@ -288,13 +297,17 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       ptx::mbar_init(&ctl->acc_full[i], 1);
       ptx::mbar_init(&ctl->acc_empty[i], kEpiWarps);  // one arrival per promotion warp
     }
+    for (int i = 0; i < kScaleStages; ++i) {
+      ptx::mbar_init(&ctl->sc_full[i], 1);
+      ptx::mbar_init(&ctl->sc_empty[i], kEpiWarps);
+    }
     ctl->abort_flag = 0;
     ptx::fence_barrier_init();
     ptx::fence_proxy_async();
     ptx::prefetch_tensormap(&map_a);
     ptx::prefetch_tensormap(&map_b);
   }
-  if (warp == kIssuers) {
+  if (warp == kFirstMmaWarp) {
     ptx::tmem_alloc(&ctl->tmem_base, kTmemCols);
     ptx::tmem_relinquish();
   }
@@ -349,6 +362,9 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const uint32_t empty0 = ptx::smem_u32(&ctl->empty[0]);
   const uint32_t acc_full0 = ptx::smem_u32(&ctl->acc_full[0]);
   const uint32_t acc_empty0 = ptx::smem_u32(&ctl->acc_empty[0]);
+  const uint32_t sc_full0 = ptx::smem_u32(&ctl->sc_full[0]);
+  const uint32_t sc_empty0 = ptx::smem_u32(&ctl->sc_empty[0]);
+  float4* scale_ring = reinterpret_cast<float4*>(smem + kScaleOffset);  // [kScaleStages][BM]
   const uint32_t stage0 = ptx::smem_u32(stage_base);
 
   const bool leader = ptx::elect_one();  // the lane that issues TMA and tcgen05 instructions
@@ -405,30 +421,26 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                            &g_device_status, 8);
       if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t*>(ctlw) = epoch0 + (uint32_t)row_blocks;
     }
-  } else if (warp < kIssuers) {
-    // ===== TMA producers.  Issuing a TMA or an MMA and touching an mbarrier each cost the issuing
-    // thread on the order of a hundred cycles, and the tensor pipe does not queue far ahead, so one
-    // warp per role cannot feed it: two warps per role take the k-blocks of the CTA alternately.
-    uint32_t stage = 0, phase = 0, g = 0;
+  } else if (warp == 0) {
+    // ===== TMA producer
+    uint32_t stage = 0, phase = 0;
     uint32_t armed = 0, armed_phase = 0;  // bit i: this warp has armed stage i / the phase bit of its last arming
     for (int32_t t = blockIdx.x; t < total_tiles; t += tile_stride) {
       const Tile tl = get_tile<GROUPED, AR ? kGroupMAr : kGroupM>(p, tile_start, t);
       bool ok = true;
-      for (int32_t kb = tl.kb0; kb < tl.kb1; ++kb, ++g) {
-        if ((g & (kIssuers - 1)) == (uint32_t)warp) {
-          if (!wait_bar<false>(empty0 + stage * 8, phase ^ 1)) {
-            record_timeout(ctl, 1);
-            ok = false;
-            break;
-          }
-          armed |= 1u << stage;
-          armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
-          if (leader) {
-            const uint32_t dst = stage0 + stage * kStageBytes;
-            ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, kStageBytes);
-            ptx::tma_load_2d_a(dst, &map_a, full0 + stage * 8, kb * BK, tl.row0);
-            ptx::tma_load_3d_a(dst + kTileABytes, &map_b, full0 + stage * 8, kb * BK, tl.n0, tl.expert);
-          }
+      for (int32_t kb = tl.kb0; kb < tl.kb1; ++kb) {
+        if (!wait_bar<false>(empty0 + stage * 8, phase ^ 1)) {
+          record_timeout(ctl, 1);
+          ok = false;
+          break;
+        }
+        armed |= 1u << stage;
+        armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
+        if (leader) {
+          const uint32_t dst = stage0 + stage * kStageBytes;
+          ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, kStageBytes);
+          ptx::tma_load_2d_a(dst, &map_a, full0 + stage * 8, kb * BK, tl.row0);
+          ptx::tma_load_3d_a(dst + kTileABytes, &map_b, full0 + stage * 8, kb * BK, tl.n0, tl.expert);
         }
         if (++stage == kRing) { stage = 0; phase ^= 1; }
       }
@@ -443,15 +455,57 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     // Tail: tcgen05.commit arrives on the `empty` barriers asynchronously and nobody waits for the last ones, so the
     // CTA could exit (and the next kernel's CTA re-initialise barriers at the same shared-memory addresses) while
     // such an arrival is still in flight.  Acquire every stage once more before leaving.
-    if (warp == 0 && !ctl->abort_flag) {
+    if (!ctl->abort_flag) {
       for (int i = 0; i < kRing; ++i) {
         if (!wait_bar<false>(empty0 + stage * 8, phase ^ 1)) { record_timeout(ctl, 5); break; }
         if (++stage == kRing) { stage = 0; phase ^= 1; }
       }
     }
-  } else if (warp < 2 * kIssuers) {
+  } else if (warp == 1) {
+    // ===== scale loader: lane l serves the tile rows l, l + 32, l + 64, l + 96
+    uint32_t stage = 0, phase = 0;
+    for (int32_t t = blockIdx.x; t < total_tiles; t += tile_stride) {
+      const Tile tl = get_tile<GROUPED, AR ? kGroupMAr : kGroupM>(p, tile_start, t);
+      const float* sa_row[BM / 32];
+#pragma unroll
+      for (int j = 0; j < BM / 32; ++j) {
+        const int32_t row = min(tl.row0 + lane + 32 * j, p.total_rows - 1);
+        sa_row[j] = p.sa + (int64_t)row * p.sa_stride_m;
+        if constexpr (GROUPED) {
+          if (p.rows_per_expert > 0)
+            sa_row[j] = p.sa + (int64_t)tl.expert * p.sa_stride_e +
+                        (int64_t)(row - tl.expert * p.rows_per_expert) * p.sa_stride_m;
+        }
+      }
+      const float* sb_blk = p.sb + (int64_t)tl.expert * p.sb_stride_e + (int64_t)(tl.n0 / BN) * p.sb_stride_n;
+      bool ok = true;
+      for (int32_t kb0 = tl.kb0; kb0 < tl.kb1; kb0 += kScaleGroup) {
+        float a[BM / 32][kScaleGroup], b[kScaleGroup];
+#pragma unroll
+        for (int u = 0; u < kScaleGroup; ++u) {
+          const int32_t kb = min(kb0 + u, tl.kb1 - 1);
+          const int64_t ka = (int64_t)kb * p.sa_stride_k;
+          b[u] = __ldg(sb_blk + (int64_t)kb * p.sb_stride_k);
+#pragma unroll
+          for (int j = 0; j < BM / 32; ++j) a[j][u] = __ldg(sa_row[j] + ka);
+        }
+        if (!wait_bar<false>(sc_empty0 + stage * 8, phase ^ 1)) {
+          record_timeout(ctl, 9);
+          ok = false;
+          break;
+        }
+#pragma unroll
+        for (int j = 0; j < BM / 32; ++j)
+          scale_ring[stage * BM + lane + 32 * j] = make_float4(a[j][0] * b[0], a[j][1] * b[1], a[j][2] * b[2], a[j][3] * b[3]);
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_a(sc_full0 + stage * 8);
+        if (++stage == kScaleStages) { stage = 0; phase ^= 1; }
+      }
+      if (!ok || ctl->abort_flag) break;
+    }
+  } else if (warp < kFirstPromoWarp) {
     // ===== MMA issuers (k-blocks alternate between the two warps; each k-block has its own TMEM stage)
-    const uint32_t me = warp - kIssuers;
+    const uint32_t me = warp - kFirstMmaWarp;
     constexpr uint32_t idesc = ptx::make_idesc_e4m3_f32(BM, BN);
     const uint64_t desc0 = ptx::make_kmajor_sw128_desc(stage0);
     uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, g = 0;
@@ -498,44 +552,33 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   } else {
     // ===== promotion + epilogue (warps 4..11); TMEM lane quarter = warp % 4, column half = (warp - 4) / 4
     const int q = warp & 3;
-    const int col0 = ((warp - 2 * kIssuers) >> 2) * kEpiCols;
+    const int col0 = ((warp - kFirstPromoWarp) >> 2) * kEpiCols;
     const int r_in_tile = q * 32 + lane;
-    uint32_t acc_stage = 0, acc_phase = 0;
+    uint32_t acc_stage = 0, acc_phase = 0, sc_stage = 0, sc_phase = 0;
     float2 acc[kEpiCols / 2];
     uint32_t push_epoch = 0;
     if constexpr (PUSH) push_epoch = *reinterpret_cast<const volatile uint32_t*>(p.push.ctl) + 1u;
     for (int32_t t = blockIdx.x; t < total_tiles; t += tile_stride) {
       const Tile tl = get_tile<GROUPED, AR ? kGroupMAr : kGroupM>(p, tile_start, t);
       const int32_t row = tl.row0 + r_in_tile;
-      const int32_t row_c = min(row, p.total_rows - 1);
-      const float* sa_row = p.sa + (int64_t)row_c * p.sa_stride_m;
-      if constexpr (GROUPED) {
-        if (p.rows_per_expert > 0)
-          sa_row = p.sa + (int64_t)tl.expert * p.sa_stride_e +
-                   (int64_t)(row_c - tl.expert * p.rows_per_expert) * p.sa_stride_m;
-      }
-      const float* sb_blk = p.sb + (int64_t)tl.expert * p.sb_stride_e + (int64_t)(tl.n0 / BN) * p.sb_stride_n;
 #pragma unroll
       for (int j = 0; j < kEpiCols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
-      float sa_ring[kScaleAhead], sb_ring[kScaleAhead];
-#pragma unroll
-      for (int u = 0; u < kScaleAhead; ++u) {
-        const int32_t kc = min(tl.kb0 + u, tl.kb1 - 1);
-        sa_ring[u] = __ldg(sa_row + (int64_t)kc * p.sa_stride_k);
-        sb_ring[u] = __ldg(sb_blk + (int64_t)kc * p.sb_stride_k);
-      }
       bool ok = true;
-      for (int32_t kb0 = tl.kb0; kb0 < tl.kb1 && ok; kb0 += kScaleAhead) {
+      for (int32_t kb0 = tl.kb0; kb0 < tl.kb1 && ok; kb0 += kScaleGroup) {
+        if (!wait_bar<false>(sc_full0 + sc_stage * 8, sc_phase)) {
+          record_timeout(ctl, 10);
+          ok = false;
+          break;
+        }
+        const float4 sv = scale_ring[sc_stage * BM + r_in_tile];
+        const float sc[kScaleGroup] = {sv.x, sv.y, sv.z, sv.w};
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_a(sc_empty0 + sc_stage * 8);
+        if (++sc_stage == kScaleStages) { sc_stage = 0; sc_phase ^= 1; }
 #pragma unroll
-        for (int u = 0; u < kScaleAhead; ++u) {
-          const int32_t kb = kb0 + u;
-          if (kb >= tl.kb1) break;
-          const float scale = sa_ring[u] * sb_ring[u];
-          {  // fetch the scales of k-block kb + kScaleAhead into the slot just consumed
-            const int32_t kn = min(kb + kScaleAhead, tl.kb1 - 1);
-            sa_ring[u] = __ldg(sa_row + (int64_t)kn * p.sa_stride_k);
-            sb_ring[u] = __ldg(sb_blk + (int64_t)kn * p.sb_stride_k);
-          }
+        for (int u = 0; u < kScaleGroup; ++u) {
+          if (kb0 + u >= tl.kb1) break;
+          const float scale = sc[u];
           const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc_stage * BN + col0;
           const float2 scale2 = make_float2(scale, scale);
           {
@@ -565,7 +608,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         const int32_t n_first = tl.n0 + col0;
         const int32_t tile_id = (tl.row0 / BM) * p.n_tiles + tl.n0 / BN;
         const int owner = tile_id % p.push.world;
-        const int wi = warp - 2 * kIssuers;
+        const int wi = warp - kFirstPromoWarp;
         uint32_t* stg = reinterpret_cast<uint32_t*>(smem + kStagingOffset) + wi * 32 * kStageWords;
         const int32_t row_base = tl.row0 + q * 32;  // the warp's rows are row_base + 0..31
         const uint32_t set = push_epoch & 1u;
@@ -632,7 +675,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   // ---------------------------------------------------------------- tear-down
   ptx::tc_fence_before();
   __syncthreads();
-  if (warp == kIssuers) {
+  if (warp == kFirstMmaWarp) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, kTmemCols);
   }
