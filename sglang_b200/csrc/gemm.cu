@@ -58,7 +58,6 @@ constexpr int kGroupMAr = 16;  // the same in the GEMM with the fused all-reduce
                                // reduced over the ranks, and the reduction of the LAST group is not hidden (8 measured
                                // 2-3 % slower at eight ranks: twice the barriers for half the exposed tail)
 constexpr size_t kScaleOffset = (((size_t)kStages * kStageBytes + 256 /*barriers*/ + (kMaxExperts + 1) * sizeof(int32_t)) + 15) / 16 * 16;
-constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + kScaleOffset + (size_t)kScaleStages * BM * sizeof(float4);
 
 // Push epilogue (dense, one tile per (m, n)): instead of writing `out`, every output tile is stored into the receive
 // buffer of every rank, in the slot of this rank, and flagged there.  Receive buffer of a rank:
@@ -79,12 +78,15 @@ struct PushParams {
   int32_t scatter;  // 0: every tile goes to every rank (one-shot); 1: tile t goes to rank t % world only (two-shot)
 };
 
-// Push epilogue staging: every promotion warp turns "one output row per lane" into "rows of contiguous bytes per store"
-// through a private [32 rows][kStageWords] patch of shared memory, 16 payload words per row and pass.
+// Epilogue staging: every promotion warp turns "one output row per lane" into "rows of contiguous bytes per store"
+// through a private [32 rows][kStageWords] patch of shared memory, 16 payload words per row and pass.  Stored straight
+// from the registers a warp's 16-byte stores touch 32 rows each, one L1 wavefront per row: 2048 of them per tile, more than
+// the tile's whole K loop where K is short (K = 1536: 640 cycles per k-block with the epilogue against 437 at K = 7168).
 constexpr int kStageWords = 20;  // 80-byte row stride: 16-byte aligned, conflict-free for the per-lane uint4 writes
 constexpr size_t kStagingBytes = (size_t)kEpiWarps * 32 * kStageWords * sizeof(uint32_t);
 constexpr size_t kStagingOffset = kScaleOffset + (size_t)kScaleStages * BM * sizeof(float4);
-constexpr size_t kSmemBytesPush = 1024 + kStagingOffset + kStagingBytes;
+constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + kStagingOffset + kStagingBytes;
+static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
 
 struct GemmParams {
   const float* sa;
@@ -230,22 +232,6 @@ template <>
 __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
-}
-
-// acc holds kEpiCols consecutive columns starting at column n_first of the output row
-template <typename OutT>
-__device__ __forceinline__ void store_row(const float2 (&acc)[kEpiCols / 2], OutT* out_row, int32_t n_first, int32_t N) {
-#pragma unroll
-  for (int c = 0; c < kEpiCols / 8; ++c) {
-    if (n_first + c * 8 < N) {
-      uint4 u;
-      u.x = pack2<OutT>(acc[c * 4 + 0].x, acc[c * 4 + 0].y);
-      u.y = pack2<OutT>(acc[c * 4 + 1].x, acc[c * 4 + 1].y);
-      u.z = pack2<OutT>(acc[c * 4 + 2].x, acc[c * 4 + 2].y);
-      u.w = pack2<OutT>(acc[c * 4 + 3].x, acc[c * 4 + 3].y);
-      *reinterpret_cast<uint4*>(out_row + c * 8) = u;
-    }
-  }
 }
 
 // acc[j] += v[2j], v[2j+1] * scale, two columns per instruction
@@ -644,9 +630,9 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                         (((int64_t)set * kMaxPeers + p.push.rank) * kPushMaxTiles + tile_id) * kEpiWarps + wi;
           ptx::st_release_sys_u32(f, push_epoch);
         }
-      } else if (row < tl.row_end) {
-        const int32_t n_first = tl.n0 + col0;
-        if (p.partial != nullptr) {
+      } else if (p.partial != nullptr) {
+        if (row < tl.row_end) {
+          const int32_t n_first = tl.n0 + col0;
           float* dst = p.partial + ((int64_t)tl.split * p.total_rows + row) * p.N + n_first;
 #pragma unroll
           for (int c = 0; c < kEpiCols / 4; ++c) {
@@ -654,10 +640,23 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
               *reinterpret_cast<float4*>(dst + c * 4) =
                   make_float4(acc[2 * c].x, acc[2 * c].y, acc[2 * c + 1].x, acc[2 * c + 1].y);
           }
-        } else if (p.out_dtype == SGLB200_BF16) {
-          store_row<__nv_bfloat16>(acc, static_cast<__nv_bfloat16*>(p.out) + (int64_t)row * p.ldc + n_first, n_first, p.N);
-        } else {
-          store_row<__half>(acc, static_cast<__half*>(p.out) + (int64_t)row * p.ldc + n_first, n_first, p.N);
+        }
+      } else {
+        const int32_t n_first = tl.n0 + col0, row_base = tl.row0 + q * 32;
+        uint32_t* stg = reinterpret_cast<uint32_t*>(smem + kStagingOffset) + (warp - kFirstPromoWarp) * 32 * kStageWords;
+        uint16_t* out = static_cast<uint16_t*>(p.out) + (int64_t)row_base * p.ldc + n_first;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // 32 columns (64 bytes of a row) per pass
+          uint32_t v[16];
+#pragma unroll
+          for (int w = 0; w < 16; ++w)
+            v[w] = p.out_dtype == SGLB200_BF16 ? pack2<__nv_bfloat16>(acc[16 * h + w].x, acc[16 * h + w].y)
+                                               : pack2<__half>(acc[16 * h + w].x, acc[16 * h + w].y);
+          warp_rows_via_smem(stg, v, lane, [&](int r, int w, uint4 val) {
+            const int32_t c = 32 * h + 2 * w;  // 8 columns from n_first + c (N % 8 == 0)
+            if (row_base + r < tl.row_end && n_first + c < p.N)
+              *reinterpret_cast<uint4*>(out + (int64_t)r * p.ldc + c) = val;
+          });
         }
       }
       if constexpr (AR) {
@@ -1058,7 +1057,7 @@ int set_smem_attr_once() {
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !done[dev]) {
     cudaError_t e = cudaFuncSetAttribute(fp8_block_gemm_kernel<GROUPED, PUSH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(PUSH ? kSmemBytesPush : kSmemBytes));
+                                         (int)kSmemBytes);
     if (e != cudaSuccess) return fail(SGLB200_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     done[dev] = true;
   }
@@ -1199,7 +1198,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
     if (int rc = set_smem_attr_once<false, true>()) return rc;
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
     const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
-    fp8_block_gemm_kernel<false, true><<<grid, kThreads, kSmemBytesPush, st>>>(map_a, map_b, p);
+    fp8_block_gemm_kernel<false, true><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
   } else {
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles * p.k_splits;
     const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
