@@ -66,9 +66,9 @@ int sglb200_get_num_sms(void);
  * few-rows kernel: operands swapped, 128 weight rows x 16 / 32 / 64 activation rows per MMA, only the weights of
  * experts that have rows are streamed.  This is the decode case of a mixture-of-experts layer, where the 128 x 128
  * kernel spends a full tile of tensor-core work (and, with fp32 scales, of promotion) on a handful of rows: no slower
- * in a burst, but sustained that work runs the board into its power cap at half the SM clock.  Default 20 (measured
- * cross-over on the DeepSeek-V3 layer shape under sustained load: faster up to ~24 rows per expert, level at 32-48);
- * 0 = always the 128 x 128 kernels; at most 64.  With UE8M0 scales the few-rows kernel decodes the exponent bytes and
+ * in a burst, but sustained that work runs the board into its power cap at half the SM clock.  Default 20, which stands for
+ * the library's own measured rule (fp32 scales: up to 48 rows on average; UE8M0 scales: up to 20); any other value is
+ * taken as the limit itself, 0 = always the 128 x 128 kernels; at most 64.  With UE8M0 scales the few-rows kernel decodes the exponent bytes and
  * applies the scales in fp32 after each k-block (exact for powers of two).
  * The results of the two kernels are bit-identical (same products, same fp32 accumulation order per k-block).
  * Process-wide, read at every launch.
@@ -338,6 +338,19 @@ int sglb200_silu_and_mul(const void* input, void* output, int64_t num_rows, int6
 int sglb200_fp8_blockwise_scaled_masked_grouped_mm(const void* a, const void* b, const float* sa, const float* sb,
                                                    void* out, const int32_t* masked_m, int64_t num_groups,
                                                    int64_t max_m, int64_t N, int64_t K, int64_t lda, int64_t ldb,
+                                                   int64_t ldb_e, int64_t ldc, int64_t sa_stride_g, int64_t sa_stride_m,
+                                                   int64_t sa_stride_k, int64_t sb_stride_e, int64_t sb_stride_n,
+                                                   int64_t sb_stride_k, int out_dtype, void* stream);
+
+/*
+ * The same with the number of rows the caller expects per group on average (expected_m, DeepGEMM's argument of that name;
+ * <= 0: unknown).  It only chooses the kernel: any masked_m up to max_m gives the same result.  The row bound max_m says
+ * little about the rows in use (a dispatcher sizes it for the worst case), and few rows per group are served best by the
+ * weight-streaming kernel.
+ */
+int sglb200_fp8_blockwise_scaled_masked_grouped_mm_expected(const void* a, const void* b, const float* sa, const float* sb,
+                                                   void* out, const int32_t* masked_m, int64_t num_groups,
+                                                   int64_t max_m, int64_t expected_m, int64_t N, int64_t K, int64_t lda, int64_t ldb,
                                                    int64_t ldb_e, int64_t ldc, int64_t sa_stride_g, int64_t sa_stride_m,
                                                    int64_t sa_stride_k, int64_t sb_stride_e, int64_t sb_stride_n,
                                                    int64_t sb_stride_k, int out_dtype, void* stream);

@@ -37,6 +37,8 @@ SIGNATURES = {
                                                 _L, _L, _L, _I, _P],
     "sglb200_fp8_blockwise_scaled_masked_grouped_mm": [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L,
                                                        _L, _L, _L, _L, _I, _P],
+    "sglb200_fp8_blockwise_scaled_masked_grouped_mm_expected": [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L,
+                                                                _L, _L, _L, _L, _L, _L, _I, _P],
     "sglb200_prepare_moe_input": [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _P],
     "sglb200_shuffle_rows": [_P, _P, _P, _L, _L, _P],
     "sglb200_apply_shuffle_mul_sum": [_P, _P, _P, _P, _L, _L, _L, _I, _I, _P],

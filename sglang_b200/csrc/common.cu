@@ -18,7 +18,7 @@ int fail(int code, const char* fmt, ...) {
 }
 
 static int g_num_sms_limit = 0;  // 0: no limit
-int g_grouped_few_rows_max = 20;  // grouped GEMMs with at most this many rows per expert on average take the few-rows kernel
+int g_grouped_few_rows_max = kGroupedFewRowsDefault;  // sglb200_set_grouped_few_rows
 
 int device_info(DeviceInfo* out) {
   static DeviceInfo cache[64];

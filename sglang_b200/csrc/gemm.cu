@@ -1069,7 +1069,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
                 int64_t lda, int64_t ldb, int64_t ldb_e, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k,
                 int64_t sb_stride_e, int64_t sb_stride_n, int64_t sb_stride_k, int out_dtype, void* stream,
                 float* workspace = nullptr, int64_t workspace_floats = 0, const PushParams* push = nullptr,
-                int64_t rows_per_expert = 0, int64_t sa_stride_e = 0) {
+                int64_t rows_per_expert = 0, int64_t sa_stride_e = 0, int64_t expected_rows = 0) {
   const bool grouped = expert_offsets != nullptr || rows_per_expert > 0;
   SGLB_REQUIRE(total_rows >= 0 && N >= 0 && K >= 0, SGLB200_ERR_SHAPE, "M=%lld N=%lld K=%lld: negative size",
                (long long)total_rows, (long long)N, (long long)K);
@@ -1131,7 +1131,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
 
   if (grouped && !push) {
     // few rows per expert: the weight-streaming kernel with swapped operands (gemm_smallm.cu)
-    if (const int chunk = smallm_grouped_chunk(total_rows, num_experts, rows_per_expert))
+    if (const int chunk = smallm_grouped_chunk(total_rows, num_experts, rows_per_expert, expected_rows))
       return smallm_grouped_gemm(chunk, a, b, sa, sb, out, expert_offsets, problem_sizes, rows_per_expert > 0 ? 1 : 3,
                                  total_rows, num_experts, rows_per_expert, N, K, lda, ldb, ldb_e, ldc, sa_stride_e,
                                  sa_stride_m, sa_stride_k, sb_stride_e, sb_stride_n, sb_stride_k, out_dtype, di.sm_count,
@@ -1236,9 +1236,9 @@ extern "C" int sglb200_fp8_blockwise_scaled_grouped_mm(const void* a, const void
                            sa_stride_m, sa_stride_k, sb_stride_e, sb_stride_n, sb_stride_k, out_dtype, stream);
 }
 
-extern "C" int sglb200_fp8_blockwise_scaled_masked_grouped_mm(const void* a, const void* b, const float* sa,
+extern "C" int sglb200_fp8_blockwise_scaled_masked_grouped_mm_expected(const void* a, const void* b, const float* sa,
                                                               const float* sb, void* out, const int32_t* masked_m,
-                                                              int64_t num_groups, int64_t max_m, int64_t N, int64_t K,
+                                                              int64_t num_groups, int64_t max_m, int64_t expected_m, int64_t N, int64_t K,
                                                               int64_t lda, int64_t ldb, int64_t ldb_e, int64_t ldc,
                                                               int64_t sa_stride_g, int64_t sa_stride_m,
                                                               int64_t sa_stride_k, int64_t sb_stride_e,
@@ -1250,7 +1250,20 @@ extern "C" int sglb200_fp8_blockwise_scaled_masked_grouped_mm(const void* a, con
   SGLB_REQUIRE(masked_m != nullptr, SGLB200_ERR_NULL, "masked_m must not be NULL");
   return sglb::gemm_common(a, b, sa, sb, out, nullptr, masked_m, num_groups * max_m, num_groups, N, K, lda, ldb, ldb_e, ldc,
                            sa_stride_m, sa_stride_k, sb_stride_e, sb_stride_n, sb_stride_k, out_dtype, stream, nullptr, 0,
-                           nullptr, max_m, sa_stride_g);
+                           nullptr, max_m, sa_stride_g, expected_m);
+}
+
+extern "C" int sglb200_fp8_blockwise_scaled_masked_grouped_mm(const void* a, const void* b, const float* sa,
+                                                              const float* sb, void* out, const int32_t* masked_m,
+                                                              int64_t num_groups, int64_t max_m, int64_t N, int64_t K,
+                                                              int64_t lda, int64_t ldb, int64_t ldb_e, int64_t ldc,
+                                                              int64_t sa_stride_g, int64_t sa_stride_m,
+                                                              int64_t sa_stride_k, int64_t sb_stride_e,
+                                                              int64_t sb_stride_n, int64_t sb_stride_k, int out_dtype,
+                                                              void* stream) {
+  return sglb200_fp8_blockwise_scaled_masked_grouped_mm_expected(a, b, sa, sb, out, masked_m, num_groups, max_m, 0, N, K, lda,
+                                                                 ldb, ldb_e, ldc, sa_stride_g, sa_stride_m, sa_stride_k,
+                                                                 sb_stride_e, sb_stride_n, sb_stride_k, out_dtype, stream);
 }
 
 extern "C" int64_t sglb200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, int64_t N, int64_t K) {

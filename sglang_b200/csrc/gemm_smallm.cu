@@ -1,22 +1,23 @@
 // Block-scaled FP8 GEMM for few rows of activations (M <= 128: the decode case), weight-streaming bound.
 //
 // The roles of the operands are swapped: the tensor core computes C^T = W * A^T, a tile being 128 WEIGHT rows (the MMA's
-// M) by MT token columns (the MMA's N, MT = 16 / 32 / 64).  An accumulator stage is then only MT TMEM columns wide, so 8 to
-// 16 k-blocks are in flight between the MMA warp and the promotion warps instead of 4, and a shared-memory stage is 16 KB
-// of weights plus MT x 128 bytes of activations, so 8 to 10 stages (128 to 160 KB of weights) are in flight per SM: the
-// kernel is bound by HBM, not by the accumulator hand-off of the 128 x 128 kernel.  K can be cut into ranges that run on
-// different SMs (fp32 partial sums, added by splitk_reduce_kernel) when N / 128 tiles alone cannot occupy the SMs.
-// From 65 to 128 rows the tile is 128 x 128 (4 accumulator stages, 7 shared-memory stages) and eight promotion warps
-// share every accumulator stage, four per 64 token columns: what is left of the advantage over the 128 x 128 kernel is
-// the deeper weight ring and the single role per warp (measured 7-15 % at 96-128 rows).
+// M) by MT token columns (the MMA's N, MT = 16 / 32 / 64 / 128, and as few of them as the item has rows).  An accumulator
+// stage is then only MT TMEM columns wide, so 4 to 16 k-blocks are in flight between the MMA warp and the promotion warps, and
+// a shared-memory stage is 16 KB of weights plus MT x 128 bytes of activations, 6 to 11 of them: 64 KB of weights in flight
+// per SM already bring a plain stream of such tiles to 90 % of the HBM rate, 128 KB to all of it.  K can be cut into ranges
+// that run on different SMs (fp32 partial sums, added by splitk_reduce_kernel) when N / 128 tiles alone cannot occupy the SMs.
+// From 65 to 128 rows eight promotion warps share every accumulator stage, four per 64 token columns.
+// Measured against scales that every promotion warp fetched and spread by shuffles, weights from HBM (B200):
+// N=36864 K=7168 M=32 / 64 / 128: 46.6 / 54.8 / 75.0 -> 41.8 / 43.3 / 55.1 us (6.1 TB/s at 64 rows);
+// N=24576 K=1536 M=16 / 64 / 128: 8.4 / 15.4 / 21.8 -> 7.7 / 9.8 / 13.9 us.
 //
 // GROUPED variant (one weight matrix per expert, few rows per expert: the decode case of a mixture-of-experts layer): a
 // work item is (expert, 128 weight rows, chunk of MT of the expert's rows).  The row ranges come from the same device
 // tables as in the 128 x 128 grouped kernel; an expert with more than MT rows gets several chunks (its weight tile is
 // then re-read, from L2), an expert without rows gets no item, so only the weights of routed experts are streamed.
 //
-// warp 0: TMA producer; warp 1: TMEM owner + MMA issuer; warps 2..5: promotion (tcgen05.ld, acc += p * sa[token] * sb)
-// and the transposed store.  All waits are bounded.
+// warp 0: TMA producer; warp 1: TMEM owner + MMA issuer; warp 2: scale loader (sa[token] * sb into shared memory); warps 4..7
+// (..11): promotion (tcgen05.ld, acc += p * scale) and the transposed store.  All waits are bounded.
 //
 // The kernel is launched with programmatic stream serialization: it may start while the kernel before it (the
 // activation quantiser, or the previous layer's reduce kernel) is still running.  Its set-up and the WEIGHT tiles of the
@@ -53,24 +54,30 @@ namespace {
 constexpr int BN = 128, BK = 128;  // weight rows per tile, K per block
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kWBytes = BN * BK;
-constexpr int kScaleAhead = 4;
+constexpr int kScaleGroup = 4;   // k-blocks per stage of the scale ring
+constexpr int kScaleStages = 4;
+constexpr uint32_t kCtlBytes = 640;
+constexpr uint32_t kPatchRow = 80, kPatchBytes = 16 * kPatchRow;  // epilogue patch of a warp: 16 tokens x 64 bytes, padded
 
 constexpr int kMaxExperts = 1024;
 
-// NSUB = 2 (dense, 64 < M <= 128): the MMA covers MT * NSUB = 128 activation rows (one instruction shape 128 x 128, so
-// the issuing thread's cost per k-block stays that of the narrow tiles) and a second set of four promotion warps takes
-// the second half of every accumulator stage's columns, so the registers per thread stay those of 64 rows.
+// NSUB = 2 (65 to 128 rows per item): the MMA covers up to MT * NSUB = 128 activation rows and a second set of four
+// promotion warps takes the second half of every accumulator stage's columns, so the registers per thread stay those of
+// 64 rows.
 template <int MT, int NSUB = 1>
 struct Cfg {
-  static constexpr int kTile = MT * NSUB;  // activation rows per work item = the MMA's N = TMEM columns per stage
-  static constexpr int kStages = kTile == 128 ? 7 : (kTile == 64 ? 8 : 10);
+  static constexpr int kTile = MT * NSUB;  // most activation rows per work item = TMEM columns per stage
+  static constexpr int kStages = kTile == 128 ? 6 : (kTile == 64 ? 8 : (kTile == 32 ? 10 : 11));
   static constexpr int kAcc = (512 / kTile) < 16 ? (512 / kTile) : 16;
-  static constexpr int kThreads = 64 + 128 * NSUB;
+  static constexpr int kThreads = 128 + 128 * NSUB;
   static constexpr uint32_t kABytes = kTile * BK;
   static constexpr uint32_t kStageBytes = kWBytes + kABytes;
-  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStageBytes + 512;
+  static constexpr uint32_t kScaleBytes = kScaleStages * kScaleGroup * kTile * sizeof(float);
+  static constexpr size_t kPatchOffset = (size_t)kStages * kStageBytes + kScaleBytes;
+  static constexpr size_t kSmem = 1024 + kPatchOffset + 4 * NSUB * kPatchBytes + kCtlBytes;
   // grouped: the table of first work items per expert follows the control block
   static constexpr size_t kSmemGrouped = kSmem + (kMaxExperts + 1) * sizeof(int32_t) + 12;
+  static_assert(kSmemGrouped <= 227 * 1024, "shared memory of one CTA");
 };
 
 struct SmallParams {
@@ -106,7 +113,7 @@ __device__ __forceinline__ void expert_rows(const SmallParams& p, int32_t e, int
   }
 }
 
-template <int MT, bool GROUPED>
+template <int TILE, bool GROUPED>
 __device__ __forceinline__ Item get_item(const SmallParams& p, const int32_t* item_start, int32_t t) {
   Item it;
   if constexpr (!GROUPED) {
@@ -125,13 +132,14 @@ __device__ __forceinline__ Item get_item(const SmallParams& p, const int32_t* it
     }
     int32_t r0, cnt;
     expert_rows(p, lo, &r0, &cnt);
-    const int32_t chunks = (cnt + MT - 1) / MT;
+    const int32_t chunks = (cnt + TILE - 1) / TILE;
     const int32_t local = t - item_start[lo];
     it.e = lo;
     it.nt = local / chunks;
     const int32_t ch = local - it.nt * chunks;
-    it.row0 = r0 + ch * MT;
-    it.rows = min(MT, cnt - ch * MT);
+    const int32_t per = (cnt + chunks - 1) / chunks;  // chunks of even size: the MMA is as wide as the chunk
+    it.row0 = r0 + ch * per;
+    it.rows = min(per, cnt - ch * per);
     it.kb0 = 0;
     it.kb1 = p.k_tiles;
     it.split = 0;
@@ -140,44 +148,56 @@ __device__ __forceinline__ Item get_item(const SmallParams& p, const int32_t* it
 }
 
 struct Ctl {
-  uint64_t full[10];
-  uint64_t empty[10];
+  uint64_t full[12];
+  uint64_t empty[12];
   uint64_t acc_full[16];
   uint64_t acc_empty[16];
+  uint64_t sc_full[kScaleStages];
+  uint64_t sc_empty[kScaleStages];
   uint32_t tmem_base;
   volatile int32_t abort_flag;
   int32_t total;
 };
-static_assert(sizeof(Ctl) <= 512, "control block");
+static_assert(sizeof(Ctl) <= kCtlBytes, "control block");
 
 __device__ __forceinline__ void timeout(Ctl* ctl, int code) {
   ctl->abort_flag = 1;
   atomicCAS(&g_smallm_status, 0, code);
 }
 
-// 32 lanes x N consecutive fp32 columns
-template <int N>
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* r);
+// 16 lanes x 8 * G fp32 columns in the accumulator-fragment arrangement: registers 4g + {0, 1} of thread t hold lane t / 4,
+// columns 8g + 2 * (t % 4) + {0, 1}; registers 4g + {2, 3} the same columns of lane t / 4 + 8.
+template <int G>
+__device__ __forceinline__ void tmem_ld_16x256(uint32_t taddr, uint32_t* r);
 template <>
-__device__ __forceinline__ void tmem_ld_cols<16>(uint32_t taddr, uint32_t* r) {
+__device__ __forceinline__ void tmem_ld_16x256<2>(uint32_t taddr, uint32_t* r) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
       : "r"(taddr)
       : "memory");
 }
 template <>
-__device__ __forceinline__ void tmem_ld_cols<32>(uint32_t taddr, uint32_t* r) {
+__device__ __forceinline__ void tmem_ld_16x256<4>(uint32_t taddr, uint32_t* r) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+template <>
+__device__ __forceinline__ void tmem_ld_16x256<8>(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
       "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr)
       : "memory");
 }
@@ -201,16 +221,32 @@ __device__ __forceinline__ float load_scale(const float* base, int32_t kc, int64
   }
 }
 
+// Four 8 x 8 matrices of 16-bit values in fragment arrangement, stored transposed: lane l passes the address of row l % 8 of
+// matrix l / 8.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c),
+               "r"(d)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t pack16(float a, float b, int out_dtype) {
+  if (out_dtype == SGLB200_BF16) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+  }
+  __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+
 template <int MT, bool UE, bool GROUPED, int NSUB>
-__global__ void __launch_bounds__(64 + 128 * NSUB, 1)
+__global__ void __launch_bounds__(128 + 128 * NSUB, 1)
 fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                              const SmallParams p) {
   using C = Cfg<MT, NSUB>;
-  static_assert(!GROUPED || NSUB == 1, "the grouped form has one sub-tile");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  Ctl* ctl = reinterpret_cast<Ctl*>(smem + (size_t)C::kStages * C::kStageBytes);
-  int32_t* item_start = reinterpret_cast<int32_t*>(smem + (size_t)C::kStages * C::kStageBytes + 512);
+  float* scale_ring = reinterpret_cast<float*>(smem + (size_t)C::kStages * C::kStageBytes);  // [stage][k-block][token]
+  Ctl* ctl = reinterpret_cast<Ctl*>(smem + C::kPatchOffset + 4 * NSUB * kPatchBytes);
+  int32_t* item_start = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(ctl) + kCtlBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -221,6 +257,10 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
     for (int i = 0; i < C::kAcc; ++i) {
       ptx::mbar_init(&ctl->acc_full[i], 1);
       ptx::mbar_init(&ctl->acc_empty[i], 4 * NSUB);  // one arrival per promotion warp
+    }
+    for (int i = 0; i < kScaleStages; ++i) {
+      ptx::mbar_init(&ctl->sc_full[i], 1);
+      ptx::mbar_init(&ctl->sc_empty[i], 4 * NSUB);
     }
     ctl->abort_flag = 0;
     ptx::fence_barrier_init();
@@ -243,7 +283,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         if (e < p.num_experts) {
           int32_t r0, cnt;
           expert_rows(p, e, &r0, &cnt);
-          v = ((cnt + MT - 1) / MT) * p.n_tiles;
+          v = ((cnt + C::kTile - 1) / C::kTile) * p.n_tiles;
         }
         int32_t incl = v;
 #pragma unroll
@@ -269,201 +309,267 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
   const int32_t total = ctl->total;
   const uint32_t full0 = ptx::smem_u32(&ctl->full[0]), empty0 = ptx::smem_u32(&ctl->empty[0]);
   const uint32_t acc_full0 = ptx::smem_u32(&ctl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctl->acc_empty[0]);
+  const uint32_t sc_full0 = ptx::smem_u32(&ctl->sc_full[0]), sc_empty0 = ptx::smem_u32(&ctl->sc_empty[0]);
   const uint32_t stage0 = ptx::smem_u32(smem);
 
   if (threadIdx.x == 0) ptx::grid_dep_launch();  // the next kernel of the stream may begin its own set-up
 
   const bool leader = ptx::elect_one();  // the lane that issues TMA and tcgen05 instructions
-  if (warp == 0) {
-    // ===== TMA producer.  Pass 0 runs before griddepcontrol.wait: the weight tiles of the first k-blocks (at most one
-    // ring of stages, whose barriers are fresh) are requested; pass 1 adds their activation tiles and then continues
-    // with whole stages.
-    uint32_t pre = 0;
-    uint32_t armed = 0, armed_phase = 0;  // bit i: stage i was armed / the phase bit of its last arming
-    for (int pass = GROUPED ? 1 : 0; pass < 2; ++pass) {
-      uint32_t stage = 0, phase = 0, idx = 0;
-      bool ok = true;
-      for (int32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
-        const Item it = get_item<MT, GROUPED>(p, item_start, t);
-        const int32_t nt = it.nt;
-        for (int32_t kb = it.kb0; kb < it.kb1; ++kb, ++idx) {
-          const uint32_t dst = stage0 + stage * C::kStageBytes;
-          if (pass == 0) {
-            if (idx >= (uint32_t)C::kStages) { ok = false; break; }
-            if (leader) {
-              ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, C::kStageBytes);
-              ptx::tma_load_3d_a(dst, &map_w, full0 + stage * 8, kb * BK, nt * BN, 0);
-            }
-            armed |= 1u << stage;
-            armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
-            pre = idx + 1;
-          } else if (idx < pre) {
-            if (leader) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, 0);
-          } else {
-            if (!ptx::mbar_wait_a(empty0 + stage * 8, phase ^ 1)) {
-              timeout(ctl, 11);
-              ok = false;
-              break;
-            }
-            if (leader) {
-              ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, C::kStageBytes);
-              ptx::tma_load_3d_a(dst, &map_w, full0 + stage * 8, kb * BK, nt * BN, it.e);
-              ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, it.row0);
-            }
-            armed |= 1u << stage;
-            armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
-          }
-          if (++stage == C::kStages) { stage = 0; phase ^= 1; }
-        }
-        if (ctl->abort_flag) ok = false;
-      }
-      if (pass == 0) {
-        ptx::grid_dep_wait();  // the activations are written by the kernel before this one
-      } else if (ctl->abort_flag) {
-        // bulk copies must not be in flight when the CTA exits: wait (bounded) for every stage that may still be armed
-        for (int i = 0; i < C::kStages; ++i)
-          if (armed & (1u << i)) ptx::mbar_wait_a(full0 + i * 8, (armed_phase >> i) & 1u, 20000000ull);
-      } else {
-        // the last tcgen05.commit arrivals on `empty` must have landed before the CTA's shared memory is reused
-        for (int i = 0; i < C::kStages; ++i) {
-          if (!ptx::mbar_wait_a(empty0 + stage * 8, phase ^ 1)) { timeout(ctl, 15); break; }
-          if (++stage == C::kStages) { stage = 0; phase ^= 1; }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    // ===== MMA issuer: D[128 weight rows][MT tokens] (+)= W_tile * A_tile^T, one TMEM stage per k-block
-    constexpr uint32_t idesc = ptx::make_idesc_e4m3_f32(BN, C::kTile);
-    const uint64_t desc0 = ptx::make_kmajor_sw128_desc(stage0);
-    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-    for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
-      int32_t kb0 = 0, kb1 = p.k_tiles;
-      if constexpr (!GROUPED) {
-        const int32_t split = t / p.n_tiles;
-        kb0 = split * p.kb_per_split;
-        kb1 = min(kb0 + p.kb_per_split, p.k_tiles);
-      }
-      bool ok = true;
-      for (int32_t kb = kb0; kb < kb1; ++kb) {
-        if (!ptx::mbar_wait_a(acc_empty0 + acc * 8, acc_phase ^ 1)) { timeout(ctl, 12); ok = false; break; }
-        if (!ptx::mbar_wait_a(full0 + stage * 8, phase)) { timeout(ctl, 13); ok = false; break; }
-        ptx::tc_fence_after();
-        if (leader) {
-          const uint64_t w_desc = desc0 + (uint64_t)(stage * (C::kStageBytes >> 4));
-          const uint64_t a_desc = w_desc + (kWBytes >> 4);
-          const uint32_t d_tmem = tmem_base + acc * C::kTile;
-          ptx::mma_f8f6f4(d_tmem, w_desc, a_desc, idesc, 0);
-#pragma unroll
-          for (uint32_t k = 1; k < BK / 32; ++k) ptx::mma_f8f6f4(d_tmem, w_desc + 2 * k, a_desc + 2 * k, idesc, 1);
-          ptx::mma_commit_a(empty0 + stage * 8);
-          ptx::mma_commit_a(acc_full0 + acc * 8);
-        }
-        if (++stage == C::kStages) { stage = 0; phase ^= 1; }
-        if (++acc == C::kAcc) { acc = 0; acc_phase ^= 1; }
-      }
-      if (!ok || ctl->abort_flag) break;
-    }
-  } else {
-    // ===== promotion + transposed store; TMEM lane quarter = warp % 4 (warps 2, 3, 4, 5 -> quarters 2, 3, 0, 1)
-    if constexpr (!GROUPED)
-      ptx::grid_dep_wait();  // the activation scales come from the kernel before this one, and it may still read `out` / `partial`
+  // Register split (NSUB = 2): eight promotion warps with 64 accumulators, 64 loaded sums and the scales in flight want more
+  // than the 168 registers that 384 threads start with; the other four warps need few: 128 * 96 + 256 * 200 = 63488 <=
+  // 384 * 168.  No call may sit in a region with a changed limit, hence the inlined waits.
+  if (warp >= 4) {
+    if constexpr (NSUB == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    // ===== promotion + transposed store; TMEM lane quarter = warp % 4.  A warp owns 32 weight rows (columns of the output)
+    // and MT tokens.  The sums are loaded in fragment arrangement (tmem_ld_16x256), in which a thread meets only MT / 4
+    // tokens: with one weight row per thread (32x32b loads) every thread needs every token's scale, and the 64 KB of
+    // broadcast scale reads per k-block of 128 tokens kept the shared memory busier than the loads and the MMAs.
+    // (16x256b loads are slower, 125 against 74 cycles per k-block of 128 x 128, and still far from the bound.)
+    if constexpr (!GROUPED) ptx::grid_dep_wait();  // the kernel before this one may still read `out` / `partial`
+    constexpr int G = MT / 8;  // groups of eight tokens
     const int q = warp & 3;
-    const int sub = NSUB == 1 ? 0 : (warp - 2) >> 2;  // which sub-tile of the item this warp promotes
-    constexpr int kPerLane = MT / 32 > 0 ? MT / 32 : 1;  // tokens whose activation scale this lane fetches
-    uint32_t acc_stage = 0, acc_phase = 0;
-    float acc[MT];
+    const int sub = NSUB == 1 ? 0 : (warp - 4) >> 2;  // which sub-tile of the item this warp promotes
+    const int tr = lane >> 2, tc = 2 * (lane & 3);    // this thread's row inside 8 weight rows / column inside 8 tokens
+    uint8_t* patch = reinterpret_cast<uint8_t*>(smem) + C::kPatchOffset + (size_t)(warp - 4) * kPatchBytes;
+    uint32_t acc_stage = 0, acc_phase = 0, sc_stage = 0, sc_phase = 0;
+    float2 acc[2][G][2];  // [lanes 0-15 / 16-31][token group][rows tr / tr + 8]: two neighbouring tokens
     for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
-      const Item it = get_item<MT, GROUPED>(p, item_start, t);
-      const int32_t split = it.split, nt = it.nt, kb0 = it.kb0, kb1 = it.kb1;
-      const int32_t n = nt * BN + q * 32 + lane;
-      const float* sb_blk = p.sb + (int64_t)nt * p.sb_stride_n;
+      const Item it = get_item<C::kTile, GROUPED>(p, item_start, t);
+      const int32_t kb0 = it.kb0, kb1 = it.kb1;
       const int32_t row0 = it.row0 + sub * MT, rows = max(0, min(MT, it.rows - sub * MT));
-      const float* sa_base = p.sa + (int64_t)row0 * p.sa_stride_m;
-      if constexpr (GROUPED) {
-        sb_blk += (int64_t)it.e * p.sb_stride_e;
-        if (p.rows_per_expert > 0)
-          sa_base = p.sa + (int64_t)it.e * p.sa_stride_e + (int64_t)(row0 - it.e * p.rows_per_expert) * p.sa_stride_m;
-      }
 #pragma unroll
-      for (int j = 0; j < MT; ++j) acc[j] = 0.f;
-      // lane l holds the scale of token l (and l + 32); tokens past M get 0 (their products are 0 anyway)
-      const float* sa_tok[kPerLane];
-      bool tok_ok[kPerLane];
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int h = 0; h < kPerLane; ++h) {
-        const int32_t tok = lane + 32 * h;
-        tok_ok[h] = tok < rows && tok < MT;
-        sa_tok[h] = sa_base + (int64_t)(tok_ok[h] ? tok : 0) * p.sa_stride_m;
-      }
-      float sa_ring[kScaleAhead][kPerLane], sb_ring[kScaleAhead];
-#pragma unroll
-      for (int u = 0; u < kScaleAhead; ++u) {
-        const int32_t kc = min(kb0 + u, kb1 - 1);
-#pragma unroll
-        for (int h = 0; h < kPerLane; ++h) sa_ring[u][h] = tok_ok[h] ? load_scale<UE>(sa_tok[h], kc, p.sa_stride_k) : 0.f;
-        sb_ring[u] = load_scale<UE>(sb_blk, kc, p.sb_stride_k);
-      }
+        for (int g = 0; g < G; ++g) acc[h][g][0] = acc[h][g][1] = make_float2(0.f, 0.f);
       bool ok = true;
-      for (int32_t kbb = kb0; kbb < kb1 && ok; kbb += kScaleAhead) {
+      for (int32_t kbb = kb0; kbb < kb1 && ok; kbb += kScaleGroup) {
+        if (!ptx::mbar_wait_inl_a(sc_full0 + sc_stage * 8, sc_phase)) {
+          timeout(ctl, 17);
+          ok = false;
+          break;
+        }
+        const float* sc_row = scale_ring + (size_t)sc_stage * kScaleGroup * C::kTile + sub * MT + tc;
 #pragma unroll
-        for (int u = 0; u < kScaleAhead; ++u) {
-          const int32_t kb = kbb + u;
-          if (kb >= kb1) break;
-          float s[kPerLane];
+        for (int u = 0; u < kScaleGroup; ++u) {
+          if (kbb + u >= kb1) break;
+          float2 s[G];
 #pragma unroll
-          for (int h = 0; h < kPerLane; ++h) s[h] = sa_ring[u][h] * sb_ring[u];
-          {
-            const int32_t kn = min(kb + kScaleAhead, kb1 - 1);
-#pragma unroll
-            for (int h = 0; h < kPerLane; ++h)
-              sa_ring[u][h] = tok_ok[h] ? load_scale<UE>(sa_tok[h], kn, p.sa_stride_k) : 0.f;
-            sb_ring[u] = load_scale<UE>(sb_blk, kn, p.sb_stride_k);
-          }
-          if (!ptx::mbar_wait_a(acc_full0 + acc_stage * 8, acc_phase)) {
+          for (int g = 0; g < G; ++g) s[g] = *reinterpret_cast<const float2*>(sc_row + u * C::kTile + 8 * g);
+          if (!ptx::mbar_wait_inl_a(acc_full0 + acc_stage * 8, acc_phase)) {
             timeout(ctl, 14);
             ok = false;
             break;
           }
           ptx::tc_fence_after();
           const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc_stage * C::kTile + sub * MT;
-          uint32_t v[MT];
-          if constexpr (MT == 64) {
-            tmem_ld_cols<32>(taddr, v);
-            tmem_ld_cols<32>(taddr + 32, v + 32);
-          } else {
-            tmem_ld_cols<MT>(taddr, v);
+          uint32_t v[2 * 4 * G];
+          if (NSUB == 1 || rows > 0) {  // uniform over the warp
+            tmem_ld_16x256<G>(taddr, v);
+            tmem_ld_16x256<G>(taddr + (16u << 16), v + 4 * G);
+            tmem_ld_fence<8 * G>(v);
           }
-          tmem_ld_fence<MT>(v);
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive_a(acc_empty0 + acc_stage * 8);
+          if (NSUB == 1 || rows > 0) {
 #pragma unroll
-          for (int j = 0; j < MT; ++j) {
-            const float sj = __shfl_sync(0xffffffffu, s[j / 32], j & 31);
-            acc[j] = fmaf(__uint_as_float(v[j]), sj, acc[j]);
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  const int i = (h * G + g) * 4 + 2 * r;
+                  acc[h][g][r] = __ffma2_rn(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), s[g], acc[h][g][r]);
+                }
           }
           if (++acc_stage == C::kAcc) { acc_stage = 0; acc_phase ^= 1; }
         }
+        __syncwarp();  // every lane has read this group's scales
+        if (lane == 0) ptx::mbar_arrive_a(sc_empty0 + sc_stage * 8);
+        if (++sc_stage == kScaleStages) { sc_stage = 0; sc_phase ^= 1; }
       }
       if (!ok || ctl->abort_flag) break;
-      // transposed store: for every token the warp writes 32 consecutive outputs
-      if (n < p.N) {
-        if (p.partial != nullptr) {
-          float* dst = p.partial + ((int64_t)split * p.M + row0) * p.N + n;
+      const int32_t n_warp = it.nt * BN + q * 32;  // first of the warp's 32 output columns
+      if (p.partial != nullptr) {
+        float* dst = p.partial + ((int64_t)it.split * p.M + row0) * p.N + n_warp;
 #pragma unroll
-          for (int j = 0; j < MT; ++j)
-            if (j < rows) dst[(int64_t)j * p.N] = acc[j];
-        } else if (p.out_dtype == SGLB200_BF16) {
-          __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.out) + (int64_t)row0 * p.ldc + n;
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int j = 0; j < MT; ++j)
-            if (j < rows) dst[(int64_t)j * p.ldc] = __float2bfloat16_rn(acc[j]);
-        } else {
-          __half* dst = static_cast<__half*>(p.out) + (int64_t)row0 * p.ldc + n;
+          for (int r = 0; r < 2; ++r) {
+            const int32_t c = h * 16 + r * 8 + tr;
+            if (n_warp + c < p.N) {
 #pragma unroll
-          for (int j = 0; j < MT; ++j)
-            if (j < rows) dst[(int64_t)j * p.ldc] = __float2half_rn(acc[j]);
+              for (int g = 0; g < G; ++g) {
+                const int32_t tok = 8 * g + tc;
+                if (tok < rows) dst[(int64_t)tok * p.N + c] = acc[h][g][r].x;
+                if (tok + 1 < rows) dst[(int64_t)(tok + 1) * p.N + c] = acc[h][g][r].y;
+              }
+            }
+          }
+      } else {
+        // 16 tokens per pass through the warp's patch: transposed there by stmatrix, read back as 64 bytes of a token's row
+        const uint32_t st_addr = ptx::smem_u32(patch) + (uint32_t)(lane & 7) * kPatchRow + (uint32_t)(lane >> 3) * 16;
+        char* out = static_cast<char*>(p.out) + ((int64_t)row0 * p.ldc + n_warp) * 2;
+#pragma unroll
+        for (int g = 0; g < G; g += 2) {
+          if (8 * g >= rows) break;
+          __syncwarp();  // the previous pass has been read out
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            stmatrix_x4_trans(st_addr + i * 8 * kPatchRow, pack16(acc[0][g + i][0].x, acc[0][g + i][0].y, p.out_dtype),
+                              pack16(acc[0][g + i][1].x, acc[0][g + i][1].y, p.out_dtype),
+                              pack16(acc[1][g + i][0].x, acc[1][g + i][0].y, p.out_dtype),
+                              pack16(acc[1][g + i][1].x, acc[1][g + i][1].y, p.out_dtype));
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int32_t tl = i * 8 + (lane >> 2), tok = 8 * g + tl, c = (lane & 3) * 8;
+            const uint4 val = *reinterpret_cast<const uint4*>(patch + tl * kPatchRow + c * 2);
+            if (tok < rows && n_warp + c < p.N)  // N % 8 == 0
+              *reinterpret_cast<uint4*>(out + ((int64_t)tok * p.ldc + c) * 2) = val;
+          }
         }
+      }
+    }
+  } else {
+    if constexpr (NSUB == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+    if (warp == 0) {
+      // ===== TMA producer.  Pass 0 runs before griddepcontrol.wait: the weight tiles of the first k-blocks (at most one
+      // ring of stages, whose barriers are fresh) are requested; pass 1 adds their activation tiles and then continues
+      // with whole stages.
+      uint32_t pre = 0;
+      uint32_t armed = 0, armed_phase = 0;  // bit i: stage i was armed / the phase bit of its last arming
+      for (int pass = GROUPED ? 1 : 0; pass < 2; ++pass) {
+        uint32_t stage = 0, phase = 0, idx = 0;
+        bool ok = true;
+        for (int32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
+          const Item it = get_item<C::kTile, GROUPED>(p, item_start, t);
+          const int32_t nt = it.nt;
+          for (int32_t kb = it.kb0; kb < it.kb1; ++kb, ++idx) {
+            const uint32_t dst = stage0 + stage * C::kStageBytes;
+            if (pass == 0) {
+              if (idx >= (uint32_t)C::kStages) { ok = false; break; }
+              if (leader) {
+                ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, C::kStageBytes);
+                ptx::tma_load_3d_a(dst, &map_w, full0 + stage * 8, kb * BK, nt * BN, 0);
+              }
+              armed |= 1u << stage;
+              armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
+              pre = idx + 1;
+            } else if (idx < pre) {
+              if (leader) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, 0);
+            } else {
+              if (!ptx::mbar_wait_inl_a(empty0 + stage * 8, phase ^ 1)) {
+                timeout(ctl, 11);
+                ok = false;
+                break;
+              }
+              if (leader) {
+                ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, C::kStageBytes);
+                ptx::tma_load_3d_a(dst, &map_w, full0 + stage * 8, kb * BK, nt * BN, it.e);
+                ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, it.row0);
+              }
+              armed |= 1u << stage;
+              armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
+            }
+            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+          }
+          if (ctl->abort_flag) ok = false;
+        }
+        if (pass == 0) {
+          ptx::grid_dep_wait();  // the activations are written by the kernel before this one
+        } else if (ctl->abort_flag) {
+          // bulk copies must not be in flight when the CTA exits: wait (bounded) for every stage that may still be armed
+          for (int i = 0; i < C::kStages; ++i)
+            if (armed & (1u << i)) ptx::mbar_wait_inl_a(full0 + i * 8, (armed_phase >> i) & 1u, 20000000ull);
+        } else {
+          // the last tcgen05.commit arrivals on `empty` must have landed before the CTA's shared memory is reused
+          for (int i = 0; i < C::kStages; ++i) {
+            if (!ptx::mbar_wait_inl_a(empty0 + stage * 8, phase ^ 1)) { timeout(ctl, 15); break; }
+            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+          }
+        }
+      }
+    } else if (warp == 1) {
+      // ===== MMA issuer: D[128 weight rows][tokens] (+)= W_tile * A_tile^T, one TMEM stage per k-block; the instruction is
+      // as wide as the item's rows (in steps of 16), so a ragged chunk costs neither time nor power for its padding
+      const uint64_t desc0 = ptx::make_kmajor_sw128_desc(stage0);
+      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+      for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
+        const Item it = get_item<C::kTile, GROUPED>(p, item_start, t);
+        const int32_t kb0 = it.kb0, kb1 = it.kb1;
+        const uint32_t idesc = ptx::make_idesc_e4m3_f32(BN, (uint32_t)(it.rows + 15) / 16 * 16);
+        bool ok = true;
+        for (int32_t kb = kb0; kb < kb1; ++kb) {
+          if (!ptx::mbar_wait_inl_a(acc_empty0 + acc * 8, acc_phase ^ 1)) { timeout(ctl, 12); ok = false; break; }
+          if (!ptx::mbar_wait_inl_a(full0 + stage * 8, phase)) { timeout(ctl, 13); ok = false; break; }
+          ptx::tc_fence_after();
+          if (leader) {
+            const uint64_t w_desc = desc0 + (uint64_t)(stage * (C::kStageBytes >> 4));
+            const uint64_t a_desc = w_desc + (kWBytes >> 4);
+            const uint32_t d_tmem = tmem_base + acc * C::kTile;
+            ptx::mma_f8f6f4(d_tmem, w_desc, a_desc, idesc, 0);
+#pragma unroll
+            for (uint32_t k = 1; k < BK / 32; ++k) ptx::mma_f8f6f4(d_tmem, w_desc + 2 * k, a_desc + 2 * k, idesc, 1);
+            ptx::mma_commit_a(empty0 + stage * 8);
+            ptx::mma_commit_a(acc_full0 + acc * 8);
+          }
+          if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+          if (++acc == C::kAcc) { acc = 0; acc_phase ^= 1; }
+        }
+        if (!ok || ctl->abort_flag) break;
+      }
+    } else if (warp == 2) {
+      // ===== scale loader: per group of four k-blocks the products sa[token, kb] * sb[nt, kb], 0 for tokens past the item's
+      // rows (the accumulator columns there hold leftovers and are not stored).  The loads of the next group are in flight
+      // while this group waits for its place in the ring.
+      if constexpr (!GROUPED) ptx::grid_dep_wait();  // the activation scales come from the kernel before this one
+      constexpr int kPerLane = C::kTile / 32 > 0 ? C::kTile / 32 : 1;
+      uint32_t stage = 0, phase = 0;
+      for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
+        const Item it = get_item<C::kTile, GROUPED>(p, item_start, t);
+        const float* sb_blk = p.sb + (int64_t)it.nt * p.sb_stride_n;
+        const float* sa_base = p.sa + (int64_t)it.row0 * p.sa_stride_m;
+        if constexpr (GROUPED) {
+          sb_blk += (int64_t)it.e * p.sb_stride_e;
+          if (p.rows_per_expert > 0)
+            sa_base = p.sa + (int64_t)it.e * p.sa_stride_e + (int64_t)(it.row0 - it.e * p.rows_per_expert) * p.sa_stride_m;
+        }
+        float a[kPerLane][kScaleGroup], b[kScaleGroup];
+        auto fetch = [&](int32_t first) {
+#pragma unroll
+          for (int u = 0; u < kScaleGroup; ++u) {
+            const int32_t kb = min(first + u, it.kb1 - 1);
+            b[u] = load_scale<UE>(sb_blk, kb, p.sb_stride_k);
+#pragma unroll
+            for (int h = 0; h < kPerLane; ++h) {
+              const int32_t tok = lane + 32 * h;
+              a[h][u] = tok < it.rows ? load_scale<UE>(sa_base + (int64_t)tok * p.sa_stride_m, kb, p.sa_stride_k) : 0.f;
+            }
+          }
+        };
+        fetch(it.kb0);
+        bool ok = true;
+        for (int32_t kb0 = it.kb0; kb0 < it.kb1; kb0 += kScaleGroup) {
+          float v[kPerLane][kScaleGroup];
+#pragma unroll
+          for (int h = 0; h < kPerLane; ++h)
+#pragma unroll
+            for (int u = 0; u < kScaleGroup; ++u) v[h][u] = a[h][u] * b[u];
+          if (kb0 + kScaleGroup < it.kb1) fetch(kb0 + kScaleGroup);
+          if (!ptx::mbar_wait_inl_a(sc_empty0 + stage * 8, phase ^ 1)) { timeout(ctl, 16); ok = false; break; }
+          float* dst = scale_ring + (size_t)stage * kScaleGroup * C::kTile;
+#pragma unroll
+          for (int h = 0; h < kPerLane; ++h)
+            if (C::kTile >= 32 || lane < C::kTile) {
+#pragma unroll
+              for (int u = 0; u < kScaleGroup; ++u) dst[u * C::kTile + lane + 32 * h] = v[h][u];
+            }
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_a(sc_full0 + stage * 8);
+          if (++stage == kScaleStages) { stage = 0; phase ^= 1; }
+        }
+        if (!ok || ctl->abort_flag) break;
       }
     }
   }
@@ -602,12 +708,26 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
   }
 }
 
+// Above this average the 128 x 128 tile kernel is level with or ahead of chunks of up to 128 rows (256 experts, N=7168 K=2048:
+// 896 against 920 us at 64 rows, 1327 against 1410 at 128); at 32 rows the chunks win (875 against 689 us).  The UE8M0 tile
+// kernel has no promotion to pay for and draws level much earlier (whole layer at 32 rows: 1940 us it, 1990 the chunks).
+constexpr int64_t kWideRowsMax = 48, kWideRowsMaxUe8m0 = 20;
+
 // Rows per chunk of the grouped few-rows kernel for `total_rows` rows spread over `num_experts` experts (or
 // rows_per_expert rows at most per expert in the masked layout); 0 = the 128 x 128 grouped kernel is the better choice.
-int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert) {
-  const int64_t avg = rows_per_expert > 0 ? rows_per_expert : (total_rows + num_experts - 1) / num_experts;
-  if (avg > g_grouped_few_rows_max) return 0;
-  if (rows_per_expert > 0) return avg <= 16 ? 16 : (avg <= 32 ? 32 : 64);  // masked layout: the row bound is known
+int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows, bool ue8m0) {
+  if (g_grouped_few_rows_max == 0) return 0;
+  int64_t avg = (total_rows + num_experts - 1) / num_experts;
+  if (rows_per_expert > 0) {  // masked layout: the row bound is known, the rows in use only if the caller expects a number
+    if (expected_rows <= 0 || expected_rows > rows_per_expert) {
+      if (rows_per_expert > g_grouped_few_rows_max) return 0;
+      return rows_per_expert <= 16 ? 16 : (rows_per_expert <= 32 ? 32 : 64);
+    }
+    avg = expected_rows;
+  }
+  // the setter's default stands for the rule above; a caller who sets another limit gets exactly that
+  const int64_t rule = ue8m0 ? kWideRowsMaxUe8m0 : kWideRowsMax;
+  if (avg > (g_grouped_few_rows_max == kGroupedFewRowsDefault ? rule : g_grouped_few_rows_max)) return 0;
   return avg <= 8 ? 16 : (avg <= 24 ? 32 : 64);
 }
 

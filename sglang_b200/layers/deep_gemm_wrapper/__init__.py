@@ -1,7 +1,7 @@
 """Grouped block-FP8 GEMM entry points with the signatures of
 ``python/sglang/srt/layers/deep_gemm_wrapper/entrypoint.py`` (there they forward to the third-party DeepGEMM
-package; here they call the library's grouped kernel).  No JIT, no warm-up hook: ``expected_m`` is accepted and
-unused."""
+package; here they call the library's grouped kernel).  No JIT, no warm-up hook: ``expected_m`` only chooses between the
+weight-streaming kernel and the 128 x 128 tile kernel."""
 
 from __future__ import annotations
 
@@ -43,8 +43,9 @@ def grouped_gemm_nt_f8f8bf16_masked(lhs: Tuple[torch.Tensor, torch.Tensor], rhs:
     if G == 0 or max_m == 0 or N == 0:
         return
     with torch.cuda.device(a.device):
-        check(lib().sglb200_fp8_blockwise_scaled_masked_grouped_mm(
-            a.data_ptr(), w.data_ptr(), a_s.data_ptr(), w_s.data_ptr(), out.data_ptr(), masked_m.data_ptr(), G, max_m, N, K,
+        check(lib().sglb200_fp8_blockwise_scaled_masked_grouped_mm_expected(
+            a.data_ptr(), w.data_ptr(), a_s.data_ptr(), w_s.data_ptr(), out.data_ptr(), masked_m.data_ptr(), G, max_m,
+            int(expected_m), N, K,
             a.stride(1), w.stride(1), w.stride(0), out.stride(1), a_s.stride(0), a_s.stride(1), a_s.stride(2), w_s.stride(0),
             w_s.stride(1), w_s.stride(2), dtype_code(out.dtype), torch.cuda.current_stream(a.device).cuda_stream),
             "grouped_gemm_nt_f8f8bf16_masked")

@@ -1,0 +1,43 @@
+"""The weight-streaming kernel at the edges of its token tiles (16 / 32 / 64 / 128 columns, chunks of uneven rows) and the
+masked layout with an expected row count, which picks the kernel and must not change the result."""
+
+import pytest
+import torch
+
+import oracle
+from helpers import assert_gemm_close, make_activations, make_weight
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 15, 17, 33, 63, 65, 80, 127, 128])
+@pytest.mark.parametrize("N,K,dtype", [(264, 640, torch.bfloat16), (1160, 2048, torch.float16)])
+def test_token_tile_edges(M, N, K, dtype):
+    from sglang_b200._lib import lib
+    from sglang_b200.layers.quantization import w8a8_block_fp8_matmul
+    a, a_s = oracle.per_token_group_quant_fp8(make_activations(M, K, seed=M), 128)
+    w, w_s = make_weight(N, K, seed=N)
+    got = w8a8_block_fp8_matmul(a.cuda(), w.cuda(), a_s.cuda(), w_s.cuda(), [128, 128], dtype)
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    assert_gemm_close(got, oracle.w8a8_block_fp8_matmul(a, w, a_s, w_s, output_dtype=dtype), f"M={M}")
+
+
+@pytest.mark.parametrize("expected", [0, 1, 9, 24, 48, 100])
+def test_masked_layout_with_expected_rows(expected):
+    from sglang_b200.layers.deep_gemm_wrapper import grouped_gemm_nt_f8f8bf16_masked
+    G, max_m, N, K = 5, 100, 384, 640
+    masked = torch.tensor([100, 0, 1, 37, 65], dtype=torch.int32)
+    q, s = oracle.per_token_group_quant_fp8(make_activations(G * max_m, K, seed=7), 128)
+    ws = [make_weight(N, K, seed=20 + g) for g in range(G)]
+    out = torch.full((G, max_m, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    grouped_gemm_nt_f8f8bf16_masked((q.view(G, max_m, K).cuda(), s.view(G, max_m, -1).cuda()),
+                                    (torch.stack([w[0] for w in ws]).cuda(), torch.stack([w[1] for w in ws]).cuda()), out,
+                                    masked.cuda(), expected)
+    out = out.cpu()
+    for g in range(G):
+        m = int(masked[g])
+        assert (out[g, m:] == 7.0).all(), f"group {g}: rows past masked_m were written"
+        if m:
+            ref = oracle.w8a8_block_fp8_matmul(q.view(G, max_m, K)[g, :m], ws[g][0], s.view(G, max_m, -1)[g, :m], ws[g][1])
+            assert_gemm_close(out[g, :m], ref, f"group {g}")
