@@ -159,15 +159,15 @@ int sglb200_fp8_blockwise_scaled_mm(const void* a, const void* b, const float* s
                                     int64_t sb_stride_k, int out_dtype, void* stream);
 
 /*
- * G with split-K for small M.  When the output tiles alone cannot occupy the SMs (M <= 128 at most shapes) the kernel is
- * bound by streaming the weights; cutting K into ranges that run on different SMs restores the bandwidth.  The ranges
- * write fp32 partial sums to `workspace` ([splits, M, N] floats) and a second small kernel adds them in ascending
- * split order and casts.  sglb200_fp8_blockwise_scaled_mm_workspace_bytes() returns the size this needs for a shape on
- * the current device (0 = split-K would not be used); with workspace == NULL or a workspace that is too small the call
- * is exactly sglb200_fp8_blockwise_scaled_mm.  The workspace is scratch: contents on entry are ignored, calls on the
- * same stream may share it.  Replaces the per-call cudaMalloc'ed CUTLASS workspace of the reference
- * (sgl-kernel/csrc/gemm/fp8_blockwise_gemm_kernel.cu:162-163) and its stream-K path
- * (sgl-kernel/csrc/cutlass_extensions/gemm/fp8_blockwise_gemm_sm90_dispatch.cuh:179-197).
+ * G with scratch for split-K.  When the output tiles alone cannot occupy the SMs the kernel is bound by streaming the
+ * weights; cutting K into ranges that run on different SMs restores the bandwidth.  Above 128 rows the ranges write fp32
+ * partial sums to `workspace` ([splits, M, N] floats) and a second small kernel adds them in ascending split order and
+ * casts; up to 128 rows the CTAs of a cluster share a tile's K and add up on the chip, with or without `workspace`.
+ * sglb200_fp8_blockwise_scaled_mm_workspace_bytes() returns a sufficient size for a shape on the current device (0 = K is
+ * not cut); with workspace == NULL or a workspace that is too small the call is exactly sglb200_fp8_blockwise_scaled_mm.
+ * The workspace is scratch: contents on entry are ignored, calls on the same stream may share it.  Replaces the per-call
+ * cudaMalloc'ed CUTLASS workspace of the reference (sgl-kernel/csrc/gemm/fp8_blockwise_gemm_kernel.cu:162-163) and its
+ * stream-K path (sgl-kernel/csrc/cutlass_extensions/gemm/fp8_blockwise_gemm_sm90_dispatch.cuh:179-197).
  */
 int64_t sglb200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int sglb200_fp8_blockwise_scaled_mm_ws(const void* a, const void* b, const float* sa, const float* sb, void* out,
@@ -175,6 +175,21 @@ int sglb200_fp8_blockwise_scaled_mm_ws(const void* a, const void* b, const float
                                        int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n,
                                        int64_t sb_stride_k, int out_dtype, void* workspace, int64_t workspace_bytes,
                                        void* stream);
+
+/*
+ * L  The linear layer in one call: per-token-group quantisation of x, block-scaled GEMM, optional bias.
+ *   x [M, K] (dtype = SGLB200_BF16 | SGLB200_F16) contiguous, K % 128 == 0;  w [N, K] e4m3 contiguous, N % 8 == 0
+ *   w_scale: scale_ue8m0 == 0: fp32 [ceil(N/128), K/128];  != 0: int32 words [ceil(N/128), ceil(K/512)] of four exponent
+ *            bytes (the activation scales are then powers of two too); element (n, k) at n * stride_n + k * stride_k
+ *   bias [N] of dtype or NULL: added to the rounded product, one more rounding, as `output += bias` does
+ *   out [M, N] of dtype, contiguous;  eps as in sglb200_per_token_group_quant_fp8 (already rounded to dtype)
+ *   scratch: sglb200_fp8_block_linear_scratch_bytes(M, N, K, scale_ue8m0) bytes, 256-byte aligned, contents arbitrary.
+ * Replaces: w8a8_block_fp8_linear  python/sglang/srt/layers/quantization/fp8_utils.py:184-301.
+ */
+int sglb200_fp8_block_linear(const void* x, const void* w, const void* w_scale, const void* bias, void* out, int64_t M,
+                             int64_t N, int64_t K, int64_t w_scale_stride_n, int64_t w_scale_stride_k, int scale_ue8m0,
+                             float eps, int dtype, void* scratch, int64_t scratch_bytes, void* stream);
+int64_t sglb200_fp8_block_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int scale_ue8m0);
 
 /*
  * G with split-K for callers that cannot allocate.  No counterpart in the reference.
@@ -234,9 +249,9 @@ int sglb200_fp8_blockwise_scaled_mm_pair(const void* a, const void* b, const flo
 int sglb200_fp8_ue8m0_scaled_mm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, void* out,
                                 int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int64_t sfa_ld,
                                 int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype, void* stream);
-/* The same with optional split-K scratch for M <= 64 (size: sglb200_fp8_blockwise_scaled_mm_workspace_bytes; NULL = no
- * split).  Up to 64 rows both entries run the weight-streaming kernel of sglb200_fp8_blockwise_scaled_mm, which decodes
- * the exponent bytes itself (the scales stay exact powers of two); above that the block-scaling kernel. */
+/* The same with the scratch argument of sglb200_fp8_blockwise_scaled_mm_ws, which is checked and not needed.  Up to 64 rows
+ * both entries run the weight-streaming kernel of sglb200_fp8_blockwise_scaled_mm, which decodes the exponent bytes itself
+ * (the scales stay exact powers of two); above that the block-scaling kernel. */
 int sglb200_fp8_ue8m0_scaled_mm_ws(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, void* out,
                                    int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int64_t sfa_ld,
                                    int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype, void* workspace,

@@ -30,13 +30,21 @@ int make_map_sw128(CUtensorMap* map, const void* base, int rank, const uint64_t*
 
 // The few-rows (M <= smallm_max_rows()) weight-streaming GEMM, gemm_smallm.cu
 int smallm_max_rows();
-int smallm_splits(int64_t N, int64_t K, int sm_count);
+constexpr int kMaxCluster = 8;
+int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count);  // CTAs that share a tile's K, 1..kMaxCluster
 int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K,
                 int64_t lda, int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n,
-                int64_t sb_stride_k, int out_dtype, float* partial, int64_t partial_floats, int sm_count, void* stream,
-                int* splits_used, bool always_partial = false, bool ue8m0 = false);
-void launch_splitk_reduce(const float* partial, void* out, int64_t M, int64_t N, int64_t ldc, int splits, int out_dtype,
-                          int sm_count, void* stream);  // gemm.cu
+                int64_t sb_stride_k, int out_dtype, const void* bias, float* partial, int64_t partial_floats, int sm_count,
+                void* stream, int* splits_used, bool ue8m0);
+void launch_splitk_reduce(const float* partial, void* out, const void* bias, int64_t M, int64_t N, int64_t ldc, int splits,
+                          int out_dtype, int sm_count, void* stream);  // gemm.cu
+// Per-token-group quantisation (groups of 128) of whole rows, quant.cu
+int quant_rows(const void* input, int in_dtype, void* out_q, void* out_s, int64_t rows, int64_t hidden, float eps, bool ue8m0,
+               int64_t s_stride_row, int64_t s_stride_group, void* stream);
+// The UE8M0 GEMM of the linear layer, gemm_ue8m0.cu
+int ue8m0_linear_gemm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, const void* bias, void* out, int64_t M,
+                      int64_t N, int64_t K, int64_t sfa_ld, int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype,
+                      void* stream);
 int smallm_take_device_status();
 int nvls_take_device_status();  // nvls.cu
 constexpr int kGroupedFewRowsDefault = 20;
@@ -57,21 +65,33 @@ int pair_gemm(int bn, const void* a, const void* b, const float* sa, const float
               int64_t sb_stride_n, int64_t sb_stride_k, int out_dtype, int sm_count, void* stream);
 
 // Launch with programmatic stream serialization allowed: the kernel may begin before the previous kernel of the stream
-// has finished and must call ptx::grid_dep_wait() before it touches anything that kernel writes or reads.
+// has finished and must call ptx::grid_dep_wait() before it touches anything that kernel writes or reads.  With cluster > 1
+// in clusters of that many CTAs.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                              Args&&... args) {
+inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                      int cluster, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              Args&&... args) {
+  return launch_pdl_cluster(kernel, grid, block, smem, stream, 1, args...);
 }
 
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }

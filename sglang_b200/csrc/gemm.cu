@@ -92,6 +92,7 @@ struct GemmParams {
   const float* sa;
   const float* sb;
   void* out;
+  const void* bias;               // dense, optional: [N] of the output type, added to the rounded result
   const int32_t* expert_offsets;  // null: dense (or the masked layout, see rows_per_expert)
   const int32_t* problem_sizes;   // grouped, optional: rows of expert e = problem_sizes[count_stride * e]
   int32_t count_stride;           // 3 for a [E, 3] problem-size table, 1 for a plain per-expert row count
@@ -654,8 +655,14 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                                                : pack2<__half>(acc[16 * h + w].x, acc[16 * h + w].y);
           warp_rows_via_smem(stg, v, lane, [&](int r, int w, uint4 val) {
             const int32_t c = 32 * h + 2 * w;  // 8 columns from n_first + c (N % 8 == 0)
-            if (row_base + r < tl.row_end && n_first + c < p.N)
+            if (row_base + r < tl.row_end && n_first + c < p.N) {
+              if constexpr (!GROUPED && !AR) {
+                if (p.bias != nullptr)
+                  val = ptx::add_bias8(val, __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + n_first + c)),
+                                       p.out_dtype);
+              }
               *reinterpret_cast<uint4*>(out + (int64_t)r * p.ldc + c) = val;
+            }
           });
         }
       }
@@ -683,8 +690,8 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 // out[m, n] = cast(sum_s partial[s][m][n]); 8 columns per thread, splits added in ascending order
 template <typename OutT>
 __global__ void __launch_bounds__(256)
-splitk_reduce_kernel(const float* __restrict__ partial, OutT* __restrict__ out, int32_t M, int32_t N, int64_t ldc,
-                     int32_t splits) {
+splitk_reduce_kernel(const float* __restrict__ partial, OutT* __restrict__ out, const void* __restrict__ bias, int32_t M,
+                     int32_t N, int64_t ldc, int32_t splits, int32_t out_dtype) {
   ptx::grid_dep_launch();  // the next kernel may begin its set-up (and a GEMM its weight streaming) beside this one
   ptx::grid_dep_wait();    // the partial sums come from the kernel before this one
   const int32_t vec_per_row = N / 8;
@@ -706,6 +713,7 @@ splitk_reduce_kernel(const float* __restrict__ partial, OutT* __restrict__ out, 
     u.y = pack2<OutT>(a[2], a[3]);
     u.z = pack2<OutT>(a[4], a[5]);
     u.w = pack2<OutT>(a[6], a[7]);
+    if (bias != nullptr) u = ptx::add_bias8(u, __ldg(reinterpret_cast<const uint4*>(static_cast<const OutT*>(bias) + c)), out_dtype);
     *reinterpret_cast<uint4*>(out + (int64_t)m * ldc + c) = u;
   }
 }
@@ -1020,18 +1028,18 @@ int make_map_sw128(CUtensorMap* map, const void* base, int rank, const uint64_t*
   return SGLB200_OK;
 }
 
-void launch_splitk_reduce(const float* partial, void* out, int64_t M, int64_t N, int64_t ldc, int splits, int out_dtype,
-                          int sm_count, void* stream) {
+void launch_splitk_reduce(const float* partial, void* out, const void* bias, int64_t M, int64_t N, int64_t ldc, int splits,
+                          int out_dtype, int sm_count, void* stream) {
   const int64_t vecs = M * (N / 8);
   int rgrid = (int)((vecs + 255) / 256);
   if (rgrid > sm_count * 8) rgrid = sm_count * 8;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (out_dtype == SGLB200_BF16) {
-    launch_pdl(splitk_reduce_kernel<__nv_bfloat16>, dim3(rgrid), dim3(256), 0, st, partial, static_cast<__nv_bfloat16*>(out),
-               (int32_t)M, (int32_t)N, ldc, (int32_t)splits);
+    launch_pdl(splitk_reduce_kernel<__nv_bfloat16>, dim3(rgrid), dim3(256), 0, st, partial, static_cast<__nv_bfloat16*>(out), bias,
+               (int32_t)M, (int32_t)N, ldc, (int32_t)splits, (int32_t)out_dtype);
   } else {
-    launch_pdl(splitk_reduce_kernel<__half>, dim3(rgrid), dim3(256), 0, st, partial, static_cast<__half*>(out), (int32_t)M,
-               (int32_t)N, ldc, (int32_t)splits);
+    launch_pdl(splitk_reduce_kernel<__half>, dim3(rgrid), dim3(256), 0, st, partial, static_cast<__half*>(out), bias, (int32_t)M,
+               (int32_t)N, ldc, (int32_t)splits, (int32_t)out_dtype);
   }
 }
 
@@ -1069,7 +1077,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
                 int64_t lda, int64_t ldb, int64_t ldb_e, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k,
                 int64_t sb_stride_e, int64_t sb_stride_n, int64_t sb_stride_k, int out_dtype, void* stream,
                 float* workspace = nullptr, int64_t workspace_floats = 0, const PushParams* push = nullptr,
-                int64_t rows_per_expert = 0, int64_t sa_stride_e = 0, int64_t expected_rows = 0) {
+                int64_t rows_per_expert = 0, int64_t sa_stride_e = 0, int64_t expected_rows = 0, const void* bias = nullptr) {
   const bool grouped = expert_offsets != nullptr || rows_per_expert > 0;
   SGLB_REQUIRE(total_rows >= 0 && N >= 0 && K >= 0, SGLB200_ERR_SHAPE, "M=%lld N=%lld K=%lld: negative size",
                (long long)total_rows, (long long)N, (long long)K);
@@ -1100,11 +1108,11 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
                di.cc_major, di.cc_minor);
 
   if (!grouped && push && total_rows <= smallm_max_rows() && workspace != nullptr &&
-      (int64_t)smallm_splits(N, K, di.sm_count) * total_rows * N <= workspace_floats) {
+      (int64_t)smallm_cluster(total_rows, N, K, di.sm_count) * total_rows * N <= workspace_floats) {
     // few rows, exchanged: the weight-streaming kernel leaves fp32 sums, a second kernel casts and pushes them
     int splits = 1;
     if (int rc = smallm_gemm(a, b, sa, sb, out, total_rows, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n,
-                             sb_stride_k, out_dtype, workspace, workspace_floats, di.sm_count, stream, &splits, true))
+                             sb_stride_k, out_dtype, nullptr, workspace, workspace_floats, di.sm_count, stream, &splits, false))
       return rc;
     const int32_t n_tiles = (int32_t)((N + BN - 1) / BN);
     const int32_t tiles = (int32_t)((total_rows + BM - 1) / BM) * n_tiles;
@@ -1120,13 +1128,8 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
   }
   if (!grouped && !push && total_rows <= smallm_max_rows()) {
     // few rows: the weight-streaming kernel with swapped operands (gemm_smallm.cu)
-    int splits = 1;
-    if (int rc = smallm_gemm(a, b, sa, sb, out, total_rows, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n,
-                             sb_stride_k, out_dtype, workspace, workspace_floats, di.sm_count, stream, &splits))
-      return rc;
-    if (splits > 1) launch_splitk_reduce(workspace, out, total_rows, N, ldc, splits, out_dtype, di.sm_count, stream);
-    SGLB_CHECK_LAUNCH("splitk_reduce_kernel");
-    return SGLB200_OK;
+    return smallm_gemm(a, b, sa, sb, out, total_rows, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k,
+                       out_dtype, bias, nullptr, 0, di.sm_count, stream, nullptr, false);
   }
 
   if (grouped && !push) {
@@ -1155,6 +1158,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
   p.sa = sa;
   p.sb = sb;
   p.out = out;
+  p.bias = bias;
   p.expert_offsets = expert_offsets;
   p.problem_sizes = problem_sizes;
   p.count_stride = rows_per_expert > 0 ? 1 : 3;
@@ -1206,7 +1210,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
     fp8_block_gemm_kernel<false, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, static_cast<const GemmParams&>(p));
     if (p.partial != nullptr) {
       SGLB_CHECK_LAUNCH("fp8_block_gemm_kernel");
-      launch_splitk_reduce(p.partial, out, total_rows, N, ldc, p.k_splits, out_dtype, di.sm_count, stream);
+      launch_splitk_reduce(p.partial, out, bias, total_rows, N, ldc, p.k_splits, out_dtype, di.sm_count, stream);
     }
   }
   SGLB_CHECK_LAUNCH("fp8_block_gemm_kernel");
@@ -1271,7 +1275,10 @@ extern "C" int64_t sglb200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, in
   sglb::DeviceInfo di;
   int sms = 148;
   if (sglb::device_info(&di) == SGLB200_OK) sms = di.sm_count;
-  const int splits = M <= sglb::smallm_max_rows() ? sglb::smallm_splits(N, K, sms) : sglb::splitk_choice(M, N, K, sms);
+  // up to 128 rows K is added up inside a cluster and the scratch goes unused; the size stays an upper bound of what a split
+  // of that shape may need, so that callers who hold it keep working
+  const int splits = M > sglb::smallm_max_rows() ? sglb::splitk_choice(M, N, K, sms)
+                     : sglb::smallm_cluster(M, N, K, sms) > 1 ? sglb::kMaxCluster : 1;
   return splits > 1 ? (int64_t)splits * M * N * (int64_t)sizeof(float) : 0;
 }
 
@@ -1286,6 +1293,65 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm_ws(const void* a, const void* b, 
   return sglb::gemm_common(a, b, sa, sb, out, nullptr, nullptr, M, 1, N, K, lda, ldb, 0, ldc, sa_stride_m, sa_stride_k,
                            0, sb_stride_n, sb_stride_k, out_dtype, stream, static_cast<float*>(workspace),
                            workspace ? workspace_bytes / (int64_t)sizeof(float) : 0);
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// The linear layer in one call: quantise, multiply, add the bias.  Scratch: [GEMM scratch | activation scales | codes].
+// ---------------------------------------------------------------------------------------------------------
+namespace sglb {
+namespace {
+struct LinearScratch {
+  int64_t gemm_bytes, scales_at, codes_at, bytes, ld;
+};
+LinearScratch linear_scratch(int64_t M, int64_t N, int64_t K, bool ue8m0, int sms) {
+  LinearScratch l;
+  const int splits = !ue8m0 && M > smallm_max_rows() ? splitk_choice(M, N, K, sms) : 1;
+  l.gemm_bytes = splits > 1 ? (int64_t)splits * M * N * (int64_t)sizeof(float) : 0;
+  l.ld = (M + 3) / 4 * 4;
+  const int64_t words = ue8m0 ? (K / 128 + 3) / 4 : K / 128;
+  l.scales_at = (l.gemm_bytes + 511) / 512 * 512;
+  l.codes_at = l.scales_at + (words * l.ld * 4 + 511) / 512 * 512;
+  l.bytes = l.codes_at + M * K;
+  return l;
+}
+}  // namespace
+}  // namespace sglb
+
+extern "C" int64_t sglb200_fp8_block_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int scale_ue8m0) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  sglb::DeviceInfo di;
+  int sms = 148;
+  if (sglb::device_info(&di) == SGLB200_OK) sms = di.sm_count;
+  return sglb::linear_scratch(M, N, K, scale_ue8m0 != 0, sms).bytes;
+}
+
+extern "C" int sglb200_fp8_block_linear(const void* x, const void* w, const void* w_scale, const void* bias, void* out, int64_t M,
+                                        int64_t N, int64_t K, int64_t w_scale_stride_n, int64_t w_scale_stride_k,
+                                        int scale_ue8m0, float eps, int dtype, void* scratch, int64_t scratch_bytes,
+                                        void* stream) {
+  SGLB_REQUIRE(dtype == SGLB200_BF16 || dtype == SGLB200_F16, SGLB200_ERR_DTYPE, "dtype=%d: only bf16 (0) and f16 (1)", dtype);
+  SGLB_REQUIRE(M >= 0 && N >= 0 && K >= 0 && K % 128 == 0, SGLB200_ERR_SHAPE, "M=%lld N=%lld K=%lld: K in whole groups of 128",
+               (long long)M, (long long)N, (long long)K);
+  if (M == 0 || N == 0) return SGLB200_OK;
+  SGLB_REQUIRE(K > 0, SGLB200_ERR_SHAPE, "K must be positive");
+  SGLB_REQUIRE(scratch != nullptr && sglb::aligned(scratch, 256), SGLB200_ERR_ALIGN, "scratch must be 256-byte aligned");
+  SGLB_REQUIRE(bias == nullptr || sglb::aligned(bias, 16), SGLB200_ERR_ALIGN, "bias must be 16-byte aligned");
+  sglb::DeviceInfo di;
+  if (int rc = sglb::device_info(&di)) return rc;
+  const bool ue = scale_ue8m0 != 0;
+  const sglb::LinearScratch l = sglb::linear_scratch(M, N, K, ue, di.sm_count);
+  SGLB_REQUIRE(scratch_bytes >= l.bytes, SGLB200_ERR_WORKSPACE, "scratch_bytes=%lld: %lld needed", (long long)scratch_bytes,
+               (long long)l.bytes);
+  char* base = static_cast<char*>(scratch);
+  void *scales = base + l.scales_at, *codes = base + l.codes_at;
+  if (int rc = sglb::quant_rows(x, dtype, codes, scales, M, K, eps, ue, 1, l.ld, stream)) return rc;
+  if (ue)
+    return sglb::ue8m0_linear_gemm(codes, w, static_cast<const int32_t*>(scales), static_cast<const int32_t*>(w_scale), bias, out, M,
+                                   N, K, l.ld, w_scale_stride_n, w_scale_stride_k, dtype, stream);
+  return sglb::gemm_common(codes, w, static_cast<const float*>(scales), static_cast<const float*>(w_scale), out, nullptr, nullptr, M,
+                           1, N, K, K, K, 0, N, 1, l.ld, 0, w_scale_stride_n, w_scale_stride_k, dtype, stream,
+                           l.gemm_bytes > 0 ? static_cast<float*>(scratch) : nullptr, l.gemm_bytes / (int64_t)sizeof(float), nullptr,
+                           0, 0, 0, bias);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -1372,7 +1438,7 @@ extern "C" int64_t sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes(int64_t 
   sglb::DeviceInfo di;
   int sms = 148;
   if (sglb::device_info(&di) == SGLB200_OK) sms = di.sm_count;
-  return (int64_t)sglb::smallm_splits(N, K, sms) * M * N * (int64_t)sizeof(float);
+  return (int64_t)sglb::smallm_cluster(M, N, K, sms) * M * N * (int64_t)sizeof(float);
 }
 
 extern "C" int64_t sglb200_peer_recv_bytes(int64_t slot_elems) {
@@ -1617,6 +1683,7 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm_allreduce(const void* a, const vo
   p.sa = sa;
   p.sb = sb;
   p.out = out;
+  p.bias = nullptr;
   p.expert_offsets = nullptr;
   p.problem_sizes = nullptr;
   p.count_stride = 3;

@@ -171,6 +171,7 @@ fp8_block_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
     n0 = nt * BN;
   };
 
+  const bool leader = ptx::elect_one();  // the lane that issues TMA and tcgen05 instructions
   // Registers move from the four producer / MMA warps (one warpgroup, one instruction) to the promotion warps.
   if constexpr (C::kRealloc) {
     if (warp < kFirstPromoWarp) {
@@ -179,7 +180,6 @@ fp8_block_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
       asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
     }
   }
-  const bool leader = ptx::elect_one();  // the lane that issues TMA and tcgen05 instructions
   if (warp < kProducers) {
     uint32_t stage = 0, phase = 0, g = 0;
     uint32_t armed = 0, armed_phase = 0;  // bit i: this warp has armed stage i / the phase bit of its last arming

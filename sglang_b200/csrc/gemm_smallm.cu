@@ -4,8 +4,10 @@
 // M) by MT token columns (the MMA's N, MT = 16 / 32 / 64 / 128, and as few of them as the item has rows).  An accumulator
 // stage is then only MT TMEM columns wide, so 4 to 16 k-blocks are in flight between the MMA warp and the promotion warps, and
 // a shared-memory stage is 16 KB of weights plus MT x 128 bytes of activations, 6 to 11 of them: 64 KB of weights in flight
-// per SM already bring a plain stream of such tiles to 90 % of the HBM rate, 128 KB to all of it.  K can be cut into ranges
-// that run on different SMs (fp32 partial sums, added by splitk_reduce_kernel) when N / 128 tiles alone cannot occupy the SMs.
+// per SM already bring a plain stream of such tiles to 90 % of the HBM rate, 128 KB to all of it.  When
+// N / 128 tiles alone cannot occupy the SMs, the CTAs of a cluster cut a tile's K among themselves and rank 0 adds their sums up
+// out of their shared memory (smallm_cluster): against fp32 partial sums in memory and a kernel that adds them, quantiser
+// included, N=576 K=7168 M=1 / 48: 9.6 / 14.1 -> 6.8 / 11.1 us, N=7168 K=16384 M=48 32.3 -> 27.1, N=10240 K=8192 M=48 27.0 -> 22.1.
 // From 65 to 128 rows eight promotion warps share every accumulator stage, four per 64 token columns.
 // Measured against scales that every promotion warp fetched and spread by shuffles, weights from HBM (B200):
 // N=36864 K=7168 M=32 / 64 / 128: 46.6 / 54.8 / 75.0 -> 41.8 / 43.3 / 55.1 us (6.1 TB/s at 64 rows);
@@ -27,6 +29,8 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "ptx.cuh"
@@ -59,6 +63,8 @@ constexpr int kScaleStages = 4;
 constexpr uint32_t kCtlBytes = 640;
 constexpr uint32_t kPatchRow = 80, kPatchBytes = 16 * kPatchRow;  // epilogue patch of a warp: 16 tokens x 64 bytes, padded
 
+constexpr int kAuxRegs = 96, kPromoRegs = 200;  // register split of the NSUB = 2 form (four and eight warps)
+
 constexpr int kMaxExperts = 1024;
 
 // NSUB = 2 (65 to 128 rows per item): the MMA covers up to MT * NSUB = 128 activation rows and a second set of four
@@ -84,7 +90,9 @@ struct SmallParams {
   const float* sa;  // UE8M0 variant: int32 words, four exponent bytes (k-blocks 4g .. 4g + 3) per word
   const float* sb;
   void* out;
-  float* partial;  // [splits][M][N] fp32 when k_splits > 1
+  const void* bias;  // [N] of the output type, or NULL: added to the rounded result
+  float* partial;    // fp32 sums [splits][M][N] instead of `out`
+  int32_t cluster;   // > 1: the CTAs of a cluster share one tile's K, rank 0 adds their sums up (k_splits == cluster)
   int32_t M, N, K;
   int32_t n_tiles, k_tiles, k_splits, kb_per_split;
   int64_t ldc;
@@ -113,12 +121,17 @@ __device__ __forceinline__ void expert_rows(const SmallParams& p, int32_t e, int
   }
 }
 
-template <int TILE, bool GROUPED>
+template <int TILE, bool GROUPED, bool CLUSTER>
 __device__ __forceinline__ Item get_item(const SmallParams& p, const int32_t* item_start, int32_t t) {
   Item it;
   if constexpr (!GROUPED) {
-    it.split = t / p.n_tiles;
-    it.nt = t - it.split * p.n_tiles;
+    if constexpr (CLUSTER) {
+      it.nt = t / p.cluster;
+      it.split = t - it.nt * p.cluster;
+    } else {
+      it.split = t / p.n_tiles;
+      it.nt = t - it.split * p.n_tiles;
+    }
     it.kb0 = it.split * p.kb_per_split;
     it.kb1 = min(it.kb0 + p.kb_per_split, p.k_tiles);
     it.e = 0;
@@ -237,8 +250,12 @@ __device__ __forceinline__ uint32_t pack16(float a, float b, int out_dtype) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-template <int MT, bool UE, bool GROUPED, int NSUB>
-__global__ void __launch_bounds__(128 + 128 * NSUB, 1)
+// CLUSTER is a template parameter because the mere presence of the adding-up code cost the main loop of the other form up to
+// 18 % (N=36864 K=7168 M=113: 57 -> 68 us) through its register allocation.
+template <int MT, bool UE, bool GROUPED, int NSUB, bool CLUSTER>
+// NSUB = 1 has 256 threads; the bound of 320 keeps it at 200 registers, so that a block of the quantiser or of another small
+// kernel (256 threads of 48) fits beside it and programmatic dependent launch really overlaps the two.
+__global__ void __launch_bounds__(NSUB == 1 ? 320 : 384, 1)
 fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                              const SmallParams p) {
   using C = Cfg<MT, NSUB>;
@@ -319,7 +336,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
   // than the 168 registers that 384 threads start with; the other four warps need few: 128 * 96 + 256 * 200 = 63488 <=
   // 384 * 168.  No call may sit in a region with a changed limit, hence the inlined waits.
   if (warp >= 4) {
-    if constexpr (NSUB == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    if constexpr (NSUB == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPromoRegs));
     // ===== promotion + transposed store; TMEM lane quarter = warp % 4.  A warp owns 32 weight rows (columns of the output)
     // and MT tokens.  The sums are loaded in fragment arrangement (tmem_ld_16x256), in which a thread meets only MT / 4
     // tokens: with one weight row per thread (32x32b loads) every thread needs every token's scale, and the 64 KB of
@@ -332,9 +349,10 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
     const int tr = lane >> 2, tc = 2 * (lane & 3);    // this thread's row inside 8 weight rows / column inside 8 tokens
     uint8_t* patch = reinterpret_cast<uint8_t*>(smem) + C::kPatchOffset + (size_t)(warp - 4) * kPatchBytes;
     uint32_t acc_stage = 0, acc_phase = 0, sc_stage = 0, sc_phase = 0;
+    [[maybe_unused]] bool met = false;  // this warp has passed the cluster's first barrier
     float2 acc[2][G][2];  // [lanes 0-15 / 16-31][token group][rows tr / tr + 8]: two neighbouring tokens
     for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
-      const Item it = get_item<C::kTile, GROUPED>(p, item_start, t);
+      const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
       const int32_t kb0 = it.kb0, kb1 = it.kb1;
       const int32_t row0 = it.row0 + sub * MT, rows = max(0, min(MT, it.rows - sub * MT));
 #pragma unroll
@@ -390,6 +408,45 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       }
       if (!ok || ctl->abort_flag) break;
       const int32_t n_warp = it.nt * BN + q * 32;  // first of the warp's 32 output columns
+      if constexpr (CLUSTER) {
+        {
+          // One tile per cluster, K cut into as many ranges.  The others leave their sums, fragment order, in their own shared
+          // memory (the ring of stages: all of its loads and MMAs are done) and rank 0 adds them in the order of K.
+          constexpr int kWarps = 4 * NSUB;
+          float4* mine = reinterpret_cast<float4*>(smem) + (size_t)(warp - 4) * 2 * G * 32 + lane;
+          if (it.split != 0) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int g = 0; g < G; ++g)
+                if (8 * g < rows)
+                  mine[(h * G + g) * 32] = make_float4(acc[h][g][0].x, acc[h][g][0].y, acc[h][g][1].x, acc[h][g][1].y);
+          }
+          met = true;
+          ptx::cluster_arrive_release();
+          ptx::cluster_wait_acquire();
+          static_assert((size_t)kWarps * 2 * G * 32 * sizeof(float4) <= (size_t)C::kStages * C::kStageBytes, "sums of a tile");
+          if (it.split == 0) {
+            const uint32_t local = ptx::smem_u32(mine);
+            for (int32_t r = 1; r < p.cluster; ++r) {
+              const uint32_t src = ptx::mapa_shared(local, (uint32_t)r);
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+                  if (8 * g < rows) {
+                    const float4 v = ptx::ld_cluster_f4(src + (h * G + g) * 32 * (uint32_t)sizeof(float4));
+                    acc[h][g][0].x += v.x;
+                    acc[h][g][0].y += v.y;
+                    acc[h][g][1].x += v.z;
+                    acc[h][g][1].y += v.w;
+                  }
+            }
+          } else {
+            continue;
+          }
+        }
+      }
       if (p.partial != nullptr) {
         float* dst = p.partial + ((int64_t)it.split * p.M + row0) * p.N + n_warp;
 #pragma unroll
@@ -410,29 +467,47 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         // 16 tokens per pass through the warp's patch: transposed there by stmatrix, read back as 64 bytes of a token's row
         const uint32_t st_addr = ptx::smem_u32(patch) + (uint32_t)(lane & 7) * kPatchRow + (uint32_t)(lane >> 3) * 16;
         char* out = static_cast<char*>(p.out) + ((int64_t)row0 * p.ldc + n_warp) * 2;
+        auto store = [&](auto with_bias) {
+          const char* bias = static_cast<const char*>(p.bias);
 #pragma unroll
-        for (int g = 0; g < G; g += 2) {
-          if (8 * g >= rows) break;
-          __syncwarp();  // the previous pass has been read out
+          for (int g = 0; g < G; g += 2) {
+            if (8 * g >= rows) break;
+            __syncwarp();  // the previous pass has been read out
 #pragma unroll
-          for (int i = 0; i < 2; ++i)
-            stmatrix_x4_trans(st_addr + i * 8 * kPatchRow, pack16(acc[0][g + i][0].x, acc[0][g + i][0].y, p.out_dtype),
-                              pack16(acc[0][g + i][1].x, acc[0][g + i][1].y, p.out_dtype),
-                              pack16(acc[1][g + i][0].x, acc[1][g + i][0].y, p.out_dtype),
-                              pack16(acc[1][g + i][1].x, acc[1][g + i][1].y, p.out_dtype));
-          __syncwarp();
+            for (int i = 0; i < 2; ++i)
+              stmatrix_x4_trans(st_addr + i * 8 * kPatchRow, pack16(acc[0][g + i][0].x, acc[0][g + i][0].y, p.out_dtype),
+                                pack16(acc[0][g + i][1].x, acc[0][g + i][1].y, p.out_dtype),
+                                pack16(acc[1][g + i][0].x, acc[1][g + i][0].y, p.out_dtype),
+                                pack16(acc[1][g + i][1].x, acc[1][g + i][1].y, p.out_dtype));
+            __syncwarp();
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int32_t tl = i * 8 + (lane >> 2), tok = 8 * g + tl, c = (lane & 3) * 8;
-            const uint4 val = *reinterpret_cast<const uint4*>(patch + tl * kPatchRow + c * 2);
-            if (tok < rows && n_warp + c < p.N)  // N % 8 == 0
-              *reinterpret_cast<uint4*>(out + ((int64_t)tok * p.ldc + c) * 2) = val;
+            for (int i = 0; i < 2; ++i) {
+              const int32_t tl = i * 8 + (lane >> 2), tok = 8 * g + tl, c = (lane & 3) * 8;
+              uint4 val = *reinterpret_cast<const uint4*>(patch + tl * kPatchRow + c * 2);
+              if (tok < rows && n_warp + c < p.N) {  // N % 8 == 0
+                if constexpr (decltype(with_bias)::value)
+                  val = ptx::add_bias8(val, __ldg(reinterpret_cast<const uint4*>(bias + (int64_t)(n_warp + c) * 2)), p.out_dtype);
+                *reinterpret_cast<uint4*>(out + ((int64_t)tok * p.ldc + c) * 2) = val;
+              }
+            }
           }
+        };
+        if constexpr (GROUPED) {
+          store(std::false_type{});
+        } else {
+          if (p.bias == nullptr) store(std::false_type{});
+          else store(std::true_type{});
         }
       }
     }
+    if constexpr (CLUSTER) {
+      if (!met) {  // after a time-out: the other CTAs of the cluster still wait for this warp
+        ptx::cluster_arrive_release();
+        ptx::cluster_wait_acquire();
+      }
+    }
   } else {
-    if constexpr (NSUB == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+    if constexpr (NSUB == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kAuxRegs));
     if (warp == 0) {
       // ===== TMA producer.  Pass 0 runs before griddepcontrol.wait: the weight tiles of the first k-blocks (at most one
       // ring of stages, whose barriers are fresh) are requested; pass 1 adds their activation tiles and then continues
@@ -443,7 +518,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         uint32_t stage = 0, phase = 0, idx = 0;
         bool ok = true;
         for (int32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
-          const Item it = get_item<C::kTile, GROUPED>(p, item_start, t);
+          const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
           const int32_t nt = it.nt;
           for (int32_t kb = it.kb0; kb < it.kb1; ++kb, ++idx) {
             const uint32_t dst = stage0 + stage * C::kStageBytes;
@@ -496,7 +571,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       const uint64_t desc0 = ptx::make_kmajor_sw128_desc(stage0);
       uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
       for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
-        const Item it = get_item<C::kTile, GROUPED>(p, item_start, t);
+        const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
         const int32_t kb0 = it.kb0, kb1 = it.kb1;
         const uint32_t idesc = ptx::make_idesc_e4m3_f32(BN, (uint32_t)(it.rows + 15) / 16 * 16);
         bool ok = true;
@@ -527,7 +602,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       constexpr int kPerLane = C::kTile / 32 > 0 ? C::kTile / 32 : 1;
       uint32_t stage = 0, phase = 0;
       for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
-        const Item it = get_item<C::kTile, GROUPED>(p, item_start, t);
+        const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
         const float* sb_blk = p.sb + (int64_t)it.nt * p.sb_stride_n;
         const float* sa_base = p.sa + (int64_t)it.row0 * p.sa_stride_m;
         if constexpr (GROUPED) {
@@ -572,33 +647,50 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         if (!ok || ctl->abort_flag) break;
       }
     }
+    if constexpr (CLUSTER) {  // the barrier at which the promotion warps meet those of the other CTAs counts every thread
+      ptx::cluster_arrive_release();
+      ptx::cluster_wait_acquire();
+    }
   }
 
   ptx::tc_fence_before();
   __syncthreads();
+  if constexpr (CLUSTER) {  // no CTA leaves, and no shared memory goes, before rank 0 has read the sums
+    ptx::cluster_arrive_release();
+    ptx::cluster_wait_acquire();
+  }
   if (warp == 1) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
-template <int MT, bool UE, bool GROUPED, int NSUB = 1>
+template <int MT, bool UE, bool GROUPED, int NSUB = 1, bool CLUSTER = false>
 int launch(const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams& p, int sm_count, cudaStream_t st,
-           int64_t max_items) {
+           int64_t max_items, int cluster = 1) {
   constexpr size_t smem = GROUPED ? Cfg<MT, NSUB>::kSmemGrouped : Cfg<MT, NSUB>::kSmem;
   constexpr int kThreads = Cfg<MT, NSUB>::kThreads;
   static bool done[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB>,
+    cudaError_t e = cudaFuncSetAttribute(fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB, CLUSTER>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SGLB200_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    if (NSUB == 2) {
+      // setmaxnreg.inc draws on the registers the block was launched with and waits for good if they do not suffice: a
+      // build whose register count is too low for the split must not be launched
+      cudaFuncAttributes fa;
+      e = cudaFuncGetAttributes(&fa, fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB, CLUSTER>);
+      if (e != cudaSuccess || fa.numRegs * kThreads < 128 * kAuxRegs + 256 * kPromoRegs)
+        return fail(SGLB200_ERR_LAUNCH, "fp8_block_gemm_smallm_kernel: %d registers a thread are too few for its register split",
+                    e == cudaSuccess ? fa.numRegs : 0);
+    }
     done[dev] = true;
   }
   const int grid = (int)(max_items < sm_count ? max_items : sm_count);
-  const cudaError_t le = launch_pdl(fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB>, dim3(grid), dim3(kThreads), smem, st,
-                                    map_w, map_a, p);
+  const cudaError_t le = launch_pdl_cluster(fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB, CLUSTER>, dim3(grid), dim3(kThreads), smem, st,
+                                            cluster, map_w, map_a, p);
   if (le != cudaSuccess) {
     cudaGetLastError();
     return fail(SGLB200_ERR_LAUNCH, "fp8_block_gemm_smallm_kernel: %s", cudaGetErrorString(le));
@@ -606,40 +698,58 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams
   return SGLB200_OK;
 }
 
+// one tile per cluster, as many clusters as tiles
+template <bool UE>
+int launch_cluster(int MT, bool two, const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams& p, cudaStream_t st,
+                   int64_t items) {
+  const int grid = (int)items, c = p.cluster;
+  if (two) return launch<64, UE, false, 2, true>(map_w, map_a, p, grid, st, items, c);
+  switch (MT) {
+    case 16: return launch<16, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
+    case 32: return launch<32, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
+    default: return launch<64, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
+  }
+}
+
 }  // namespace
 
 int smallm_max_rows() { return 128; }
 
-// K-splits for a small-M problem.  Cost model in units of one k-block of one work item: a split count s gives
-// ceil(n_tiles * s / SMs) waves of work items, each ceil(k_tiles / s) k-blocks deep plus a fixed cost per item (pipeline
-// fill, store), plus the second kernel that adds the partial sums when s > 1.  The cheapest s wins; ties go to fewer splits.
-int smallm_splits(int64_t N, int64_t K, int sm_count) {
+// CTAs per cluster that share one tile's K (1, 2, 4 or 8) for a dense problem.  Cost model in nanoseconds, from runs with one
+// tile per CTA at 1.9 GHz: a k-block takes one CTA `step` (the MMA issuer at 16 columns, the promotion above), or longer once
+// the CTAs together ask for more than HBM delivers (16 KB of weights each at 6.5 TB/s); adding up over the cluster costs a
+// barrier and one pass over the sums.  Larger clusters leave SMs of a GPC unused.
+int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count) {
   const int64_t n_tiles = (N + BN - 1) / BN, k_tiles = (K + BK - 1) / BK;
-  constexpr int64_t kItemCost = 3, kReduceCost = 8;
+  const int64_t step = M <= 16 ? 195 : (M <= 32 ? 215 : (M <= 64 ? 240 : 360));
   int best = 1;
-  int64_t best_cost = ((n_tiles + sm_count - 1) / sm_count) * (k_tiles + kItemCost);
-  for (int64_t s = 2; s <= 32 && s * 2 <= k_tiles; ++s) {
-    const int64_t kb = (k_tiles + s - 1) / s;
-    const int64_t used = (k_tiles + kb - 1) / kb;  // splits that actually get k-blocks
-    if (used != s) continue;
-    const int64_t cost = ((n_tiles * s + sm_count - 1) / sm_count) * (kb + kItemCost) + kReduceCost;
+  int64_t best_cost = INT64_MAX;
+  for (int c = 1; c <= kMaxCluster; c *= 2) {
+    if (c > 1 && k_tiles < 2 * c) break;
+    const int64_t kb = (k_tiles + c - 1) / c;
+    if ((k_tiles + kb - 1) / kb != c) continue;  // every CTA of the cluster must get k-blocks
+    // CTAs resident at once, about; a cluster takes one tile, so more tiles than fit are left to CTAs that walk the list
+    const int64_t ctas = n_tiles * c, fit = c <= 2 ? sm_count : sm_count - 4 * c;
+    if (c > 1 && ctas > fit) break;
+    const int64_t waves = (ctas + fit - 1) / fit, hbm = (ctas < fit ? ctas : fit) * 16384 * 10 / 65000;
+    int64_t cost = waves * kb * (step > hbm ? step : hbm);
+    if (c > 1) cost += (M <= 16 ? 900 : 1500) + (int64_t)(c - 1) * (M <= 16 ? 60 : (M <= 64 ? 200 : 500));
     if (cost < best_cost) {
       best_cost = cost;
-      best = (int)s;
+      best = c;
     }
   }
   return best;
 }
 
-// Launches the small-M kernel (arguments already validated by the caller).  With `partial` != NULL and splits > 1 the
-// kernel leaves fp32 partial sums [splits][M][N] there and the caller adds them up; *splits_used reports which.  With
-// always_partial the fp32 sums go to `partial` even for a single split (the caller converts and moves them itself).
+// Launches the small-M kernel (arguments already validated by the caller).  `partial` != NULL: the fp32 sums [splits][M][N]
+// go there, *splits_used of them, and the caller converts and moves them itself.
 // With ue8m0 the scale pointers are packed exponent words (sa: word (m, kg) at m * sa_stride_m + kg * sa_stride_k; sb
 // likewise per 128 weight rows) and the scales are the exact powers of two they encode.
 int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K,
                 int64_t lda, int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n,
-                int64_t sb_stride_k, int out_dtype, float* partial, int64_t partial_floats, int sm_count, void* stream,
-                int* splits_used, bool always_partial, bool ue8m0) {
+                int64_t sb_stride_k, int out_dtype, const void* bias, float* partial, int64_t partial_floats, int sm_count,
+                void* stream, int* splits_used, bool ue8m0) {
   const int MT = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
   const bool two = M > 64;  // 128 activation rows per work item, two sets of promotion warps
   alignas(64) CUtensorMap map_w, map_a;
@@ -654,10 +764,11 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
     if (int rc = make_map_sw128(&map_a, a, 2, dims, str, (uint32_t)(M > 64 ? 128 : MT), CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
       return rc;
   }
-  SmallParams p;
+  SmallParams p = {};
   p.sa = sa;
   p.sb = sb;
   p.out = out;
+  p.bias = bias;
   p.M = (int32_t)M;
   p.N = (int32_t)N;
   p.K = (int32_t)K;
@@ -669,27 +780,24 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
   p.sb_stride_n = sb_stride_n;
   p.sb_stride_k = sb_stride_k;
   p.out_dtype = out_dtype;
-  p.partial = nullptr;
-  p.k_splits = 1;
-  p.kb_per_split = p.k_tiles;
-  p.expert_offsets = nullptr;
-  p.problem_sizes = nullptr;
   p.count_stride = 1;
-  p.rows_per_expert = 0;
   p.num_experts = 1;
-  p.sa_stride_e = 0;
-  p.sb_stride_e = 0;
-  const int splits = smallm_splits(N, K, sm_count);
-  if (partial != nullptr && splits > 1 && (int64_t)splits * M * N <= partial_floats) {
+  p.cluster = 1;
+  int splits = 1;
+  if (partial != nullptr) {
     p.partial = partial;
-    p.kb_per_split = (p.k_tiles + splits - 1) / splits;
-    p.k_splits = (p.k_tiles + p.kb_per_split - 1) / p.kb_per_split;
-  } else if (always_partial) {
-    p.partial = partial;  // one slice of fp32 sums instead of `out` (the caller checked its size)
+    splits = smallm_cluster(M, N, K, sm_count);  // the same ranges, added in the same order: the same bits as `out`
+    if ((int64_t)splits * M * N > partial_floats) splits = 1;
+  } else {
+    splits = p.cluster = smallm_cluster(M, N, K, sm_count);
   }
-  *splits_used = p.k_splits;
+  p.kb_per_split = (p.k_tiles + splits - 1) / splits;
+  p.k_splits = (p.k_tiles + p.kb_per_split - 1) / p.kb_per_split;
+  if (splits_used) *splits_used = p.k_splits;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t items = (int64_t)p.n_tiles * p.k_splits;
+  if (p.cluster > 1)
+    return ue8m0 ? launch_cluster<true>(MT, two, map_w, map_a, p, st, items) : launch_cluster<false>(MT, two, map_w, map_a, p, st, items);
   if (two) {
     return ue8m0 ? launch<64, true, false, 2>(map_w, map_a, p, sm_count, st, items)
                  : launch<64, false, false, 2>(map_w, map_a, p, sm_count, st, items);
@@ -750,11 +858,10 @@ int smallm_grouped_gemm(int chunk, const void* a, const void* b, const float* sa
     const uint64_t str[1] = {(uint64_t)lda};
     if (int rc = make_map_sw128(&map_a, a, 2, dims, str, (uint32_t)chunk, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)) return rc;
   }
-  SmallParams p;
+  SmallParams p = {};
   p.sa = sa;
   p.sb = sb;
   p.out = out;
-  p.partial = nullptr;
   p.M = (int32_t)total_rows;
   p.N = (int32_t)N;
   p.K = (int32_t)K;

@@ -72,6 +72,7 @@ struct Params {
   const int32_t* sfa;  // packed exponents of A: word (m, kg) at sfa[kg * sfa_ld + m * sfa_stride_m]
   const int32_t* sfb;  // of B: word (e, nb, kg) at sfb[e * sfb_stride_e + nb * sfb_stride_n + kg * sfb_stride_k]
   void* out;
+  const void* bias;  // dense, optional: [N] of the output type, added to the rounded result
   const int32_t* expert_offsets;  // grouped: rows of expert e are [expert_offsets[e], expert_offsets[e + 1])
   int32_t M, N, K, num_experts;   // M = total rows of a / out
   int32_t m_tiles, n_tiles, k_tiles, k_groups;
@@ -153,20 +154,17 @@ __device__ __forceinline__ uint32_t pack_pair<__half>(float a, float b) {
 }
 
 template <typename OutT>
-__device__ __forceinline__ void store32(const uint32_t (&a)[32], const uint32_t (&b)[32], bool use_b, OutT* dst,
-                                        int32_t n_first, int32_t N) {
+__device__ __forceinline__ void store32(const uint32_t (&a)[32], const OutT* bias, OutT* dst, int32_t n_first, int32_t N,
+                                        int out_dtype) {
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     if (n_first + c * 8 < N) {
-      float v[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        v[j] = __uint_as_float(a[c * 8 + j]) + (use_b ? __uint_as_float(b[c * 8 + j]) : 0.f);
       uint4 u;
-      u.x = pack_pair<OutT>(v[0], v[1]);
-      u.y = pack_pair<OutT>(v[2], v[3]);
-      u.z = pack_pair<OutT>(v[4], v[5]);
-      u.w = pack_pair<OutT>(v[6], v[7]);
+      u.x = pack_pair<OutT>(__uint_as_float(a[c * 8]), __uint_as_float(a[c * 8 + 1]));
+      u.y = pack_pair<OutT>(__uint_as_float(a[c * 8 + 2]), __uint_as_float(a[c * 8 + 3]));
+      u.z = pack_pair<OutT>(__uint_as_float(a[c * 8 + 4]), __uint_as_float(a[c * 8 + 5]));
+      u.w = pack_pair<OutT>(__uint_as_float(a[c * 8 + 6]), __uint_as_float(a[c * 8 + 7]));
+      if (bias != nullptr) u = ptx::add_bias8(u, __ldg(reinterpret_cast<const uint4*>(bias + n_first + c * 8)), out_dtype);
       *reinterpret_cast<uint4*>(dst + c * 8) = u;
     }
   }
@@ -409,11 +407,12 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           const int32_t n_first = n0 + col0 + c * 32;
           const int32_t n_limit = min(p.N, n0 + col0 + kEpiCols);  // do not store beyond this warp's 112 columns
           if (p.out_dtype == SGLB200_BF16) {
-            store32<__nv_bfloat16>(va, va, false, static_cast<__nv_bfloat16*>(p.out) + (int64_t)row * p.ldc + n_first,
-                                   n_first, n_limit);
+            store32<__nv_bfloat16>(va, static_cast<const __nv_bfloat16*>(p.bias),
+                                   static_cast<__nv_bfloat16*>(p.out) + (int64_t)row * p.ldc + n_first, n_first, n_limit,
+                                   SGLB200_BF16);
           } else {
-            store32<__half>(va, va, false, static_cast<__half*>(p.out) + (int64_t)row * p.ldc + n_first, n_first,
-                            n_limit);
+            store32<__half>(va, static_cast<const __half*>(p.bias), static_cast<__half*>(p.out) + (int64_t)row * p.ldc + n_first,
+                            n_first, n_limit, SGLB200_F16);
           }
         }
       }
@@ -444,8 +443,8 @@ namespace {
 int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, void* out,
                  const int32_t* expert_offsets, int64_t M, int64_t num_experts, int64_t N, int64_t K, int64_t lda,
                  int64_t ldb, int64_t ldb_e, int64_t ldc, int64_t sfa_ld, int64_t sfa_stride_m, int64_t sfb_stride_e,
-                 int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype, void* stream, float* workspace = nullptr,
-                 int64_t workspace_floats = 0) {
+                 int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype, void* stream,
+                 const void* bias = nullptr) {
   const bool grouped = expert_offsets != nullptr;
   SGLB_REQUIRE(M >= 0 && N >= 0 && K >= 0, SGLB200_ERR_SHAPE, "M=%lld N=%lld K=%lld: negative size", (long long)M,
                (long long)N, (long long)K);
@@ -479,14 +478,9 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
   if (!grouped && M <= 64) {
     // few rows: the weight-streaming kernel with swapped operands decodes the exponent bytes itself (gemm_smallm.cu);
     // from 65 rows up the block-scaled tile kernel below, which has no promotion, is the faster one
-    int splits = 1;
-    if (int rc = smallm_gemm(a, b, reinterpret_cast<const float*>(sfa), reinterpret_cast<const float*>(sfb), out, M, N, K,
-                             lda, ldb, ldc, sfa_stride_m, sfa_ld, sfb_stride_n, sfb_stride_k, out_dtype, workspace,
-                             workspace_floats, di.sm_count, stream, &splits, false, true))
-      return rc;
-    if (splits > 1) launch_splitk_reduce(workspace, out, M, N, ldc, splits, out_dtype, di.sm_count, stream);
-    SGLB_CHECK_LAUNCH("splitk_reduce_kernel");
-    return SGLB200_OK;
+    return smallm_gemm(a, b, reinterpret_cast<const float*>(sfa), reinterpret_cast<const float*>(sfb), out, M, N, K, lda, ldb, ldc,
+                       sfa_stride_m, sfa_ld, sfb_stride_n, sfb_stride_k, out_dtype, bias, nullptr, 0, di.sm_count, stream, nullptr,
+                       true);
   }
 
   if (grouped) {
@@ -515,6 +509,7 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
   p.sfa = sfa;
   p.sfb = sfb;
   p.out = out;
+  p.bias = bias;
   p.expert_offsets = expert_offsets;
   p.M = (int32_t)M;
   p.N = (int32_t)N;
@@ -558,6 +553,13 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
   return SGLB200_OK;
 }
 }  // namespace
+
+int ue8m0_linear_gemm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, const void* bias, void* out, int64_t M,
+                      int64_t N, int64_t K, int64_t sfa_ld, int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype,
+                      void* stream) {
+  return ue8m0_common(a, b, sfa, sfb, out, nullptr, M, 1, N, K, K, K, 0, N, sfa_ld, 1, 0, sfb_stride_n, sfb_stride_k, out_dtype,
+                      stream, bias);
+}
 }  // namespace sglb
 
 extern "C" int sglb200_fp8_ue8m0_scaled_mm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb,
@@ -579,8 +581,7 @@ extern "C" int sglb200_fp8_ue8m0_scaled_mm_ws(const void* a, const void* b, cons
   SGLB_REQUIRE(workspace_bytes >= 0 && (workspace == nullptr || sglb::aligned(workspace, 16)), SGLB200_ERR_ALIGN,
                "workspace must be 16-byte aligned");
   return sglb::ue8m0_common(a, b, sfa, sfb, out, nullptr, M, 1, N, K, lda, ldb, 0, ldc, sfa_ld, 1, 0, sfb_stride_n,
-                            sfb_stride_k, out_dtype, stream, static_cast<float*>(workspace),
-                            workspace ? workspace_bytes / (int64_t)sizeof(float) : 0);
+                            sfb_stride_k, out_dtype, stream);
 }
 
 extern "C" int sglb200_fp8_ue8m0_scaled_grouped_mm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb,

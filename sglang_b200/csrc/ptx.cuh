@@ -2,8 +2,12 @@
 // broadcast forms), tcgen05 (TMEM allocation, MMA, commit, load) and the matrix descriptors.
 #pragma once
 #include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "../../include/sglb200.h"
 
 namespace sglb {
 namespace ptx {
@@ -40,6 +44,22 @@ __device__ __forceinline__ bool elect_one() {
       "}\n"
       : "=r"(p));
   return p != 0;
+}
+
+// ---------------------------------------------------------------- 16-bit epilogue arithmetic
+// Two packed results plus two packed biases; every sum is rounded once, as an addition to the stored 16-bit result is.
+__device__ __forceinline__ uint32_t add16x2(uint32_t v, uint32_t b, int out_dtype) {
+  if (out_dtype == SGLB200_BF16) {
+    const __nv_bfloat162 r = __hadd2(*reinterpret_cast<__nv_bfloat162*>(&v), *reinterpret_cast<__nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&r);
+  }
+  const __half2 r = __hadd2(*reinterpret_cast<__half2*>(&v), *reinterpret_cast<__half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// Eight packed 16-bit results plus eight packed biases, each sum rounded once.
+__device__ __forceinline__ uint4 add_bias8(uint4 v, uint4 b, int out_dtype) {
+  return make_uint4(add16x2(v.x, b.x, out_dtype), add16x2(v.y, b.y, out_dtype), add16x2(v.z, b.z, out_dtype),
+                    add16x2(v.w, b.w, out_dtype));
 }
 
 // ---------------------------------------------------------------- mbarrier
@@ -292,6 +312,17 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the two halves for every thread of the cluster by itself (warps of one CTA may arrive from different program points)
+__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(cluster_addr)
+               : "memory");
+  return v;
 }
 // Arrival on an mbarrier of any CTA of the cluster (address from mapa_shared).  Default semantics (release at CTA
 // scope): a cluster-scope release makes the arriving warp wait for a cluster-wide fence, measured at more than a

@@ -351,6 +351,12 @@ int quant_entry(const void* input, int in_dtype, void* out_q, void* out_s, void*
 }
 
 }  // namespace
+
+int quant_rows(const void* input, int in_dtype, void* out_q, void* out_s, int64_t rows, int64_t hidden, float eps, bool ue8m0,
+               int64_t s_stride_row, int64_t s_stride_group, void* stream) {
+  return quant_entry<false>(input, in_dtype, out_q, out_s, nullptr, rows, hidden, 128, eps, -448.f, 448.f, ue8m0, s_stride_row,
+                            s_stride_group, stream);
+}
 }  // namespace sglb
 
 extern "C" int sglb200_per_token_group_quant_fp8(const void* input, int in_dtype, void* out_q, void* out_s,

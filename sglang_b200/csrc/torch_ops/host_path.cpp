@@ -155,7 +155,9 @@ PyObject* block_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (ws.scalar_type() != (ue ? at::kInt : at::kFloat) || ws.dim() != 2 || ws.size(0) != NB || ws.size(1) != (ue ? KG : KB) ||
       ws.device() != x.device())
     Py_RETURN_NONE;
-  if (bp && (bp->device() != x.device() || bp->scalar_type() != t || bp->requires_grad())) Py_RETURN_NONE;
+  if (bp && (bp->device() != x.device() || bp->scalar_type() != t || bp->requires_grad() ||
+             bp->dim() != 1 || bp->size(0) != N || bp->stride(0) != 1 || reinterpret_cast<uintptr_t>(bp->const_data_ptr()) % 16 != 0))
+    Py_RETURN_NONE;
   const int64_t M = x.numel() / K;
   return guarded([&]() -> PyObject* {
     const c10::Device dev = x.device();
@@ -165,33 +167,12 @@ PyObject* block_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     at::DimVector shape(x.sizes().begin(), x.sizes().end());
     shape[dim - 1] = N;
     at::Tensor out = empty(shape, t, dev);
-    // one block: split-K scratch | scales (M-major, rows padded to 4) | codes
-    const int64_t ld = up(M, 4), words = ue ? KG : KB;
-    int64_t ws_bytes = !ue || M <= 64 ? sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) : 0;
-    const int64_t scale_at = up(ws_bytes, 512), code_at = scale_at + up(words * ld * 4, 512);
-    c10::DataPtr block = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)(code_at + M * K));
-    char* base = static_cast<char*>(block.get());
-    void *scratch = ws_bytes > 0 ? base : nullptr, *scales = base + scale_at, *codes = base + code_at;
-    const int code = code16(t);
-    check_rc(sglb200_per_token_group_quant_fp8(x.const_data_ptr(), code, codes, scales, M, K, 128, eps_in_dtype(1e-10, t),
-                                               -448.f, 448.f, ue, 1, ld, stream),
-             "sgl_per_token_group_quant_8bit");
-    if (ue)
-      check_rc(sglb200_fp8_ue8m0_scaled_mm_ws(codes, w.const_data_ptr(), static_cast<const int32_t*>(scales),
-                                              ws.const_data_ptr<int32_t>(), out.mutable_data_ptr(), M, N, K, K, K, N, ld,
-                                              ws.stride(0), ws.stride(1), code, scratch, ws_bytes, stream),
-               "w8a8_block_fp8_matmul_ue8m0");
-    else if (ws_bytes > 0)
-      check_rc(sglb200_fp8_blockwise_scaled_mm_ws(codes, w.const_data_ptr(), static_cast<const float*>(scales),
-                                                  ws.const_data_ptr<float>(), out.mutable_data_ptr(), M, N, K, K, K, N, 1, ld,
-                                                  ws.stride(0), ws.stride(1), code, scratch, ws_bytes, stream),
-               "fp8_blockwise_scaled_mm (split-K)");
-    else
-      check_rc(sglb200_fp8_blockwise_scaled_mm(codes, w.const_data_ptr(), static_cast<const float*>(scales),
-                                               ws.const_data_ptr<float>(), out.mutable_data_ptr(), M, N, K, K, K, N, 1, ld,
-                                               ws.stride(0), ws.stride(1), code, stream),
-               "fp8_blockwise_scaled_mm");
-    if (bp) out.add_(*bp);
+    const int64_t bytes = sglb200_fp8_block_linear_scratch_bytes(M, N, K, ue);
+    c10::DataPtr scratch = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)bytes);
+    check_rc(sglb200_fp8_block_linear(x.const_data_ptr(), w.const_data_ptr(), ws.const_data_ptr(),
+                                      bp ? bp->const_data_ptr() : nullptr, out.mutable_data_ptr(), M, N, K, ws.stride(0),
+                                      ws.stride(1), ue, eps_in_dtype(1e-10, t), code16(t), scratch.get(), bytes, stream),
+             "fp8_block_linear");
     return THPVariable_Wrap(std::move(out));
   });
 }

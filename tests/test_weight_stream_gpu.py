@@ -41,3 +41,32 @@ def test_masked_layout_with_expected_rows(expected):
         if m:
             ref = oracle.w8a8_block_fp8_matmul(q.view(G, max_m, K)[g, :m], ws[g][0], s.view(G, max_m, -1)[g, :m], ws[g][1])
             assert_gemm_close(out[g, :m], ref, f"group {g}")
+
+
+@pytest.mark.parametrize("ue8m0", [False, True])
+@pytest.mark.parametrize("M,N,K", [(1, 576, 7168), (5, 8, 128), (16, 7168, 2048), (33, 1000, 1024), (64, 10240, 1536),
+                                   (113, 2112, 7168), (128, 136, 4096), (129, 576, 2048), (300, 392, 1024)])
+def test_linear_layer_with_bias(M, N, K, ue8m0):
+    """The one-call linear layer against its parts: quantiser, GEMM entry, then the bias in the output type.  The shapes
+    put K on one CTA, on a few and on all of them, and cross the row limits of the kernels."""
+    from sglang_b200._lib import lib
+    from sglang_b200.layers.quantization.fp8 import Fp8Config, Fp8LinearMethod
+    dtype = torch.float16 if N % 16 else torch.bfloat16
+    layer, method = torch.nn.Module(), Fp8LinearMethod(Fp8Config())
+    method.create_weights(layer, K, [N], K, N, dtype, device="cuda")
+    w, w_s = oracle.block_quant_weight(torch.randn(N, K, generator=torch.Generator().manual_seed(N)) * 0.02, scale_ue8m0=ue8m0)
+    layer.weight.data.copy_(w)
+    layer.weight_scale_inv.data.copy_(w_s)
+    method.process_weights_after_loading(layer)
+    assert (layer.weight_scale_ue8m0 is not None) == ue8m0
+    x = make_activations(M, K, seed=M).to(dtype)
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(3)).to(dtype)
+    q, s = oracle.per_token_group_quant_fp8(x, 128, scale_ue8m0=ue8m0)
+    ref = oracle.w8a8_block_fp8_matmul(q, w, s, w_s, output_dtype=dtype)
+    xd, bd = x.cuda(), bias.cuda()
+    plain, again, biased = method.apply(layer, xd), method.apply(layer, xd), method.apply(layer, xd, bd)
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    assert torch.equal(plain, again), "the sum over the SMs depends on their order"
+    assert torch.equal(biased, plain + bd)
+    assert_gemm_close(plain, ref, f"{M}x{N}x{K}", allow_one_ulp=True)
