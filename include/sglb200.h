@@ -331,6 +331,26 @@ int sglb200_apply_shuffle_mul_sum(const void* input, void* output, const int32_t
                                   void* stream);
 
 /*
+ * ME  The block-FP8 expert layer in one call: out[t] = sum_j w[t, j] * expert_{ids[t, j]}(x[t]), each expert a SiLU-gated MLP.
+ *   x [M, H] and out [M, H] of dtype (SGLB200_BF16 | SGLB200_F16), contiguous; out may be x
+ *   w1 [E, 2I, H] (gate rows first), w2 [E, H, I] e4m3, contiguous;  H, I multiples of 128
+ *   w1_scale / w2_scale: fp32 per 128x128 block, or with scale_ue8m0 int32 words of four exponent bytes along K; the strides
+ *   (expert, row block, k-block or word) are host arrays of three
+ *   topk_weights [M, topk] fp32, topk_ids [M, topk] int32, contiguous; ids outside [0, E) contribute nothing.  A slot's factor is
+ *   topk_weights * weight_factor rounded to dtype, its product is rounded to dtype, the sum is fp32.  topk <= 32.
+ *   scratch: sglb200_fused_experts_scratch_bytes() bytes, 256-byte aligned, contents arbitrary.
+ * Same arithmetic as the single steps (sglb200_prepare_moe_input, quantiser, grouped GEMMs, fused SiLU quantiser,
+ * sglb200_apply_shuffle_mul_sum with round_products).
+ * Replaces: cutlass_fused_experts_fp8  python/sglang/srt/layers/moe/cutlass_moe.py:21-205.
+ */
+int sglb200_fused_experts(const void* x, int dtype, const void* w1, const void* w2, const void* w1_scale,
+                          const void* w2_scale, const int64_t* w1_scale_strides, const int64_t* w2_scale_strides,
+                          const float* topk_weights, const int32_t* topk_ids, float weight_factor, void* out, int64_t M,
+                          int64_t H, int64_t I, int64_t E, int64_t topk, int scale_ue8m0, float eps, void* scratch,
+                          int64_t scratch_bytes, void* stream);
+int64_t sglb200_fused_experts_scratch_bytes(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int scale_ue8m0);
+
+/*
  * SA — out[t, :] = round(silu(in[t, :d])) * in[t, d:], d = hidden; in [num_rows, 2*hidden].
  * Replaces: silu_and_mul  sgl-kernel/csrc/elementwise/activation.cu:82-101 (schema common_extension.cc:82-83).
  */

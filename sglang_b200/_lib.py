@@ -41,6 +41,8 @@ SIGNATURES = {
                                                        _L, _L, _L, _L, _I, _P],
     "sglb200_fp8_blockwise_scaled_masked_grouped_mm_expected": [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L,
                                                                 _L, _L, _L, _L, _L, _L, _I, _P],
+    "sglb200_fused_experts": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _F, _P, _L, _L, _L, _L, _L, _I, _F, _P, _L, _P],
+    "sglb200_fused_experts_scratch_bytes": [_L, _L, _L, _L, _L, _I],
     "sglb200_prepare_moe_input": [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _P],
     "sglb200_shuffle_rows": [_P, _P, _P, _L, _L, _P],
     "sglb200_apply_shuffle_mul_sum": [_P, _P, _P, _P, _L, _L, _L, _I, _I, _P],
@@ -88,7 +90,7 @@ SIGNATURES = {
 _RESTYPES = {"sglb200_fp8_blockwise_scaled_mm_workspace_bytes": c_int64,
              "sglb200_fp8_blockwise_scaled_mm_noalloc_max_bytes": c_int64,
              "sglb200_fp8_block_linear_scratch_bytes": c_int64,
-             "sglb200_ep_buffer_bytes": c_int64, "sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes": c_int64, "sglb200_peer_flag_bytes": c_int64, "sglb200_nvls_flag_bytes": c_int64, "sglb200_peer_recv_bytes": c_int64, "sglb200_status_string": c_char_p, "sglb200_last_error_detail": c_char_p, "sglb200_version": c_char_p}
+             "sglb200_fused_experts_scratch_bytes": c_int64, "sglb200_ep_buffer_bytes": c_int64, "sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes": c_int64, "sglb200_peer_flag_bytes": c_int64, "sglb200_nvls_flag_bytes": c_int64, "sglb200_peer_recv_bytes": c_int64, "sglb200_status_string": c_char_p, "sglb200_last_error_detail": c_char_p, "sglb200_version": c_char_p}
 
 _lib = None
 

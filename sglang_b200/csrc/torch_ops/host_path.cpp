@@ -177,9 +177,125 @@ PyObject* block_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   });
 }
 
+// ---------------------------------------------------------------------------------------------- router
+// topk_softmax(logits, topk, renormalize) -> (weights, ids)
+PyObject* topk_softmax(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 3) Py_RETURN_NONE;
+  const at::Tensor* lp = tensor_or_null(args[0]);
+  if (!lp || !PyLong_Check(args[1])) Py_RETURN_NONE;
+  const at::Tensor& x = *lp;
+  const int64_t topk = PyLong_AsLong(args[1]);
+  const at::ScalarType t = x.scalar_type();
+  if (!x.is_cuda() || x.dim() != 2 || !x.is_contiguous() || !(is16(t) || t == at::kFloat) || x.numel() == 0) Py_RETURN_NONE;
+  if (topk < 1 || topk > x.size(1)) Py_RETURN_NONE;
+  const bool renorm = PyObject_IsTrue(args[2]) == 1;
+  return guarded([&]() -> PyObject* {
+    const c10::Device dev = x.device();
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    const int64_t M = x.size(0);
+    at::Tensor w = empty({M, topk}, at::kFloat, dev), ids = empty({M, topk}, at::kInt, dev);
+    check_rc(sglb200_topk_softmax(x.const_data_ptr(), t == at::kFloat ? SGLB200_F32 : code16(t), w.mutable_data_ptr<float>(),
+                                  ids.mutable_data_ptr<int32_t>(), M, x.size(1), topk, renorm, stream),
+             "topk_softmax");
+    PyObject* out = PyTuple_New(2);
+    if (!out) return nullptr;
+    PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(w)));
+    PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(std::move(ids)));
+    return out;
+  });
+}
+
+// ---------------------------------------------------------------------------------------------- expert layer
+// fused_experts(x, w1, w2, s1, s2, topk_weights, topk_ids, weight_factor, out or None, ue8m0) -> out
+PyObject* fused_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 10) Py_RETURN_NONE;
+  const at::Tensor* t[7];
+  for (int i = 0; i < 7; ++i)
+    if (!(t[i] = tensor_or_null(args[i]))) Py_RETURN_NONE;
+  const at::Tensor &x = *t[0], &w1 = *t[1], &w2 = *t[2], &s1 = *t[3], &s2 = *t[4], &tw = *t[5], &ids = *t[6];
+  const double factor = PyFloat_AsDouble(args[7]);
+  if (PyErr_Occurred()) return nullptr;
+  const at::Tensor* op = args[8] == Py_None ? nullptr : tensor_or_null(args[8]);
+  if (args[8] != Py_None && !op) Py_RETURN_NONE;
+  const bool ue = args[9] == Py_True;
+  const at::ScalarType dt = x.scalar_type();
+  if (!x.is_cuda() || !is16(dt) || x.dim() != 2 || !x.is_contiguous() || x.numel() == 0) Py_RETURN_NONE;
+  for (int i = 1; i < 7; ++i)
+    if (t[i]->device() != x.device()) Py_RETURN_NONE;
+  if (w1.dim() != 3 || w2.dim() != 3 || !w1.is_contiguous() || !w2.is_contiguous() || w1.scalar_type() != at::kFloat8_e4m3fn ||
+      w2.scalar_type() != at::kFloat8_e4m3fn)
+    Py_RETURN_NONE;
+  const int64_t M = x.size(0), H = x.size(1), E = w1.size(0), I = w1.size(1) / 2, topk = ids.dim() == 2 ? ids.size(1) : 0;
+  if (E < 1 || E > 1024 || w1.size(1) != 2 * I || w1.size(2) != H || w2.size(0) != E || w2.size(1) != H || w2.size(2) != I)
+    Py_RETURN_NONE;
+  if (H % 128 != 0 || I == 0 || I % 128 != 0) Py_RETURN_NONE;
+  const at::ScalarType st = ue ? at::kInt : at::kFloat;
+  const int64_t k1 = ue ? (H / 128 + 3) / 4 : H / 128, k2 = ue ? (I / 128 + 3) / 4 : I / 128;
+  if (s1.scalar_type() != st || s2.scalar_type() != st || s1.dim() != 3 || s2.dim() != 3 || s1.size(0) != E || s2.size(0) != E ||
+      s1.size(1) != 2 * I / 128 || s1.size(2) != k1 || s2.size(1) != H / 128 || s2.size(2) != k2)
+    Py_RETURN_NONE;
+  if (topk < 1 || topk > 32 || M * topk > (1 << 24) || tw.dim() != 2 || tw.size(0) != M || tw.size(1) != topk || ids.size(0) != M ||
+      tw.scalar_type() != at::kFloat || ids.scalar_type() != at::kInt || !tw.is_contiguous() || !ids.is_contiguous())
+    Py_RETURN_NONE;
+  if (op && (op->device() != x.device() || op->scalar_type() != dt || op->dim() != 2 || op->size(0) != M || op->size(1) != H ||
+             !op->is_contiguous()))
+    Py_RETURN_NONE;
+  return guarded([&]() -> PyObject* {
+    const c10::Device dev = x.device();
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    at::Tensor out = op ? *op : empty({M, H}, dt, dev);
+    const int64_t bytes = sglb200_fused_experts_scratch_bytes(M, H, I, E, topk, ue);
+    c10::DataPtr scratch = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)bytes);
+    check_rc(sglb200_fused_experts(x.const_data_ptr(), code16(dt), w1.const_data_ptr(), w2.const_data_ptr(), s1.const_data_ptr(),
+                                   s2.const_data_ptr(), s1.strides().data(), s2.strides().data(), tw.const_data_ptr<float>(),
+                                   ids.const_data_ptr<int32_t>(), (float)factor, out.mutable_data_ptr(), M, H, I, E, topk, ue,
+                                   eps_in_dtype(1e-10, dt), scratch.get(), bytes, stream),
+             "fused_experts");
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
+// grouped_masked(a, a_s, w, w_s, out, masked_m, expected_m) -> True
+PyObject* grouped_masked(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 7) Py_RETURN_NONE;
+  const at::Tensor* t[6];
+  for (int i = 0; i < 6; ++i)
+    if (!(t[i] = tensor_or_null(args[i]))) Py_RETURN_NONE;
+  const at::Tensor &a = *t[0], &as = *t[1], &w = *t[2], &ws = *t[3], &out = *t[4], &mm = *t[5];
+  if (!PyLong_Check(args[6])) Py_RETURN_NONE;
+  const int64_t expected = PyLong_AsLong(args[6]);
+  if (!a.is_cuda() || a.dim() != 3 || w.dim() != 3 || a.scalar_type() != at::kFloat8_e4m3fn || w.scalar_type() != at::kFloat8_e4m3fn ||
+      !a.is_contiguous() || w.stride(2) != 1)
+    Py_RETURN_NONE;
+  for (int i = 1; i < 6; ++i)
+    if (t[i]->device() != a.device()) Py_RETURN_NONE;
+  const int64_t G = a.size(0), max_m = a.size(1), K = a.size(2), N = w.size(1), kt = (K + 127) / 128, nt = (N + 127) / 128;
+  if (G == 0 || max_m == 0 || N == 0 || w.size(0) != G || w.size(2) != K) Py_RETURN_NONE;
+  if (out.dim() != 3 || out.size(0) != G || out.size(1) != max_m || out.size(2) != N || !out.is_contiguous() || !is16(out.scalar_type()))
+    Py_RETURN_NONE;
+  if (as.scalar_type() != at::kFloat || as.dim() != 3 || as.size(0) != G || as.size(1) != max_m || as.size(2) != kt ||
+      ws.scalar_type() != at::kFloat || ws.dim() != 3 || ws.size(0) != G || ws.size(1) != nt || ws.size(2) != kt)
+    Py_RETURN_NONE;
+  if (mm.scalar_type() != at::kInt || !mm.is_contiguous() || mm.numel() != G) Py_RETURN_NONE;
+  return guarded([&]() -> PyObject* {
+    const c10::Device dev = a.device();
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    check_rc(sglb200_fp8_blockwise_scaled_masked_grouped_mm_expected(
+                 a.const_data_ptr(), w.const_data_ptr(), as.const_data_ptr<float>(), ws.const_data_ptr<float>(), out.mutable_data_ptr(),
+                 mm.const_data_ptr<int32_t>(), G, max_m, expected, N, K, a.stride(1), w.stride(1), w.stride(0), out.stride(1),
+                 as.stride(0), as.stride(1), as.stride(2), ws.stride(0), ws.stride(1), ws.stride(2), code16(out.scalar_type()),
+                 c10::cuda::getCurrentCUDAStream(dev.index()).stream()),
+             "grouped_gemm_nt_f8f8bf16_masked");
+    Py_RETURN_TRUE;
+  });
+}
+
+#define SGLB_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
-    {"quant", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(quant)), METH_FASTCALL, nullptr},
-    {"block_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(block_linear)), METH_FASTCALL, nullptr},
+    SGLB_METHOD(quant),         SGLB_METHOD(block_linear),   SGLB_METHOD(topk_softmax),
+    SGLB_METHOD(fused_experts), SGLB_METHOD(grouped_masked),
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_sglb200_host", nullptr, -1, kMethods};

@@ -10,7 +10,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from ..._lib import check, dtype_code, lib
+from ..._lib import check, dtype_code, host, lib
 
 FP8 = torch.float8_e4m3fn
 
@@ -28,6 +28,8 @@ def grouped_gemm_nt_f8f8bf16_masked(lhs: Tuple[torch.Tensor, torch.Tensor], rhs:
     int32.  Rows at and past ``masked_m[g]`` are left untouched."""
     a, a_s = lhs
     w, w_s = rhs
+    if host().grouped_masked(a, a_s, w, w_s, out, masked_m, expected_m):
+        return
     _req(a.is_cuda and a.dtype == FP8 and a.dim() == 3 and a.is_contiguous(), "lhs must be a contiguous [G, max_m, K] e4m3 tensor")
     _req(w.dtype == FP8 and w.dim() == 3 and w.stride(2) == 1, "rhs must be [G, N, K] e4m3 with K contiguous")
     G, max_m, K = a.shape

@@ -15,7 +15,7 @@ from typing import List, NamedTuple, Optional
 
 import torch
 
-from ..._lib import check, dtype_code, lib
+from ..._lib import check, dtype_code, host, lib
 from ...sgl_kernel import apply_shuffle_mul_sum, prepare_moe_input, shuffle_rows
 from ..quantization.fp8_kernel import sglang_per_token_group_quant_fp8
 
@@ -78,6 +78,11 @@ def fused_experts_block_fp8(hidden_states: torch.Tensor, w1: torch.Tensor, w2: t
     output (``fused_moe_triton_kernels.py``, ``MUL_ROUTED_WEIGHT`` on the first kernel); top-1 routing only, as the
     reference's callers require.
     """
+    if not no_combine and not apply_router_weight_on_input:
+        done = host().fused_experts(hidden_states, w1, w2, w1_scale, w2_scale, topk_weights, topk_ids,
+                                    1.0 if routed_scaling_factor is None else routed_scaling_factor, out, False)
+        if done is not None:
+            return done
     assert hidden_states.dim() == 2 and hidden_states.is_contiguous()
     if hidden_states.size(0) == 0:
         if no_combine:
@@ -244,6 +249,10 @@ def fused_experts_block_fp8_ue8m0(hidden_states: torch.Tensor, w1: torch.Tensor,
     group scales: the reference's Blackwell route through DeepGEMM
     (``python/sglang/srt/layers/moe/moe_runner/deep_gemm.py:131-207``, ``DEEPGEMM_SCALE_UE8M0``).  Same pipeline as
     :func:`fused_experts_block_fp8`; both grouped GEMMs run on the tensor core's block-scaling path."""
+    done = host().fused_experts(hidden_states, w1, w2, w1_sf, w2_sf, topk_weights, topk_ids,
+                                1.0 if routed_scaling_factor is None else routed_scaling_factor, None, True)
+    if done is not None:
+        return done
     from ...sgl_kernel import sgl_per_token_group_quant_8bit
     assert hidden_states.dim() == 2 and hidden_states.is_contiguous()
     M, H = hidden_states.shape

@@ -8,6 +8,7 @@ from typing import Optional, Tuple
 
 import torch
 
+from ..._lib import host
 from ...sgl_kernel import moe_align_block_size as _sgl_moe_align_block_size
 from ...sgl_kernel import topk_softmax
 
@@ -20,6 +21,10 @@ def fused_topk(hidden_states: torch.Tensor, gating_output: torch.Tensor, topk: i
     assert hidden_states.shape[0] == gating_output.shape[0], "Number of tokens mismatch"
     if num_token_non_padded is not None or expert_location_dispatch_info is not None:
         raise RuntimeError("num_token_non_padded / expert_location_dispatch_info are not implemented")
+    if gating_output.device == hidden_states.device:
+        done = host().topk_softmax(gating_output, topk, renormalize)
+        if done is not None:
+            return done
     M = hidden_states.shape[0]
     topk_weights = torch.empty(M, topk, dtype=torch.float32, device=hidden_states.device)
     topk_ids = torch.empty(M, topk, dtype=torch.int32, device=hidden_states.device)
