@@ -9,8 +9,8 @@
 //     (quant_math.cuh), evaluated two lanes at a time with the packed fp32x2 FMA of sm_100;
 //   * codes are converted two at a time (cvt.rn.satfinite.e4m3x2.f32) and the sign bit is taken
 //     from the input so that -0 stays -0.
-// Every thread has UNROLL groups (4 x 16 B) in flight.  Algorithmic bytes per group of 128 bf16:
-// 256 read + 128 written + 4 (float scale) or 1 (UE8M0 byte).
+// A thread has all its loads (four of 16 bytes: two groups, or gate and up of one) in flight before the first use.
+// Algorithmic bytes per group of 128 bf16: 256 read (fused: 512) + 128 written + 4 (float scale) or 1 (UE8M0 byte).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -23,8 +23,15 @@
 namespace sglb {
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kUnroll = 2;
+// Block and groups per thread of the 16-bit kernels.  The fused form holds gate and up (64 bytes a lane and group) and spends
+// about three times the instructions of the plain one, so it wants small blocks that drain and refill independently: 32768 x
+// 2048 takes 68 us with 128 threads and one group, 76 with 256 and one, 72 with 128 and two, 78 with 256 and two; for the plain
+// form 256 and two is the best or level at every size.
+template <bool FUSE>
+constexpr int kThreads16 = FUSE ? 128 : 256;
+template <bool FUSE>
+constexpr int kUnroll16 = FUSE ? 1 : 2;
+constexpr int kThreads = 256;  // fp32 input
 
 struct QuantParams {
   const void* in;
@@ -47,9 +54,10 @@ struct QuantParams {
 // 16-bit input types.  LPG = lanes per group = group_size / 16; each lane owns vectors `lane` and
 // `lane + LPG` of its group (group_size 16: one lane, both vectors).
 template <typename T, int LPG, bool UE8M0, bool FUSE_SILU, bool CLAMP>
-__global__ void __launch_bounds__(kThreads) group_quant16_kernel(const QuantParams p) {
+__global__ void __launch_bounds__(kThreads16<FUSE_SILU>) group_quant16_kernel(const QuantParams p) {
   static_assert(sizeof(T) == 2, "16-bit element types only");
-  constexpr int kGroupsPerIter = kThreads / LPG;
+  constexpr int kUnroll = kUnroll16<FUSE_SILU>;
+  constexpr int kGroupsPerIter = kThreads16<FUSE_SILU> / LPG;
   constexpr int kGroupSize = LPG * 16;
   constexpr int kSecond = (LPG == 1 && kGroupSize == 16) ? 1 : LPG;  // vector index of the second load
   const uint32_t tg = threadIdx.x / LPG;
@@ -62,7 +70,7 @@ __global__ void __launch_bounds__(kThreads) group_quant16_kernel(const QuantPara
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();
 
-  uint4 raw[kUnroll][2];
+  uint4 raw[kUnroll][2], up[FUSE_SILU ? kUnroll : 1][2];
   uint32_t row[kUnroll], grp[kUnroll];
   int64_t s_off[kUnroll];  // offset of the row's scales
   bool live[kUnroll];
@@ -82,22 +90,14 @@ __global__ void __launch_bounds__(kThreads) group_quant16_kernel(const QuantPara
       if (p.masked_m != nullptr && (int32_t)local >= __ldg(p.masked_m + b)) live[i] = false;
     }
     raw[i][0] = raw[i][1] = make_uint4(0, 0, 0, 0);
+    if constexpr (FUSE_SILU) up[i][0] = up[i][1] = make_uint4(0, 0, 0, 0);
     if (live[i]) {
       if constexpr (FUSE_SILU) {
         const T* g = static_cast<const T*>(p.in) + (size_t)row[i] * p.hidden * 2 + (size_t)grp[i] * kGroupSize;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const uint32_t vec = lane + h * kSecond;
-          const uint4 gv = __ldcs(reinterpret_cast<const uint4*>(g) + vec);
-          const uint4 uv = __ldcs(reinterpret_cast<const uint4*>(g + p.hidden) + vec);
-          const uint32_t* gw = reinterpret_cast<const uint32_t*>(&gv);
-          const uint32_t* uw = reinterpret_cast<const uint32_t*>(&uv);
-          uint32_t* ow = reinterpret_cast<uint32_t*>(&raw[i][h]);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 gf = Elem<T>::pair(gw[j]), uf = Elem<T>::pair(uw[j]);
-            ow[j] = Elem<T>::pack(Elem<T>::round(silu_f32(gf.x)) * uf.x, Elem<T>::round(silu_f32(gf.y)) * uf.y);
-          }
+          raw[i][h] = __ldcs(reinterpret_cast<const uint4*>(g) + lane + h * kSecond);
+          up[i][h] = __ldcs(reinterpret_cast<const uint4*>(g + p.hidden) + lane + h * kSecond);
         }
       } else {
         const uint4* g = reinterpret_cast<const uint4*>(static_cast<const T*>(p.in) + (size_t)tt * kGroupSize);
@@ -105,6 +105,12 @@ __global__ void __launch_bounds__(kThreads) group_quant16_kernel(const QuantPara
         raw[i][1] = __ldcs(g + lane + kSecond);
       }
     }
+  }
+  if constexpr (FUSE_SILU) {
+#pragma unroll
+    for (int i = 0; i < kUnroll; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) raw[i][h] = silu_mul8<T>(raw[i][h], up[i][h]);
   }
 
 #pragma unroll
@@ -235,14 +241,14 @@ __global__ void __launch_bounds__(kThreads) group_quant32_kernel(const QuantPara
 
 template <typename T, int LPG, bool FUSE>
 int launch16(const QuantParams& p, bool ue8m0, bool clamp, cudaStream_t stream) {
-  constexpr int kGroupsPerBlock = (kThreads / LPG) * kUnroll;
+  constexpr int kGroupsPerBlock = (kThreads16<FUSE> / LPG) * kUnroll16<FUSE>;
   const uint32_t blocks = (p.num_groups + kGroupsPerBlock - 1) / kGroupsPerBlock;
   if (ue8m0) {
-    if (clamp) launch_pdl(group_quant16_kernel<T, LPG, true, FUSE, true>, dim3(blocks), dim3(kThreads), 0, stream, p);
-    else launch_pdl(group_quant16_kernel<T, LPG, true, FUSE, false>, dim3(blocks), dim3(kThreads), 0, stream, p);
+    if (clamp) launch_pdl(group_quant16_kernel<T, LPG, true, FUSE, true>, dim3(blocks), dim3(kThreads16<FUSE>), 0, stream, p);
+    else launch_pdl(group_quant16_kernel<T, LPG, true, FUSE, false>, dim3(blocks), dim3(kThreads16<FUSE>), 0, stream, p);
   } else {
-    if (clamp) launch_pdl(group_quant16_kernel<T, LPG, false, FUSE, true>, dim3(blocks), dim3(kThreads), 0, stream, p);
-    else launch_pdl(group_quant16_kernel<T, LPG, false, FUSE, false>, dim3(blocks), dim3(kThreads), 0, stream, p);
+    if (clamp) launch_pdl(group_quant16_kernel<T, LPG, false, FUSE, true>, dim3(blocks), dim3(kThreads16<FUSE>), 0, stream, p);
+    else launch_pdl(group_quant16_kernel<T, LPG, false, FUSE, false>, dim3(blocks), dim3(kThreads16<FUSE>), 0, stream, p);
   }
   SGLB_CHECK_LAUNCH("group_quant16_kernel");
   return SGLB200_OK;

@@ -36,6 +36,10 @@ struct Elem<__nv_bfloat16> {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
   }
+  static __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {  // products of the pairs, rounded to T
+    const __nv_bfloat162 h = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
 };
 
 template <>
@@ -59,6 +63,10 @@ struct Elem<__half> {
     __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
   }
+  static __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {  // products of the pairs, rounded to T
+    const __half2 h = __hmul2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
 };
 
 template <>
@@ -78,6 +86,47 @@ __device__ __forceinline__ float2 quotient2(float2 x, float2 rr, float2 neg_ss) 
   const float2 q0 = __fmul2_rn(x, rr);
   const float2 rem = __ffma2_rn(q0, neg_ss, x);
   return __ffma2_rn(rem, rr, q0);
+}
+
+// x / (1 + exp(-x)) rounded to T, times u, rounded to T, on eight packed pairs.  The quotient is the approximate reciprocal
+// (one ulp) and one Markstein correction q0 + (x - q0 t) r, whose error is 2^-46 before its single rounding; for |x| <= 80
+// nothing in it under- or overflows and it agrees with the IEEE division for every bf16 and every fp16 x (all of them are
+// tested).  The division routine is a call with special cases per element: the fused quantiser spent 104 us on 32768 x 2048
+// with it (issue-bound, half the copy rate of HBM), 68 without.
+template <typename T>
+__device__ __forceinline__ uint4 silu_mul8(const uint4& g, const uint4& u) {
+  const uint32_t* gw = reinterpret_cast<const uint32_t*>(&g);
+  const uint32_t* uw = reinterpret_cast<const uint32_t*>(&u);
+  uint4 out;
+  uint32_t* ow = reinterpret_cast<uint32_t*>(&out);
+  const bool fast = Elem<T>::vec_absmax(g) <= 80.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 x = Elem<T>::pair(gw[j]);
+    const float2 t = make_float2(1.0f + expf(-x.x), 1.0f + expf(-x.y));
+    float2 r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(t.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(t.y));
+    const float2 q0 = __fmul2_rn(x, r);
+    const float2 rem = __ffma2_rn(q0, make_float2(-t.x, -t.y), x);
+    const float2 q = __ffma2_rn(rem, r, q0);
+    // the sign comes from x: the FMA chain gives +0 for x = -0
+    ow[j] = Elem<T>::mul2((Elem<T>::pack(q.x, q.y) & 0x7fff7fffu) | (gw[j] & 0x80008000u), uw[j]);
+  }
+  if (!fast) {
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t a = j == 0 ? g.x : j == 1 ? g.y : j == 2 ? g.z : g.w;
+      const uint32_t b = j == 0 ? u.x : j == 1 ? u.y : j == 2 ? u.z : u.w;
+      const float2 x = Elem<T>::pair(a);
+      const uint32_t o = Elem<T>::mul2(Elem<T>::pack(silu_f32(x.x), silu_f32(x.y)), b);
+      if (j == 0) out.x = o;
+      else if (j == 1) out.y = o;
+      else if (j == 2) out.z = o;
+      else out.w = o;
+    }
+  }
+  return out;
 }
 
 __device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
