@@ -206,9 +206,9 @@ combine_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __r
   const bool small = vecs * 8 != hidden;  // rows of fewer than eight elements
   for (int32_t c0 = 0; c0 < (small ? 1 : vecs); c0 += blockDim.x) {
     const int32_t c = c0 + threadIdx.x;
-    float acc[8];
+    float2 acc[4];
 #pragma unroll
-    for (int x = 0; x < 8; ++x) acc[x] = 0.f;
+    for (int x = 0; x < 4; ++x) acc[x] = make_float2(0.f, 0.f);
     for (int32_t j0 = 0; j0 < topk; j0 += kCombineSlots) {
       if (c0 == 0 || topk > kCombineSlots) {  // otherwise the slots of the first pass are still there
         __syncthreads();
@@ -227,8 +227,8 @@ combine_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __r
           for (int j = 0; j < kCombineSlots; ++j)
             if (s_src[j] >= 0) {
               const float v = Cvt<T>::f(in[(int64_t)s_src[j] * hidden + threadIdx.x]);
-              if constexpr (ROUND) acc[0] += Cvt<T>::f(Cvt<T>::t(s_w[j] * v));
-              else acc[0] = fmaf(s_w[j], v, acc[0]);
+              if constexpr (ROUND) acc[0].x += Cvt<T>::f(Cvt<T>::t(s_w[j] * v));
+              else acc[0].x = fmaf(s_w[j], v, acc[0].x);
             }
         continue;
       }
@@ -241,25 +241,22 @@ combine_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __r
       for (int j = 0; j < kCombineSlots; ++j) {
         if (s_src[j] < 0) continue;
         const float w = s_w[j];
-        const T* h = reinterpret_cast<const T*>(&u[j]);
+        const uint32_t* h = reinterpret_cast<const uint32_t*>(&u[j]);
+        // the factor is a T, so with ROUND the packed product has the bits of the rounded fp32 one; the sums stay fp32
+        const uint32_t ww = Elem<T>::pack(w, w);
 #pragma unroll
-        for (int x = 0; x < 8; ++x) {
-          if constexpr (ROUND) {
-            acc[x] += Cvt<T>::f(Cvt<T>::t(w * Cvt<T>::f(h[x])));
-          } else {
-            acc[x] = fmaf(w, Cvt<T>::f(h[x]), acc[x]);
-          }
+        for (int x = 0; x < 4; ++x) {
+          if constexpr (ROUND) acc[x] = __fadd2_rn(acc[x], Elem<T>::pair(Elem<T>::mul2(ww, h[x])));
+          else acc[x] = __ffma2_rn(make_float2(w, w), Elem<T>::pair(h[x]), acc[x]);
         }
       }
     }
     if (small) {
-      if ((int)threadIdx.x < hidden) out[i * hidden + threadIdx.x] = Cvt<T>::t(acc[0]);
+      if ((int)threadIdx.x < hidden) out[i * hidden + threadIdx.x] = Cvt<T>::t(acc[0].x);
     } else if (c < vecs) {
-      uint4 o;
-      T* oh = reinterpret_cast<T*>(&o);
-#pragma unroll
-      for (int x = 0; x < 8; ++x) oh[x] = Cvt<T>::t(acc[x]);
-      reinterpret_cast<uint4*>(out + i * hidden)[c] = o;
+      reinterpret_cast<uint4*>(out + i * hidden)[c] =
+          make_uint4(Elem<T>::pack(acc[0].x, acc[0].y), Elem<T>::pack(acc[1].x, acc[1].y), Elem<T>::pack(acc[2].x, acc[2].y),
+                     Elem<T>::pack(acc[3].x, acc[3].y));
     }
   }
 }
