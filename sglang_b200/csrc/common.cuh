@@ -32,10 +32,16 @@ int make_map_sw128(CUtensorMap* map, const void* base, int rank, const uint64_t*
 int smallm_max_rows();
 constexpr int kMaxCluster = 8;
 int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count);  // CTAs that share a tile's K, 1..kMaxCluster
+// Rows that are not quantised yet: `a` of smallm_gemm is [M, K] of the output type, contiguous, K in whole groups of 128, and the
+// kernel quantises them itself with this floor; M <= smallm_quant_rows(), `sa` and `partial` unused
+struct RawRows {
+  float eps;
+};
+int smallm_quant_rows();
 int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K,
                 int64_t lda, int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n,
                 int64_t sb_stride_k, int out_dtype, const void* bias, float* partial, int64_t partial_floats, int sm_count,
-                void* stream, int* splits_used, bool ue8m0);
+                void* stream, int* splits_used, bool ue8m0, const RawRows* raw = nullptr);
 void launch_splitk_reduce(const float* partial, void* out, const void* bias, int64_t M, int64_t N, int64_t ldc, int splits,
                           int out_dtype, int sm_count, void* stream);  // gemm.cu
 // Per-token-group quantisation (groups of 128) of whole rows, quant.cu

@@ -1318,7 +1318,7 @@ LinearScratch linear_scratch(int64_t M, int64_t N, int64_t K, bool ue8m0, int sm
 }  // namespace sglb
 
 extern "C" int64_t sglb200_fp8_block_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int scale_ue8m0) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (M <= sglb::smallm_quant_rows() || N <= 0 || K <= 0) return 0;
   sglb::DeviceInfo di;
   int sms = 148;
   if (sglb::device_info(&di) == SGLB200_OK) sms = di.sm_count;
@@ -1334,11 +1334,24 @@ extern "C" int sglb200_fp8_block_linear(const void* x, const void* w, const void
                (long long)M, (long long)N, (long long)K);
   if (M == 0 || N == 0) return SGLB200_OK;
   SGLB_REQUIRE(K > 0, SGLB200_ERR_SHAPE, "K must be positive");
-  SGLB_REQUIRE(scratch != nullptr && sglb::aligned(scratch, 256), SGLB200_ERR_ALIGN, "scratch must be 256-byte aligned");
   SGLB_REQUIRE(bias == nullptr || sglb::aligned(bias, 16), SGLB200_ERR_ALIGN, "bias must be 16-byte aligned");
   sglb::DeviceInfo di;
   if (int rc = sglb::device_info(&di)) return rc;
   const bool ue = scale_ue8m0 != 0;
+  if (M <= sglb::smallm_quant_rows()) {  // no quantiser kernel, no scratch
+    SGLB_REQUIRE(N % 8 == 0, SGLB200_ERR_SHAPE, "N=%lld must be a multiple of 8 (16-byte output rows)", (long long)N);
+    SGLB_REQUIRE(N < ((int64_t)1 << 31) - 256 && K < ((int64_t)1 << 31) - 256, SGLB200_ERR_SHAPE, "a dimension exceeds 2^31");
+    SGLB_REQUIRE(x && w && w_scale && out, SGLB200_ERR_NULL, "x, w, w_scale and out must not be NULL");
+    SGLB_REQUIRE(sglb::aligned(x, 16) && sglb::aligned(w, 16) && sglb::aligned(out, 16) && sglb::aligned(w_scale, 4), SGLB200_ERR_ALIGN,
+                 "x, w and out must be 16-byte aligned and the scale pointer 4-byte aligned");
+    SGLB_REQUIRE(eps >= 0.f, SGLB200_ERR_SHAPE, "eps must be >= 0");
+    SGLB_REQUIRE(di.cc_major == 10, SGLB200_ERR_ARCH, "compute capability %d.%d: this library is built for sm_100a only", di.cc_major,
+                 di.cc_minor);
+    const sglb::RawRows raw = {eps};
+    return sglb::smallm_gemm(x, w, nullptr, static_cast<const float*>(w_scale), out, M, N, K, K, K, N, 0, 0, w_scale_stride_n,
+                             w_scale_stride_k, dtype, bias, nullptr, 0, di.sm_count, stream, nullptr, ue, &raw);
+  }
+  SGLB_REQUIRE(scratch != nullptr && sglb::aligned(scratch, 256), SGLB200_ERR_ALIGN, "scratch must be 256-byte aligned");
   const sglb::LinearScratch l = sglb::linear_scratch(M, N, K, ue, di.sm_count);
   SGLB_REQUIRE(scratch_bytes >= l.bytes, SGLB200_ERR_WORKSPACE, "scratch_bytes=%lld: %lld needed", (long long)scratch_bytes,
                (long long)l.bytes);

@@ -18,7 +18,8 @@
 // tables as in the 128 x 128 grouped kernel; an expert with more than MT rows gets several chunks (its weight tile is
 // then re-read, from L2), an expert without rows gets no item, so only the weights of routed experts are streamed.
 //
-// warp 0: TMA producer; warp 1: TMEM owner + MMA issuer; warp 2: scale loader (sa[token] * sb into shared memory); warps 4..7
+// warp 0: TMA producer; warp 1: TMEM owner + MMA issuer; warp 2: scale loader (sa[token] * sb into shared memory), or
+// at one or two rows warps 2 and 3: quantisers (QUANT); warps 4..7
 // (..11): promotion (tcgen05.ld, acc += p * scale) and the transposed store.  All waits are bounded.
 //
 // The kernel is launched with programmatic stream serialization: it may start while the kernel before it (the
@@ -34,6 +35,8 @@
 
 #include "common.cuh"
 #include "ptx.cuh"
+#include "quant_math.cuh"
+#include "quant_vec.cuh"
 
 namespace sglb {
 
@@ -103,6 +106,9 @@ struct SmallParams {
   const int32_t* problem_sizes;   // optional: rows of expert e = problem_sizes[count_stride * e]
   int32_t count_stride, rows_per_expert, num_experts;
   int64_t sa_stride_e, sb_stride_e;
+  // QUANT form: rows not quantised yet, [M, K] of the output type, and the quantiser's floor
+  const void* x;
+  float eps;
 };
 
 // one unit of work: rows [row0, row0 + rows) of the activations against weight rows [nt * 128, +128) of expert e,
@@ -252,7 +258,81 @@ __device__ __forceinline__ uint32_t pack16(float a, float b, int out_dtype) {
 
 // CLUSTER is a template parameter because the mere presence of the adding-up code cost the main loop of the other form up to
 // 18 % (N=36864 K=7168 M=113: 57 -> 68 us) through its register allocation.
-template <int MT, bool UE, bool GROUPED, int NSUB, bool CLUSTER>
+// Warps 2 and 3 of the QUANT form (one or two rows): the activations come as they are, and these two warps quantise them on their
+// way into the ring, four k-blocks each in turn, with the arithmetic of the separate quantiser.  Every CTA does so for all k-blocks
+// it multiplies; at one or two rows a group of four k-blocks is one or two passes of a warp, less than the weights take to
+// arrive, and it saves a launch and the hand-over between two kernels.  With four passes it no longer hides.  Replayed graph of
+// calls over rotating weights, quantiser kernel -> this, N x K: M=1 576 x 7168 6.6 -> 6.1 us, 24576 x 1536 9.6 -> 9.05, 7168 x
+// 16384 23.4 -> 21.9, 36864 x 7168 43.0 -> 40.4; M=2 6.95 -> 6.3, 9.7 -> 9.3, 23.7 -> 23.0, 42.2 -> 41.5; M=4 7.0 -> 7.4, 10.5 ->
+// 12.9, 23.9 -> 31.2, 42.6 -> 53.
+constexpr int kQuantRows = 2;
+
+template <typename T, int MT, bool UE, bool CLUSTER>
+__device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, uint8_t* smem, float* scale_ring, uint32_t me, int lane,
+                                              int32_t total) {
+  using C = Cfg<MT>;
+  const uint32_t full0 = ptx::smem_u32(&ctl->full[0]), empty0 = ptx::smem_u32(&ctl->empty[0]);
+  const uint32_t sc_full0 = ptx::smem_u32(&ctl->sc_full[0]), sc_empty0 = ptx::smem_u32(&ctl->sc_empty[0]);
+  // eight lanes (sixteen elements each) take a row of a k-block; a pass of the warp covers the rows of `per_pass` k-blocks
+  static_assert(kScaleGroup == 4 && kQuantRows == 2, "four rows of k-blocks per pass");
+  const int rows = p.M, per_pass = kScaleGroup / rows;
+  const int sub = lane & 7, r = (lane >> 3) & (rows - 1), ko = (lane >> 3) / rows;
+  const uint4* row = reinterpret_cast<const uint4*>(static_cast<const T*>(p.x) + (int64_t)r * p.K) + 2 * sub;
+  const uint32_t piece = kWBytes + (uint32_t)(r * 128 + ((sub ^ r) << 4));  // 128-byte swizzle
+  const float inv_max = __frcp_rn(448.0f);
+  uint32_t stage = 0, phase = 0, sc_stage = 0, sc_phase = 0, turn = 0;
+  for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
+    const Item it = get_item<C::kTile, false, CLUSTER>(p, nullptr, t);
+    const float* sb_blk = p.sb + (int64_t)it.nt * p.sb_stride_n;
+    for (int32_t kb0 = it.kb0; kb0 < it.kb1; kb0 += kScaleGroup, turn ^= 1) {
+      if (turn == me) {
+        uint4 v[kQuantRows][2];
+        float b[kQuantRows];
+#pragma unroll
+        for (int u = 0; u < kQuantRows; ++u) {
+          if (u >= rows) break;
+          const int32_t kb = min(kb0 + u * per_pass + ko, it.kb1 - 1);
+          v[u][0] = __ldg(row + (int64_t)kb * (BK / 8));
+          v[u][1] = __ldg(row + (int64_t)kb * (BK / 8) + 1);
+          b[u] = load_scale<UE>(sb_blk, kb, p.sb_stride_k);
+        }
+        if (!ptx::mbar_wait_inl_a(sc_empty0 + sc_stage * 8, sc_phase ^ 1)) { timeout(ctl, 16); return; }
+        float* dst = scale_ring + (size_t)sc_stage * kScaleGroup * C::kTile + r;
+#pragma unroll
+        for (int u = 0; u < kQuantRows; ++u) {
+          if (u >= rows || kb0 + u * per_pass >= it.kb1) break;
+          float amax = fmaxf(p.eps, fmaxf(Elem<T>::vec_absmax(v[u][0]), Elem<T>::vec_absmax(v[u][1])));
+#pragma unroll
+          for (int m = 4; m >= 1; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
+          const float s = group_scale_fast(amax, 448.0f, inv_max, UE);
+          const uint4 codes = encode16_e4m3<T>(v[u][0], v[u][1], s);
+          if (sub == 0) dst[(u * per_pass + ko) * C::kTile] = s * b[u];
+          const int n = min(per_pass, it.kb1 - kb0 - u * per_pass);  // k-blocks of this pass
+          uint32_t mine = stage;
+          for (int i = 0; i < n; ++i) {
+            if (!ptx::mbar_wait_inl_a(empty0 + stage * 8, phase ^ 1)) { timeout(ctl, 11); return; }
+            if (i == ko) mine = stage;
+            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+          }
+          if (ko < n) *reinterpret_cast<uint4*>(smem + (size_t)mine * C::kStageBytes + piece) = codes;
+          ptx::fence_proxy_async();  // the MMA reads shared memory through the asynchronous proxy
+          __syncwarp();
+          if (ko < n && (lane & (8 * rows - 1)) == 0) ptx::mbar_arrive_a(full0 + mine * 8);
+        }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_a(sc_full0 + sc_stage * 8);
+      } else {
+        stage += min(kScaleGroup, it.kb1 - kb0);
+        if (stage >= (uint32_t)C::kStages) { stage -= C::kStages; phase ^= 1; }
+      }
+      if (++sc_stage == kScaleStages) { sc_stage = 0; sc_phase ^= 1; }
+    }
+    if (ctl->abort_flag) return;
+  }
+}
+
+// QUANT: see quantise_rows.
+template <int MT, bool UE, bool GROUPED, int NSUB, bool CLUSTER, bool QUANT>
 // NSUB = 1 has 256 threads; the bound of 320 keeps it at 200 registers, so that a block of the quantiser or of another small
 // kernel (256 threads of 48) fits beside it and programmatic dependent launch really overlaps the two.
 __global__ void __launch_bounds__(NSUB == 1 ? 320 : 384, 1)
@@ -268,7 +348,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::kStages; ++i) {
-      ptx::mbar_init(&ctl->full[i], 1);
+      ptx::mbar_init(&ctl->full[i], QUANT ? 2 : 1);  // the weights' bytes; QUANT: and the warp that wrote the codes
       ptx::mbar_init(&ctl->empty[i], 1);
     }
     for (int i = 0; i < C::kAcc; ++i) {
@@ -283,7 +363,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
     ptx::fence_barrier_init();
     ptx::fence_proxy_async();
     ptx::prefetch_tensormap(&map_w);
-    ptx::prefetch_tensormap(&map_a);
+    if constexpr (!QUANT) ptx::prefetch_tensormap(&map_a);
   }
   if (warp == 1) {
     ptx::tmem_alloc(&ctl->tmem_base, kTmemCols);
@@ -525,14 +605,15 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
             if (pass == 0) {
               if (idx >= (uint32_t)C::kStages) { ok = false; break; }
               if (leader) {
-                ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, C::kStageBytes);
+                ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, QUANT ? kWBytes : C::kStageBytes);
                 ptx::tma_load_3d_a(dst, &map_w, full0 + stage * 8, kb * BK, nt * BN, 0);
               }
               armed |= 1u << stage;
               armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
               pre = idx + 1;
             } else if (idx < pre) {
-              if (leader) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, 0);
+              if constexpr (!QUANT)
+                if (leader) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, 0);
             } else {
               if (!ptx::mbar_wait_inl_a(empty0 + stage * 8, phase ^ 1)) {
                 timeout(ctl, 11);
@@ -540,9 +621,9 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
                 break;
               }
               if (leader) {
-                ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, C::kStageBytes);
+                ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, QUANT ? kWBytes : C::kStageBytes);
                 ptx::tma_load_3d_a(dst, &map_w, full0 + stage * 8, kb * BK, nt * BN, it.e);
-                ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, it.row0);
+                if constexpr (!QUANT) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, it.row0);
               }
               armed |= 1u << stage;
               armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
@@ -594,6 +675,11 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         }
         if (!ok || ctl->abort_flag) break;
       }
+    } else if (QUANT) {
+      // ===== quantisers (warps 2 and 3)
+      ptx::grid_dep_wait();  // the rows come from the kernel before this one
+      if (p.out_dtype == SGLB200_BF16) quantise_rows<__nv_bfloat16, MT, UE, CLUSTER>(p, ctl, smem, scale_ring, warp - 2, lane, total);
+      else quantise_rows<__half, MT, UE, CLUSTER>(p, ctl, smem, scale_ring, warp - 2, lane, total);
     } else if (warp == 2) {
       // ===== scale loader: per group of four k-blocks the products sa[token, kb] * sb[nt, kb], 0 for tokens past the item's
       // rows (the accumulator columns there hold leftovers and are not stored).  The loads of the next group are in flight
@@ -665,7 +751,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
   }
 }
 
-template <int MT, bool UE, bool GROUPED, int NSUB = 1, bool CLUSTER = false>
+template <int MT, bool UE, bool GROUPED, int NSUB = 1, bool CLUSTER = false, bool QUANT = false>
 int launch(const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams& p, int sm_count, cudaStream_t st,
            int64_t max_items, int cluster = 1) {
   constexpr size_t smem = GROUPED ? Cfg<MT, NSUB>::kSmemGrouped : Cfg<MT, NSUB>::kSmem;
@@ -674,14 +760,14 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB, CLUSTER>,
+    cudaError_t e = cudaFuncSetAttribute(fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB, CLUSTER, QUANT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SGLB200_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     if (NSUB == 2) {
       // setmaxnreg.inc draws on the registers the block was launched with and waits for good if they do not suffice: a
       // build whose register count is too low for the split must not be launched
       cudaFuncAttributes fa;
-      e = cudaFuncGetAttributes(&fa, fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB, CLUSTER>);
+      e = cudaFuncGetAttributes(&fa, fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB, CLUSTER, QUANT>);
       if (e != cudaSuccess || fa.numRegs * kThreads < 128 * kAuxRegs + 256 * kPromoRegs)
         return fail(SGLB200_ERR_LAUNCH, "fp8_block_gemm_smallm_kernel: %d registers a thread are too few for its register split",
                     e == cudaSuccess ? fa.numRegs : 0);
@@ -689,7 +775,7 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams
     done[dev] = true;
   }
   const int grid = (int)(max_items < sm_count ? max_items : sm_count);
-  const cudaError_t le = launch_pdl_cluster(fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB, CLUSTER>, dim3(grid), dim3(kThreads), smem, st,
+  const cudaError_t le = launch_pdl_cluster(fp8_block_gemm_smallm_kernel<MT, UE, GROUPED, NSUB, CLUSTER, QUANT>, dim3(grid), dim3(kThreads), smem, st,
                                             cluster, map_w, map_a, p);
   if (le != cudaSuccess) {
     cudaGetLastError();
@@ -714,6 +800,8 @@ int launch_cluster(int MT, bool two, const CUtensorMap& map_w, const CUtensorMap
 }  // namespace
 
 int smallm_max_rows() { return 128; }
+
+int smallm_quant_rows() { return kQuantRows; }
 
 // CTAs per cluster that share one tile's K (1, 2, 4 or 8) for a dense problem.  Cost model in nanoseconds, from runs with one
 // tile per CTA at 1.9 GHz: a k-block takes one CTA `step` (the MMA issuer at 16 columns, the promotion above), or longer once
@@ -749,7 +837,7 @@ int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count) {
 int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K,
                 int64_t lda, int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n,
                 int64_t sb_stride_k, int out_dtype, const void* bias, float* partial, int64_t partial_floats, int sm_count,
-                void* stream, int* splits_used, bool ue8m0) {
+                void* stream, int* splits_used, bool ue8m0, const RawRows* raw) {
   const int MT = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
   const bool two = M > 64;  // 128 activation rows per work item, two sets of promotion warps
   alignas(64) CUtensorMap map_w, map_a;
@@ -758,7 +846,7 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
     const uint64_t str[2] = {(uint64_t)ldb, (uint64_t)ldb * (uint64_t)N};
     if (int rc = make_map_sw128(&map_w, b, 3, dims, str, BN, CU_TENSOR_MAP_L2_PROMOTION_L2_256B)) return rc;
   }
-  {
+  if (raw == nullptr) {
     const uint64_t dims[2] = {(uint64_t)K, (uint64_t)M};
     const uint64_t str[1] = {(uint64_t)lda};
     if (int rc = make_map_sw128(&map_a, a, 2, dims, str, (uint32_t)(M > 64 ? 128 : MT), CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
@@ -796,6 +884,15 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
   if (splits_used) *splits_used = p.k_splits;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t items = (int64_t)p.n_tiles * p.k_splits;
+  if (raw != nullptr) {
+    p.x = a;
+    p.eps = raw->eps;
+    if (p.cluster > 1)
+      return ue8m0 ? launch<16, true, false, 1, true, true>(map_w, map_w, p, (int)items, st, items, p.cluster)
+                   : launch<16, false, false, 1, true, true>(map_w, map_w, p, (int)items, st, items, p.cluster);
+    return ue8m0 ? launch<16, true, false, 1, false, true>(map_w, map_w, p, sm_count, st, items)
+                 : launch<16, false, false, 1, false, true>(map_w, map_w, p, sm_count, st, items);
+  }
   if (p.cluster > 1)
     return ue8m0 ? launch_cluster<true>(MT, two, map_w, map_a, p, st, items) : launch_cluster<false>(MT, two, map_w, map_a, p, st, items);
   if (two) {

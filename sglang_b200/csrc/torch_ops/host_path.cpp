@@ -168,7 +168,8 @@ PyObject* block_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     shape[dim - 1] = N;
     at::Tensor out = empty(shape, t, dev);
     const int64_t bytes = sglb200_fp8_block_linear_scratch_bytes(M, N, K, ue);
-    c10::DataPtr scratch = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)bytes);
+    c10::DataPtr scratch;
+    if (bytes > 0) scratch = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)bytes);
     check_rc(sglb200_fp8_block_linear(x.const_data_ptr(), w.const_data_ptr(), ws.const_data_ptr(),
                                       bp ? bp->const_data_ptr() : nullptr, out.mutable_data_ptr(), M, N, K, ws.stride(0),
                                       ws.stride(1), ue, eps_in_dtype(1e-10, t), code16(t), scratch.get(), bytes, stream),

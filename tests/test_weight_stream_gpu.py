@@ -70,3 +70,35 @@ def test_linear_layer_with_bias(M, N, K, ue8m0):
     assert torch.equal(plain, again), "the sum over the SMs depends on their order"
     assert torch.equal(biased, plain + bd)
     assert_gemm_close(plain, ref, f"{M}x{N}x{K}", allow_one_ulp=True)
+
+
+@pytest.mark.parametrize("ue8m0", [False, True])
+@pytest.mark.parametrize("M,N,K,dtype", [(1, 576, 7168, torch.bfloat16), (2, 136, 640, torch.float16), (1, 24576, 1152, torch.bfloat16),
+                                         (2, 20000, 896, torch.float16), (3, 7168, 2048, torch.bfloat16)])
+def test_rows_quantised_by_the_gemm_itself(M, N, K, dtype, ue8m0):
+    """Up to two rows the GEMM quantises its activations: the bits of the separate quantiser and the same GEMM.  The shapes put K on
+    one CTA and on clusters, several tiles on a CTA, and end K inside a group of four k-blocks."""
+    from sglang_b200._lib import lib
+    from sglang_b200.layers.quantization import w8a8_block_fp8_matmul
+    from sglang_b200.layers.quantization.fp8_kernel import sglang_per_token_group_quant_fp8
+    from sglang_b200.layers.quantization.fp8 import Fp8Config, Fp8LinearMethod
+    layer, method = torch.nn.Module(), Fp8LinearMethod(Fp8Config())
+    method.create_weights(layer, K, [N], K, N, dtype, device="cuda")
+    w, w_s = oracle.block_quant_weight(torch.randn(N, K, generator=torch.Generator().manual_seed(N)) * 0.02, scale_ue8m0=ue8m0)
+    layer.weight.data.copy_(w)
+    layer.weight_scale_inv.data.copy_(w_s)
+    method.process_weights_after_loading(layer)
+    x = make_activations(M, K, seed=M).to(dtype)
+    if not ue8m0:
+        x[0, :128] = 0  # a group without a maximum
+    x[M - 1, -1] = -0.0
+    x = x.cuda()
+    got = method.apply(layer, x)
+    if ue8m0:
+        q, s = oracle.per_token_group_quant_fp8(x.cpu(), 128, scale_ue8m0=True)
+    else:
+        q, s = sglang_per_token_group_quant_fp8(x, 128)
+    want = w8a8_block_fp8_matmul(q.cuda(), w.cuda(), s.cuda(), w_s.cuda(), [128, 128], dtype)
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    assert torch.equal(got, want)
