@@ -8,7 +8,7 @@
 // N / 128 tiles alone cannot occupy the SMs, the CTAs of a cluster cut a tile's K among themselves and rank 0 adds their sums up
 // out of their shared memory (smallm_cluster): against fp32 partial sums in memory and a kernel that adds them, quantiser
 // included, N=576 K=7168 M=1 / 48: 9.6 / 14.1 -> 6.8 / 11.1 us, N=7168 K=16384 M=48 32.3 -> 27.1, N=10240 K=8192 M=48 27.0 -> 22.1.
-// From 65 to 128 rows eight promotion warps share every accumulator stage, four per 64 token columns.
+// From 65 to 128 rows eight or sixteen promotion warps share every accumulator stage.
 // Measured against scales that every promotion warp fetched and spread by shuffles, weights from HBM (B200):
 // N=36864 K=7168 M=32 / 64 / 128: 46.6 / 54.8 / 75.0 -> 41.8 / 43.3 / 55.1 us (6.1 TB/s at 64 rows);
 // N=24576 K=1536 M=16 / 64 / 128: 8.4 / 15.4 / 21.8 -> 7.7 / 9.8 / 13.9 us.
@@ -70,9 +70,11 @@ constexpr int kAuxRegs = 96, kPromoRegs = 200;  // register split of the NSUB = 
 
 constexpr int kMaxExperts = 1024;
 
-// NSUB = 2 (65 to 128 rows per item): the MMA covers up to MT * NSUB = 128 activation rows and a second set of four
-// promotion warps takes the second half of every accumulator stage's columns, so the registers per thread stay those of
-// 64 rows.
+// NSUB > 1 (65 to 128 rows per item): the MMA covers up to MT * NSUB = 128 activation rows and every set of four promotion warps
+// takes its MT of every accumulator stage's columns.  Alone on a tile, four sets of 32 columns are the better split: 16 warps hide
+// each other's chain of wait, load, hand-back and FMA (N=10240 K=8192 M=113 31.3 -> 30.1 us, N=24576 K=1536 18.7 -> 17.6, N=36864
+// K=7168 65 -> 59 against two sets of 64).  In a cluster two sets of 64 are: with the code that adds the sums up, 96 registers do
+// not hold four sets' (N=7168 K=16384 M=113 36.7 against 40.1 us).
 template <int MT, int NSUB = 1>
 struct Cfg {
   static constexpr int kTile = MT * NSUB;  // most activation rows per work item = TMEM columns per stage
@@ -335,7 +337,7 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
 template <int MT, bool UE, bool GROUPED, int NSUB, bool CLUSTER, bool QUANT>
 // NSUB = 1 has 256 threads; the bound of 320 keeps it at 200 registers, so that a block of the quantiser or of another small
 // kernel (256 threads of 48) fits beside it and programmatic dependent launch really overlaps the two.
-__global__ void __launch_bounds__(NSUB == 1 ? 320 : 384, 1)
+__global__ void __launch_bounds__(NSUB == 1 ? 320 : 128 + 128 * NSUB, 1)
 fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                              const SmallParams p) {
   using C = Cfg<MT, NSUB>;
@@ -789,7 +791,8 @@ template <bool UE>
 int launch_cluster(int MT, bool two, const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams& p, cudaStream_t st,
                    int64_t items) {
   const int grid = (int)items, c = p.cluster;
-  if (two) return launch<64, UE, false, 2, true>(map_w, map_a, p, grid, st, items, c);
+  if constexpr (!UE)
+    if (two) return launch<64, false, false, 2, true>(map_w, map_a, p, grid, st, items, c);
   switch (MT) {
     case 16: return launch<16, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
     case 32: return launch<32, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
@@ -839,7 +842,8 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
                 int64_t sb_stride_k, int out_dtype, const void* bias, float* partial, int64_t partial_floats, int sm_count,
                 void* stream, int* splits_used, bool ue8m0, const RawRows* raw) {
   const int MT = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
-  const bool two = M > 64;  // 128 activation rows per work item, two sets of promotion warps
+  const bool two = M > 64;  // up to 128 activation rows per work item, several sets of promotion warps (fp32 scales only)
+  if (two && ue8m0) return fail(SGLB200_ERR_SHAPE, "UE8M0 scales: at most 64 rows, not %lld", (long long)M);
   alignas(64) CUtensorMap map_w, map_a;
   {
     const uint64_t dims[3] = {(uint64_t)K, (uint64_t)N, 1};
@@ -894,11 +898,8 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
                  : launch<16, false, false, 1, false, true>(map_w, map_w, p, sm_count, st, items);
   }
   if (p.cluster > 1)
-    return ue8m0 ? launch_cluster<true>(MT, two, map_w, map_a, p, st, items) : launch_cluster<false>(MT, two, map_w, map_a, p, st, items);
-  if (two) {
-    return ue8m0 ? launch<64, true, false, 2>(map_w, map_a, p, sm_count, st, items)
-                 : launch<64, false, false, 2>(map_w, map_a, p, sm_count, st, items);
-  }
+    return ue8m0 ? launch_cluster<true>(MT, false, map_w, map_a, p, st, items) : launch_cluster<false>(MT, two, map_w, map_a, p, st, items);
+  if (two) return launch<32, false, false, 4>(map_w, map_a, p, sm_count, st, items);
   if (ue8m0) {
     switch (MT) {
       case 16: return launch<16, true, false>(map_w, map_a, p, sm_count, st, items);
