@@ -659,8 +659,19 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         const uint32_t idesc = ptx::make_idesc_e4m3_f32(BN, (uint32_t)(it.rows + 15) / 16 * 16);
         bool ok = true;
         for (int32_t kb = kb0; kb < kb1; ++kb) {
-          if (!ptx::mbar_wait_inl_a(acc_empty0 + acc * 8, acc_phase ^ 1)) { timeout(ctl, 12); ok = false; break; }
-          if (!ptx::mbar_wait_inl_a(full0 + stage * 8, phase)) { timeout(ctl, 13); ok = false; break; }
+          if constexpr (MT == 16 && NSUB == 1) {
+            // Both waits at once, one half of the warp each: with 16 columns a k-block costs this warp little else (N=10240 K=8192
+            // M=1 18.1 -> 16.1 us a call, N=24576 K=1536 M=16 10.2 -> 9.8); with more it gained nothing.
+            const bool op = (lane & 1) != 0;
+            if (!__all_sync(0xffffffffu, ptx::mbar_wait_inl_a(op ? full0 + stage * 8 : acc_empty0 + acc * 8, op ? phase : acc_phase ^ 1))) {
+              timeout(ctl, 12);
+              ok = false;
+              break;
+            }
+          } else {
+            if (!ptx::mbar_wait_inl_a(acc_empty0 + acc * 8, acc_phase ^ 1)) { timeout(ctl, 12); ok = false; break; }
+            if (!ptx::mbar_wait_inl_a(full0 + stage * 8, phase)) { timeout(ctl, 13); ok = false; break; }
+          }
           ptx::tc_fence_after();
           if (leader) {
             const uint64_t w_desc = desc0 + (uint64_t)(stage * (C::kStageBytes >> 4));
