@@ -1045,17 +1045,26 @@ void launch_splitk_reduce(const float* partial, void* out, const void* bias, int
 
 namespace {
 
-// Number of k-splits for a dense problem: only when the output tiles alone cannot occupy the SMs (small M, where the
-// kernel streams the weights once and is HBM-bound), enough splits for about two work items per SM, each at least
-// four k-blocks deep.  Returns 1 when split-K does not apply.
+// Number of k-splits for a dense problem whose output tiles alone leave SMs idle; 1 = none.  Cost model in nanoseconds from runs
+// at 1.9 GHz: a k-block takes a CTA 230 and a work item 500 more; splitting costs the reduce kernel (3500) and the partial sums'
+// way to memory and back (8 bytes each at about 5 TB/s).  The rule before aimed at two items per SM whatever the sums cost, and
+// often hit three waves: N=4096 K=4096 M=256 27.9 us (now 17), N=1536 K=7168 M=512 30.0 (22), N=3072 K=1536 M=256 13.4 (10).
 int splitk_choice(int64_t M, int64_t N, int64_t K, int sm_count) {
   const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int64_t k_tiles = (K + BK - 1) / BK;
-  if (tiles * 2 > sm_count || k_tiles < 8) return 1;
-  int64_t splits = (2 * (int64_t)sm_count + tiles - 1) / tiles;
-  if (splits > k_tiles / 4) splits = k_tiles / 4;
-  if (splits > 32) splits = 32;
-  return splits < 2 ? 1 : (int)splits;
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int64_t c = 1; c <= 32 && (c == 1 || (c * 4 <= k_tiles && tiles * c <= 2 * (int64_t)sm_count)); ++c) {
+    const int64_t kb = (k_tiles + c - 1) / c;
+    if ((k_tiles + kb - 1) / kb != c) continue;  // every split must get k-blocks
+    const int64_t waves = (tiles * c + sm_count - 1) / sm_count;
+    const int64_t cost = waves * (kb * 230 + 500) + (c > 1 ? 3500 + c * M * N * 8 / 5000 : 0);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = (int)c;
+    }
+  }
+  return best;
 }
 
 template <bool GROUPED, bool PUSH>
