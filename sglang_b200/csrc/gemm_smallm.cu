@@ -802,8 +802,7 @@ template <bool UE>
 int launch_cluster(int MT, bool two, const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams& p, cudaStream_t st,
                    int64_t items) {
   const int grid = (int)items, c = p.cluster;
-  if constexpr (!UE)
-    if (two) return launch<64, false, false, 2, true>(map_w, map_a, p, grid, st, items, c);
+  if (two) return launch<64, UE, false, 2, true>(map_w, map_a, p, grid, st, items, c);
   switch (MT) {
     case 16: return launch<16, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
     case 32: return launch<32, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
@@ -853,8 +852,7 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
                 int64_t sb_stride_k, int out_dtype, const void* bias, float* partial, int64_t partial_floats, int sm_count,
                 void* stream, int* splits_used, bool ue8m0, const RawRows* raw) {
   const int MT = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
-  const bool two = M > 64;  // up to 128 activation rows per work item, several sets of promotion warps (fp32 scales only)
-  if (two && ue8m0) return fail(SGLB200_ERR_SHAPE, "UE8M0 scales: at most 64 rows, not %lld", (long long)M);
+  const bool two = M > 64;  // up to 128 activation rows per work item, several sets of promotion warps
   alignas(64) CUtensorMap map_w, map_a;
   {
     const uint64_t dims[3] = {(uint64_t)K, (uint64_t)N, 1};
@@ -909,8 +907,11 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
                  : launch<16, false, false, 1, false, true>(map_w, map_w, p, sm_count, st, items);
   }
   if (p.cluster > 1)
-    return ue8m0 ? launch_cluster<true>(MT, false, map_w, map_a, p, st, items) : launch_cluster<false>(MT, two, map_w, map_a, p, st, items);
-  if (two) return launch<32, false, false, 4>(map_w, map_a, p, sm_count, st, items);
+    return ue8m0 ? launch_cluster<true>(MT, two, map_w, map_a, p, st, items) : launch_cluster<false>(MT, two, map_w, map_a, p, st, items);
+  if (two) {
+    if (ue8m0) return fail(SGLB200_ERR_SHAPE, "UE8M0 scales: at most 64 rows unless K is shared, not %lld", (long long)M);
+    return launch<32, false, false, 4>(map_w, map_a, p, sm_count, st, items);
+  }
   if (ue8m0) {
     switch (MT) {
       case 16: return launch<16, true, false>(map_w, map_a, p, sm_count, st, items);

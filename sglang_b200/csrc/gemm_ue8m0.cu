@@ -475,9 +475,11 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
   SGLB_REQUIRE(di.cc_major == 10, SGLB200_ERR_ARCH, "compute capability %d.%d: this library is built for sm_100a only",
                di.cc_major, di.cc_minor);
 
-  if (!grouped && M <= 64) {
+  if (!grouped && (M <= 64 || (M <= smallm_max_rows() && smallm_cluster(M, N, K, di.sm_count) > 1))) {
     // few rows: the weight-streaming kernel with swapped operands decodes the exponent bytes itself (gemm_smallm.cu);
-    // from 65 rows up the block-scaled tile kernel below, which has no promotion, is the faster one
+    // from 65 rows up the block-scaled tile kernel below, which has no promotion, is level or faster (N=24576 K=1536 M=100 15.9
+    // against 17.9 us), except where it would leave most SMs idle and the other shares K inside clusters (N=2112 K=7168 M=100
+    // 26.2 against 15.9, N=7168 K=16384 53 against 36)
     return smallm_gemm(a, b, reinterpret_cast<const float*>(sfa), reinterpret_cast<const float*>(sfb), out, M, N, K, lda, ldb, ldc,
                        sfa_stride_m, sfa_ld, sfb_stride_n, sfb_stride_k, out_dtype, bias, nullptr, 0, di.sm_count, stream, nullptr,
                        true);
