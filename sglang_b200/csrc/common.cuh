@@ -50,7 +50,8 @@ int quant_rows(const void* input, int in_dtype, void* out_q, void* out_s, int64_
 // The UE8M0 GEMM of the linear layer, gemm_ue8m0.cu
 int ue8m0_linear_gemm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, const void* bias, void* out, int64_t M,
                       int64_t N, int64_t K, int64_t sfa_ld, int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype,
-                      void* stream);
+                      void* stream, float* workspace, int64_t workspace_floats);
+int ue8m0_splits(int64_t M, int64_t N, int64_t K, int sm_count);  // with `workspace` of that many [M][N] fp32 sums
 int smallm_take_device_status();
 int nvls_take_device_status();  // nvls.cu
 constexpr int kGroupedFewRowsDefault = 20;

@@ -1314,7 +1314,7 @@ struct LinearScratch {
 };
 LinearScratch linear_scratch(int64_t M, int64_t N, int64_t K, bool ue8m0, int sms) {
   LinearScratch l;
-  const int splits = !ue8m0 && M > smallm_max_rows() ? splitk_choice(M, N, K, sms) : 1;
+  const int splits = ue8m0 ? ue8m0_splits(M, N, K, sms) : (M > smallm_max_rows() ? splitk_choice(M, N, K, sms) : 1);
   l.gemm_bytes = splits > 1 ? (int64_t)splits * M * N * (int64_t)sizeof(float) : 0;
   l.ld = (M + 3) / 4 * 4;
   const int64_t words = ue8m0 ? (K / 128 + 3) / 4 : K / 128;
@@ -1369,7 +1369,8 @@ extern "C" int sglb200_fp8_block_linear(const void* x, const void* w, const void
   if (int rc = sglb::quant_rows(x, dtype, codes, scales, M, K, eps, ue, 1, l.ld, stream)) return rc;
   if (ue)
     return sglb::ue8m0_linear_gemm(codes, w, static_cast<const int32_t*>(scales), static_cast<const int32_t*>(w_scale), bias, out, M,
-                                   N, K, l.ld, w_scale_stride_n, w_scale_stride_k, dtype, stream);
+                                   N, K, l.ld, w_scale_stride_n, w_scale_stride_k, dtype, stream, l.gemm_bytes > 0 ? static_cast<float*>(scratch) : nullptr,
+                                   l.gemm_bytes / (int64_t)sizeof(float));
   return sglb::gemm_common(codes, w, static_cast<const float*>(scales), static_cast<const float*>(w_scale), out, nullptr, nullptr, M,
                            1, N, K, K, K, 0, N, 1, l.ld, 0, w_scale_stride_n, w_scale_stride_k, dtype, stream,
                            l.gemm_bytes > 0 ? static_cast<float*>(scratch) : nullptr, l.gemm_bytes / (int64_t)sizeof(float), nullptr,

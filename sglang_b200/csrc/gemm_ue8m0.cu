@@ -78,6 +78,8 @@ struct Params {
   int32_t m_tiles, n_tiles, k_tiles, k_groups;
   int64_t ldc, sfa_ld, sfa_stride_m, sfb_stride_e, sfb_stride_n, sfb_stride_k;
   int32_t out_dtype;
+  float* partial;  // SPLIT: fp32 sums [k_splits][M][N] instead of `out`
+  int32_t k_splits, kg_per_split;
 };
 
 struct Ctl {
@@ -95,12 +97,23 @@ static_assert(sizeof(Ctl) <= 256, "control block");
 
 struct TileUe {
   int32_t m0, row_end, n0, expert;
+  int32_t split, kg0, kg1;  // groups of four k-blocks [kg0, kg1)
 };
 
 // dense: grouped-M raster; grouped: tile table of the experts (prefix sums in shared memory), n-major inside an expert
-template <bool GROUPED>
+template <bool GROUPED, bool SPLIT>
 __device__ __forceinline__ TileUe tile_coords(const Params& p, const int32_t* tile_start, int32_t t) {
   TileUe tl;
+  tl.split = 0;
+  tl.kg0 = 0;
+  tl.kg1 = p.k_groups;
+  if constexpr (SPLIT) {
+    const int32_t tiles = p.m_tiles * p.n_tiles;
+    tl.split = t / tiles;
+    t -= tl.split * tiles;
+    tl.kg0 = tl.split * p.kg_per_split;
+    tl.kg1 = min(tl.kg0 + p.kg_per_split, p.k_groups);
+  }
   if constexpr (!GROUPED) {
     const int32_t per_group = kGroupM * p.n_tiles;
     const int32_t gid = t / per_group;
@@ -170,7 +183,9 @@ __device__ __forceinline__ void store32(const uint32_t (&a)[32], const OutT* bia
   }
 }
 
-template <bool GROUPED>
+// SPLIT (dense): a work item is (tile, range of K) and leaves fp32 sums for splitk_reduce_kernel; the other forms do without the
+// range arithmetic.
+template <bool GROUPED, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const Params p) {
@@ -229,7 +244,7 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       }
     }
   } else {
-    if (threadIdx.x == 0) ctl->total_tiles = p.m_tiles * p.n_tiles;
+    if (threadIdx.x == 0) ctl->total_tiles = p.m_tiles * p.n_tiles * (SPLIT ? p.k_splits : 1);
   }
   ptx::tc_fence_before();
   __syncthreads();
@@ -251,9 +266,10 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     // ===== TMA producers
     uint32_t stage = 0, phase = 0, g = 0;
     for (int32_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-      const TileUe tl = tile_coords<GROUPED>(p, tile_start, t);
+      const TileUe tl = tile_coords<GROUPED, SPLIT>(p, tile_start, t);
       bool ok = true;
-      for (int32_t kb = 0; kb < p.k_tiles; ++kb, ++g) {
+      const int32_t kb1 = SPLIT ? min(tl.kg1 * 4, p.k_tiles) : p.k_tiles;
+      for (int32_t kb = SPLIT ? tl.kg0 * 4 : 0; kb < kb1; ++kb, ++g) {
         if ((g & 1) == (uint32_t)warp) {
           if (!ptx::mbar_wait_a(empty0 + stage * 8, phase ^ 1)) {
             timeout(ctl, 11);
@@ -289,7 +305,13 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       bool ok = ptx::mbar_wait_a(acc_empty0 + as * 8, ((tile_i >> 1) & 1) ^ 1);
       if (!ok) timeout(ctl, 12);
       const uint32_t d_tmem = tmem_base + as * BN;
-      for (int32_t kg = 0; kg < p.k_groups && ok; ++kg, ++q) {
+      int32_t kg0 = 0, kg1 = p.k_groups;
+      if constexpr (SPLIT) {
+        const TileUe tl = tile_coords<GROUPED, SPLIT>(p, tile_start, t);
+        kg0 = tl.kg0;
+        kg1 = tl.kg1;
+      }
+      for (int32_t kg = kg0; kg < kg1 && ok; ++kg, ++q) {
         const uint32_t buf = q % kSfBufs;
         if (!ptx::mbar_wait_a(sf_full0 + buf * 8, (q / kSfBufs) & 1)) {
           timeout(ctl, 13);
@@ -317,7 +339,7 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             const uint64_t a_desc = desc0 + (uint64_t)(stage * (kStageBytes >> 4));
             const uint64_t b_desc = a_desc + (kTileABytes >> 4);
             const uint32_t idesc = ptx::make_idesc_mxf8(BM, BN, (uint32_t)(kb & 3));
-            ptx::mma_mxf8_block_scaled(d_tmem, a_desc, b_desc, idesc, sf_col, sf_col + 4, kb > 0 ? 1u : 0u);
+            ptx::mma_mxf8_block_scaled(d_tmem, a_desc, b_desc, idesc, sf_col, sf_col + 4, kb > kg0 * 4 ? 1u : 0u);
 #pragma unroll
             for (uint32_t k = 1; k < BK / 32; ++k)
               ptx::mma_mxf8_block_scaled(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, sf_col, sf_col + 4, 1u);
@@ -334,10 +356,10 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const int32_t nb_last = (p.N + 127) / 128 - 1;
     uint32_t q = 0;
     for (int32_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-      const TileUe tl = tile_coords<GROUPED>(p, tile_start, t);
+      const TileUe tl = tile_coords<GROUPED, SPLIT>(p, tile_start, t);
       const int32_t m0 = tl.m0, n0 = tl.n0;
       bool ok = true;
-      for (int32_t kg = 0; kg < p.k_groups; ++kg, ++q) {
+      for (int32_t kg = SPLIT ? tl.kg0 : 0; kg < (SPLIT ? tl.kg1 : p.k_groups); ++kg, ++q) {
         const uint32_t buf = q % kSfBufs;
         if (!ptx::mbar_wait_a(sf_empty0 + buf * 8, ((q / kSfBufs) & 1) ^ 1)) {
           timeout(ctl, 15);
@@ -380,7 +402,7 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const int col0 = ((warp - kEpiWarp0) >> 2) * kEpiCols;
     uint32_t tile_i = 0;
     for (int32_t t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_i) {
-      const TileUe tl = tile_coords<GROUPED>(p, tile_start, t);
+      const TileUe tl = tile_coords<GROUPED, SPLIT>(p, tile_start, t);
       const int32_t m0 = tl.m0, n0 = tl.n0;
       const uint32_t as = tile_i & 1;
       if (!ptx::mbar_wait_a(acc_full0 + as * 8, (tile_i >> 1) & 1)) {
@@ -406,7 +428,14 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         if (row < tl.row_end) {
           const int32_t n_first = n0 + col0 + c * 32;
           const int32_t n_limit = min(p.N, n0 + col0 + kEpiCols);  // do not store beyond this warp's 112 columns
-          if (p.out_dtype == SGLB200_BF16) {
+          if constexpr (SPLIT) {
+            float4* dst = reinterpret_cast<float4*>(p.partial + ((int64_t)tl.split * p.M + row) * p.N + n_first);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (n_first + 4 * j < n_limit)
+                dst[j] = make_float4(__uint_as_float(va[4 * j]), __uint_as_float(va[4 * j + 1]), __uint_as_float(va[4 * j + 2]),
+                                     __uint_as_float(va[4 * j + 3]));
+          } else if (p.out_dtype == SGLB200_BF16) {
             store32<__nv_bfloat16>(va, static_cast<const __nv_bfloat16*>(p.bias),
                                    static_cast<__nv_bfloat16*>(p.out) + (int64_t)row * p.ldc + n_first, n_first, n_limit,
                                    SGLB200_BF16);
@@ -440,11 +469,39 @@ extern "C" int sglb200_debug_set_status_mirror(int* device_visible_host_ptr) {
 
 namespace sglb {
 namespace {
+bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count) {
+  return M <= 64 || (M <= smallm_max_rows() && smallm_cluster(M, N, K, sm_count) > 1);
+}
+}  // namespace
+
+// K ranges (whole groups of four k-blocks) of a dense problem whose tiles alone leave SMs idle, for callers with scratch; 1 = none.
+// Cost model in nanoseconds at 1.9 GHz: a k-block takes a CTA 380, a work item 800 more; splitting costs the reduce kernel (3500)
+// and the partial sums' way to memory and back (8 bytes each at about 5 TB/s).
+int ue8m0_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
+  if (takes_few_rows(M, N, K, sm_count)) return 1;
+  const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), groups = (K + 4 * BK - 1) / (4 * BK);
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int64_t c = 1; c <= 32 && (c == 1 || (c <= groups && tiles * c <= 2 * (int64_t)sm_count)); ++c) {
+    const int64_t kg = (groups + c - 1) / c;
+    if ((groups + kg - 1) / kg != c) continue;  // every range must get k-blocks
+    const int64_t waves = (tiles * c + sm_count - 1) / sm_count;
+    const int64_t cost = waves * (kg * 4 * 380 + 800) + (c > 1 ? 3500 + c * M * N * 8 / 5000 : 0);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = (int)c;
+    }
+  }
+  return best;
+}
+
+namespace {
 int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, void* out,
                  const int32_t* expert_offsets, int64_t M, int64_t num_experts, int64_t N, int64_t K, int64_t lda,
                  int64_t ldb, int64_t ldb_e, int64_t ldc, int64_t sfa_ld, int64_t sfa_stride_m, int64_t sfb_stride_e,
                  int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype, void* stream,
-                 const void* bias = nullptr) {
+                 const void* bias = nullptr,
+                 float* workspace = nullptr, int64_t workspace_floats = 0) {
   const bool grouped = expert_offsets != nullptr;
   SGLB_REQUIRE(M >= 0 && N >= 0 && K >= 0, SGLB200_ERR_SHAPE, "M=%lld N=%lld K=%lld: negative size", (long long)M,
                (long long)N, (long long)K);
@@ -475,7 +532,7 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
   SGLB_REQUIRE(di.cc_major == 10, SGLB200_ERR_ARCH, "compute capability %d.%d: this library is built for sm_100a only",
                di.cc_major, di.cc_minor);
 
-  if (!grouped && (M <= 64 || (M <= smallm_max_rows() && smallm_cluster(M, N, K, di.sm_count) > 1))) {
+  if (!grouped && takes_few_rows(M, N, K, di.sm_count)) {
     // few rows: the weight-streaming kernel with swapped operands decodes the exponent bytes itself (gemm_smallm.cu);
     // from 65 rows up the block-scaled tile kernel below, which has no promotion, is level or faster (N=24576 K=1536 M=100 15.9
     // against 17.9 us), except where it would leave most SMs idle and the other shares K inside clusters (N=2112 K=7168 M=100
@@ -528,28 +585,44 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
   p.sfb_stride_n = sfb_stride_n;
   p.sfb_stride_k = sfb_stride_k;
   p.out_dtype = out_dtype;
+  p.partial = nullptr;
+  p.k_splits = 1;
+  p.kg_per_split = p.k_groups;
+  if (!grouped && workspace != nullptr) {
+    const int splits = ue8m0_splits(M, N, K, di.sm_count);
+    if (splits > 1 && (int64_t)splits * M * N <= workspace_floats) {
+      p.partial = workspace;
+      p.kg_per_split = (p.k_groups + splits - 1) / splits;
+      p.k_splits = splits;
+    }
+  }
 
-  static bool attr_done[2][64] = {{false}};
+  static bool attr_done[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !attr_done[grouped][dev]) {
-    cudaError_t e = grouped ? cudaFuncSetAttribute(fp8_ue8m0_gemm_kernel<true>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes)
-                            : cudaFuncSetAttribute(fp8_ue8m0_gemm_kernel<false>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (e != cudaSuccess) return fail(SGLB200_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    attr_done[grouped][dev] = true;
+  if (dev >= 0 && dev < 64 && !attr_done[dev]) {
+    for (auto* kernel : {fp8_ue8m0_gemm_kernel<true, false>, fp8_ue8m0_gemm_kernel<false, false>, fp8_ue8m0_gemm_kernel<false, true>}) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+      if (e != cudaSuccess) return fail(SGLB200_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    }
+    attr_done[dev] = true;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (grouped) {
     // an upper bound on the tile count without reading the device: every expert can add one ragged m-tile
     const int64_t max_tiles = ((M + BM - 1) / BM + num_experts) * p.n_tiles;
     const int grid = (int)(max_tiles < di.sm_count ? max_tiles : di.sm_count);
-    fp8_ue8m0_gemm_kernel<true><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
+    fp8_ue8m0_gemm_kernel<true, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
   } else {
-    const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
+    const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles * p.k_splits;
     const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
-    fp8_ue8m0_gemm_kernel<false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
+    if (p.k_splits > 1) {
+      fp8_ue8m0_gemm_kernel<false, true><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
+      SGLB_CHECK_LAUNCH("fp8_ue8m0_gemm_kernel");
+      launch_splitk_reduce(p.partial, out, bias, M, N, ldc, p.k_splits, out_dtype, di.sm_count, stream);
+    } else {
+      fp8_ue8m0_gemm_kernel<false, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
+    }
   }
   SGLB_CHECK_LAUNCH("fp8_ue8m0_gemm_kernel");
   return SGLB200_OK;
@@ -558,9 +631,9 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
 
 int ue8m0_linear_gemm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, const void* bias, void* out, int64_t M,
                       int64_t N, int64_t K, int64_t sfa_ld, int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype,
-                      void* stream) {
+                      void* stream, float* workspace, int64_t workspace_floats) {
   return ue8m0_common(a, b, sfa, sfb, out, nullptr, M, 1, N, K, K, K, 0, N, sfa_ld, 1, 0, sfb_stride_n, sfb_stride_k, out_dtype,
-                      stream, bias);
+                      stream, bias, workspace, workspace_floats);
 }
 }  // namespace sglb
 

@@ -45,7 +45,7 @@ def test_masked_layout_with_expected_rows(expected):
 
 @pytest.mark.parametrize("ue8m0", [False, True])
 @pytest.mark.parametrize("M,N,K", [(1, 576, 7168), (5, 8, 128), (16, 7168, 2048), (33, 1000, 1024), (64, 10240, 1536),
-                                   (113, 2112, 7168), (128, 136, 4096), (129, 576, 2048), (300, 392, 1024)])
+                                   (113, 2112, 7168), (128, 136, 4096), (129, 576, 2048), (300, 392, 1024), (200, 264, 2176), (385, 1000, 4480)])
 def test_linear_layer_with_bias(M, N, K, ue8m0):
     """The one-call linear layer against its parts: quantiser, GEMM entry, then the bias in the output type.  The shapes
     put K on one CTA, on a few and on all of them, and cross the row limits of the kernels."""
