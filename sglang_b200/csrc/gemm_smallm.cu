@@ -929,11 +929,14 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
 // Above this average the 128 x 128 tile kernel is level with or ahead of chunks of up to 128 rows (256 experts, N=7168 K=2048:
 // 896 against 920 us at 64 rows, 1327 against 1410 at 128); at 32 rows the chunks win (875 against 689 us).  The UE8M0 tile
 // kernel has no promotion to pay for and draws level much earlier (whole layer at 32 rows: 1940 us it, 1990 the chunks).
-constexpr int64_t kWideRowsMax = 48, kWideRowsMaxUe8m0 = 20;
+// With a K of a few k-blocks an item is mostly start and store, of which the UE8M0 tile kernel has less (its epilogue overlaps the
+// next tile): the layer of 256 experts, 7168 columns, K=256 in the second GEMM takes 131 / 242 / 296 us with the chunks at 16 / 128 /
+// 256 tokens, 123 / 216 / 246 without.  The fp32 tile kernel gains nothing from that (325 against 376 us at 256 tokens).
+constexpr int64_t kWideRowsMax = 48, kWideRowsMaxUe8m0 = 20, kShortKUe8m0 = 512;
 
 // Rows per chunk of the grouped few-rows kernel for `total_rows` rows spread over `num_experts` experts (or
 // rows_per_expert rows at most per expert in the masked layout); 0 = the 128 x 128 grouped kernel is the better choice.
-int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows, bool ue8m0) {
+int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows, int64_t K, bool ue8m0) {
   if (g_grouped_few_rows_max == 0) return 0;
   int64_t avg = (total_rows + num_experts - 1) / num_experts;
   if (rows_per_expert > 0) {  // masked layout: the row bound is known, the rows in use only if the caller expects a number
@@ -944,7 +947,7 @@ int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_p
     avg = expected_rows;
   }
   // the setter's default stands for the rule above; a caller who sets another limit gets exactly that
-  const int64_t rule = ue8m0 ? kWideRowsMaxUe8m0 : kWideRowsMax;
+  const int64_t rule = !ue8m0 ? kWideRowsMax : (K <= kShortKUe8m0 ? 0 : kWideRowsMaxUe8m0);
   if (avg > (g_grouped_few_rows_max == kGroupedFewRowsDefault ? rule : g_grouped_few_rows_max)) return 0;
   return avg <= 8 ? 16 : (avg <= 24 ? 32 : 64);
 }
