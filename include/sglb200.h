@@ -164,7 +164,7 @@ int sglb200_fp8_blockwise_scaled_mm(const void* a, const void* b, const float* s
  * partial sums to `workspace` ([splits, M, N] floats) and a second small kernel adds them in ascending split order and
  * casts; up to 128 rows the CTAs of a cluster share a tile's K and add up on the chip, with or without `workspace`.
  * sglb200_fp8_blockwise_scaled_mm_workspace_bytes() returns a sufficient size for a shape on the current device (0 = K is
- * not cut); with workspace == NULL or a workspace that is too small the call is exactly sglb200_fp8_blockwise_scaled_mm.
+ * not cut; up to 128 rows the size of a split through memory, which this kernel does without); with workspace == NULL or a workspace that is too small the call is exactly sglb200_fp8_blockwise_scaled_mm.
  * The workspace is scratch: contents on entry are ignored, calls on the same stream may share it.  Replaces the per-call
  * cudaMalloc'ed CUTLASS workspace of the reference (sgl-kernel/csrc/gemm/fp8_blockwise_gemm_kernel.cu:162-163) and its
  * stream-K path (sgl-kernel/csrc/cutlass_extensions/gemm/fp8_blockwise_gemm_sm90_dispatch.cuh:179-197).
@@ -201,7 +201,8 @@ int64_t sglb200_fp8_block_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, 
  * allocate where they run the GEMM: an engine that gave all device memory to its own pool, a region in which
  * allocation is forbidden, a C caller without an allocator.
  *   - Shapes whose split-K scratch (sglb200_fp8_blockwise_scaled_mm_workspace_bytes) exceeds the built-in buffer are
- *     REJECTED with SGLB200_ERR_WORKSPACE (nothing is launched); shapes that do not use split-K run as usual.
+ *     REJECTED with SGLB200_ERR_WORKSPACE (nothing is launched), except above 128 rows where the output tiles alone
+ *     (128 x 128) occupy more than half of the SMs: those run with K uncut.  Shapes that do not use split-K run as usual.
  *   - The first call on each device looks the array's device address up (cudaGetSymbolAddress, that device current);
  *     make that first call outside any stream capture.
  *   - Every call on a device shares the one array, which keeps whatever the previous call left in it.  The kernels

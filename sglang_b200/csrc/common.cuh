@@ -32,6 +32,7 @@ int make_map_sw128(CUtensorMap* map, const void* base, int rank, const uint64_t*
 int smallm_max_rows();
 constexpr int kMaxCluster = 8;
 int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count);  // CTAs that share a tile's K, 1..kMaxCluster
+int smallm_splits(int64_t N, int64_t K, int sm_count);  // K ranges of a split through memory: sizes scratch, see there
 // Rows that are not quantised yet: `a` of smallm_gemm is [M, K] of the output type, contiguous, K in whole groups of 128, and the
 // kernel quantises them itself with this floor; M <= smallm_quant_rows(), `sa` and `partial` unused
 struct RawRows {

@@ -1284,10 +1284,8 @@ extern "C" int64_t sglb200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, in
   sglb::DeviceInfo di;
   int sms = 148;
   if (sglb::device_info(&di) == SGLB200_OK) sms = di.sm_count;
-  // up to 128 rows K is added up inside a cluster and the scratch goes unused; the size stays an upper bound of what a split
-  // of that shape may need, so that callers who hold it keep working
-  const int splits = M > sglb::smallm_max_rows() ? sglb::splitk_choice(M, N, K, sms)
-                     : sglb::smallm_cluster(M, N, K, sms) > 1 ? sglb::kMaxCluster : 1;
+  // up to smallm_max_rows() K is added up inside a cluster and the scratch goes unused
+  const int splits = M > sglb::smallm_max_rows() ? sglb::splitk_choice(M, N, K, sms) : sglb::smallm_splits(N, K, sms);
   return splits > 1 ? (int64_t)splits * M * N * (int64_t)sizeof(float) : 0;
 }
 
@@ -1424,8 +1422,15 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm_noalloc(const void* a, const void
                                                        int64_t ldb, int64_t ldc, int64_t sa_stride_m,
                                                        int64_t sa_stride_k, int64_t sb_stride_n, int64_t sb_stride_k,
                                                        int out_dtype, void* stream) {
-  const int64_t need = sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K);
-  if (need > sglb::kStaticWsFloats * (int64_t)sizeof(float)) {
+  int64_t need = sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K);
+  const bool fits = need <= sglb::kStaticWsFloats * (int64_t)sizeof(float);
+  if (!fits && M > sglb::smallm_max_rows()) {
+    // tiles that occupy more than half of the SMs by themselves: cutting K helps, but the call runs well without
+    sglb::DeviceInfo di;
+    const int sms = sglb::device_info(&di) == SGLB200_OK ? di.sm_count : 148;
+    if (((M + sglb::BM - 1) / sglb::BM) * ((N + sglb::BN - 1) / sglb::BN) * 2 > sms) need = 0;
+  }
+  if (!fits && need > 0) {
     return sglb::fail(SGLB200_ERR_WORKSPACE,
                       "M=%lld N=%lld K=%lld needs %lld bytes of split-K scratch; the built-in buffer holds %lld "
                       "(use sglb200_fp8_blockwise_scaled_mm_ws with your own buffer, or sglb200_fp8_blockwise_scaled_mm)",

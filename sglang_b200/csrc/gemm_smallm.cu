@@ -843,6 +843,27 @@ int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count) {
   return best;
 }
 
+// K ranges that fp32 partial sums in memory would be cut into, in units of one k-block of one work item: an item costs its
+// k-blocks plus 3 (fill, store), the kernel that adds the sums 8.  The kernels here add up on the chip and write no such sums; this is
+// what sglb200_fp8_blockwise_scaled_mm_workspace_bytes answers up to smallm_max_rows() and what the built-in buffer's limit is held
+// against.  Callers sized buffers by it and know from it which shapes the no-allocation entry takes, so it stays as it is.
+int smallm_splits(int64_t N, int64_t K, int sm_count) {
+  const int64_t n_tiles = (N + BN - 1) / BN, k_tiles = (K + BK - 1) / BK;
+  constexpr int64_t kItemCost = 3, kReduceCost = 8;
+  int best = 1;
+  int64_t best_cost = ((n_tiles + sm_count - 1) / sm_count) * (k_tiles + kItemCost);
+  for (int64_t s = 2; s <= 32 && s * 2 <= k_tiles; ++s) {
+    const int64_t kb = (k_tiles + s - 1) / s;
+    if ((k_tiles + kb - 1) / kb != s) continue;  // every range must get k-blocks
+    const int64_t cost = ((n_tiles * s + sm_count - 1) / sm_count) * (kb + kItemCost) + kReduceCost;
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = (int)s;
+    }
+  }
+  return best;
+}
+
 // Launches the small-M kernel (arguments already validated by the caller).  `partial` != NULL: the fp32 sums [splits][M][N]
 // go there, *splits_used of them, and the caller converts and moves them itself.
 // With ue8m0 the scale pointers are packed exponent words (sa: word (m, kg) at m * sa_stride_m + kg * sa_stride_k; sb

@@ -235,3 +235,22 @@ def test_host_validation_of_the_multicast_and_few_rows_entries(built_lib):
     assert L.sglb200_set_grouped_few_rows(65) == -1 and L.sglb200_set_grouped_few_rows(-1) == -1
     assert L.sglb200_set_grouped_few_rows(0) == 0 and L.sglb200_get_grouped_few_rows() == 0
     assert L.sglb200_set_grouped_few_rows(before) == 0 and L.sglb200_get_grouped_few_rows() == before == 20
+
+
+@pytest.mark.parametrize("M,N,K,served", [
+    (65, 8192, 8192, True), (128, 8192, 8192, True), (74, 7168, 16384, True), (117, 7168, 18432, True),
+    (103, 5120, 2560, True), (128, 576, 7168, True), (118, 7168, 16384, False), (128, 7168, 16384, False),
+    (240, 5888, 18432, True), (684, 2048, 28672, True), (2978, 512, 28672, True)])
+def test_shapes_the_no_allocation_entry_takes(built_lib, M, N, K, served):
+    """The refusal comes before any pointer is looked at: a served shape gets past it and fails on the NULL operands (or,
+    with scratch, on the missing device).  The sizes lie on both sides of 16 MiB of partial sums, and above 128 rows where
+    a split would be larger than that but the tiles alone occupy the SMs (the answers are those for 148 SMs, which the
+    library assumes without a device)."""
+    from sglang_b200._lib import lib
+    L = lib()
+    if L.sglb200_get_num_sms() not in (0, 148):
+        pytest.skip("sizes chosen for 148 SMs")
+    rc = L.sglb200_fp8_blockwise_scaled_mm_noalloc(None, None, None, None, None, M, N, K, K, K, N, 1, M, K // 128, 1, 0, None)
+    assert (rc != -7) == served and rc != 0
+    if M <= 128:
+        assert (L.sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) <= 16 << 20) == served

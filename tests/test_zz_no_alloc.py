@@ -69,3 +69,21 @@ def test_noalloc_entry_rejects_oversized_scratch_and_runs_large_m():
     assert L.sglb200_fp8_blockwise_scaled_mm_noalloc(*_args(aq, a_s, wq, ws, out), stream) == 0
     torch.cuda.synchronize()
     assert_gemm_close(out, oracle.w8a8_block_fp8_matmul(aq_c, wq_c, as_c, ws_c), "large M through no-alloc entry")
+
+
+@pytest.mark.parametrize("M,N,K", [(100, 8192, 8192), (384, 3968, 28672)])
+def test_noalloc_entry_runs_where_a_split_would_not_fit(M, N, K):
+    """Shapes whose partial sums would need more than the built-in buffer, but which run without them: up to 128 rows K is
+    added up on the chip, above that the tiles alone occupy the SMs.  Same bits as the plain entry."""
+    from sglang_b200._lib import check, lib
+    L = lib()
+    stream = torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(M)
+    aq, wq = (torch.randn(r, K, device="cuda", generator=g).to(torch.float8_e4m3fn) for r in (M, N))
+    a_s, ws = (torch.rand(r, K // 128, device="cuda", generator=g) + 0.5 for r in (M, -(-N // 128)))
+    want, got = (torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    check(L.sglb200_fp8_blockwise_scaled_mm(*_args(aq, a_s, wq, ws, want), stream), "plain entry")
+    check(L.sglb200_fp8_blockwise_scaled_mm_noalloc(*_args(aq, a_s, wq, ws, got), stream), "no-alloc entry")
+    torch.cuda.synchronize()
+    assert L.sglb200_read_device_status() == 0
+    assert torch.isfinite(got).all() and torch.equal(got, want)
