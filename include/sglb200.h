@@ -251,9 +251,12 @@ int sglb200_fp8_blockwise_scaled_mm_pair(const void* a, const void* b, const flo
 int sglb200_fp8_ue8m0_scaled_mm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, void* out,
                                 int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int64_t sfa_ld,
                                 int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype, void* stream);
-/* The same with the scratch argument of sglb200_fp8_blockwise_scaled_mm_ws, which is checked and not needed.  Up to 64 rows
- * both entries run the weight-streaming kernel of sglb200_fp8_blockwise_scaled_mm, which decodes the exponent bytes itself
- * (the scales stay exact powers of two); above that the block-scaling kernel. */
+/* The same with scratch, as sglb200_fp8_blockwise_scaled_mm_ws: where the output tiles alone leave SMs idle, K is cut into
+ * ranges whose fp32 sums go through `workspace` (sglb200_fp8_ue8m0_scaled_mm_scratch_bytes() bytes; 0 = not needed); with
+ * NULL or a smaller workspace the call is exactly the entry above.  Up to 64 rows, and up to 128 where the CTAs of a cluster
+ * share K, both entries run the weight-streaming kernel of sglb200_fp8_blockwise_scaled_mm, which decodes the exponent bytes
+ * itself (the scales stay exact powers of two) and needs no scratch; otherwise the block-scaling kernel. */
+int64_t sglb200_fp8_ue8m0_scaled_mm_scratch_bytes(int64_t M, int64_t N, int64_t K);
 int sglb200_fp8_ue8m0_scaled_mm_ws(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, void* out,
                                    int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int64_t sfa_ld,
                                    int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype, void* workspace,

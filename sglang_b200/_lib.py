@@ -33,6 +33,7 @@ SIGNATURES = {
     "sglb200_fp8_blockwise_scaled_mm_pair": [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L, _I, _I, _P],
     "sglb200_fp8_ue8m0_scaled_mm": [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _I, _P],
     "sglb200_fp8_ue8m0_scaled_mm_ws": [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _I, _P, _L, _P],
+    "sglb200_fp8_ue8m0_scaled_mm_scratch_bytes": [_L, _L, _L],
     "sglb200_fp8_ue8m0_scaled_grouped_mm": [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L,
                                             _I, _P],
     "sglb200_fp8_blockwise_scaled_grouped_mm": [_P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L,
@@ -90,6 +91,7 @@ SIGNATURES = {
 _RESTYPES = {"sglb200_fp8_blockwise_scaled_mm_workspace_bytes": c_int64,
              "sglb200_fp8_blockwise_scaled_mm_noalloc_max_bytes": c_int64,
              "sglb200_fp8_block_linear_scratch_bytes": c_int64,
+             "sglb200_fp8_ue8m0_scaled_mm_scratch_bytes": c_int64,
              "sglb200_fused_experts_scratch_bytes": c_int64, "sglb200_ep_buffer_bytes": c_int64, "sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes": c_int64, "sglb200_peer_flag_bytes": c_int64, "sglb200_nvls_flag_bytes": c_int64, "sglb200_peer_recv_bytes": c_int64, "sglb200_status_string": c_char_p, "sglb200_last_error_detail": c_char_p, "sglb200_version": c_char_p}
 
 _lib = None

@@ -656,7 +656,16 @@ extern "C" int sglb200_fp8_ue8m0_scaled_mm_ws(const void* a, const void* b, cons
   SGLB_REQUIRE(workspace_bytes >= 0 && (workspace == nullptr || sglb::aligned(workspace, 16)), SGLB200_ERR_ALIGN,
                "workspace must be 16-byte aligned");
   return sglb::ue8m0_common(a, b, sfa, sfb, out, nullptr, M, 1, N, K, lda, ldb, 0, ldc, sfa_ld, 1, 0, sfb_stride_n,
-                            sfb_stride_k, out_dtype, stream);
+                            sfb_stride_k, out_dtype, stream, nullptr, static_cast<float*>(workspace),
+                            workspace ? workspace_bytes / (int64_t)sizeof(float) : 0);
+}
+
+extern "C" int64_t sglb200_fp8_ue8m0_scaled_mm_scratch_bytes(int64_t M, int64_t N, int64_t K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  sglb::DeviceInfo di;
+  const int sms = sglb::device_info(&di) == SGLB200_OK ? di.sm_count : 148;
+  const int splits = sglb::ue8m0_splits(M, N, K, sms);
+  return splits > 1 ? (int64_t)splits * M * N * (int64_t)sizeof(float) : 0;
 }
 
 extern "C" int sglb200_fp8_ue8m0_scaled_grouped_mm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb,

@@ -154,3 +154,36 @@ def test_fused_experts_ue8m0_matches_oracle(M, E, topk, H, I):
     from sglang_b200._lib import lib
     assert lib().sglb200_read_device_status() == 0
     assert_gemm_close(out, ref, "fused experts, UE8M0", allow_one_ulp=True)
+
+
+@pytest.mark.parametrize("M,N,K", [(200, 264, 2176), (129, 576, 7168), (385, 1000, 4480), (300, 136, 2064), (113, 7168, 512)])
+def test_matmul_cuts_k_like_the_linear_layer(M, N, K):
+    """Few output tiles: the matmul takes scratch and cuts K as the linear layer does (its bits), also where K ends inside a
+    k-block, which the layer does not take.  The last shape needs no scratch."""
+    from sglang_b200._lib import check, lib
+    from sglang_b200.layers.quantization import pack_ue8m0_scales, w8a8_block_fp8_matmul_ue8m0
+    from sglang_b200.layers.quantization.fp8_utils import w8a8_block_fp8_linear_ue8m0
+    L = lib()
+    g = torch.Generator().manual_seed(M + K)
+    x = torch.randn(M, K, generator=g).bfloat16()
+    wq, ws = oracle.block_quant_weight(torch.randn(N, K, generator=g) * 0.02, scale_ue8m0=True)
+    pad = -K % 128
+    aq, a_s = oracle.per_token_group_quant_fp8(torch.nn.functional.pad(x, (0, pad)), 128, scale_ue8m0=True)
+    aq = aq[:, :K].contiguous()
+    a, w, sw = aq.cuda(), wq.cuda(), pack_ue8m0_scales(ws.cuda())
+    sa = pack_ue8m0_scales(a_s).cuda().t().contiguous().t()  # M-major, as the quantiser writes it
+    got = w8a8_block_fp8_matmul_ue8m0(a, w, sa, sw)
+    assert_gemm_close(got, oracle.w8a8_block_fp8_matmul(aq, wq, a_s, ws), f"{M}x{N}x{K}", allow_one_ulp=True)
+    if pad == 0:
+        assert torch.equal(got, w8a8_block_fp8_linear_ue8m0(x.cuda(), w, sw))
+    need = L.sglb200_fp8_ue8m0_scaled_mm_scratch_bytes(M, N, K)
+    assert (need > 0) == (N < 7168)
+    if need:
+        scratch = torch.full((need // 4,), float("nan"), device="cuda")
+        out = torch.empty_like(got)
+        check(L.sglb200_fp8_ue8m0_scaled_mm_ws(a.data_ptr(), w.data_ptr(), sa.data_ptr(), sw.data_ptr(), out.data_ptr(), M, N, K, K, K,
+                                               N, sa.stride(1), sw.stride(0), sw.stride(1), 0, scratch.data_ptr(), need,
+                                               torch.cuda.current_stream().cuda_stream), "workspace entry")
+        assert torch.equal(out, got) and torch.isfinite(scratch).all(), "every partial sum is written"
+    torch.cuda.synchronize()
+    assert L.sglb200_read_device_status() == 0
