@@ -67,14 +67,17 @@ int sglb200_get_num_sms(void);
  * experts that have rows are streamed.  This is the decode case of a mixture-of-experts layer, where the 128 x 128
  * kernel spends a full tile of tensor-core work (and, with fp32 scales, of promotion) on a handful of rows: no slower
  * in a burst, but sustained that work runs the board into its power cap at half the SM clock.  Default 20, which stands for
- * the library's own measured rule (fp32 scales: up to 48 rows on average; UE8M0 scales: up to 20); any other value is
- * taken as the limit itself, 0 = always the 128 x 128 kernels; at most 64.  With UE8M0 scales the few-rows kernel decodes the exponent bytes and
- * applies the scales in fp32 after each k-block (exact for powers of two).
- * The results of the two kernels are bit-identical (same products, same fp32 accumulation order per k-block).
+ * the library's own measured rule (fp32 scales: up to 48 rows on average; UE8M0 scales: up to 20, and never where K <= 512); any
+ * other value is taken as the limit itself, 0 = always the 128 x 128 kernels; at most 64.  The limit 20 itself is asked for as
+ * 20 | SGLB200_FEW_ROWS_EXACT.  The getter answers what the setter takes, so that a caller can put back what it found.
+ * With UE8M0 scales the few-rows kernel decodes the exponent bytes and applies the scales in fp32 after each k-block (exact
+ * for powers of two).  With fp32 scales the results of the two kernels are bit-identical (same products, same fp32
+ * accumulation order per k-block); with UE8M0 scales an output may differ by one unit in its last place.
  * Process-wide, read at every launch.
  * Replaces: the small-M tile configurations of the reference's grouped kernel,
  *           sgl-kernel/csrc/moe/fp8_blockwise_moe_kernel.cu:440-560 (dispatch on the row count).
  */
+#define SGLB200_FEW_ROWS_EXACT 0x100
 int sglb200_set_grouped_few_rows(int max_avg_rows);
 int sglb200_get_grouped_few_rows(void);
 

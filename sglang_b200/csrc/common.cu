@@ -74,9 +74,11 @@ int sglb200_set_num_sms(int num_sms) {
 }
 
 int sglb200_set_grouped_few_rows(int max_avg_rows) {
-  if (max_avg_rows < 0 || max_avg_rows > 64)
+  const int limit = max_avg_rows & ~SGLB200_FEW_ROWS_EXACT;
+  if (max_avg_rows < 0 || limit > 64)
     return sglb::fail(SGLB200_ERR_SHAPE, "max_avg_rows=%d: 0 (never) .. 64", max_avg_rows);
-  sglb::g_grouped_few_rows_max = max_avg_rows;
+  // the mark is kept only where it says something, so that the getter answers a limit as it was given
+  sglb::g_grouped_few_rows_max = limit == sglb::kGroupedFewRowsDefault ? max_avg_rows : limit;
   return SGLB200_OK;
 }
 

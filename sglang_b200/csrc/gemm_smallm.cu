@@ -958,18 +958,19 @@ constexpr int64_t kWideRowsMax = 48, kWideRowsMaxUe8m0 = 20, kShortKUe8m0 = 512;
 // Rows per chunk of the grouped few-rows kernel for `total_rows` rows spread over `num_experts` experts (or
 // rows_per_expert rows at most per expert in the masked layout); 0 = the 128 x 128 grouped kernel is the better choice.
 int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows, int64_t K, bool ue8m0) {
-  if (g_grouped_few_rows_max == 0) return 0;
+  const int setting = g_grouped_few_rows_max, limit = setting & ~SGLB200_FEW_ROWS_EXACT;
+  if (limit == 0) return 0;
   int64_t avg = (total_rows + num_experts - 1) / num_experts;
   if (rows_per_expert > 0) {  // masked layout: the row bound is known, the rows in use only if the caller expects a number
     if (expected_rows <= 0 || expected_rows > rows_per_expert) {
-      if (rows_per_expert > g_grouped_few_rows_max) return 0;
+      if (rows_per_expert > limit) return 0;
       return rows_per_expert <= 16 ? 16 : (rows_per_expert <= 32 ? 32 : 64);
     }
     avg = expected_rows;
   }
   // the setter's default stands for the rule above; a caller who sets another limit gets exactly that
   const int64_t rule = !ue8m0 ? kWideRowsMax : (K <= kShortKUe8m0 ? 0 : kWideRowsMaxUe8m0);
-  if (avg > (g_grouped_few_rows_max == kGroupedFewRowsDefault ? rule : g_grouped_few_rows_max)) return 0;
+  if (avg > (setting == kGroupedFewRowsDefault ? rule : limit)) return 0;
   return avg <= 8 ? 16 : (avg <= 24 ? 32 : 64);
 }
 
@@ -1034,3 +1035,9 @@ int smallm_grouped_gemm(int chunk, const void* a, const void* b, const float* sa
 }
 
 }  // namespace sglb
+
+// Test hook (not in the public header): the grouped kernel's choice for a call without touching a device.
+extern "C" int sglb200_debug_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows,
+                                           int64_t K, int ue8m0) {
+  return sglb::smallm_grouped_chunk(total_rows, num_experts, rows_per_expert, expected_rows, K, ue8m0 != 0);
+}

@@ -254,3 +254,28 @@ def test_shapes_the_no_allocation_entry_takes(built_lib, M, N, K, served):
     assert (rc != -7) == served and rc != 0
     if M <= 128:
         assert (L.sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) <= 16 << 20) == served
+
+
+def test_few_rows_limit_of_twenty_itself(built_lib):
+    """20 stands for the library's rule; with the mark it is the limit itself, and what the getter answers restores either."""
+    import ctypes
+    from sglang_b200._lib import lib
+    L, exact = lib(), 0x100
+    chunk = L.sglb200_debug_grouped_chunk
+    chunk.argtypes, chunk.restype = [ctypes.c_int64] * 5 + [ctypes.c_int], ctypes.c_int
+    average = lambda rows, k=2048, ue8m0=0: chunk(rows * 64, 64, 0, 0, k, ue8m0)
+    before = L.sglb200_get_grouped_few_rows()
+    try:
+        assert before == 20 and [average(r) for r in (20, 21, 48, 49)] == [32, 32, 64, 0]
+        assert average(20, ue8m0=1) == 32 and average(21, ue8m0=1) == 0
+        assert L.sglb200_set_grouped_few_rows(20 | exact) == 0
+        assert [average(r) for r in (20, 21, 48)] == [32, 0, 0] and average(20, 512, 1) == 32
+        mark = L.sglb200_get_grouped_few_rows()
+        assert L.sglb200_set_grouped_few_rows(30 | exact) == 0 and L.sglb200_get_grouped_few_rows() == 30
+        assert average(30) == 64 and average(31) == 0
+        assert L.sglb200_set_grouped_few_rows(mark) == 0 and average(21) == 0
+        assert L.sglb200_set_grouped_few_rows(65 | exact) == -1 and L.sglb200_set_grouped_few_rows(0x200 | 20) == -1
+        assert L.sglb200_set_grouped_few_rows(0) == 0 and average(1) == 0
+    finally:
+        assert L.sglb200_set_grouped_few_rows(before) == 0
+    assert average(48) == 64
