@@ -67,7 +67,8 @@ int sglb200_get_num_sms(void);
  * experts that have rows are streamed.  This is the decode case of a mixture-of-experts layer, where the 128 x 128
  * kernel spends a full tile of tensor-core work (and, with fp32 scales, of promotion) on a handful of rows: no slower
  * in a burst, but sustained that work runs the board into its power cap at half the SM clock.  Default 20, which stands for
- * the library's own measured rule (fp32 scales: up to 48 rows on average; UE8M0 scales: up to 20, and never where K <= 512); any
+ * the library's own measured rule (fp32 scales: up to 48 rows on average; UE8M0 scales: up to 20, and not
+ * where K <= 512 and there are more than about 1400 pieces of 128 weight rows in the experts that have rows); any
  * other value is taken as the limit itself, 0 = always the 128 x 128 kernels; at most 64.  The limit 20 itself is asked for as
  * 20 | SGLB200_FEW_ROWS_EXACT.  The getter answers what the setter takes, so that a caller can put back what it found.
  * With UE8M0 scales the few-rows kernel decodes the exponent bytes and applies the scales in fp32 after each k-block (exact

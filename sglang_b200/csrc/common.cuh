@@ -58,7 +58,8 @@ int nvls_take_device_status();  // nvls.cu
 constexpr int kGroupedFewRowsDefault = 20;  // stands for the library's rule; the limit 20 itself carries SGLB200_FEW_ROWS_EXACT
 extern int g_grouped_few_rows_max;  // common.cu; as given to sglb200_set_grouped_few_rows
 // The grouped form of the few-rows kernel (one weight matrix per expert, few rows per expert); chunk 0 = do not use it
-int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows, int64_t K, bool ue8m0);
+int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows, int64_t N, int64_t K,
+                         bool ue8m0);
 int smallm_grouped_gemm(int chunk, const void* a, const void* b, const float* sa, const float* sb, void* out,
                         const int32_t* expert_offsets, const int32_t* problem_sizes, int count_stride, int64_t total_rows,
                         int64_t num_experts, int64_t rows_per_expert, int64_t N, int64_t K, int64_t lda, int64_t ldb,

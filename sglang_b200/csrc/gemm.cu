@@ -1143,7 +1143,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
 
   if (grouped && !push) {
     // few rows per expert: the weight-streaming kernel with swapped operands (gemm_smallm.cu)
-    if (const int chunk = smallm_grouped_chunk(total_rows, num_experts, rows_per_expert, expected_rows, K, false))
+    if (const int chunk = smallm_grouped_chunk(total_rows, num_experts, rows_per_expert, expected_rows, N, K, false))
       return smallm_grouped_gemm(chunk, a, b, sa, sb, out, expert_offsets, problem_sizes, rows_per_expert > 0 ? 1 : 3,
                                  total_rows, num_experts, rows_per_expert, N, K, lda, ldb, ldb_e, ldc, sa_stride_e,
                                  sa_stride_m, sa_stride_k, sb_stride_e, sb_stride_n, sb_stride_k, out_dtype, di.sm_count,

@@ -31,6 +31,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <cmath>
 #include <type_traits>
 
 #include "common.cuh"
@@ -951,13 +952,24 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
 // 896 against 920 us at 64 rows, 1327 against 1410 at 128); at 32 rows the chunks win (875 against 689 us).  The UE8M0 tile
 // kernel has no promotion to pay for and draws level much earlier (whole layer at 32 rows: 1940 us it, 1990 the chunks).
 // With a K of a few k-blocks an item is mostly start and store, of which the UE8M0 tile kernel has less (its epilogue overlaps the
-// next tile): the layer of 256 experts, 7168 columns, K=256 in the second GEMM takes 131 / 242 / 296 us with the chunks at 16 / 128 /
-// 256 tokens, 123 / 216 / 246 without.  The fp32 tile kernel gains nothing from that (325 against 376 us at 256 tokens).
+// next tile), once there are enough items for that to outweigh its later start (it is launched without programmatic overlap).
+// Measured on 11 layers of 8 to 256 experts and 2048 to 7168 columns, K = 128 to 512, 0.5 to 20 rows per expert: with up to 1400
+// items (128 weight rows of an expert that has rows) the chunks take 0.67 to 1.05 of the tile kernel's time (64 x 2048 x 256 at 4
+// rows: 12.3 against 14.4 us), with more 0.95 to 1.48 (256 x 7168 x 256 at 1 / 16 rows: 94 / 164 against 74 / 114 us).  K = 1024
+// still gives 1.0 to 1.12 there and K = 2048 0.94 to 1.02.  The fp32 tile kernel gains nothing from a short K (layer of 256 x 7168 x 256 at
+// 256 tokens: 325 against 376 us).
 constexpr int64_t kWideRowsMax = 48, kWideRowsMaxUe8m0 = 20, kShortKUe8m0 = 512;
+constexpr double kShortKItems = 1400.;
+
+// Work items of one chunk per expert that `rows` rows routed evenly at random make.
+double routed_items(int64_t rows, int64_t num_experts, int64_t N) {
+  return -std::expm1(-(double)rows / (double)num_experts) * (double)num_experts * (double)((N + BN - 1) / BN);
+}
 
 // Rows per chunk of the grouped few-rows kernel for `total_rows` rows spread over `num_experts` experts (or
 // rows_per_expert rows at most per expert in the masked layout); 0 = the 128 x 128 grouped kernel is the better choice.
-int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows, int64_t K, bool ue8m0) {
+int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows, int64_t N, int64_t K,
+                         bool ue8m0) {
   const int setting = g_grouped_few_rows_max, limit = setting & ~SGLB200_FEW_ROWS_EXACT;
   if (limit == 0) return 0;
   int64_t avg = (total_rows + num_experts - 1) / num_experts;
@@ -969,7 +981,8 @@ int smallm_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_p
     avg = expected_rows;
   }
   // the setter's default stands for the rule above; a caller who sets another limit gets exactly that
-  const int64_t rule = !ue8m0 ? kWideRowsMax : (K <= kShortKUe8m0 ? 0 : kWideRowsMaxUe8m0);
+  const bool short_k = ue8m0 && K <= kShortKUe8m0 && routed_items(total_rows, num_experts, N) > kShortKItems;
+  const int64_t rule = !ue8m0 ? kWideRowsMax : (short_k ? 0 : kWideRowsMaxUe8m0);
   if (avg > (setting == kGroupedFewRowsDefault ? rule : limit)) return 0;
   return avg <= 8 ? 16 : (avg <= 24 ? 32 : 64);
 }
@@ -1038,6 +1051,6 @@ int smallm_grouped_gemm(int chunk, const void* a, const void* b, const float* sa
 
 // Test hook (not in the public header): the grouped kernel's choice for a call without touching a device.
 extern "C" int sglb200_debug_grouped_chunk(int64_t total_rows, int64_t num_experts, int64_t rows_per_expert, int64_t expected_rows,
-                                           int64_t K, int ue8m0) {
-  return sglb::smallm_grouped_chunk(total_rows, num_experts, rows_per_expert, expected_rows, K, ue8m0 != 0);
+                                           int64_t N, int64_t K, int ue8m0) {
+  return sglb::smallm_grouped_chunk(total_rows, num_experts, rows_per_expert, expected_rows, N, K, ue8m0 != 0);
 }

@@ -262,8 +262,8 @@ def test_few_rows_limit_of_twenty_itself(built_lib):
     from sglang_b200._lib import lib
     L, exact = lib(), 0x100
     chunk = L.sglb200_debug_grouped_chunk
-    chunk.argtypes, chunk.restype = [ctypes.c_int64] * 5 + [ctypes.c_int], ctypes.c_int
-    average = lambda rows, k=2048, ue8m0=0: chunk(rows * 64, 64, 0, 0, k, ue8m0)
+    chunk.argtypes, chunk.restype = [ctypes.c_int64] * 6 + [ctypes.c_int], ctypes.c_int
+    average = lambda rows, k=2048, ue8m0=0: chunk(rows * 64, 64, 0, 0, 7168, k, ue8m0)
     before = L.sglb200_get_grouped_few_rows()
     try:
         assert before == 20 and [average(r) for r in (20, 21, 48, 49)] == [32, 32, 64, 0]
@@ -279,3 +279,15 @@ def test_few_rows_limit_of_twenty_itself(built_lib):
     finally:
         assert L.sglb200_set_grouped_few_rows(before) == 0
     assert average(48) == 64
+
+
+@pytest.mark.parametrize("rows,experts,n,k,chunk", [
+    (64, 64, 2048, 256, 16), (1280, 64, 2048, 512, 32), (32, 32, 7168, 512, 16), (128, 32, 7168, 128, 0),
+    (256, 256, 7168, 256, 0), (5120, 256, 7168, 512, 0), (256, 256, 7168, 640, 16), (5120, 256, 7168, 2048, 32), (1, 256, 7168, 128, 16)])
+def test_short_k_leaves_the_few_rows_kernel_only_in_large_layers(built_lib, rows, experts, n, k, chunk):
+    """UE8M0 grouped GEMM with K of at most 512: small layers stay with the few-rows kernel, on both sides of the bound."""
+    import ctypes
+    from sglang_b200._lib import lib
+    fn = lib().sglb200_debug_grouped_chunk
+    fn.argtypes, fn.restype = [ctypes.c_int64] * 6 + [ctypes.c_int], ctypes.c_int
+    assert fn(rows, experts, 0, 0, n, k, 1) == chunk
