@@ -168,12 +168,14 @@ int sglb200_fp8_blockwise_scaled_mm(const void* a, const void* b, const float* s
  * partial sums to `workspace` ([splits, M, N] floats) and a second small kernel adds them in ascending split order and
  * casts; up to 128 rows the CTAs of a cluster share a tile's K and add up on the chip, with or without `workspace`.
  * sglb200_fp8_blockwise_scaled_mm_workspace_bytes() returns a sufficient size for a shape on the current device (0 = K is
- * not cut; up to 128 rows the size of a split through memory, which this kernel does without); with workspace == NULL or a workspace that is too small the call is exactly sglb200_fp8_blockwise_scaled_mm.
+ * not cut; up to 128 rows the size of a split through memory, which this kernel does without).
+ * sglb200_fp8_blockwise_scaled_mm_scratch_bytes() returns what the call really makes use of (0 = a workspace changes nothing).  With workspace == NULL or a workspace that is too small the call is exactly sglb200_fp8_blockwise_scaled_mm.
  * The workspace is scratch: contents on entry are ignored, calls on the same stream may share it.  Replaces the per-call
  * cudaMalloc'ed CUTLASS workspace of the reference (sgl-kernel/csrc/gemm/fp8_blockwise_gemm_kernel.cu:162-163) and its
  * stream-K path (sgl-kernel/csrc/cutlass_extensions/gemm/fp8_blockwise_gemm_sm90_dispatch.cuh:179-197).
  */
 int64_t sglb200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, int64_t N, int64_t K);
+int64_t sglb200_fp8_blockwise_scaled_mm_scratch_bytes(int64_t M, int64_t N, int64_t K);
 int sglb200_fp8_blockwise_scaled_mm_ws(const void* a, const void* b, const float* sa, const float* sb, void* out,
                                        int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc,
                                        int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n,

@@ -26,6 +26,7 @@ SIGNATURES = {
     "sglb200_fp8_blockwise_scaled_mm": [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L, _I, _P],
     "sglb200_fp8_blockwise_scaled_mm_ws": [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L, _I, _P, _L, _P],
     "sglb200_fp8_blockwise_scaled_mm_workspace_bytes": [_L, _L, _L],
+    "sglb200_fp8_blockwise_scaled_mm_scratch_bytes": [_L, _L, _L],
     "sglb200_fp8_blockwise_scaled_mm_noalloc": [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _L, _I, _P],
     "sglb200_fp8_blockwise_scaled_mm_noalloc_max_bytes": [],
     "sglb200_fp8_block_linear": [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _I, _F, _I, _P, _L, _P],
@@ -89,6 +90,7 @@ SIGNATURES = {
                                                   _L, _L, _L, _L, _L, _I, _P],
 }
 _RESTYPES = {"sglb200_fp8_blockwise_scaled_mm_workspace_bytes": c_int64,
+             "sglb200_fp8_blockwise_scaled_mm_scratch_bytes": c_int64,
              "sglb200_fp8_blockwise_scaled_mm_noalloc_max_bytes": c_int64,
              "sglb200_fp8_block_linear_scratch_bytes": c_int64,
              "sglb200_fp8_ue8m0_scaled_mm_scratch_bytes": c_int64,
@@ -146,11 +148,10 @@ def check(status: int, what: str) -> None:
 def blockwise_mm(a_ptr, b_ptr, sa_ptr, sb_ptr, out_ptr, M, N, K, lda, ldb, ldc, sa_m, sa_k, sb_n, sb_k, out_code, device,
                  stream) -> None:
     """One dense block-scaled GEMM launch; picks the split-K entry with a torch-allocated scratch buffer when the
-    library asks for one (more than 128 rows but few output tiles), else the plain entry."""
+    library makes use of one (few output tiles, K not added up on the chip), else the plain entry."""
     import torch
     L = lib()
-    # up to 128 rows the kernel adds its K ranges up on the chip
-    ws_bytes = L.sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) if M > 128 else 0
+    ws_bytes = L.sglb200_fp8_blockwise_scaled_mm_scratch_bytes(M, N, K)
     if ws_bytes > 0:
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=device)
         check(L.sglb200_fp8_blockwise_scaled_mm_ws(a_ptr, b_ptr, sa_ptr, sb_ptr, out_ptr, M, N, K, lda, ldb, ldc, sa_m,

@@ -1067,6 +1067,11 @@ int splitk_choice(int64_t M, int64_t N, int64_t K, int sm_count) {
   return best;
 }
 
+// K ranges whose sums a dense call puts into its scratch; up to smallm_max_rows() K is added up on the chip
+int dense_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
+  return M > smallm_max_rows() ? splitk_choice(M, N, K, sm_count) : 1;
+}
+
 template <bool GROUPED, bool PUSH>
 int set_smem_attr_once() {
   static bool done[64] = {false};
@@ -1192,7 +1197,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
   p.kb_per_split = p.k_tiles;
   if (push) p.push = *push;
   if (!grouped && workspace != nullptr && !push) {
-    const int splits = splitk_choice(total_rows, N, K, di.sm_count);
+    const int splits = dense_splits(total_rows, N, K, di.sm_count);
     if (splits > 1 && (int64_t)splits * total_rows * N <= workspace_floats) {
       p.partial = workspace;
       p.kb_per_split = (p.k_tiles + splits - 1) / splits;
@@ -1289,6 +1294,14 @@ extern "C" int64_t sglb200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, in
   return splits > 1 ? (int64_t)splits * M * N * (int64_t)sizeof(float) : 0;
 }
 
+extern "C" int64_t sglb200_fp8_blockwise_scaled_mm_scratch_bytes(int64_t M, int64_t N, int64_t K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  sglb::DeviceInfo di;
+  const int sms = sglb::device_info(&di) == SGLB200_OK ? di.sm_count : 148;
+  const int splits = sglb::dense_splits(M, N, K, sms);
+  return splits > 1 ? (int64_t)splits * M * N * (int64_t)sizeof(float) : 0;
+}
+
 extern "C" int sglb200_fp8_blockwise_scaled_mm_ws(const void* a, const void* b, const float* sa, const float* sb,
                                                   void* out, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
                                                   int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k,
@@ -1312,7 +1325,7 @@ struct LinearScratch {
 };
 LinearScratch linear_scratch(int64_t M, int64_t N, int64_t K, bool ue8m0, int sms) {
   LinearScratch l;
-  const int splits = ue8m0 ? ue8m0_splits(M, N, K, sms) : (M > smallm_max_rows() ? splitk_choice(M, N, K, sms) : 1);
+  const int splits = ue8m0 ? ue8m0_splits(M, N, K, sms) : dense_splits(M, N, K, sms);
   l.gemm_bytes = splits > 1 ? (int64_t)splits * M * N * (int64_t)sizeof(float) : 0;
   l.ld = (M + 3) / 4 * 4;
   const int64_t words = ue8m0 ? (K / 128 + 3) / 4 : K / 128;

@@ -51,8 +51,7 @@ torch::Tensor fp8_blockwise_scaled_mm(const torch::Tensor& mat_a, const torch::T
   if (M == 0 || N == 0) return out;
   const int64_t lda = M > 1 ? mat_a.stride(0) : std::max<int64_t>(mat_a.stride(0), K);
   const int64_t ldb = N > 1 ? mat_b.stride(1) : std::max<int64_t>(mat_b.stride(1), K);
-  // up to 128 rows the kernel adds its K ranges up on the chip
-  const int64_t ws_bytes = M > 128 ? sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) : 0;
+  const int64_t ws_bytes = sglb200_fp8_blockwise_scaled_mm_scratch_bytes(M, N, K);
   if (ws_bytes > 0) {  // few output tiles: split-K scratch from torch's caching allocator
     auto ws = torch::empty({ws_bytes}, mat_a.options().dtype(at::kByte));
     check_rc(sglb200_fp8_blockwise_scaled_mm_ws(mat_a.data_ptr(), mat_b.data_ptr(), scales_a.data_ptr<float>(),

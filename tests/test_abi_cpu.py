@@ -291,3 +291,17 @@ def test_short_k_leaves_the_few_rows_kernel_only_in_large_layers(built_lib, rows
     fn = lib().sglb200_debug_grouped_chunk
     fn.argtypes, fn.restype = [ctypes.c_int64] * 6 + [ctypes.c_int], ctypes.c_int
     assert fn(rows, experts, 0, 0, n, k, 1) == chunk
+
+
+@pytest.mark.parametrize("M,N,K,ranges", [(1, 576, 7168, 0), (128, 576, 7168, 0), (128, 7168, 16384, 0), (129, 576, 7168, 8),
+                                          (4096, 7168, 16384, 0)])
+def test_scratch_that_a_dense_call_uses(built_lib, M, N, K, ranges):
+    """What the wrappers allocate: nothing where K is added up on the chip or not cut, else one fp32 output per range.  The
+    linear layer's scratch holds the same."""
+    from sglang_b200._lib import lib
+    L = lib()
+    used = L.sglb200_fp8_blockwise_scaled_mm_scratch_bytes(M, N, K)
+    assert used == ranges * M * N * 4 and used <= L.sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K)
+    if M > 2:
+        rest = (K // 128) * (-(-M // 4) * 4) * 4 + M * K
+        assert used + rest <= L.sglb200_fp8_block_linear_scratch_bytes(M, N, K, 0) <= used + rest + 1024
