@@ -662,13 +662,15 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         for (int32_t kb = kb0; kb < kb1; ++kb) {
           if constexpr (MT == 16 && NSUB == 1) {
             // Both waits at once, one half of the warp each: with 16 columns a k-block costs this warp little else (N=10240 K=8192
-            // M=1 18.1 -> 16.1 us a call, N=24576 K=1536 M=16 10.2 -> 9.8); with more it gained nothing.
+            // M=1 18.1 -> 16.1 us a call, N=24576 K=1536 M=16 10.2 -> 9.8); with more it gained nothing.  The vote does not order
+            // memory, and the issuing lane has seen only one of the two barriers: the warp barrier passes on what the others saw.
             const bool op = (lane & 1) != 0;
             if (!__all_sync(0xffffffffu, ptx::mbar_wait_inl_a(op ? full0 + stage * 8 : acc_empty0 + acc * 8, op ? phase : acc_phase ^ 1))) {
               timeout(ctl, 12);
               ok = false;
               break;
             }
+            __syncwarp();
           } else {
             if (!ptx::mbar_wait_inl_a(acc_empty0 + acc * 8, acc_phase ^ 1)) { timeout(ctl, 12); ok = false; break; }
             if (!ptx::mbar_wait_inl_a(full0 + stage * 8, phase)) { timeout(ctl, 13); ok = false; break; }
