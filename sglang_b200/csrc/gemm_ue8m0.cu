@@ -265,6 +265,7 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   if (warp < 2) {
     // ===== TMA producers
     uint32_t stage = 0, phase = 0, g = 0;
+    uint32_t armed = 0, armed_phase = 0;  // bit i: this warp has armed stage i / the phase bit of its last arming
     for (int32_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
       const TileUe tl = tile_coords<GROUPED, SPLIT>(p, tile_start, t);
       bool ok = true;
@@ -276,6 +277,8 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             ok = false;
             break;
           }
+          armed |= 1u << stage;
+          armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
           if (leader) {
             const uint32_t dst = stage0 + stage * kStageBytes;
             ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, kStageBytes);
@@ -286,6 +289,12 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
       if (!ok || ctl->abort_flag) break;
+    }
+    // After a time-out somewhere in the CTA: a CTA must not exit while bulk copies into its shared memory are in flight, so
+    // each producer waits (20 ms at most per stage) for the loads it issued.
+    if (ctl->abort_flag) {
+      for (uint32_t i = 0; i < (uint32_t)kStages; ++i)
+        if (armed & (1u << i)) ptx::mbar_wait_a(full0 + i * 8, (armed_phase >> i) & 1u, 20000000ull);
     }
     // Tail: tcgen05.commit arrives on the `empty` barriers asynchronously.  Nobody waits for the last ones, so
     // without this the CTA could exit (and the next kernel's CTA re-initialise barriers at the same shared-memory
