@@ -186,6 +186,7 @@ PyObject* topk_softmax(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (!lp || !PyLong_Check(args[1])) Py_RETURN_NONE;
   const at::Tensor& x = *lp;
   const int64_t topk = PyLong_AsLong(args[1]);
+  if (PyErr_Occurred()) return nullptr;
   const at::ScalarType t = x.scalar_type();
   if (!x.is_cuda() || x.dim() != 2 || !x.is_contiguous() || !(is16(t) || t == at::kFloat) || x.numel() == 0) Py_RETURN_NONE;
   if (topk < 1 || topk > x.size(1)) Py_RETURN_NONE;
@@ -267,6 +268,7 @@ PyObject* grouped_masked(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const at::Tensor &a = *t[0], &as = *t[1], &w = *t[2], &ws = *t[3], &out = *t[4], &mm = *t[5];
   if (!PyLong_Check(args[6])) Py_RETURN_NONE;
   const int64_t expected = PyLong_AsLong(args[6]);
+  if (PyErr_Occurred()) return nullptr;
   if (!a.is_cuda() || a.dim() != 3 || w.dim() != 3 || a.scalar_type() != at::kFloat8_e4m3fn || w.scalar_type() != at::kFloat8_e4m3fn ||
       !a.is_contiguous() || w.stride(2) != 1)
     Py_RETURN_NONE;

@@ -112,8 +112,9 @@ class Fp8LinearMethod:
 
     def apply(self, layer: Module, x: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``Fp8LinearMethod.apply`` (``fp8.py:453-499``, block-quant branch ``:482-489``)."""
-        # Module.__getattr__ costs about a microsecond per parameter; the parameter table is a plain attribute
-        params = layer._parameters
+        # Module.__getattr__ costs about a microsecond per parameter; the parameter table is a plain attribute, which a
+        # layer object that is no Module does not have
+        params = getattr(layer, "_parameters", {})
         weight = params.get("weight")
         if weight is None:
             weight = layer.weight

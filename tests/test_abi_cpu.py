@@ -305,3 +305,24 @@ def test_scratch_that_a_dense_call_uses(built_lib, M, N, K, ranges):
     if M > 2:
         rest = (K // 128) * (-(-M // 4) * 4) * 4 + M * K
         assert used + rest <= L.sglb200_fp8_block_linear_scratch_bytes(M, N, K, 0) <= used + rest + 1024
+
+
+def test_host_path_reports_integers_out_of_range(built_lib):
+    """An integer argument that does not fit is an OverflowError, raised before anything is launched, and leaves no pending
+    exception behind."""
+    from sglang_b200._lib import host
+    t = torch.zeros(2, 4)
+    with pytest.raises(OverflowError):
+        host().topk_softmax(t, 1 << 80, True)
+    with pytest.raises(OverflowError):
+        host().grouped_masked(t, t, t, t, t, t, 1 << 80)
+    assert host().topk_softmax(t, 1, True) is None  # a CPU tensor: left to the Python route
+
+
+def test_linear_method_takes_a_layer_that_is_no_module(built_lib):
+    """Only ``weight`` and ``weight_scale_inv`` are asked of the layer; CPU tensors are then refused by the op itself."""
+    from types import SimpleNamespace
+    from sglang_b200.layers.quantization.fp8 import Fp8Config, Fp8LinearMethod
+    layer = SimpleNamespace(weight=torch.zeros(128, 128).to(torch.float8_e4m3fn), weight_scale_inv=torch.ones(1, 1))
+    with pytest.raises(RuntimeError, match="CUDA tensor"):
+        Fp8LinearMethod(Fp8Config()).apply(layer, torch.zeros(2, 128, dtype=torch.bfloat16))
