@@ -36,8 +36,15 @@ PyObject* raise(const LibraryError& e) {
   return nullptr;
 }
 
+// The tensor behind `o`, or NULL where its sizes or its memory cannot simply be asked for (sparse and nested tensors, symbolic
+// sizes, tracing subclasses): those are left to the Python route.
 inline const at::Tensor* tensor_or_null(PyObject* o) {
-  return THPVariable_CheckExact(o) || THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
+  if (!THPVariable_CheckExact(o) && !THPVariable_Check(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  if (!t.defined() || t.layout() != at::kStrided || t.is_nested() || t.key_set().has(c10::DispatchKey::Python) ||
+      t.unsafeGetTensorImpl()->has_symbolic_sizes_strides())
+    return nullptr;
+  return &t;
 }
 
 inline int64_t up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
@@ -56,12 +63,14 @@ inline at::Tensor empty(at::IntArrayRef sizes, at::ScalarType t, c10::Device dev
   return at::Tensor(at::detail::empty_cuda(sizes, t, dev, c10::nullopt));
 }
 
-// Runs `f`; what it throws becomes the Python exception that torch or the Python route would raise.
-template <typename F>
-PyObject* guarded(F&& f) {
+using Function = PyObject*(PyObject* const* args, Py_ssize_t n);
+
+// The C entry of `f`, checks included: what it throws becomes the Python exception that torch or the Python route would raise.
+template <Function* f>
+PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   try {
-    return f();
+    return f(args, n);
   } catch (const LibraryError& e) {
     return raise(e);
   }
@@ -70,7 +79,7 @@ PyObject* guarded(F&& f) {
 
 // ---------------------------------------------------------------------------------------------- quantiser
 // quant(x, group_size, eps, fp8_min, fp8_max, column_major, tma_aligned, ue8m0, fuse_silu, masked_m) -> (codes, scales)
-PyObject* quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* quant(PyObject* const* args, Py_ssize_t n) {
   if (n != 10) Py_RETURN_NONE;
   const at::Tensor* xp = tensor_or_null(args[0]);
   const at::Tensor* mp = args[9] == Py_None ? nullptr : tensor_or_null(args[9]);
@@ -96,50 +105,48 @@ PyObject* quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (dim != 3 || !mp->is_cuda() || mp->scalar_type() != at::kInt || !mp->is_contiguous() || mp->numel() != E) Py_RETURN_NONE;
     mptr = mp->const_data_ptr<int32_t>();
   }
-  return guarded([&]() -> PyObject* {
-    const c10::Device dev = x.device();
-    const c10::cuda::OptionalCUDAGuard guard(dev);
-    void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    const int64_t W = ue ? (G + 3) / 4 : G;                       // scale words per row
-    const int64_t ld = col ? (tma ? up(M, 4) : M) : W;            // stride between word columns (or rows)
-    const at::ScalarType st = ue ? at::kInt : at::kFloat;
-    at::Tensor q, s;
-    if (dim == 2) {
-      q = empty({M, hidden}, at::kFloat8_e4m3fn, dev);
-      s = col ? empty({W, ld}, st, dev) : empty({M, W}, st, dev);
-      if (col) s.unsafeGetTensorImpl()->set_sizes_and_strides(at::IntArrayRef({M, W}), at::IntArrayRef({1, ld}));
-    } else {
-      q = empty({E, M, hidden}, at::kFloat8_e4m3fn, dev);
-      s = col ? empty({E, W, ld}, st, dev) : empty({E, M, W}, st, dev);
-      if (col) s.unsafeGetTensorImpl()->set_sizes_and_strides(at::IntArrayRef({E, M, W}), at::IntArrayRef({W * ld, 1, ld}));
-    }
-    const int code = t == at::kFloat ? SGLB200_F32 : code16(t);
-    const float e = eps_in_dtype(eps, t);
-    if (dim == 3)
-      check_rc(sglb200_group_quant_fp8_batched(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), E, M, hidden,
-                                               (int)gs, e, (float)lo, (float)hi, ue, silu, mptr, s.stride(0), s.stride(1),
-                                               s.stride(2), stream),
-               "sgl_per_token_group_quant_8bit(masked)");
-    else if (silu)
-      check_rc(sglb200_silu_mul_group_quant_fp8(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), nullptr, M,
-                                                hidden, (int)gs, e, (float)lo, (float)hi, ue, s.stride(0), s.stride(1), stream),
-               "sgl_per_token_group_quant_8bit(fuse_silu_and_mul)");
-    else
-      check_rc(sglb200_per_token_group_quant_fp8(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), M, hidden,
-                                                 (int)gs, e, (float)lo, (float)hi, ue, s.stride(0), s.stride(1), stream),
-               "sgl_per_token_group_quant_8bit");
-    PyObject* out = PyTuple_New(2);
-    if (!out) return nullptr;
-    PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(q)));
-    PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(std::move(s)));
-    return out;
-  });
+  const c10::Device dev = x.device();
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const int64_t W = ue ? (G + 3) / 4 : G;                       // scale words per row
+  const int64_t ld = col ? (tma ? up(M, 4) : M) : W;            // stride between word columns (or rows)
+  const at::ScalarType st = ue ? at::kInt : at::kFloat;
+  at::Tensor q, s;
+  if (dim == 2) {
+    q = empty({M, hidden}, at::kFloat8_e4m3fn, dev);
+    s = col ? empty({W, ld}, st, dev) : empty({M, W}, st, dev);
+    if (col) s.unsafeGetTensorImpl()->set_sizes_and_strides(at::IntArrayRef({M, W}), at::IntArrayRef({1, ld}));
+  } else {
+    q = empty({E, M, hidden}, at::kFloat8_e4m3fn, dev);
+    s = col ? empty({E, W, ld}, st, dev) : empty({E, M, W}, st, dev);
+    if (col) s.unsafeGetTensorImpl()->set_sizes_and_strides(at::IntArrayRef({E, M, W}), at::IntArrayRef({W * ld, 1, ld}));
+  }
+  const int code = t == at::kFloat ? SGLB200_F32 : code16(t);
+  const float e = eps_in_dtype(eps, t);
+  if (dim == 3)
+    check_rc(sglb200_group_quant_fp8_batched(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), E, M, hidden,
+                                             (int)gs, e, (float)lo, (float)hi, ue, silu, mptr, s.stride(0), s.stride(1),
+                                             s.stride(2), stream),
+             "sgl_per_token_group_quant_8bit(masked)");
+  else if (silu)
+    check_rc(sglb200_silu_mul_group_quant_fp8(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), nullptr, M,
+                                              hidden, (int)gs, e, (float)lo, (float)hi, ue, s.stride(0), s.stride(1), stream),
+             "sgl_per_token_group_quant_8bit(fuse_silu_and_mul)");
+  else
+    check_rc(sglb200_per_token_group_quant_fp8(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), M, hidden,
+                                               (int)gs, e, (float)lo, (float)hi, ue, s.stride(0), s.stride(1), stream),
+             "sgl_per_token_group_quant_8bit");
+  PyObject* out = PyTuple_New(2);
+  if (!out) return nullptr;
+  PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(q)));
+  PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(std::move(s)));
+  return out;
 }
 
 // ---------------------------------------------------------------------------------------------- linear layer
 // block_linear(x, weight, weight_scale, bias, ue8m0) -> out: quantise the activations, multiply, add the bias.
 // weight_scale is fp32 [ceil(N/128), K/128], or with ue8m0 the packed int32 words [ceil(N/128), ceil(K/512)].
-PyObject* block_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* block_linear(PyObject* const* args, Py_ssize_t n) {
   if (n != 5) Py_RETURN_NONE;
   const at::Tensor *xp = tensor_or_null(args[0]), *wp = tensor_or_null(args[1]), *sp = tensor_or_null(args[2]);
   const at::Tensor* bp = args[3] == Py_None ? nullptr : tensor_or_null(args[3]);
@@ -159,28 +166,26 @@ PyObject* block_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
              bp->dim() != 1 || bp->size(0) != N || bp->stride(0) != 1 || reinterpret_cast<uintptr_t>(bp->const_data_ptr()) % 16 != 0))
     Py_RETURN_NONE;
   const int64_t M = x.numel() / K;
-  return guarded([&]() -> PyObject* {
-    const c10::Device dev = x.device();
-    const c10::cuda::OptionalCUDAGuard guard(dev);
-    const c10::cuda::CUDAStream cs = c10::cuda::getCurrentCUDAStream(dev.index());
-    void* stream = cs.stream();
-    at::DimVector shape(x.sizes().begin(), x.sizes().end());
-    shape[dim - 1] = N;
-    at::Tensor out = empty(shape, t, dev);
-    const int64_t bytes = sglb200_fp8_block_linear_scratch_bytes(M, N, K, ue);
-    c10::DataPtr scratch;
-    if (bytes > 0) scratch = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)bytes);
-    check_rc(sglb200_fp8_block_linear(x.const_data_ptr(), w.const_data_ptr(), ws.const_data_ptr(),
-                                      bp ? bp->const_data_ptr() : nullptr, out.mutable_data_ptr(), M, N, K, ws.stride(0),
-                                      ws.stride(1), ue, eps_in_dtype(1e-10, t), code16(t), scratch.get(), bytes, stream),
-             "fp8_block_linear");
-    return THPVariable_Wrap(std::move(out));
-  });
+  const c10::Device dev = x.device();
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  const c10::cuda::CUDAStream cs = c10::cuda::getCurrentCUDAStream(dev.index());
+  void* stream = cs.stream();
+  at::DimVector shape(x.sizes().begin(), x.sizes().end());
+  shape[dim - 1] = N;
+  at::Tensor out = empty(shape, t, dev);
+  const int64_t bytes = sglb200_fp8_block_linear_scratch_bytes(M, N, K, ue);
+  c10::DataPtr scratch;
+  if (bytes > 0) scratch = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)bytes);
+  check_rc(sglb200_fp8_block_linear(x.const_data_ptr(), w.const_data_ptr(), ws.const_data_ptr(),
+                                    bp ? bp->const_data_ptr() : nullptr, out.mutable_data_ptr(), M, N, K, ws.stride(0),
+                                    ws.stride(1), ue, eps_in_dtype(1e-10, t), code16(t), scratch.get(), bytes, stream),
+           "fp8_block_linear");
+  return THPVariable_Wrap(std::move(out));
 }
 
 // ---------------------------------------------------------------------------------------------- router
 // topk_softmax(logits, topk, renormalize) -> (weights, ids)
-PyObject* topk_softmax(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* topk_softmax(PyObject* const* args, Py_ssize_t n) {
   if (n != 3) Py_RETURN_NONE;
   const at::Tensor* lp = tensor_or_null(args[0]);
   if (!lp || !PyLong_Check(args[1])) Py_RETURN_NONE;
@@ -191,26 +196,24 @@ PyObject* topk_softmax(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (!x.is_cuda() || x.dim() != 2 || !x.is_contiguous() || !(is16(t) || t == at::kFloat) || x.numel() == 0) Py_RETURN_NONE;
   if (topk < 1 || topk > x.size(1)) Py_RETURN_NONE;
   const bool renorm = PyObject_IsTrue(args[2]) == 1;
-  return guarded([&]() -> PyObject* {
-    const c10::Device dev = x.device();
-    const c10::cuda::OptionalCUDAGuard guard(dev);
-    void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    const int64_t M = x.size(0);
-    at::Tensor w = empty({M, topk}, at::kFloat, dev), ids = empty({M, topk}, at::kInt, dev);
-    check_rc(sglb200_topk_softmax(x.const_data_ptr(), t == at::kFloat ? SGLB200_F32 : code16(t), w.mutable_data_ptr<float>(),
-                                  ids.mutable_data_ptr<int32_t>(), M, x.size(1), topk, renorm, stream),
-             "topk_softmax");
-    PyObject* out = PyTuple_New(2);
-    if (!out) return nullptr;
-    PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(w)));
-    PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(std::move(ids)));
-    return out;
-  });
+  const c10::Device dev = x.device();
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const int64_t M = x.size(0);
+  at::Tensor w = empty({M, topk}, at::kFloat, dev), ids = empty({M, topk}, at::kInt, dev);
+  check_rc(sglb200_topk_softmax(x.const_data_ptr(), t == at::kFloat ? SGLB200_F32 : code16(t), w.mutable_data_ptr<float>(),
+                                ids.mutable_data_ptr<int32_t>(), M, x.size(1), topk, renorm, stream),
+           "topk_softmax");
+  PyObject* out = PyTuple_New(2);
+  if (!out) return nullptr;
+  PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(w)));
+  PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(std::move(ids)));
+  return out;
 }
 
 // ---------------------------------------------------------------------------------------------- expert layer
 // fused_experts(x, w1, w2, s1, s2, topk_weights, topk_ids, weight_factor, out or None, ue8m0) -> out
-PyObject* fused_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* fused_experts(PyObject* const* args, Py_ssize_t n) {
   if (n != 10) Py_RETURN_NONE;
   const at::Tensor* t[7];
   for (int i = 0; i < 7; ++i)
@@ -243,24 +246,22 @@ PyObject* fused_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (op && (op->device() != x.device() || op->scalar_type() != dt || op->dim() != 2 || op->size(0) != M || op->size(1) != H ||
              !op->is_contiguous()))
     Py_RETURN_NONE;
-  return guarded([&]() -> PyObject* {
-    const c10::Device dev = x.device();
-    const c10::cuda::OptionalCUDAGuard guard(dev);
-    void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    at::Tensor out = op ? *op : empty({M, H}, dt, dev);
-    const int64_t bytes = sglb200_fused_experts_scratch_bytes(M, H, I, E, topk, ue);
-    c10::DataPtr scratch = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)bytes);
-    check_rc(sglb200_fused_experts(x.const_data_ptr(), code16(dt), w1.const_data_ptr(), w2.const_data_ptr(), s1.const_data_ptr(),
-                                   s2.const_data_ptr(), s1.strides().data(), s2.strides().data(), tw.const_data_ptr<float>(),
-                                   ids.const_data_ptr<int32_t>(), (float)factor, out.mutable_data_ptr(), M, H, I, E, topk, ue,
-                                   eps_in_dtype(1e-10, dt), scratch.get(), bytes, stream),
-             "fused_experts");
-    return THPVariable_Wrap(std::move(out));
-  });
+  const c10::Device dev = x.device();
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  at::Tensor out = op ? *op : empty({M, H}, dt, dev);
+  const int64_t bytes = sglb200_fused_experts_scratch_bytes(M, H, I, E, topk, ue);
+  c10::DataPtr scratch = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)bytes);
+  check_rc(sglb200_fused_experts(x.const_data_ptr(), code16(dt), w1.const_data_ptr(), w2.const_data_ptr(), s1.const_data_ptr(),
+                                 s2.const_data_ptr(), s1.strides().data(), s2.strides().data(), tw.const_data_ptr<float>(),
+                                 ids.const_data_ptr<int32_t>(), (float)factor, out.mutable_data_ptr(), M, H, I, E, topk, ue,
+                                 eps_in_dtype(1e-10, dt), scratch.get(), bytes, stream),
+           "fused_experts");
+  return THPVariable_Wrap(std::move(out));
 }
 
 // grouped_masked(a, a_s, w, w_s, out, masked_m, expected_m) -> True
-PyObject* grouped_masked(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* grouped_masked(PyObject* const* args, Py_ssize_t n) {
   if (n != 7) Py_RETURN_NONE;
   const at::Tensor* t[6];
   for (int i = 0; i < 6; ++i)
@@ -282,20 +283,18 @@ PyObject* grouped_masked(PyObject*, PyObject* const* args, Py_ssize_t n) {
       ws.scalar_type() != at::kFloat || ws.dim() != 3 || ws.size(0) != G || ws.size(1) != nt || ws.size(2) != kt)
     Py_RETURN_NONE;
   if (mm.scalar_type() != at::kInt || !mm.is_contiguous() || mm.numel() != G) Py_RETURN_NONE;
-  return guarded([&]() -> PyObject* {
-    const c10::Device dev = a.device();
-    const c10::cuda::OptionalCUDAGuard guard(dev);
-    check_rc(sglb200_fp8_blockwise_scaled_masked_grouped_mm_expected(
-                 a.const_data_ptr(), w.const_data_ptr(), as.const_data_ptr<float>(), ws.const_data_ptr<float>(), out.mutable_data_ptr(),
-                 mm.const_data_ptr<int32_t>(), G, max_m, expected, N, K, a.stride(1), w.stride(1), w.stride(0), out.stride(1),
-                 as.stride(0), as.stride(1), as.stride(2), ws.stride(0), ws.stride(1), ws.stride(2), code16(out.scalar_type()),
-                 c10::cuda::getCurrentCUDAStream(dev.index()).stream()),
-             "grouped_gemm_nt_f8f8bf16_masked");
-    Py_RETURN_TRUE;
-  });
+  const c10::Device dev = a.device();
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  check_rc(sglb200_fp8_blockwise_scaled_masked_grouped_mm_expected(
+               a.const_data_ptr(), w.const_data_ptr(), as.const_data_ptr<float>(), ws.const_data_ptr<float>(), out.mutable_data_ptr(),
+               mm.const_data_ptr<int32_t>(), G, max_m, expected, N, K, a.stride(1), w.stride(1), w.stride(0), out.stride(1),
+               as.stride(0), as.stride(1), as.stride(2), ws.stride(0), ws.stride(1), ws.stride(2), code16(out.scalar_type()),
+               c10::cuda::getCurrentCUDAStream(dev.index()).stream()),
+           "grouped_gemm_nt_f8f8bf16_masked");
+  Py_RETURN_TRUE;
 }
 
-#define SGLB_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr}
+#define SGLB_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(entry<name>)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
     SGLB_METHOD(quant),         SGLB_METHOD(block_linear),   SGLB_METHOD(topk_softmax),
     SGLB_METHOD(fused_experts), SGLB_METHOD(grouped_masked),

@@ -326,3 +326,33 @@ def test_linear_method_takes_a_layer_that_is_no_module(built_lib):
     layer = SimpleNamespace(weight=torch.zeros(128, 128).to(torch.float8_e4m3fn), weight_scale_inv=torch.ones(1, 1))
     with pytest.raises(RuntimeError, match="CUDA tensor"):
         Fp8LinearMethod(Fp8Config()).apply(layer, torch.zeros(2, 128, dtype=torch.bfloat16))
+
+
+def test_host_path_leaves_tensors_without_plain_memory_alone(built_lib):
+    """Traced tensors (static and symbolic sizes) and sparse ones that claim to be on a GPU: every function of the host path
+    answers None and the process lives.  In a child process, which an exception escaping from C++ would end."""
+    code = """
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from torch.fx.experimental.symbolic_shapes import ShapeEnv
+from sglang_b200._lib import host
+mode = FakeTensorMode(shape_env=ShapeEnv())
+with mode:
+    n = mode.shape_env.create_unbacked_symint()
+    w = torch.empty(128, 128, dtype=torch.float8_e4m3fn, device="cuda")
+    s = torch.empty(1, 1, device="cuda")
+    xs = [torch.empty(r, 128, dtype=torch.bfloat16, device="cuda") for r in (4, n)]
+    xs.append(torch.sparse_coo_tensor(torch.zeros(2, 1, dtype=torch.int64, device="cuda"),
+                                      torch.ones(1, dtype=torch.bfloat16, device="cuda"), (4, 128)))
+h = host()
+for x in xs:
+    assert x.is_cuda
+    assert h.block_linear(x, w, s, None, False) is None and h.block_linear(x, w, s, x, True) is None
+    assert h.quant(x, 128, 1e-10, -448.0, 448.0, False, False, False, False, None) is None
+    assert h.topk_softmax(x, 2, True) is None
+    assert h.fused_experts(x, x, x, x, x, x, x, 1.0, None, False) is None
+    assert h.grouped_masked(x, x, x, x, x, x, 1) is None
+print("alive")
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "alive", r.stderr[-2000:]
