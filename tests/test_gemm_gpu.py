@@ -128,8 +128,8 @@ def test_linear_method_apply():
 @pytest.mark.parametrize("M", [1, 16, 64, 128])
 @pytest.mark.parametrize("N,K", [(576, 7168), (7168, 8192), (1536, 4096)])
 def test_small_m_split_k(M, N, K):
-    """Small M: the split-K path (fp32 partial sums in a scratch buffer + reduce) against the oracle.  M <= 64 runs
-    the weight-streaming kernel with swapped operands, M = 128 the 128 x 128 kernel."""
+    """Small M where the output tiles alone leave SMs idle: the weight-streaming kernel, whose clusters cut K and add up on
+    the chip, against the oracle.  (The workspace size that the library names for such a shape is not needed here.)"""
     from sglang_b200._lib import lib
     a = make_activations(M, K, seed=M * 3 + N)
     aq, a_s = oracle.per_token_group_quant_fp8(a, 128)
@@ -141,11 +141,34 @@ def test_small_m_split_k(M, N, K):
     assert lib().sglb200_fp8_blockwise_scaled_mm_workspace_bytes(4096, N, K) == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(129, 576, 7168), (144, 1536, 4096), (200, 264, 4112), (385, 1000, 4496), (1023, 136, 8192)])
+def test_split_k_through_scratch(M, N, K):
+    """More than 128 rows and few output tiles: fp32 partial sums of K ranges in the wrapper's scratch and the kernel that
+    adds them, with ragged rows, columns and K, against the oracle and close to the uncut kernel."""
+    from sglang_b200._lib import check, lib
+    pad = -K % 128
+    a = torch.nn.functional.pad(make_activations(M, K, seed=M + N), (0, pad))
+    aq, a_s = oracle.per_token_group_quant_fp8(a, 128)
+    aq = aq[:, :K].contiguous()
+    wq, ws = make_weight(N, K, seed=N + K)
+    ref = oracle.w8a8_block_fp8_matmul(aq, wq, a_s, ws)
+    assert lib().sglb200_fp8_blockwise_scaled_mm_scratch_bytes(M, N, K) > 0, "expected split-K for this shape"
+    assert_gemm_close(_run(aq, a_s, wq, ws, m_major=True), ref, f"split-K M={M} N={N} K={K}")
+    a_d, w_d, s_d, ws_d = aq.cuda(), wq.cuda(), a_s.cuda(), ws.cuda()
+    out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    check(lib().sglb200_fp8_blockwise_scaled_mm(a_d.data_ptr(), w_d.data_ptr(), s_d.data_ptr(), ws_d.data_ptr(), out.data_ptr(),
+                                                M, N, K, K, K, N, s_d.stride(0), s_d.stride(1), ws_d.stride(0), ws_d.stride(1), 0,
+                                                torch.cuda.current_stream().cuda_stream), "mm")
+    torch.cuda.synchronize()
+    assert _status() == 0
+    assert_gemm_close(out, ref, f"uncut M={M} N={N} K={K}")
+
+
 @pytest.mark.parametrize("M", [2, 16, 17, 32, 33, 48, 64, 65, 96, 127, 128, 129])
 @pytest.mark.parametrize("N,K", [(128, 128), (576, 1024), (1536, 384), (4096, 4096), (7168, 2048)])
 def test_few_rows_kernel_boundaries(M, N, K):
-    """The weight-streaming kernel (M <= 64, token columns padded to 16 / 32 / 64) on both sides of every padding
-    boundary, with ragged N, with and without split-K, both scale layouts; M = 65 is the first size of the 128-row
+    """The weight-streaming kernel (M <= 128, token columns padded to 16 / 32 / 64 / 128) on both sides of every padding
+    boundary, with ragged N, K on one CTA and on clusters, both scale layouts; M = 129 is the first size of the 128-row
     kernel."""
     a = make_activations(M, K, seed=M * 7 + N + K)
     aq, a_s = oracle.per_token_group_quant_fp8(a, 128)
@@ -153,7 +176,7 @@ def test_few_rows_kernel_boundaries(M, N, K):
     ref = oracle.w8a8_block_fp8_matmul(aq, wq, a_s, ws)
     out = _run(aq, a_s, wq, ws, m_major=(M % 2 == 0))
     assert_gemm_close(out, ref, f"few rows M={M} N={N} K={K}")
-    from sglang_b200._lib import check, lib  # the plain entry point: same kernel, never split
+    from sglang_b200._lib import check, lib  # the plain entry point: same kernel
     a_d, w_d, s_d, ws_d = aq.cuda(), wq.cuda(), a_s.cuda(), ws.cuda()
     out2 = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
     check(lib().sglb200_fp8_blockwise_scaled_mm(a_d.data_ptr(), w_d.data_ptr(), s_d.data_ptr(), ws_d.data_ptr(),
@@ -165,7 +188,7 @@ def test_few_rows_kernel_boundaries(M, N, K):
     assert_gemm_close(out2, ref, f"few rows, plain entry M={M} N={N} K={K}")
 
 
-@pytest.mark.parametrize("M", [24, 100])  # one sub-tile of 32 rows; two sub-tiles of 64 rows
+@pytest.mark.parametrize("M", [24, 100])  # 32 token columns; 128, shared by several sets of promotion warps
 def test_few_rows_f16_ragged_k_and_strided_output(M):
     N, K = 384, 320  # K = 2.5 blocks
     a = make_activations(M, 384, seed=5)[:, :K].contiguous()

@@ -24,9 +24,9 @@ def _buffers(world, slot_elems):
 
 
 def _plain_partial(a_q, a_s, w, ws):
-    """The rank's partial product as the plain entry points compute it: for M <= 128 the few-rows kernel with the
-    library's own K-split (scratch + reduce kernel), above that the 128-row kernel without a split - in both cases the
-    kernel and the order of additions the push variant uses, stored instead of pushed."""
+    """The rank's partial product as the plain entry points compute it: for M <= 128 the few-rows kernel, which adds the K
+    ranges of a cluster up on the chip, above that the 128-row kernel without a split - in both cases the ranges and the
+    order of additions the push variant uses, stored instead of pushed."""
     from sglang_b200._lib import blockwise_mm, check, lib
     M, K = a_q.shape
     N = w.shape[0]

@@ -3,8 +3,8 @@
 Some callers of this library are not allowed to allocate device memory at the point where they run the GEMM (an
 engine that owns all device memory through its own pool, a no-allocation region, a bare C host).  For them the
 split-K scratch is a fixed array inside the library.  This file checks that entry against the existing split-K
-entry (caller-provided scratch) on two consecutive calls with different inputs, so stale scratch contents from the
-first call would show up in the second, and that shapes beyond the built-in buffer are refused.  It is collected
+entry (caller-provided scratch) on consecutive calls with different inputs, so stale scratch contents from one call
+would show up in the next (up to 128 rows K is added up on the chip and both go unused), and that shapes beyond the built-in buffer are refused.  It is collected
 last on purpose: a run that stops at the first failure has already run everything else.
 """
 
@@ -29,13 +29,15 @@ def test_noalloc_entry_matches_workspace_entry_twice():
     L = lib()
     assert L.sglb200_fp8_blockwise_scaled_mm_noalloc_max_bytes() == 16 * 1024 * 1024
     stream = torch.cuda.current_stream().cuda_stream
-    for call, (M, N, K, seed) in enumerate([(16, 7168, 8192, 1), (64, 1536, 4096, 2)]):
+    for call, (M, N, K, seed) in enumerate([(16, 7168, 8192, 1), (64, 1536, 4096, 2), (200, 576, 7168, 3),
+                                                 (144, 1536, 4096, 4)]):
         a = make_activations(M, K, seed=seed)
         aq_c, as_c = oracle.per_token_group_quant_fp8(a, 128)
         wq_c, ws_c = make_weight(N, K, seed=seed + 10)
         aq, a_s, wq, ws = aq_c.cuda(), as_c.cuda(), wq_c.cuda(), ws_c.cuda()
         need = L.sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K)
         assert 0 < need <= L.sglb200_fp8_blockwise_scaled_mm_noalloc_max_bytes(), "shape must use split-K and fit"
+        assert (L.sglb200_fp8_blockwise_scaled_mm_scratch_bytes(M, N, K) > 0) == (M > 128)
         scratch = torch.empty(need, dtype=torch.uint8, device="cuda")
         want = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
         check(L.sglb200_fp8_blockwise_scaled_mm_ws(*_args(aq, a_s, wq, ws, want), scratch.data_ptr(), need, stream),
@@ -53,7 +55,7 @@ def test_noalloc_entry_rejects_oversized_scratch_and_runs_large_m():
     from sglang_b200._lib import lib
     L = lib()
     stream = torch.cuda.current_stream().cuda_stream
-    # M=128, N=7168, K=16384 splits six ways: 22 MB of partial sums, more than the built-in 16 MiB: refused before any launch
+    # M=128, N=7168, K=16384 in five ranges: 18 MB of partial sums, more than the built-in 16 MiB: refused before any launch
     M, N, K = 128, 7168, 16384
     assert L.sglb200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) > L.sglb200_fp8_blockwise_scaled_mm_noalloc_max_bytes()
     rc = L.sglb200_fp8_blockwise_scaled_mm_noalloc(None, None, None, None, None, M, N, K, K, K, N, 1, M, K // 128, 1, 0,
