@@ -154,8 +154,8 @@ int sglb200_group_quant_fp8_batched(const void* input, int in_dtype, void* out_q
  * K need not be a multiple of 128 (the tail block is zero-filled), but K % 16 == 0.
  * fp32 accumulation; each 128-deep partial product is scaled and added in registers.
  * Any M >= 0 is accepted with no padding copy (the reference pads M to a multiple of 4).
- * Up to 128 rows the weight-streaming kernel with swapped operands runs (128 weight rows x 16 / 32 / 64 activation rows
- * per MMA; from 65 rows two such sub-tiles per work item share every weight stage), above that the 128 x 128 kernel.
+ * Up to 128 rows the weight-streaming kernel with swapped operands runs (128 weight rows x up to 16 / 32 / 64 / 128
+ * activation rows per MMA), above that the 128 x 128 kernel.
  */
 int sglb200_fp8_blockwise_scaled_mm(const void* a, const void* b, const float* sa, const float* sb, void* out,
                                     int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc,
@@ -226,9 +226,8 @@ int sglb200_fp8_blockwise_scaled_mm_noalloc(const void* a, const void* b, const 
  * two CTAs that share one tcgen05.mma.cta_group::2 over a 256 x tile_n output tile (tile_n = 128 or 256).  Each CTA
  * loads its own 128 rows of A and half of the B rows with its own TMA copies (nothing is broadcast), which lowers the
  * L2 -> shared-memory bytes per flop to 3/4 (tile_n 128) or 1/2 (tile_n 256) of the single-CTA kernel's.  An explicit
- * alternative, not the default: measured on B200 it is level with the single-CTA kernel at tile_n = 128 and behind it at
- * tile_n = 256 on most of the benchmark's shapes (the promotion of the partial sums, not operand delivery, is what bounds
- * both).  No split-K, no scratch.
+ * alternative, not the default: measured on B200 under sustained load (8192 x 36864 x 7168) it takes 2806 us at tile_n = 128
+ * and 2985 us at 256 where the single-CTA kernel takes 2401.  No split-K, no scratch.
  * Replaces: the 2-SM configuration of the reference's sm_100 kernels
  *           (KernelPtrArrayTmaWarpSpecializedBlockwise2SmSm100, sgl-kernel/csrc/moe/fp8_blockwise_moe_kernel.cu:300-310;
  *           dense launch sgl-kernel/csrc/gemm/fp8_blockwise_gemm_kernel.cu:39-196).
@@ -316,7 +315,7 @@ int sglb200_fp8_blockwise_scaled_grouped_mm(const void* a, const void* b, const 
  *   (either may be NULL); a_map [num_tokens * topk]: sorted row -> source token;
  *   c_map [num_tokens * topk]: token-major slot -> sorted row, -1 for ids outside [0, E).
  * Rows of one expert keep ascending slot order (deterministic; the reference's order is atomic order).
- * One launch, one thread block: num_tokens * topk <= 2^24, E <= 1024.
+ * One launch, one thread block per expert: num_tokens * topk <= 2^24, E <= 1024.
  */
 int sglb200_prepare_moe_input(const int32_t* topk_ids, int32_t* expert_offsets, int32_t* problem_sizes1,
                               int32_t* problem_sizes2, int32_t* a_map, int32_t* c_map, int64_t num_tokens,
@@ -484,8 +483,8 @@ int sglb200_moe_sum_reduce(const void* input, void* output, int64_t num_tokens, 
  * alternating slot sets are safe exactly because a rank's exchange e + 1 is enqueued after its exchange e); at most
  * 1024 output tiles of 128 x 128; world <= 8.
  * workspace / workspace_bytes: scratch for M <= 128 (size from sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes; 0 for
- * larger M).  With it the few-rows weight-streaming kernel computes fp32 sums (K split over the SMs where that pays) and
- * a second small kernel adds the splits, casts and does the pushing and flagging; without it (NULL) the 128-row kernel
+ * larger M).  With it the few-rows weight-streaming kernel computes fp32 sums (K in the ranges of the plain entry) and
+ * a second small kernel adds the ranges, casts and does the pushing and flagging; without it (NULL) the 128-row kernel
  * with the push epilogue runs.  Both produce the bits of the corresponding plain entry point.
  * A wait that runs out (a rank that never pushed) leaves its tile unwritten, sets device status 5
  * (sglb200_read_device_status) and does not advance the epoch, so the same exchange can be reduced again once the

@@ -14,7 +14,7 @@
 //              columns.  A thread owns one accumulator row: per k-block it pulls its 64 partial sums out
 //              of TMEM (two tcgen05.ld of 32 columns, one wait), multiplies by sa[m,kb] * sb[nb,kb] and
 //              adds into 64 fp32 registers with packed fp32x2 FMAs; after the last k-block it rounds to
-//              bf16/f16 and writes 128 contiguous bytes of the output row.  The scale of a row comes from the scale
+//              bf16/f16 and the warp stores 64-byte pieces of its rows through shared memory.  The scale of a row comes from the scale
 //              loader's ring with one 16-byte load per four k-blocks: with the promotion warps loading sa and sb
 //              themselves (two global loads with 64-bit addresses per k-block, four k-blocks ahead) a k-block took
 //              580 cycles instead of 427, whatever the latency of the loads.  Two warps per quarter hide each
@@ -1123,7 +1123,11 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
 
   if (!grouped && push && total_rows <= smallm_max_rows() && workspace != nullptr &&
       (int64_t)smallm_cluster(total_rows, N, K, di.sm_count) * total_rows * N <= workspace_floats) {
-    // few rows, exchanged: the weight-streaming kernel leaves fp32 sums, a second kernel casts and pushes them
+    // few rows, exchanged: the weight-streaming kernel leaves fp32 sums, a second kernel casts and pushes them.  K is cut as
+    // for the plain entry (smallm_cluster), which makes the bits the same.  Both kernels against the ranges that a split through
+    // memory would choose by itself (smallm_splits), one rank, M = 16 / 64 / 128: N=7168 K=16384 30.1 / 36.6 / 45.2 against 30.5 /
+    // 38.8 / 50.9 us, N=576 K=7168 10.8 / 18.1 / 26.7 against 13.6 / 33.0 / 57.8, N=8192 K=4096 level; behind only at 128 rows and
+    // K = 2048 (N=7168 21.9 against 20.4).
     int splits = 1;
     if (int rc = smallm_gemm(a, b, sa, sb, out, total_rows, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n,
                              sb_stride_k, out_dtype, nullptr, workspace, workspace_floats, di.sm_count, stream, &splits, false))

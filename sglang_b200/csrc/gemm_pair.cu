@@ -9,11 +9,12 @@
 // BN = 128: (128 + 64) x 128 / 256 = 96; BN = 256: (128 + 128) x 128 / 512 = 64; BN = 256 also halves the MMA, commit
 // and barrier operations per flop.  No load is broadcast: every CTA fetches its own tiles with its own TMA copies; only
 // mbarrier arrivals cross between the two CTAs.
-// Measured on B200 (M = 8192, the five DeepSeek-V3 shapes): BN = 128 is level with the single-CTA kernel of gemm.cu
-// (1147-1725 against 1150-1717 TFLOP/s), BN = 256 behind it on four of five shapes: with the loads removed altogether
-// the single-CTA kernel gains only 15 %, so operand delivery is not what bounds this family of kernels; the per-k-block
-// hand-over of partial sums through TMEM is, and BN = 256 has only two TMEM stages to hide it.  The kernel is therefore
-// an explicit entry point (sglb200_fp8_blockwise_scaled_mm_pair), not the default.
+// Measured on B200 over a second of load, M = 8192, BN = 128 / BN = 256 / the single-CTA kernel of gemm.cu (us a call at the
+// SM clock in MHz that the 1000 W cap left): N=36864 K=7168 2806 at 1590 / 2985 at 1717 / 2401 at 1350, N=7168 K=16384 1235 at
+// 1575 / 1407 at 1837 / 1063 at 1320, N=24576 K=1536 555 at 1785 / 538 at 1856 / 421 at 1458.  The pairs leave power unused and
+// are behind in cycles: their promotion warps still fetch the scales of every k-block themselves and store rows straight from
+// registers, which the single-CTA kernel no longer does, and BN = 256 has only two TMEM stages.  The kernel is therefore an
+// explicit entry point (sglb200_fp8_blockwise_scaled_mm_pair), not the default.
 //
 // Per CTA, 384 threads, warp-specialised as in gemm.cu:
 //   warps 0-1  TMA producers (k-blocks alternate): A [128 x 128 B] and B [BN/2 x 128 B] per k-block into a ring of

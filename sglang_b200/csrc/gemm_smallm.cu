@@ -259,8 +259,6 @@ __device__ __forceinline__ uint32_t pack16(float a, float b, int out_dtype) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// CLUSTER is a template parameter because the mere presence of the adding-up code cost the main loop of the other form up to
-// 18 % (N=36864 K=7168 M=113: 57 -> 68 us) through its register allocation.
 // Warps 2 and 3 of the QUANT form (one or two rows): the activations come as they are, and these two warps quantise them on their
 // way into the ring, four k-blocks each in turn, with the arithmetic of the separate quantiser.  Every CTA does so for all k-blocks
 // it multiplies; at one or two rows a group of four k-blocks is one or two passes of a warp, less than the weights take to
@@ -334,6 +332,8 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
   }
 }
 
+// CLUSTER is a template parameter because the mere presence of the adding-up code cost the main loop of the other form up to
+// 18 % (N=36864 K=7168 M=113: 57 -> 68 us) through its register allocation.
 // QUANT: see quantise_rows.
 template <int MT, bool UE, bool GROUPED, int NSUB, bool CLUSTER, bool QUANT>
 // NSUB = 1 has 256 threads; the bound of 320 keeps it at 200 registers, so that a block of the quantiser or of another small
@@ -815,6 +815,13 @@ int launch_cluster(int MT, bool two, const CUtensorMap& map_w, const CUtensorMap
 
 }  // namespace
 
+// Row limit of this kernel for dense calls with fp32 scales.  It was drawn when the 128 x 128 kernel took 690 cycles a k-block; that
+// one now takes 425 and this one 780 above 64 rows, and measured again (GEMM alone in a replayed graph, weights from HBM, this /
+// the tile kernel with its K split, us at M = 65, 96, 128): N=576 K=7168 11.6/11.0 12.9/11.9 15.1/12.0, N=1536 K=7168 12.5/10.9
+// 14.0/12.4 16.6/13.1, N=7168 K=16384 32.1/30.0 32.7/30.3 33.6/32.2, N=10240 K=8192 26.8/22.7 27.0/23.0 27.7/23.6, N=36864 K=7168
+// 48.2/47.3 49.0/48.3 52.2/49.3, N=57344 K=8192 99.7/91.1 101/92.5 105/93.7, N=24576 K=1536 and N=5120 K=2560 level, N=4096 K=4096
+// 10.9/10.1 11.6/12.7 12.9/12.8.  So 64 would be the better limit for most widths, and a comparison of the two kernels' cost models
+// (smallm_cluster here, splitk_choice in gemm.cu) better than either; neither is built.
 int smallm_max_rows() { return 128; }
 
 int smallm_quant_rows() { return kQuantRows; }

@@ -30,10 +30,8 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // One lane of a converged warp, always the same one for a full mask.  Issue tcgen05 / TMA instructions under this and not
-// under `lane == 0`: their operands are uniform registers, and only for an elected lane does the compiler know that the
-// values are uniform; under a lane comparison it emits a loop over the active lanes around every such instruction.
-// Measured (B200, four 128 x 128 x 32 MMAs and one commit, per k-block): 520 cycles of the issuing warp under
-// `lane == 0`, 160 elected; the TMEM hand-off ring of gemm.cu without loads 407 -> 303 cycles per k-block.
+// under `lane == 0`.  Measured (B200, four 128 x 128 x 32 MMAs and one commit, per k-block): 520 cycles of the issuing warp
+// under `lane == 0`, 160 elected; the TMEM hand-off ring of gemm.cu without loads 407 -> 303 cycles per k-block.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile(
