@@ -155,7 +155,9 @@ int sglb200_group_quant_fp8_batched(const void* input, int in_dtype, void* out_q
  * fp32 accumulation; each 128-deep partial product is scaled and added in registers.
  * Any M >= 0 is accepted with no padding copy (the reference pads M to a multiple of 4).
  * Up to 128 rows the weight-streaming kernel with swapped operands runs (128 weight rows x up to 16 / 32 / 64 / 128
- * activation rows per MMA), above that the 128 x 128 kernel.
+ * activation rows per MMA), above that the 128 x 128 kernel.  The weight-streaming kernel may be launched beside the end of
+ * the kernel before it and then reads the first tiles of `b` at once: b must not be written by a kernel that releases its
+ * dependents early (griddepcontrol.launch_dependents).  All other work of the stream is ordered as usual.
  */
 int sglb200_fp8_blockwise_scaled_mm(const void* a, const void* b, const float* sa, const float* sb, void* out,
                                     int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc,

@@ -45,7 +45,7 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
                 void* stream, int* splits_used, bool ue8m0, const RawRows* raw = nullptr);
 void launch_splitk_reduce(const float* partial, void* out, const void* bias, int64_t M, int64_t N, int64_t ldc, int splits,
                           int out_dtype, int sm_count, void* stream);  // gemm.cu
-// Per-token-group quantisation (groups of 128) of whole rows, quant.cu
+// Per-token-group quantisation (groups of 128) of the linear layer's rows, quant.cu: the GEMM after it may start beside it
 int quant_rows(const void* input, int in_dtype, void* out_q, void* out_s, int64_t rows, int64_t hidden, float eps, bool ue8m0,
                int64_t s_stride_row, int64_t s_stride_group, void* stream);
 // The UE8M0 GEMM of the linear layer, gemm_ue8m0.cu

@@ -24,8 +24,9 @@
 //
 // The kernel is launched with programmatic stream serialization: it may start while the kernel before it (the
 // activation quantiser, or the previous layer's reduce kernel) is still running.  Its set-up and the WEIGHT tiles of the
-// first ring of stages depend on nothing earlier in the stream and are issued at once; the activation tiles, the
-// activation scales and every store come after griddepcontrol.wait.  At decode sizes the fixed cost of a call (launch,
+// first ring of stages are issued at once, ahead of griddepcontrol.wait; the activation tiles, all scales and every store
+// come after it.  The kernel starts when all blocks of the one before have ended, or have released it early: no kernel of this
+// library that could have written the weights does that (quant.cu), and callers' own kernels must not.  At decode sizes the fixed cost of a call (launch,
 // set-up, first TMA round trip) is of the order of the streaming time itself, and this hides most of it.
 #include <cuda.h>
 #include <cuda_bf16.h>

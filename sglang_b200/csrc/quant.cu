@@ -49,6 +49,7 @@ struct QuantParams {
   const int32_t* masked_m;
   uint32_t rows_per_batch, bdiv_mul, bdiv_shift;
   int64_t s_stride_batch;
+  bool release_early;  // the next kernel of the stream may start beside this one
 };
 
 // 16-bit input types.  LPG = lanes per group = group_size / 16; each lane owns vectors `lane` and
@@ -65,9 +66,10 @@ __global__ void __launch_bounds__(kThreads16<FUSE_SILU>) group_quant16_kernel(co
   const uint32_t base = blockIdx.x * (uint32_t)(kGroupsPerIter * kUnroll) + tg;
   const float inv_max = __frcp_rn(p.fp8_max);
   const bool fast_scale = p.fp8_max == 448.0f;
-  // programmatic dependent launch: the GEMM that follows may begin its set-up and stream its weights beside this
-  // kernel; this kernel's own input comes from the kernel before it
-  ptx::grid_dep_launch();
+  // Programmatic dependent launch: the GEMM that follows may begin its set-up and stream its weights beside this kernel; this
+  // kernel's own input comes from the kernel before it.  Only where the codes cannot be those weights: the fused form makes
+  // activations, the plain form is released by the linear layer alone.
+  if (FUSE_SILU || p.release_early) ptx::grid_dep_launch();
   ptx::grid_dep_wait();
 
   uint4 raw[kUnroll][2], up[FUSE_SILU ? kUnroll : 1][2];
@@ -288,7 +290,7 @@ template <bool FUSE>
 int quant_entry(const void* input, int in_dtype, void* out_q, void* out_s, void* out_act, int64_t num_rows,
                 int64_t hidden, int group_size, float eps, float fp8_min, float fp8_max, int scale_ue8m0,
                 int64_t s_stride_row, int64_t s_stride_group, void* stream, int64_t rows_per_batch = 0,
-                int64_t s_stride_batch = 0, const int32_t* masked_m = nullptr) {
+                int64_t s_stride_batch = 0, const int32_t* masked_m = nullptr, bool release_early = false) {
   SGLB_REQUIRE(rows_per_batch == 0 || (in_dtype != SGLB200_F32 && rows_per_batch > 0 && num_rows % rows_per_batch == 0),
                SGLB200_ERR_SHAPE, "batched layout: 16-bit input and num_rows a multiple of rows_per_batch=%lld",
                (long long)rows_per_batch);
@@ -340,6 +342,7 @@ int quant_entry(const void* input, int in_dtype, void* out_q, void* out_s, void*
   p.rows_per_batch = (uint32_t)rows_per_batch;
   p.bdiv_mul = p.bdiv_shift = 0;
   p.s_stride_batch = s_stride_batch;
+  p.release_early = release_early;
   if (rows_per_batch > 0) {  // same round-up magic number as for the groups
     uint32_t sh = 0;
     while (((uint64_t)1 << sh) < (uint64_t)rows_per_batch) ++sh;
@@ -361,7 +364,7 @@ int quant_entry(const void* input, int in_dtype, void* out_q, void* out_s, void*
 int quant_rows(const void* input, int in_dtype, void* out_q, void* out_s, int64_t rows, int64_t hidden, float eps, bool ue8m0,
                int64_t s_stride_row, int64_t s_stride_group, void* stream) {
   return quant_entry<false>(input, in_dtype, out_q, out_s, nullptr, rows, hidden, 128, eps, -448.f, 448.f, ue8m0, s_stride_row,
-                            s_stride_group, stream);
+                            s_stride_group, stream, 0, 0, nullptr, true);
 }
 }  // namespace sglb
 

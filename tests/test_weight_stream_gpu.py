@@ -102,3 +102,29 @@ def test_rows_quantised_by_the_gemm_itself(M, N, K, dtype, ue8m0):
     torch.cuda.synchronize()
     assert lib().sglb200_read_device_status() == 0
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M", [1, 16, 128])
+def test_weights_written_by_the_kernel_before(M):
+    """The quantiser writes the codes that the next call takes as weights, into the same memory every time: the
+    weight-streaming kernel, which reads weight tiles ahead of its other operands, must see the new ones."""
+    from sglang_b200.layers.quantization import w8a8_block_fp8_matmul
+    from sglang_b200.sgl_kernel import sgl_per_token_group_quant_8bit
+    N, K = 24576, 1536
+    a, a_s = oracle.per_token_group_quant_fp8(make_activations(M, K, seed=M), 128)
+    a, a_s = a.cuda(), a_s.cuda()
+    y = [torch.randn(N, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(i)).bfloat16() for i in range(3)]
+    w, w_s = torch.empty(N, K, dtype=torch.float8_e4m3fn, device="cuda"), torch.empty(N, K // 128, device="cuda")
+    blocks = torch.ones(N // 128, K // 128, device="cuda")
+
+    def product(i, wait):
+        sgl_per_token_group_quant_8bit(y[i], w, w_s, 128, 1e-10, -448.0, 448.0)
+        if wait:
+            torch.cuda.synchronize()
+        return w8a8_block_fp8_matmul(a, w, a_s, blocks, [128, 128], torch.bfloat16)
+
+    want = [product(i, True) for i in range(3)]
+    got = [product(i % 3, False) for i in range(9)]
+    torch.cuda.synchronize()
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 3]), f"call {i} saw other weights"
