@@ -186,7 +186,8 @@ int sglb200_fp8_blockwise_scaled_mm_ws(const void* a, const void* b, const float
 
 /*
  * L  The linear layer in one call: per-token-group quantisation of x, block-scaled GEMM, optional bias.
- *   x [M, K] (dtype = SGLB200_BF16 | SGLB200_F16) contiguous, K % 128 == 0;  w [N, K] e4m3 contiguous, N % 8 == 0
+ *   x [M, K] (dtype = SGLB200_BF16 | SGLB200_F16) contiguous, K % 128 == 0;  w [N, K] e4m3 contiguous, N % 8 == 0; for the
+ *   kernel that writes w the same holds as for b of sglb200_fp8_blockwise_scaled_mm
  *   w_scale: scale_ue8m0 == 0: fp32 [ceil(N/128), K/128];  != 0: int32 words [ceil(N/128), ceil(K/512)] of four exponent
  *            bytes (the activation scales are then powers of two too); element (n, k) at n * stride_n + k * stride_k
  *   bias [N] of dtype or NULL: added to the rounded product, one more rounding, as `output += bias` does
