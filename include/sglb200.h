@@ -226,11 +226,12 @@ int sglb200_fp8_blockwise_scaled_mm_noalloc(const void* a, const void* b, const 
                                             int64_t sb_stride_k, int out_dtype, void* stream);
 /*
  * G on CTA pairs: the same result contract as sglb200_fp8_blockwise_scaled_mm (dense, any M), computed by clusters of
- * two CTAs that share one tcgen05.mma.cta_group::2 over a 256 x tile_n output tile (tile_n = 128 or 256).  Each CTA
- * loads its own 128 rows of A and half of the B rows with its own TMA copies (nothing is broadcast), which lowers the
- * L2 -> shared-memory bytes per flop to 3/4 (tile_n 128) or 1/2 (tile_n 256) of the single-CTA kernel's.  An explicit
- * alternative, not the default: measured on B200 under sustained load (8192 x 36864 x 7168) it takes 2806 us at tile_n = 128
- * and 2985 us at 256 where the single-CTA kernel takes 2401.  No split-K, no scratch.
+ * two CTAs that share tcgen05.mma.cta_group::2 over a 256 x 256 output tile.  Each CTA loads its own 128 rows of A and half of the B
+ * rows with its own TMA copies (nothing is broadcast): half of the L2 -> shared-memory bytes per flop of the 128 x 128 tiles.
+ * sglb200_fp8_blockwise_scaled_mm and its forms choose this kernel themselves where it is the faster one (gemm.cu,
+ * pair_preferred); the entry takes it always.  tile_n, 128 or 256, no longer changes anything.  The kernel fetches the
+ * activation scales by TMA: where they are not M-major (sa_stride_m == 1) with sa 16-byte aligned and sa_stride_k a multiple
+ * of 4, the call runs on the 128 x 128 tiles, with the same bits.  No split-K, no scratch.
  * Replaces: the 2-SM configuration of the reference's sm_100 kernels
  *           (KernelPtrArrayTmaWarpSpecializedBlockwise2SmSm100, sgl-kernel/csrc/moe/fp8_blockwise_moe_kernel.cu:300-310;
  *           dense launch sgl-kernel/csrc/gemm/fp8_blockwise_gemm_kernel.cu:39-196).

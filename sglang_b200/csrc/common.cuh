@@ -28,6 +28,12 @@ int device_info(DeviceInfo* out);  // returns SGLB200_OK or an error code
 int make_map_sw128(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                    uint32_t box_rows, CUtensorMapL2promotion promo);
 
+// Tensor map of an fp32 [rows][cols] tensor (scales), boxes of box_cols x 1.  Defined in gemm.cu.
+int make_map_f32(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint64_t stride_bytes, uint32_t box_cols);
+
+// Tensor map of a [rows][cols] tensor of 16-bit results for TMA stores.  Defined in gemm.cu.
+int make_map_out16(CUtensorMap* map, void* base, uint64_t cols, uint64_t rows, uint64_t stride_bytes, uint32_t box_cols, uint32_t box_rows);
+
 // The few-rows (M <= smallm_max_rows()) weight-streaming GEMM, gemm_smallm.cu
 int smallm_max_rows();
 constexpr int kMaxCluster = 8;
@@ -67,10 +73,16 @@ int smallm_grouped_gemm(int chunk, const void* a, const void* b, const float* sa
                         int64_t sb_stride_e, int64_t sb_stride_n, int64_t sb_stride_k, int out_dtype, int sm_count,
                         void* stream, bool ue8m0);
 
-// Dense GEMM on CTA pairs (256 x bn tiles, bn = 128 or 256), gemm_pair.cu
-int pair_gemm(int bn, const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N,
-              int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k,
-              int64_t sb_stride_n, int64_t sb_stride_k, int out_dtype, int sm_count, void* stream);
+// Dense GEMM on CTA pairs (256 x 256 tiles), gemm_pair.cu
+int pair_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K,
+              int64_t lda, int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n,
+              int64_t sb_stride_k, int out_dtype, const void* bias, int sm_count, void* stream);
+
+bool pair_takes_scales(const float* sa, int64_t sa_stride_m, int64_t sa_stride_k);
+// The dense GEMM on 128 x 128 tiles (few-rows kernel for few rows), gemm.cu: the pair entry's way out for other scale layouts
+int tile_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K, int64_t lda,
+              int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n, int64_t sb_stride_k,
+              int out_dtype, void* stream);
 
 // Launch with programmatic stream serialization allowed: the kernel may begin before the previous kernel of the stream
 // has finished and must call ptx::grid_dep_wait() before it touches anything that kernel writes or reads.  With cluster > 1

@@ -1028,6 +1028,30 @@ int make_map_sw128(CUtensorMap* map, const void* base, int rank, const uint64_t*
   return SGLB200_OK;
 }
 
+// rank-2 fp32 tensor [rows][cols], cols contiguous, unswizzled boxes of box_cols x 1
+int make_map_f32(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint64_t stride_bytes, uint32_t box_cols) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(SGLB200_ERR_LAUNCH, "cuTensorMapEncodeTiled is not available from the CUDA driver");
+  const cuuint64_t gdim[2] = {cols, rows}, gstr[1] = {stride_bytes};
+  const cuuint32_t box[2] = {box_cols, 1}, estr[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(SGLB200_ERR_LAUNCH, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+  return SGLB200_OK;
+}
+
+// rank-2 tensor [rows][cols] of 16-bit results, cols contiguous, 128-byte-swizzled boxes of box_rows x box_cols (64 at most)
+int make_map_out16(CUtensorMap* map, void* base, uint64_t cols, uint64_t rows, uint64_t stride_bytes, uint32_t box_cols, uint32_t box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(SGLB200_ERR_LAUNCH, "cuTensorMapEncodeTiled is not available from the CUDA driver");
+  const cuuint64_t gdim[2] = {cols, rows}, gstr[1] = {stride_bytes};
+  const cuuint32_t box[2] = {box_cols, box_rows}, estr[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, base, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(SGLB200_ERR_LAUNCH, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+  return SGLB200_OK;
+}
+
 void launch_splitk_reduce(const float* partial, void* out, const void* bias, int64_t M, int64_t N, int64_t ldc, int splits,
                           int out_dtype, int sm_count, void* stream) {
   const int64_t vecs = M * (N / 8);
@@ -1072,6 +1096,23 @@ int dense_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
   return M > smallm_max_rows() ? splitk_choice(M, N, K, sm_count) : 1;
 }
 
+// Whether CTA pairs (gemm_pair.cu, 256 x 256 tiles) take a dense call that leaves K whole, or the 128 x 128 tiles here.  Cost model
+// in nanoseconds (runs of one call at a time, 11 layers of N = 576 to 36864, K = 1024 to 16384, 160 to 4096 rows): a k-block
+// takes a pair 505 and a CTA of the tile kernel 295, the end of a tile 2000 and 1000; the pair kernel starts 2500 later.  Mostly
+// it decides by waves: N=4096 K=4096 M=3072 48.5 against 53.7 us (pair / tile), M=1536 34.1 against 28.2; N=24576 K=1536 M=4096 165
+// against 188, M=640 31.6 against 29.8; N=1536 K=7168 M=1536 28 against 17.  Under sustained load at the power cap the pairs gain
+// 12 % more, because they move half of the operand bytes (figures in gemm_pair.cu): calls of more than 2e11 operations, which take
+// 100 us and more, go to them while the model has them up to 6 % behind, smaller ones where it has them 2 % ahead.
+bool pair_preferred(int64_t M, int64_t N, int64_t K, int sm_count) {
+  if (sm_count < 2) return false;
+  const int64_t kb = (K + BK - 1) / BK, pairs = sm_count / 2;
+  const int64_t waves2 = (((M + 255) / 256) * ((N + 255) / 256) + pairs - 1) / pairs;
+  const int64_t waves1 = (((M + BM - 1) / BM) * ((N + BN - 1) / BN) + sm_count - 1) / sm_count;
+  const int64_t cost2 = 2500 + waves2 * (kb * 505 + 2000), cost1 = waves1 * (kb * 295 + 1000);
+  const bool sustained = 2.0 * (double)M * (double)N * (double)K > 2e11;
+  return cost2 * 100 < cost1 * (sustained ? 106 : 98);
+}
+
 template <bool GROUPED, bool PUSH>
 int set_smem_attr_once() {
   static bool done[64] = {false};
@@ -1091,7 +1132,8 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
                 int64_t lda, int64_t ldb, int64_t ldb_e, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k,
                 int64_t sb_stride_e, int64_t sb_stride_n, int64_t sb_stride_k, int out_dtype, void* stream,
                 float* workspace = nullptr, int64_t workspace_floats = 0, const PushParams* push = nullptr,
-                int64_t rows_per_expert = 0, int64_t sa_stride_e = 0, int64_t expected_rows = 0, const void* bias = nullptr) {
+                int64_t rows_per_expert = 0, int64_t sa_stride_e = 0, int64_t expected_rows = 0, const void* bias = nullptr,
+                bool allow_pairs = true) {
   const bool grouped = expert_offsets != nullptr || rows_per_expert > 0;
   SGLB_REQUIRE(total_rows >= 0 && N >= 0 && K >= 0, SGLB200_ERR_SHAPE, "M=%lld N=%lld K=%lld: negative size",
                (long long)total_rows, (long long)N, (long long)K);
@@ -1159,6 +1201,13 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
                                  stream, false);
   }
 
+  const int splits = !grouped && !push && workspace != nullptr ? dense_splits(total_rows, N, K, di.sm_count) : 1;
+  const bool split = splits > 1 && (int64_t)splits * total_rows * N <= workspace_floats;
+  if (!grouped && !push && !split && allow_pairs && pair_takes_scales(sa, sa_stride_m, sa_stride_k) &&
+      pair_preferred(total_rows, N, K, di.sm_count))
+    return pair_gemm(a, b, sa, sb, out, total_rows, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k, out_dtype,
+                     bias, di.sm_count, stream);
+
   alignas(64) CUtensorMap map_a, map_b;
   {
     const uint64_t dims[2] = {(uint64_t)K, (uint64_t)total_rows};
@@ -1200,13 +1249,10 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
   p.k_splits = 1;
   p.kb_per_split = p.k_tiles;
   if (push) p.push = *push;
-  if (!grouped && workspace != nullptr && !push) {
-    const int splits = dense_splits(total_rows, N, K, di.sm_count);
-    if (splits > 1 && (int64_t)splits * total_rows * N <= workspace_floats) {
-      p.partial = workspace;
-      p.kb_per_split = (p.k_tiles + splits - 1) / splits;
-      p.k_splits = (p.k_tiles + p.kb_per_split - 1) / p.kb_per_split;
-    }
+  if (split) {
+    p.partial = workspace;
+    p.kb_per_split = (p.k_tiles + splits - 1) / splits;
+    p.k_splits = (p.k_tiles + p.kb_per_split - 1) / p.kb_per_split;
   }
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1236,6 +1282,14 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
 }
 
 }  // namespace
+
+// The dense GEMM without the CTA pairs
+int tile_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K, int64_t lda,
+              int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n, int64_t sb_stride_k,
+              int out_dtype, void* stream) {
+  return gemm_common(a, b, sa, sb, out, nullptr, nullptr, M, 1, N, K, lda, ldb, 0, ldc, sa_stride_m, sa_stride_k, 0, sb_stride_n, sb_stride_k,
+                     out_dtype, stream, nullptr, 0, nullptr, 0, 0, 0, nullptr, false);
+}
 }  // namespace sglb
 
 extern "C" int sglb200_fp8_blockwise_scaled_mm(const void* a, const void* b, const float* sa, const float* sb,

@@ -128,6 +128,20 @@ __device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// The answer at once, without try_wait's suspension of the warp.
+__device__ __forceinline__ bool mbar_test_wait_a(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait (see mbar_wait).  The time-out path is out of line so the ready path stays short.
 static __device__ __noinline__ bool mbar_wait_slow_a(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
   uint64_t t0 = 0;
@@ -184,6 +198,12 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu_u32(const uint32_t* p) {
   return v;
 }
 
+__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
 // ---------------------------------------------------------------- TMA
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
@@ -215,6 +235,20 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
+}
+
+// Store of a box from shared memory, as a bulk group of its own; what lies outside the tensor is left out.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t smem_src, int32_t c0, int32_t c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];\n\t"
+      "cp.async.bulk.commit_group;" ::"l"(reinterpret_cast<uint64_t>(map)),
+      "r"(smem_src), "r"(c0), "r"(c1)
+      : "memory");
+}
+// All bulk stores this thread has issued have read their shared memory.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
 // ---------------------------------------------------------------- tcgen05 / TMEM
@@ -293,6 +327,14 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[32]) {
                : "memory");
 }
 
+// One wait for two loads.  A second tcgen05.wait::ld is not free: a loop of two 32-column loads and their FMAs takes 191 cycles
+// with a wait for each, 173 with one (eight warps).
+__device__ __forceinline__ void tmem_ld_wait2(uint32_t (&a)[32], uint32_t (&b)[32]) {
+  tmem_ld_wait(a);
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(b[i])::"memory");
+}
+
 // ---------------------------------------------------------------- CTA pairs (cta_group::2)
 // Two CTAs of a cluster (ranks 2i, 2i + 1) share one MMA: the even CTA issues it, each CTA holds its own 128 rows of
 // A, half of the B rows and the accumulators of its own 128 rows.  No cluster-broadcast load is used anywhere: each
@@ -327,6 +369,17 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
 // thousand cycles per arrival, and nothing but the arrival itself has to be seen by the other CTA here.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The same where `pred` holds, without a branch around it
+__device__ __forceinline__ void mbar_arrive_cluster_if(uint32_t cluster_addr, bool pred) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %1, 0;\n"
+      "@p mbarrier.arrive.shared::cluster.b64 _, [%0];\n"
+      "}\n" ::"r"(cluster_addr),
+      "r"((uint32_t)pred)
+      : "memory");
 }
 // TMA loads of a CTA pair: the destination is this CTA's shared memory, the completion bytes may be counted on an
 // mbarrier of the partner CTA (`bar_cluster` from mapa_shared)

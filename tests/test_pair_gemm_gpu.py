@@ -1,4 +1,4 @@
-"""The CTA-pair GEMM (tcgen05 cta_group::2, 256 x 128 and 256 x 256 tiles) through its C-ABI entry against the CPU
+"""The CTA-pair GEMM (tcgen05 cta_group::2, 256 x 256 tiles) through its C-ABI entry against the CPU
 oracle, and bit for bit against the single-CTA kernel (both add the k-blocks of a row in the same order)."""
 
 import pytest
@@ -62,6 +62,65 @@ def test_pair_gemm_full_size_rows_sample_and_f16():
         out = _pair(q, s, wq, ws, tile_n, out_dtype=torch.float16)
         torch.cuda.synchronize()
         assert_gemm_close(out[rows], ref, f"pair tile_n={tile_n} full size")
+
+
+def _m_major(scales):
+    """The scales as the quantiser's TMA-aligned layout: M-major, each group's row padded to four."""
+    m, k = scales.shape
+    buf = torch.full((k, (m + 3) // 4 * 4), float("nan"))
+    buf[:, :m] = scales.t()
+    return buf.cuda().t()[:m]
+
+
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 128), (127, 136, 272), (129, 576, 640), (256, 256, 4224), (257, 264, 1408), (770, 1000, 1024),
+                                   (2500, 5120, 384)])
+def test_pair_gemm_edges_of_tiles_bit_for_bit(M, N, K, out_dtype):
+    # tiles cut off in either direction, one to 33 k-blocks (the shuffle of the weight scales wraps at 32), a K tail, more tiles than
+    # pairs; rows behind the output stay untouched.  Row-major scales send the plain entry to the kernels that the pairs are compared with.
+    from sglang_b200._lib import check, dtype_code, lib
+    kg = (K + 127) // 128
+    a = make_activations(M, kg * 128, seed=M + N)
+    aq, a_s = oracle.per_token_group_quant_fp8(a, 128)
+    wq, ws = make_weight(N, kg * 128, seed=K + N)
+    aq[:, K:] = 0
+    ref = oracle.w8a8_block_fp8_matmul(aq, wq, a_s, ws * 0.01, output_dtype=out_dtype)
+    aq_d, wq_d, ws_d = aq.cuda()[:, :K], wq.cuda()[:, :K], (ws * 0.01).cuda()
+    out, plain = (torch.full((M + 3, N), 7.0, dtype=out_dtype, device="cuda") for _ in range(2))
+    st = torch.cuda.current_stream().cuda_stream
+    sm, sr = _m_major(a_s), a_s.cuda()
+    check(lib().sglb200_fp8_blockwise_scaled_mm_pair(
+        aq_d.data_ptr(), wq_d.data_ptr(), sm.data_ptr(), ws_d.data_ptr(), out.data_ptr(), M, N, K, kg * 128, kg * 128, N, sm.stride(0),
+        sm.stride(1), ws_d.stride(0), ws_d.stride(1), dtype_code(out_dtype), 256, st), "pair")
+    check(lib().sglb200_fp8_blockwise_scaled_mm(
+        aq_d.data_ptr(), wq_d.data_ptr(), sr.data_ptr(), ws_d.data_ptr(), plain.data_ptr(), M, N, K, kg * 128, kg * 128, N, sr.stride(0),
+        sr.stride(1), ws_d.stride(0), ws_d.stride(1), dtype_code(out_dtype), st), "mm")
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    assert_gemm_close(out[:M], ref, f"pair M={M} N={N} K={K}")
+    assert torch.equal(bits(out), bits(plain))  # the three rows behind the output included
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_linear_layer_on_pairs_adds_its_bias(dtype):
+    # 3072 x 4096 x 4096 is a size the plain entry gives to the pairs; through row-major scales it stays on the 128 x 128 tiles
+    from sglang_b200.layers.quantization import block_quant_weight_fp8, sglang_per_token_group_quant_fp8, w8a8_block_fp8_matmul
+    from sglang_b200.layers.quantization.fp8 import Fp8Config, Fp8LinearMethod
+    M, N, K = 3072, 4096, 4096
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(M, K, generator=g, device="cuda").to(dtype)
+    layer, method = torch.nn.Module(), Fp8LinearMethod(Fp8Config())
+    method.create_weights(layer, K, [N], K, N, dtype, device="cuda")
+    codes, scales = block_quant_weight_fp8(torch.randn(N, K, generator=g, device="cuda") * 0.02)
+    layer.weight.data.copy_(codes)
+    layer.weight_scale_inv.data.copy_(scales)
+    method.process_weights_after_loading(layer)
+    bias = torch.randn(N, generator=g, device="cuda").to(dtype)
+    out = method.apply(layer, x, bias)
+    q, s = sglang_per_token_group_quant_fp8(x, 128)
+    want = w8a8_block_fp8_matmul(q, codes, s, scales, [128, 128], dtype) + bias
+    torch.cuda.synchronize()
+    assert torch.equal(bits(out), bits(want))
 
 
 def test_pair_gemm_refuses_bad_arguments():
