@@ -14,7 +14,7 @@
 //              columns.  A thread owns one accumulator row: per k-block it pulls its 64 partial sums out
 //              of TMEM (two tcgen05.ld of 32 columns, one wait), multiplies by sa[m,kb] * sb[nb,kb] and
 //              adds into 64 fp32 registers with packed fp32x2 FMAs; after the last k-block it rounds to
-//              bf16/f16 and the warp stores 64-byte pieces of its rows through shared memory.  The scale of a row comes from the scale
+//              bf16/f16 and leaves through shared memory and TMA stores (store_rows).  The scale of a row comes from the scale
 //              loader's ring with one 16-byte load per four k-blocks: with the promotion warps loading sa and sb
 //              themselves (two global loads with 64-bit addresses per k-block, four k-blocks ahead) a k-block took
 //              580 cycles instead of 427, whatever the latency of the loads.  Two warps per quarter hide each
@@ -27,6 +27,8 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "nvls.cuh"
@@ -57,7 +59,6 @@ constexpr int kGroupM = 16;  // m-tiles per raster group (dense)
 constexpr int kGroupMAr = 16;  // the same in the GEMM with the fused all-reduce: a raster group is the unit that is
                                // reduced over the ranks, and the reduction of the LAST group is not hidden (8 measured
                                // 2-3 % slower at eight ranks: twice the barriers for half the exposed tail)
-constexpr size_t kScaleOffset = (((size_t)kStages * kStageBytes + 256 /*barriers*/ + (kMaxExperts + 1) * sizeof(int32_t)) + 15) / 16 * 16;
 
 // Push epilogue (dense, one tile per (m, n)): instead of writing `out`, every output tile is stored into the receive
 // buffer of every rank, in the slot of this rank, and flagged there.  Receive buffer of a rank:
@@ -78,14 +79,19 @@ struct PushParams {
   int32_t scatter;  // 0: every tile goes to every rank (one-shot); 1: tile t goes to rank t % world only (two-shot)
 };
 
-// Epilogue staging: every promotion warp turns "one output row per lane" into "rows of contiguous bytes per store"
-// through a private [32 rows][kStageWords] patch of shared memory, 16 payload words per row and pass.  Stored straight
-// from the registers a warp's 16-byte stores touch 32 rows each, one L1 wavefront per row: 2048 of them per tile, more than
-// the tile's whole K loop where K is short (K = 1536: 640 cycles per k-block with the epilogue against 437 at K = 7168).
-constexpr int kStageWords = 20;  // 80-byte row stride: 16-byte aligned, conflict-free for the per-lane uint4 writes
+// Epilogue staging, behind the ring of stages: every promotion warp packs 32 columns of its 32 rows at a time into 2 KB of shared
+// memory of its own (64-byte-swizzled), from where ONE TMA store takes them (store_rows).  The forms whose stores go to several
+// places or have to be counted (PUSH, AR) turn "one output row per lane" into "rows of contiguous bytes per store" there instead
+// (warp_rows_via_smem).  Stored straight from the registers a warp's 16-byte stores touch 32 rows each, one L1 wavefront per row.
+constexpr int kStageWords = 20;  // 80-byte row stride of warp_rows_via_smem: 16-byte aligned, conflict-free for the uint4 writes
+constexpr uint32_t kBoxBytes = 32 * 64;
 constexpr size_t kStagingBytes = (size_t)kEpiWarps * 32 * kStageWords * sizeof(uint32_t);
-constexpr size_t kStagingOffset = kScaleOffset + (size_t)kScaleStages * BM * sizeof(float4);
-constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + kStagingOffset + kStagingBytes;
+constexpr size_t kStagingOffset = (size_t)kStages * kStageBytes;
+constexpr size_t kCtlOffset = kStagingOffset + kStagingBytes;
+constexpr size_t kScaleOffset = (kCtlOffset + 256 /*barriers*/ + (kMaxExperts + 1) * sizeof(int32_t) + 15) / 16 * 16;
+constexpr int kNotes = 8;  // TileNote ring: the scale loader is at most kScaleStages tiles (of one group) ahead
+constexpr size_t kNoteOffset = kScaleOffset + (size_t)kScaleStages * BM * sizeof(float4);
+constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + kNoteOffset + kNotes * 16;
 static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
 
 struct GemmParams {
@@ -144,6 +150,16 @@ struct Tile {
   int32_t kb0, kb1;  // k-block range of this work item
   int32_t split;
 };
+
+// Where a tile's results go.  The scale loader, which walks the tiles ahead of the promotion warps, writes it for them: eight
+// warps that took the tile number apart themselves (integer divisions, a search through the experts) stood still for 900 cycles
+// between two tiles (expert layer of 256 x 7168 x 2048 at 4096 tokens 3740 -> 3510 us, dense N=24576 K=1536 M=777 40.2 -> 38.8 with
+// store_rows).  Only the coordinates come from here: loop bounds read from memory make the compiler treat the loop as divergent
+// (38.8 -> 51 us).
+struct TileNote {
+  int32_t row0, row_end, n0, split;
+};
+static_assert(sizeof(TileNote) == 16 && kNotes > kScaleStages + 1, "notes");
 
 struct SharedCtl {
   uint64_t full[kStages];
@@ -259,17 +275,58 @@ __device__ __forceinline__ void warp_rows_via_smem(uint32_t* stg, const uint32_t
   }
 }
 
+// A promotion warp's 32 rows x 64 columns, rounded, to rows [row0, row_end) of the output: 32 columns per pass into the warp's box
+// (a lane's row of 64 bytes, 16-byte pieces swizzled), then one TMA store.  Only where an expert's rows end inside the 32 do
+// the lanes store what is theirs: the store would reach into the next expert's rows.  N=24576 K=1536 M=777: 39.7 -> 38.8 us against
+// 64-byte pieces stored by the lanes (the epilogue as a whole, 1000 to 1700 cycles a tile, is 13 of 45 us there).
+template <typename OutT, bool GROUPED>
+__device__ __forceinline__ void store_rows(const GemmParams& p, const CUtensorMap& map_out, const float2* acc, uint32_t box, int32_t n0,
+                                           int32_t row0, int32_t row_end, int lane, bool leader) {
+  if (row0 >= row_end) return;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int32_t c0 = n0 + 32 * h;
+    if (c0 >= p.N) return;
+    if (leader) ptx::bulk_wait_read();  // the store before has read the box
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2* v = acc + 16 * h + 4 * i;
+      uint4 u = make_uint4(pack2<OutT>(v[0].x, v[0].y), pack2<OutT>(v[1].x, v[1].y), pack2<OutT>(v[2].x, v[2].y), pack2<OutT>(v[3].x, v[3].y));
+      if constexpr (!GROUPED) {
+        if (p.bias != nullptr && c0 + 8 * i < p.N)  // N % 8 == 0
+          u = ptx::add_bias8(u, __ldg(reinterpret_cast<const uint4*>(static_cast<const OutT*>(p.bias) + c0 + 8 * i)),
+                             std::is_same<OutT, __half>::value ? SGLB200_F16 : SGLB200_BF16);
+      }
+      ptx::st_shared_v4(box + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4), u);
+    }
+    if (GROUPED && row0 + 32 > row_end) {  // uniform over the warp
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int r = 8 * j + (lane >> 2), i = lane & 3;
+        const uint4 u = ptx::ld_shared_v4(box + r * 64 + ((i ^ ((r >> 1) & 3)) << 4));
+        if (row0 + r < row_end && c0 + 8 * i < p.N) *reinterpret_cast<uint4*>(static_cast<OutT*>(p.out) + (int64_t)(row0 + r) * p.ldc + c0 + 8 * i) = u;
+      }
+    } else {
+      ptx::fence_proxy_async();
+      __syncwarp();
+      if (leader) ptx::tma_store_2d(&map_out, box, c0, row0);
+    }
+  }
+}
+
 template <bool GROUPED, bool PUSH, bool AR = false>
 __global__ void __launch_bounds__(kThreads, 1)
 fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                      const __grid_constant__ typename ParamsOf<PUSH, AR>::type p) {
+                      const __grid_constant__ CUtensorMap map_out, const __grid_constant__ typename ParamsOf<PUSH, AR>::type p) {
   static_assert(!AR || (!GROUPED && !PUSH), "the fused all-reduce is a form of the dense kernel");
   constexpr int kRing = kStages;  // shared-memory stages in the TMA ring
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* stage_base = smem;
-  SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem + (size_t)kStages * kStageBytes);
-  int32_t* tile_start = reinterpret_cast<int32_t*>(smem + (size_t)kStages * kStageBytes + 256);
+  SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem + kCtlOffset);
+  int32_t* tile_start = reinterpret_cast<int32_t*>(smem + kCtlOffset + 256);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -352,6 +409,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const uint32_t sc_full0 = ptx::smem_u32(&ctl->sc_full[0]);
   const uint32_t sc_empty0 = ptx::smem_u32(&ctl->sc_empty[0]);
   float4* scale_ring = reinterpret_cast<float4*>(smem + kScaleOffset);  // [kScaleStages][BM]
+  TileNote* notes = reinterpret_cast<TileNote*>(smem + kNoteOffset);
   const uint32_t stage0 = ptx::smem_u32(stage_base);
 
   const bool leader = ptx::elect_one();  // the lane that issues TMA and tcgen05 instructions
@@ -450,7 +508,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
   } else if (warp == 1) {
     // ===== scale loader: lane l serves the tile rows l, l + 32, l + 64, l + 96
-    uint32_t stage = 0, phase = 0;
+    uint32_t stage = 0, phase = 0, tile_i = 0;
     for (int32_t t = blockIdx.x; t < total_tiles; t += tile_stride) {
       const Tile tl = get_tile<GROUPED, AR ? kGroupMAr : kGroupM>(p, tile_start, t);
       const float* sa_row[BM / 32];
@@ -484,6 +542,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 #pragma unroll
         for (int j = 0; j < BM / 32; ++j)
           scale_ring[stage * BM + lane + 32 * j] = make_float4(a[j][0] * b[0], a[j][1] * b[1], a[j][2] * b[2], a[j][3] * b[3]);
+        if (lane == 0 && kb0 == tl.kb0) notes[tile_i++ & (kNotes - 1)] = {tl.row0, tl.row_end, tl.n0, tl.split};
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive_a(sc_full0 + stage * 8);
         if (++stage == kScaleStages) { stage = 0; phase ^= 1; }
@@ -542,16 +601,22 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const int col0 = ((warp - kFirstPromoWarp) >> 2) * kEpiCols;
     const int r_in_tile = q * 32 + lane;
     uint32_t acc_stage = 0, acc_phase = 0, sc_stage = 0, sc_phase = 0;
+    uint32_t tile_i = 0;
     float2 acc[kEpiCols / 2];
     uint32_t push_epoch = 0;
     if constexpr (PUSH) push_epoch = *reinterpret_cast<const volatile uint32_t*>(p.push.ctl) + 1u;
     for (int32_t t = blockIdx.x; t < total_tiles; t += tile_stride) {
-      const Tile tl = get_tile<GROUPED, AR ? kGroupMAr : kGroupM>(p, tile_start, t);
-      const int32_t row = tl.row0 + r_in_tile;
+      int32_t kb_count = p.k_tiles;
+      if constexpr (!GROUPED) {
+        if (p.k_splits > 1) {
+          const Tile tl = get_tile<GROUPED, AR ? kGroupMAr : kGroupM>(p, tile_start, t);
+          kb_count = tl.kb1 - tl.kb0;
+        }
+      }
 #pragma unroll
       for (int j = 0; j < kEpiCols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
       bool ok = true;
-      for (int32_t kb0 = tl.kb0; kb0 < tl.kb1 && ok; kb0 += kScaleGroup) {
+      for (int32_t kb0 = 0; kb0 < kb_count && ok; kb0 += kScaleGroup) {
         if (!wait_bar<false>(sc_full0 + sc_stage * 8, sc_phase)) {
           record_timeout(ctl, 10);
           ok = false;
@@ -564,7 +629,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         if (++sc_stage == kScaleStages) { sc_stage = 0; sc_phase ^= 1; }
 #pragma unroll
         for (int u = 0; u < kScaleGroup; ++u) {
-          if (kb0 + u >= tl.kb1) break;
+          if (kb0 + u >= kb_count) break;
           const float scale = sc[u];
           const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc_stage * BN + col0;
           const float2 scale2 = make_float2(scale, scale);
@@ -591,6 +656,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
       }
       if (!ok || ctl->abort_flag) break;
+      const TileNote tl = notes[tile_i++ & (kNotes - 1)];
       if constexpr (PUSH) {
         const int32_t n_first = tl.n0 + col0;
         const int32_t tile_id = (tl.row0 / BM) * p.n_tiles + tl.n0 / BN;
@@ -632,6 +698,7 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           ptx::st_release_sys_u32(f, push_epoch);
         }
       } else if (p.partial != nullptr) {
+        const int32_t row = tl.row0 + r_in_tile;
         if (row < tl.row_end) {
           const int32_t n_first = tl.n0 + col0;
           float* dst = p.partial + ((int64_t)tl.split * p.total_rows + row) * p.N + n_first;
@@ -642,6 +709,10 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                   make_float4(acc[2 * c].x, acc[2 * c].y, acc[2 * c + 1].x, acc[2 * c + 1].y);
           }
         }
+      } else if constexpr (!AR) {
+        const uint32_t box = stage0 + (uint32_t)kStagingOffset + (warp - kFirstPromoWarp) * kBoxBytes;
+        if (p.out_dtype == SGLB200_BF16) store_rows<__nv_bfloat16, GROUPED>(p, map_out, acc, box, tl.n0 + col0, tl.row0 + q * 32, tl.row_end, lane, leader);
+        else store_rows<__half, GROUPED>(p, map_out, acc, box, tl.n0 + col0, tl.row0 + q * 32, tl.row_end, lane, leader);
       } else {
         const int32_t n_first = tl.n0 + col0, row_base = tl.row0 + q * 32;
         uint32_t* stg = reinterpret_cast<uint32_t*>(smem + kStagingOffset) + (warp - kFirstPromoWarp) * 32 * kStageWords;
@@ -656,11 +727,6 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           warp_rows_via_smem(stg, v, lane, [&](int r, int w, uint4 val) {
             const int32_t c = 32 * h + 2 * w;  // 8 columns from n_first + c (N % 8 == 0)
             if (row_base + r < tl.row_end && n_first + c < p.N) {
-              if constexpr (!GROUPED && !AR) {
-                if (p.bias != nullptr)
-                  val = ptx::add_bias8(val, __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + n_first + c)),
-                                       p.out_dtype);
-              }
               *reinterpret_cast<uint4*>(out + (int64_t)r * p.ldc + c) = val;
             }
           });
@@ -676,6 +742,8 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
       }
     }
+    if constexpr (!PUSH && !AR)
+      if (leader) ptx::bulk_wait_read();  // the staging must outlive its stores
   }
 
   // ---------------------------------------------------------------- tear-down
@@ -1040,14 +1108,14 @@ int make_map_f32(CUtensorMap* map, const void* base, uint64_t cols, uint64_t row
   return SGLB200_OK;
 }
 
-// rank-2 tensor [rows][cols] of 16-bit results, cols contiguous, 128-byte-swizzled boxes of box_rows x box_cols (64 at most)
+// rank-2 tensor [rows][cols] of 16-bit results, cols contiguous, boxes of box_rows x box_cols (32 or 64), swizzled over a box row
 int make_map_out16(CUtensorMap* map, void* base, uint64_t cols, uint64_t rows, uint64_t stride_bytes, uint32_t box_cols, uint32_t box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(SGLB200_ERR_LAUNCH, "cuTensorMapEncodeTiled is not available from the CUDA driver");
   const cuuint64_t gdim[2] = {cols, rows}, gstr[1] = {stride_bytes};
   const cuuint32_t box[2] = {box_cols, box_rows}, estr[2] = {1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, base, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                        box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(SGLB200_ERR_LAUNCH, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return SGLB200_OK;
 }
@@ -1255,23 +1323,26 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
     p.k_splits = (p.k_tiles + p.kb_per_split - 1) / p.kb_per_split;
   }
 
+  alignas(64) CUtensorMap map_out = map_a;  // PUSH does not use it
+  if (!push)
+    if (int rc = make_map_out16(&map_out, out, (uint64_t)N, (uint64_t)total_rows, (uint64_t)ldc * 2, 32, 32)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (grouped) {
     if (int rc = set_smem_attr_once<true, false>()) return rc;
     // an upper bound on the tile count without reading the device: every expert can add one ragged m-tile
     const int64_t max_tiles = ((total_rows + BM - 1) / BM + num_experts) * p.n_tiles;
     const int grid = (int)(max_tiles < di.sm_count ? max_tiles : di.sm_count);
-    fp8_block_gemm_kernel<true, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, static_cast<const GemmParams&>(p));
+    fp8_block_gemm_kernel<true, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_out, static_cast<const GemmParams&>(p));
   } else if (push) {
     if (int rc = set_smem_attr_once<false, true>()) return rc;
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
     const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
-    fp8_block_gemm_kernel<false, true><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
+    fp8_block_gemm_kernel<false, true><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_out, p);
   } else {
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles * p.k_splits;
     const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
     if (int rc = set_smem_attr_once<false, false>()) return rc;
-    fp8_block_gemm_kernel<false, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, static_cast<const GemmParams&>(p));
+    fp8_block_gemm_kernel<false, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_out, static_cast<const GemmParams&>(p));
     if (p.partial != nullptr) {
       SGLB_CHECK_LAUNCH("fp8_block_gemm_kernel");
       launch_splitk_reduce(p.partial, out, bias, total_rows, N, ldc, p.k_splits, out_dtype, di.sm_count, stream);
@@ -1834,7 +1905,7 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm_allreduce(const void* a, const vo
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   const int64_t gemm_ctas = tiles < di.sm_count - comm_ctas ? tiles : di.sm_count - comm_ctas;
   const int grid = (int)gemm_ctas + comm_ctas;
-  void* args[] = {(void*)&map_a, (void*)&map_b, (void*)&p};
+  void* args[] = {(void*)&map_a, (void*)&map_b, (void*)&map_a /* no TMA store in this form */, (void*)&p};
   e = cudaLaunchCooperativeKernel((const void*)fp8_block_gemm_kernel<false, false, true>, dim3(grid), dim3(kThreads), args,
                                   kSmemBytes, st);
   if (e != cudaSuccess) {

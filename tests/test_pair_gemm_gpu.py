@@ -74,10 +74,10 @@ def _m_major(scales):
 
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,N,K", [(1, 8, 128), (127, 136, 272), (129, 576, 640), (256, 256, 4224), (257, 264, 1408), (770, 1000, 1024),
-                                   (2500, 5120, 384)])
+                                   (2500, 5120, 384), (2304, 12288, 128)])
 def test_pair_gemm_edges_of_tiles_bit_for_bit(M, N, K, out_dtype):
     # tiles cut off in either direction, one to 33 k-blocks (the shuffle of the weight scales wraps at 32), a K tail, more tiles than
-    # pairs; rows behind the output stay untouched.  Row-major scales send the plain entry to the kernels that the pairs are compared with.
+    # pairs, and a dozen tiles of one k-block for every CTA of the other kernel (its ring of tile notes has eight); rows behind the output stay untouched.  Row-major scales send the plain entry to the kernels that the pairs are compared with.
     from sglang_b200._lib import check, dtype_code, lib
     kg = (K + 127) // 128
     a = make_activations(M, kg * 128, seed=M + N)
@@ -97,7 +97,9 @@ def test_pair_gemm_edges_of_tiles_bit_for_bit(M, N, K, out_dtype):
         sr.stride(1), ws_d.stride(0), ws_d.stride(1), dtype_code(out_dtype), st), "mm")
     torch.cuda.synchronize()
     assert lib().sglb200_read_device_status() == 0
-    assert_gemm_close(out[:M], ref, f"pair M={M} N={N} K={K}")
+    # one unit in the last place: the tensor core sums a k-block in another order than the oracle, and among 28 million results
+    # some lie within such a difference (2^-24 of a sum) of a rounding boundary
+    assert_gemm_close(out[:M], ref, f"pair M={M} N={N} K={K}", allow_one_ulp=True)
     assert torch.equal(bits(out), bits(plain))  # the three rows behind the output included
 
 
