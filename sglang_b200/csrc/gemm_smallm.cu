@@ -816,16 +816,19 @@ int launch_cluster(int MT, bool two, const CUtensorMap& map_w, const CUtensorMap
 
 }  // namespace
 
-// Row limit of this kernel for dense calls with fp32 scales.  It was drawn when the 128 x 128 kernel took 690 cycles a k-block; that
-// one now takes 425 and this one 780 above 64 rows, and measured again (GEMM alone in a replayed graph, weights from HBM, this /
-// the tile kernel with its K split, us at M = 65, 96, 128): N=576 K=7168 11.6/11.0 12.9/11.9 15.1/12.0, N=1536 K=7168 12.5/10.9
-// 14.0/12.4 16.6/13.1, N=7168 K=16384 32.1/30.0 32.7/30.3 33.6/32.2, N=10240 K=8192 26.8/22.7 27.0/23.0 27.7/23.6, N=36864 K=7168
-// 48.2/47.3 49.0/48.3 52.2/49.3, N=57344 K=8192 99.7/91.1 101/92.5 105/93.7, N=24576 K=1536 and N=5120 K=2560 level, N=4096 K=4096
-// 10.9/10.1 11.6/12.7 12.9/12.8.  So 64 would be the better limit for most widths, and a comparison of the two kernels' cost models
-// (smallm_cluster here, splitk_choice in gemm.cu) better than either; neither is built.
+// Row limit of this kernel, and of the scratch sizes that callers know (smallm_splits)
 int smallm_max_rows() { return 128; }
 
 int smallm_quant_rows() { return kQuantRows; }
+
+// From 65 rows up a k-block takes this kernel 780 cycles and the 128 x 128 kernel 425: where every CTA works alone, that one takes
+// the call (GEMM alone in a replayed graph, this / the tile kernel, us: 113 x 10240 x 8192 27.5/20.3, 65 x 36864 x 7168 48.6/46.6,
+// 128 x 57344 x 8192 108/94, 128 x 24576 x 1536 16.9/12.3, 100 x 5120 x 2560 11.6/9.8).  Where clusters share K most SMs
+// would be idle without them, and a split through memory is no faster (M = 96, weights from HBM: N=4096 K=4096 11.6/12.7, N=7168
+// K=16384 32.7/30.3) and needs scratch.  Both add k-blocks in the same order, so that the bits do not depend on the choice.
+bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count) {
+  return M <= 64 || (M <= smallm_max_rows() && smallm_cluster(M, N, K, sm_count) > 1);
+}
 
 // CTAs per cluster that share one tile's K (1, 2, 4 or 8) for a dense problem.  Cost model in nanoseconds, from runs with one
 // tile per CTA at 1.9 GHz: a k-block takes one CTA `step` (the MMA issuer at 16 columns, the promotion above), or longer once

@@ -477,12 +477,6 @@ extern "C" int sglb200_debug_set_status_mirror(int* device_visible_host_ptr) {
 }
 
 namespace sglb {
-namespace {
-bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count) {
-  return M <= 64 || (M <= smallm_max_rows() && smallm_cluster(M, N, K, sm_count) > 1);
-}
-}  // namespace
-
 // K ranges (whole groups of four k-blocks) of a dense problem whose tiles alone leave SMs idle, for callers with scratch; 1 = none.
 // Cost model in nanoseconds at 1.9 GHz: a k-block takes a CTA 380, a work item 800 more; splitting costs the reduce kernel (3500)
 // and the partial sums' way to memory and back (8 bytes each at about 5 TB/s).

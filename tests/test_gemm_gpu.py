@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import oracle
-from helpers import FP8, as_bf16, as_fp8, as_t, assert_gemm_close, load_golden, make_activations, make_weight
+from helpers import FP8, as_bf16, as_fp8, as_t, assert_gemm_close, bits, load_golden, make_activations, make_weight
 
 pytestmark = pytest.mark.gpu
 
@@ -207,3 +207,29 @@ def test_few_rows_f16_ragged_k_and_strided_output(M):
           "mm")
     torch.cuda.synchronize()
     assert torch.equal(wide[:, :N], out) and (wide[:, N:] == 3.0).all()
+
+
+@pytest.mark.parametrize("K", [128, 768, 1024])
+@pytest.mark.parametrize("M", [65, 128])
+def test_tile_kernel_beside_the_quantiser(M, K):
+    """65 to 128 rows on tiles of their own: the kernel starts beside the quantiser and requests a ring of weight tiles first (one
+    k-block, exactly the ring's six, more).  Calls in a row without a synchronisation between them; 129 rows run the same kernel
+    in an ordinary launch, and the bits of a row do not depend on the others."""
+    from sglang_b200.layers.quantization import block_quant_weight_fp8
+    from sglang_b200.layers.quantization.fp8 import Fp8Config, Fp8LinearMethod
+    N = 10240
+    g = torch.Generator(device="cuda").manual_seed(K)
+    layer, method = torch.nn.Module(), Fp8LinearMethod(Fp8Config())
+    method.create_weights(layer, K, [N], K, N, torch.bfloat16, device="cuda")
+    codes, scales = block_quant_weight_fp8(torch.randn(N, K, generator=g, device="cuda") * 0.02)
+    layer.weight.data.copy_(codes)
+    layer.weight_scale_inv.data.copy_(scales)
+    method.process_weights_after_loading(layer)
+    xs = [torch.randn(129, K, generator=g, device="cuda").bfloat16() for _ in range(4)]
+    few = [method.apply(layer, x[:M].contiguous(), None) for x in xs]
+    many = [method.apply(layer, x, None) for x in xs]
+    torch.cuda.synchronize()
+    from sglang_b200._lib import lib
+    assert lib().sglb200_read_device_status() == 0
+    for a, b in zip(few, many):
+        assert torch.equal(bits(a), bits(b[:M]))
