@@ -655,7 +655,7 @@ int sglb200_fp8_blockwise_scaled_mm_allreduce(const void* a, const void* b, cons
  * Device-side status word of the GEMM kernels: 0, or the code of the first bounded wait that timed out
  * (1 TMA producer, 2 or 3 MMA issuer, 4 promotion warps, 5 peer-flag wait of sglb200_peer_reduce, 6-8 the communication
  * CTAs of sglb200_fp8_blockwise_scaled_mm_allreduce, 11-18 the same
- * roles in the UE8M0 and few-rows kernels, 21-23 the expert-parallel exchange, 31-35 the CTA-pair kernel, 41-42 the multicast all-reduce).  Every
+ * roles in the UE8M0 and few-rows kernels, 21-23 the expert-parallel exchange, 31-37 the CTA-pair kernel, 51-58 its UE8M0 form, 41-42 the multicast all-reduce).  Every
  * kernel family keeps its own word; each call reads AND clears all of them and returns the first non-zero one, so a
  * status never surfaces on a later, unrelated read.  This call SYNCHRONISES the device (cudaMemcpyFromSymbol); it is for
  * tests and debugging, not for the serving path.  Returns -1 if the read itself failed.  No counterpart in the reference (its kernels have no bounded waits).

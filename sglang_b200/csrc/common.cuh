@@ -60,6 +60,11 @@ int ue8m0_linear_gemm(const void* a, const void* b, const int32_t* sfa, const in
                       int64_t N, int64_t K, int64_t sfa_ld, int64_t sfb_stride_n, int64_t sfb_stride_k, int out_dtype,
                       void* stream, float* workspace, int64_t workspace_floats);
 int ue8m0_splits(int64_t M, int64_t N, int64_t K, int sm_count);  // with `workspace` of that many [M][N] fp32 sums
+// The same GEMM on CTA pairs (256 x 224 tiles), gemm_ue8m0_pair.cu
+int64_t ue8m0_pair_cost(int64_t M, int64_t N, int64_t K, int sm_count);
+int ue8m0_pair_gemm(const void* a, const void* b, const int32_t* sfa, const int32_t* sfb, const void* bias, void* out, int64_t M, int64_t N,
+                    int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int64_t sfa_ld, int64_t sfb_stride_n, int64_t sfb_stride_k,
+                    int out_dtype, int sm_count, void* stream);
 int smallm_take_device_status();
 int nvls_take_device_status();  // nvls.cu
 constexpr int kGroupedFewRowsDefault = 20;  // stands for the library's rule; the limit 20 itself carries SGLB200_FEW_ROWS_EXACT

@@ -1957,10 +1957,11 @@ namespace sglb {
 int ue8m0_take_device_status();  // gemm_ue8m0.cu
 int ep_take_device_status();     // ep_peer.cu
 int pair_take_device_status();   // gemm_pair.cu
+int ue8m0_pair_take_device_status();  // gemm_ue8m0_pair.cu
 }
 // Reads AND clears the device-side status words of every kernel family: 0, or the code of the first bounded wait that
 // timed out (1 producer, 2/3 MMA issuer, 4 promotion warps, 5 peer flags / tail drain; 11-18 the same roles in the
-// UE8M0 and few-rows kernels; 21-23 expert-parallel exchange; 31-35 CTA-pair kernel).  All words are read and cleared on every call, so a
+// UE8M0 and few-rows kernels; 21-23 expert-parallel exchange; 31-37 CTA-pair kernel, 51-58 its UE8M0 form).  All words are read and cleared on every call, so a
 // status never outlives the call that reports it; when several are set, the first non-zero one in the order UE8M0,
 // few-rows, expert-parallel, CTA-pair, multicast all-reduce, dense is returned.  Synchronises the device: for tests and debugging, not for the
 // serving path.
@@ -1969,6 +1970,7 @@ extern "C" int sglb200_read_device_status(void) {
   const int sm = sglb::smallm_take_device_status();
   const int ep = sglb::ep_take_device_status();
   const int pr = sglb::pair_take_device_status();
+  const int up = sglb::ue8m0_pair_take_device_status();
   const int nv = sglb::nvls_take_device_status();
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, sglb::g_device_status, sizeof(int)) != cudaSuccess) {
@@ -1982,6 +1984,7 @@ extern "C" int sglb200_read_device_status(void) {
   if (sm != 0) return sm;
   if (ep != 0) return ep;
   if (pr != 0) return pr;
+  if (up != 0) return up;
   if (nv != 0) return nv;
   return v;
 }

@@ -477,15 +477,21 @@ extern "C" int sglb200_debug_set_status_mirror(int* device_visible_host_ptr) {
 }
 
 namespace sglb {
-// K ranges (whole groups of four k-blocks) of a dense problem whose tiles alone leave SMs idle, for callers with scratch; 1 = none.
-// Cost model in nanoseconds at 1.9 GHz: a k-block takes a CTA 380, a work item 800 more; splitting costs the reduce kernel (3500)
-// and the partial sums' way to memory and back (8 bytes each at about 5 TB/s).
-int ue8m0_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
-  if (takes_few_rows(M, N, K, sm_count)) return 1;
+namespace {
+// How a dense problem above the few-rows kernel's sizes is run: on CTA pairs (gemm_ue8m0_pair.cu), or here with K in `splits` ranges
+// (whole groups of four k-blocks, for callers with scratch; 1 = not cut).  Cost models in nanoseconds at 1.9 GHz: for the choice
+// among ranges a k-block takes a CTA 380 and a work item 800 more, splitting costs the reduce kernel (3500) and the partial
+// sums' way to memory and back (8 bytes each at about 5 TB/s); against the pairs a k-block of an uncut call counts 340 and a
+// tile's store, which the pairs do not pay, 1700.
+struct Plan {
+  int splits;
+  bool pair;
+};
+Plan dense_plan(int64_t M, int64_t N, int64_t K, int sm_count, bool scratch) {
   const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), groups = (K + 4 * BK - 1) / (4 * BK);
   int best = 1;
   int64_t best_cost = INT64_MAX;
-  for (int64_t c = 1; c <= 32 && (c == 1 || (c <= groups && tiles * c <= 2 * (int64_t)sm_count)); ++c) {
+  for (int64_t c = 1; c <= 32 && (c == 1 || (scratch && c <= groups && tiles * c <= 2 * (int64_t)sm_count)); ++c) {
     const int64_t kg = (groups + c - 1) / c;
     if ((groups + kg - 1) / kg != c) continue;  // every range must get k-blocks
     const int64_t waves = (tiles * c + sm_count - 1) / sm_count;
@@ -495,7 +501,14 @@ int ue8m0_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
       best = (int)c;
     }
   }
-  return best;
+  if (best == 1) best_cost = (tiles + sm_count - 1) / sm_count * ((K + BK - 1) / BK * 340 + 1700);
+  if (ue8m0_pair_cost(M, N, K, sm_count) < best_cost) return {1, true};
+  return {best, false};
+}
+}  // namespace
+
+int ue8m0_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
+  return takes_few_rows(M, N, K, sm_count) ? 1 : dense_plan(M, N, K, sm_count, true).splits;
 }
 
 namespace {
@@ -555,6 +568,15 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
                                  stream, true);
   }
 
+  Plan plan = {1, false};
+  if (!grouped) {
+    plan = dense_plan(M, N, K, di.sm_count, workspace != nullptr);
+    if ((int64_t)plan.splits * M * N > workspace_floats) plan = dense_plan(M, N, K, di.sm_count, false);
+    if (plan.pair && sfa_stride_m == 1)
+      return ue8m0_pair_gemm(a, b, sfa, sfb, bias, out, M, N, K, lda, ldb, ldc, sfa_ld, sfb_stride_n, sfb_stride_k, out_dtype, di.sm_count,
+                             stream);
+  }
+
   alignas(64) CUtensorMap map_a, map_b;
   {
     const uint64_t dims[2] = {(uint64_t)K, (uint64_t)M};
@@ -591,13 +613,10 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
   p.partial = nullptr;
   p.k_splits = 1;
   p.kg_per_split = p.k_groups;
-  if (!grouped && workspace != nullptr) {
-    const int splits = ue8m0_splits(M, N, K, di.sm_count);
-    if (splits > 1 && (int64_t)splits * M * N <= workspace_floats) {
-      p.partial = workspace;
-      p.kg_per_split = (p.k_groups + splits - 1) / splits;
-      p.k_splits = splits;
-    }
+  if (plan.splits > 1) {
+    p.partial = workspace;
+    p.kg_per_split = (p.k_groups + plan.splits - 1) / plan.splits;
+    p.k_splits = plan.splits;
   }
 
   static bool attr_done[64] = {false};

@@ -375,7 +375,12 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// The same where `pred` holds, without a branch around it
+// The same with release semantics for the whole cluster: for an arrival that publishes shared-memory writes to the other CTA's
+// tensor operations and may take its time.
+__device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The same as mbar_arrive_cluster where `pred` holds, without a branch around it
 __device__ __forceinline__ void mbar_arrive_cluster_if(uint32_t cluster_addr, bool pred) {
   asm volatile(
       "{\n"
@@ -436,6 +441,10 @@ __device__ __forceinline__ void mma_commit_pair_a(uint32_t bar) {
 __device__ __forceinline__ void tmem_cp_32x128b_warpx4(uint32_t taddr, uint64_t smem_desc) {
   asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(smem_desc) : "memory");
 }
+// The same in both CTAs of a pair, each from its own shared memory at the described offset into its own TMEM.
+__device__ __forceinline__ void tmem_cp_32x128b_warpx4_pair(uint32_t taddr, uint64_t smem_desc) {
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(smem_desc) : "memory");
+}
 // Descriptor of a scale-factor block in shared memory: 32 rows of 16 bytes, contiguous, no swizzle
 // (8-row atoms 128 bytes apart), descriptor version 1.
 __device__ __forceinline__ uint64_t make_sf_desc(uint32_t smem_addr) {
@@ -456,6 +465,20 @@ __device__ __forceinline__ void mma_mxf8_block_scaled(uint32_t d_tmem, uint64_t 
       ".reg .pred p;\n"
       "setp.ne.b32 p, %6, 0;\n"
       "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem), "r"(accumulate)
+      : "memory");
+}
+// The same over a CTA pair (M = 256, 128 rows per CTA), issued by ONE thread of the even CTA; sfa holds each CTA's own rows' factors,
+// sfb all columns' in both.
+__device__ __forceinline__ void mma_mxf8_block_scaled_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                                           uint32_t idesc, uint32_t sfa_tmem, uint32_t sfb_tmem,
+                                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %6, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], p;\n"
       "}\n" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem), "r"(accumulate)
       : "memory");

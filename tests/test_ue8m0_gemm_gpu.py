@@ -187,3 +187,55 @@ def test_matmul_cuts_k_like_the_linear_layer(M, N, K):
         assert torch.equal(out, got) and torch.isfinite(scratch).all(), "every partial sum is written"
     torch.cuda.synchronize()
     assert L.sglb200_read_device_status() == 0
+
+
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(129, 264, 1536), (256, 224, 2064), (257, 232, 1552), (777, 1000, 1536), (385, 2368, 4224),
+                                   (2900, 3208, 1664)])
+def test_dense_pairs_edges_of_tiles(M, N, K, out_dtype):
+    """The CTA-pair form: tiles cut off in either direction (224 columns, of which a CTA's half and the scale blocks of 128 end
+    elsewhere), K ending inside a group of four k-blocks and inside a k-block, more tiles than pairs.  Against the oracle, and
+    bit for bit against the single-CTA kernel, which the grouped entry runs for one expert; rows behind the output stay."""
+    from sglang_b200._lib import check, dtype_code, lib
+    from sglang_b200.layers.quantization import pack_ue8m0_scales
+    L, kg = lib(), -(-K // 128)
+    g = torch.Generator().manual_seed(M + K)
+    aq, a_s = oracle.per_token_group_quant_fp8(torch.randn(M, kg * 128, generator=g).bfloat16(), 128, scale_ue8m0=True)
+    wq, ws = oracle.block_quant_weight(torch.randn(N, kg * 128, generator=g) * 0.02, scale_ue8m0=True)
+    aq, wq = aq[:, :K].contiguous(), wq[:, :K].contiguous()
+    a, w, sw = aq.cuda(), wq.cuda(), pack_ue8m0_scales(ws.cuda())
+    sa = pack_ue8m0_scales(a_s).cuda().t().contiguous().t()
+    out, single = (torch.full((M + 3, N), 7.0, dtype=out_dtype, device="cuda") for _ in range(2))
+    offsets, st = torch.tensor([0, M], dtype=torch.int32, device="cuda"), torch.cuda.current_stream().cuda_stream
+    check(L.sglb200_fp8_ue8m0_scaled_mm(a.data_ptr(), w.data_ptr(), sa.data_ptr(), sw.data_ptr(), out.data_ptr(), M, N, K, K, K, N,
+                                        sa.stride(1), sw.stride(0), sw.stride(1), dtype_code(out_dtype), st), "mm")
+    check(L.sglb200_fp8_ue8m0_scaled_grouped_mm(a.data_ptr(), w.data_ptr(), sa.data_ptr(), sw.data_ptr(), single.data_ptr(),
+                                                offsets.data_ptr(), M, 1, N, K, K, K, N * K, N, sa.stride(0), sa.stride(1), 0,
+                                                sw.stride(0), sw.stride(1), dtype_code(out_dtype), st), "grouped mm")
+    torch.cuda.synchronize()
+    assert L.sglb200_read_device_status() == 0
+    ref = oracle.w8a8_block_fp8_matmul(aq, wq, a_s, ws, output_dtype=out_dtype)
+    assert_gemm_close(out[:M], ref, f"pairs {M}x{N}x{K}", allow_one_ulp=True)
+    assert torch.equal(out.view(torch.int16), single.view(torch.int16))
+
+
+def test_dense_pairs_add_the_bias_and_survive_repeated_launches():
+    """A full-size call through the linear layer with a bias, twenty launches in a row: the same bits as the sum taken after the call."""
+    from sglang_b200._lib import lib
+    from sglang_b200.layers.quantization.fp8 import Fp8Config, Fp8LinearMethod
+    from sglang_b200.layers.quantization.fp8_utils import per_block_cast_to_fp8
+    M, N, K = 2048, 7168, 8192
+    g = torch.Generator(device="cuda").manual_seed(5)
+    layer, method = torch.nn.Module(), Fp8LinearMethod(Fp8Config())
+    method.create_weights(layer, K, [N], K, N, torch.bfloat16, device="cuda")
+    codes, scales = per_block_cast_to_fp8(torch.randn(N, K, generator=g, device="cuda") * 0.02)
+    layer.weight.data.copy_(codes)
+    layer.weight_scale_inv.data.copy_(scales)
+    method.process_weights_after_loading(layer)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    bias = torch.randn(N, generator=g, device="cuda").bfloat16()
+    outs = [method.apply(layer, x, bias) for _ in range(20)]
+    want = method.apply(layer, x, None) + bias
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    assert all(torch.equal(o, want) for o in outs)
