@@ -320,7 +320,8 @@ __device__ __forceinline__ void store_rows(const GemmParams& p, const CUtensorMa
 template <bool GROUPED, bool PUSH, bool AR = false>
 __global__ void __launch_bounds__(kThreads, 1)
 fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                      const __grid_constant__ CUtensorMap map_out, const __grid_constant__ typename ParamsOf<PUSH, AR>::type p) {
+                      const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_rows,
+                      const __grid_constant__ typename ParamsOf<PUSH, AR>::type p) {
   static_assert(!AR || (!GROUPED && !PUSH), "the fused all-reduce is a form of the dense kernel");
   constexpr int kRing = kStages;  // shared-memory stages in the TMA ring
   extern __shared__ uint8_t smem_raw[];
@@ -505,7 +506,13 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
           if (leader) {
             ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, kStageBytes);
-            ptx::tma_load_2d_a(dst, &map_a, full0 + stage * 8, kb * BK, tl.row0);
+            if (GROUPED && tl.row_end - tl.row0 <= BM - kRowBox) {
+              // the end of an expert: rows that belong to nobody here come as zeros, from outside the tensor (see kRowBox)
+              for (int32_t r = 0; r < BM; r += kRowBox)
+                ptx::tma_load_2d_a(dst + r * BK, &map_rows, full0 + stage * 8, kb * BK, tl.row0 + r < tl.row_end ? tl.row0 + r : p.total_rows);
+            } else {
+              ptx::tma_load_2d_a(dst, &map_a, full0 + stage * 8, kb * BK, tl.row0);
+            }
             ptx::tma_load_3d_a(dst + kTileABytes, &map_b, full0 + stage * 8, kb * BK, tl.n0, tl.expert);
           }
         }
@@ -1351,18 +1358,24 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
   alignas(64) CUtensorMap map_out = map_a;  // PUSH does not use it
   if (!push)
     if (int rc = make_map_out16(&map_out, out, (uint64_t)N, (uint64_t)total_rows, (uint64_t)ldc * 2, 32, 32)) return rc;
+  alignas(64) CUtensorMap map_rows = map_a;
+  if (grouped) {
+    const uint64_t dims[2] = {(uint64_t)K, (uint64_t)total_rows};
+    const uint64_t str[1] = {(uint64_t)lda};
+    if (int rc = make_map_sw128(&map_rows, a, 2, dims, str, kRowBox, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)) return rc;
+  }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (grouped) {
     if (int rc = set_smem_attr_once<true, false>()) return rc;
     // an upper bound on the tile count without reading the device: every expert can add one ragged m-tile
     const int64_t max_tiles = ((total_rows + BM - 1) / BM + num_experts) * p.n_tiles;
     const int grid = (int)(max_tiles < di.sm_count ? max_tiles : di.sm_count);
-    fp8_block_gemm_kernel<true, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_out, static_cast<const GemmParams&>(p));
+    fp8_block_gemm_kernel<true, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_out, map_rows, static_cast<const GemmParams&>(p));
   } else if (push) {
     if (int rc = set_smem_attr_once<false, true>()) return rc;
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
     const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
-    fp8_block_gemm_kernel<false, true><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_out, p);
+    fp8_block_gemm_kernel<false, true><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_out, map_rows, p);
   } else {
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles * p.k_splits;
     const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
@@ -1371,14 +1384,14 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
     // its first weights meanwhile, as the few-rows kernel does.  Above, that gained 1 % at 777 rows and cost 3 to 7 % at 8192.
     p.early_next = total_rows <= smallm_max_rows();
     if (p.early_next) {
-      const cudaError_t e = launch_pdl(fp8_block_gemm_kernel<false, false>, dim3(grid), dim3(kThreads), kSmemBytes, st, map_a, map_b, map_out,
+      const cudaError_t e = launch_pdl(fp8_block_gemm_kernel<false, false>, dim3(grid), dim3(kThreads), kSmemBytes, st, map_a, map_b, map_out, map_rows,
                                        static_cast<const GemmParams&>(p));
       if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(SGLB200_ERR_LAUNCH, "fp8_block_gemm_kernel: %s", cudaGetErrorString(e));
       }
     } else {
-      fp8_block_gemm_kernel<false, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_out, static_cast<const GemmParams&>(p));
+      fp8_block_gemm_kernel<false, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_out, map_rows, static_cast<const GemmParams&>(p));
     }
     if (p.partial != nullptr) {
       SGLB_CHECK_LAUNCH("fp8_block_gemm_kernel");
@@ -1942,7 +1955,7 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm_allreduce(const void* a, const vo
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   const int64_t gemm_ctas = tiles < di.sm_count - comm_ctas ? tiles : di.sm_count - comm_ctas;
   const int grid = (int)gemm_ctas + comm_ctas;
-  void* args[] = {(void*)&map_a, (void*)&map_b, (void*)&map_a /* no TMA store in this form */, (void*)&p};
+  void* args[] = {(void*)&map_a, (void*)&map_b, (void*)&map_a /* no TMA store */, (void*)&map_a /* no experts */, (void*)&p};
   e = cudaLaunchCooperativeKernel((const void*)fp8_block_gemm_kernel<false, false, true>, dim3(grid), dim3(kThreads), args,
                                   kSmemBytes, st);
   if (e != cudaSuccess) {

@@ -188,7 +188,7 @@ __device__ __forceinline__ void store32(const uint32_t (&a)[32], const OutT* bia
 template <bool GROUPED, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                      const Params p) {
+                      const __grid_constant__ CUtensorMap map_rows, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sf_smem = smem + (size_t)kStages * kStageBytes;
@@ -282,7 +282,13 @@ fp8_ue8m0_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           if (leader) {
             const uint32_t dst = stage0 + stage * kStageBytes;
             ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, kStageBytes);
-            ptx::tma_load_2d_a(dst, &map_a, full0 + stage * 8, kb * BK, tl.m0);
+            if (GROUPED && tl.row_end - tl.m0 <= BM - kRowBox) {
+              // the end of an expert: rows that belong to nobody here come as zeros, from outside the tensor (see kRowBox)
+              for (int32_t r = 0; r < BM; r += kRowBox)
+                ptx::tma_load_2d_a(dst + r * BK, &map_rows, full0 + stage * 8, kb * BK, tl.m0 + r < tl.row_end ? tl.m0 + r : p.M);
+            } else {
+              ptx::tma_load_2d_a(dst, &map_a, full0 + stage * 8, kb * BK, tl.m0);
+            }
             ptx::tma_load_3d_a(dst + kTileABytes, &map_b, full0 + stage * 8, kb * BK, tl.n0, tl.expert);
           }
         }
@@ -589,6 +595,13 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
     if (int rc = make_map_sw128(&map_b, b, 3, dims, str, BN, CU_TENSOR_MAP_L2_PROMOTION_L2_256B)) return rc;
   }
 
+  alignas(64) CUtensorMap map_rows = map_a;
+  if (grouped) {
+    const uint64_t dims[2] = {(uint64_t)K, (uint64_t)M};
+    const uint64_t str[1] = {(uint64_t)lda};
+    if (int rc = make_map_sw128(&map_rows, a, 2, dims, str, kRowBox, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)) return rc;
+  }
+
   Params p;
   p.sfa = sfa;
   p.sfb = sfb;
@@ -634,16 +647,16 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
     // an upper bound on the tile count without reading the device: every expert can add one ragged m-tile
     const int64_t max_tiles = ((M + BM - 1) / BM + num_experts) * p.n_tiles;
     const int grid = (int)(max_tiles < di.sm_count ? max_tiles : di.sm_count);
-    fp8_ue8m0_gemm_kernel<true, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
+    fp8_ue8m0_gemm_kernel<true, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_rows, p);
   } else {
     const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles * p.k_splits;
     const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
     if (p.k_splits > 1) {
-      fp8_ue8m0_gemm_kernel<false, true><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
+      fp8_ue8m0_gemm_kernel<false, true><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_rows, p);
       SGLB_CHECK_LAUNCH("fp8_ue8m0_gemm_kernel");
       launch_splitk_reduce(p.partial, out, bias, M, N, ldc, p.k_splits, out_dtype, di.sm_count, stream);
     } else {
-      fp8_ue8m0_gemm_kernel<false, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, p);
+      fp8_ue8m0_gemm_kernel<false, false><<<grid, kThreads, kSmemBytes, st>>>(map_a, map_b, map_rows, p);
     }
   }
   SGLB_CHECK_LAUNCH("fp8_ue8m0_gemm_kernel");

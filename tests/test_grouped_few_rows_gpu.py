@@ -186,3 +186,47 @@ def test_fused_experts_decode_sizes_same_bits_on_both_kernels(tokens):
     assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
     ref = oracle.fused_experts_block_fp8(x, w13, w2, w13s, w2s, tw, ti)
     assert_gemm_close(outs[0], ref, f"fused experts, {tokens} tokens")
+
+
+ROW_ENDS = [1, 31, 0, 32, 33, 64, 95, 96, 97, 127, 128, 129, 224, 225, 5]  # both sides of each box of 32 rows, the last expert short
+
+
+def test_tile_kernel_at_the_ends_of_experts():
+    """A tile that an expert's end cuts loads its rows in boxes of 32 and zeros behind them, and stores blocks of 32 rows whole
+    or by the row.  fp32 scales: bit for bit what the few-rows kernel gives, and the oracle's."""
+    N, K, rows = 384, 896, sum(ROW_ENDS)
+    aq, a_s = oracle.per_token_group_quant_fp8(make_activations(rows, K, seed=1), 128)
+    wq, wsc = _weights(len(ROW_ENDS), N, K, seed=2)
+    with few_rows_limit(0):
+        tiled, offs = _run_sorted(aq, a_s, wq, wsc, ROW_ENDS)
+    with few_rows_limit(64):  # 85 rows an expert on average: above its limit, so expert by expert
+        for e, n in enumerate(ROW_ENDS):
+            if 0 < n <= 64:
+                one, _ = _run_sorted(aq[offs[e]:offs[e + 1]], a_s[offs[e]:offs[e + 1]], wq[e:e + 1], wsc[e:e + 1], [n])
+                assert torch.equal(one[:n].view(torch.int16), tiled[offs[e]:offs[e + 1]].view(torch.int16)), n
+    assert (tiled[rows:] == 7.0).all()
+    ref = torch.cat([oracle.w8a8_block_fp8_matmul(aq[offs[e]:offs[e + 1]], wq[e], a_s[offs[e]:offs[e + 1]], wsc[e])
+                     for e in range(len(ROW_ENDS)) if ROW_ENDS[e]])
+    assert_gemm_close(tiled[:rows], ref, "ends of experts", allow_one_ulp=True)
+
+
+def test_ue8m0_tile_kernel_at_the_ends_of_experts():
+    from sglang_b200._lib import check, lib
+    from sglang_b200.layers.quantization import pack_ue8m0_scales
+    N, K, rows, E = 264, 896, sum(ROW_ENDS), len(ROW_ENDS)
+    aq, a_s = oracle.per_token_group_quant_fp8(make_activations(rows, K, seed=1), 128, scale_ue8m0=True)
+    wq, wsc = _weights(E, N, K, seed=2, ue8m0=True)
+    offs = np.concatenate([[0], np.cumsum(ROW_ENDS)]).astype(np.int32)
+    a, w, sa = aq.cuda(), wq.cuda(), pack_ue8m0_scales(a_s).cuda()
+    sw = pack_ue8m0_scales(wsc.view(-1, wsc.shape[2]).cuda()).view(E, wsc.shape[1], -1)
+    out, o = torch.full((rows + 3, N), 7.0, dtype=torch.bfloat16, device="cuda"), torch.from_numpy(offs).cuda()
+    with few_rows_limit(0):
+        check(lib().sglb200_fp8_ue8m0_scaled_grouped_mm(a.data_ptr(), w.data_ptr(), sa.data_ptr(), sw.data_ptr(), out.data_ptr(), o.data_ptr(),
+                                                        rows, E, N, K, K, K, N * K, N, sa.stride(0), sa.stride(1), sw.stride(0), sw.stride(1),
+                                                        sw.stride(2), 0, torch.cuda.current_stream().cuda_stream), "grouped mm")
+        torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    assert (out[rows:] == 7.0).all()
+    ref = torch.cat([oracle.w8a8_block_fp8_matmul(aq[offs[e]:offs[e + 1]], wq[e], a_s[offs[e]:offs[e + 1]], wsc[e])
+                     for e in range(E) if ROW_ENDS[e]])
+    assert_gemm_close(out[:rows], ref, "ends of experts, UE8M0", allow_one_ulp=True)
