@@ -34,14 +34,6 @@ int make_map_f32(CUtensorMap* map, const void* base, uint64_t cols, uint64_t row
 // Tensor map of a [rows][cols] tensor of 16-bit results for TMA stores.  Defined in gemm.cu.
 int make_map_out16(CUtensorMap* map, void* base, uint64_t cols, uint64_t rows, uint64_t stride_bytes, uint32_t box_cols, uint32_t box_rows);
 
-// Grouped tile kernels: the rows of a tile that an expert's end cuts are loaded in boxes of so many, those past the end from
-// outside the tensor, as zeros.  The tensor core multiplies them all the same, but products of zeros cost it little power, and
-// power is what bounds an expert layer: with the next experts' rows in their place 256 x 7168 x 2048 at 4096 tokens (half of
-// the tiles such ends) took 3750 us, now 3540, and on a UE8M0 checkpoint at 1021 tokens (every tile) 1659, now 1587.  Running those
-// tiles on swapped operands instead, 128 weight rows by 32 or 64 tokens, was level with the former: the chain of a k-block is
-// as long, and the ordinary tiles' loop compiled worse beside it.
-constexpr int kRowBox = 32;
-
 // The few-rows (M <= smallm_max_rows()) weight-streaming GEMM, gemm_smallm.cu
 int smallm_max_rows();
 constexpr int kMaxCluster = 8;

@@ -89,6 +89,13 @@ constexpr size_t kStagingBytes = (size_t)kEpiWarps * 32 * kStageWords * sizeof(u
 constexpr size_t kStagingOffset = (size_t)kStages * kStageBytes;
 constexpr size_t kCtlOffset = kStagingOffset + kStagingBytes;
 constexpr size_t kScaleOffset = (kCtlOffset + 256 /*barriers*/ + (kMaxExperts + 1) * sizeof(int32_t) + 15) / 16 * 16;
+// Grouped: the rows of a tile that an expert's end cuts are loaded in boxes of so many, those past the end from
+// outside the tensor, as zeros.  The tensor core multiplies them all the same, but products of zeros cost it little power, and
+// power is what bounds an expert layer: with the next experts' rows in their place 256 x 7168 x 2048 at 4096 tokens (half of
+// the tiles such ends) took 3750 us, now 3540,.  Boxes of 16 keep the one producer too long (3610).  Running those
+// tiles on swapped operands instead, 128 weight rows by 32 or 64 tokens, was level with the former: the chain of a k-block is
+// as long, and the ordinary tiles' loop compiled worse beside it.
+constexpr int kRowBox = 32;
 constexpr int kNotes = 8;  // TileNote ring: the scale loader is at most kScaleStages tiles (of one group) ahead
 constexpr size_t kNoteOffset = kScaleOffset + (size_t)kScaleStages * BM * sizeof(float4);
 constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + kNoteOffset + kNotes * 16;

@@ -188,11 +188,11 @@ def test_fused_experts_decode_sizes_same_bits_on_both_kernels(tokens):
     assert_gemm_close(outs[0], ref, f"fused experts, {tokens} tokens")
 
 
-ROW_ENDS = [1, 31, 0, 32, 33, 64, 95, 96, 97, 127, 128, 129, 224, 225, 5]  # both sides of each box of 32 rows, the last expert short
+ROW_ENDS = [1, 16, 17, 31, 0, 32, 33, 64, 95, 96, 97, 112, 113, 127, 128, 129, 224, 225, 5]  # both sides of the boxes of 16 and 32 rows
 
 
 def test_tile_kernel_at_the_ends_of_experts():
-    """A tile that an expert's end cuts loads its rows in boxes of 32 and zeros behind them, and stores blocks of 32 rows whole
+    """A tile that an expert's end cuts loads its rows in boxes and zeros behind them, and stores blocks of 32 rows whole
     or by the row.  fp32 scales: bit for bit what the few-rows kernel gives, and the oracle's."""
     N, K, rows = 384, 896, sum(ROW_ENDS)
     aq, a_s = oracle.per_token_group_quant_fp8(make_activations(rows, K, seed=1), 128)
