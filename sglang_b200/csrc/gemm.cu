@@ -12,7 +12,7 @@
 //              publish the TMEM stage.
 //   warps 4-11 promotion + epilogue: two warps per TMEM lane quarter, each owning 64 of the tile's 128
 //              columns.  A thread owns one accumulator row: per k-block it pulls its 64 partial sums out
-//              of TMEM (two tcgen05.ld of 32 columns, one wait), multiplies by sa[m,kb] * sb[nb,kb] and
+//              of TMEM (one tcgen05.ld of 64 columns), multiplies by sa[m,kb] * sb[nb,kb] and
 //              adds into 64 fp32 registers with packed fp32x2 FMAs; after the last k-block it rounds to
 //              bf16/f16 and leaves through shared memory and TMA stores (store_rows).  The scale of a row comes from the scale
 //              loader's ring with one 16-byte load per four k-blocks: with the promotion warps loading sa and sb
@@ -260,9 +260,9 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
 }
 
 // acc[j] += v[2j], v[2j+1] * scale, two columns per instruction
-__device__ __forceinline__ void fma32(float2* acc, const uint32_t (&v)[32], float2 scale2) {
+__device__ __forceinline__ void fma64(float2* acc, const uint32_t (&v)[64], float2 scale2) {
 #pragma unroll
-  for (int j = 0; j < 16; ++j)
+  for (int j = 0; j < 32; ++j)
     acc[j] = __ffma2_rn(make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), scale2, acc[j]);
 }
 
@@ -678,17 +678,14 @@ fp8_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
               break;
             }
             ptx::tc_fence_after();
-            uint32_t va[32], vb[32];
-            ptx::tmem_ld_32x32(taddr, va);
-            ptx::tmem_ld_32x32(taddr + 32, vb);
-            ptx::tmem_ld_wait(va);
-            ptx::tmem_ld_wait(vb);
+            uint32_t v[64];
+            ptx::tmem_ld_32x64(taddr, v);
+            ptx::tmem_ld_wait(v);
             // every TMEM read of this stage has landed: hand the stage back to the MMA warp
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive_a(acc_empty0 + acc_stage * 8);
-            fma32(acc, va, scale2);
-            fma32(acc + 16, vb, scale2);
+            fma64(acc, v, scale2);
           }
           if (++acc_stage == kAccStages) { acc_stage = 0; acc_phase ^= 1; }
         }

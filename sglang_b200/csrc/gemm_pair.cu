@@ -9,7 +9,7 @@
 // Why pairs: the 128 x 128 tiles of gemm.cu need 32 KB of operands per SM and k-block, 15.8 TB/s out of L2 at the rate they reach,
 // which is what bounds them at high clocks, and the energy of that traffic is part of what bounds them under the power cap.
 // Here it is 16 KB per 128 x 128 x 128 of work.  Measured (B200, this / the tile kernel): a second of load at the 1000 W cap
-// 8192 x 36864 x 7168 2113 us at 1370 MHz / 2415 at 1245, 8192 x 24576 x 1536 365 / 419; one burst 4096 x 7168 x 7168 192 / 209.
+// 8192 x 36864 x 7168 2112 us / 2450, 8192 x 24576 x 1536 366 / 420; one burst 4096 x 7168 x 7168 187 / 212.
 //
 // Per CTA, 384 threads, warp-specialised:
 //   warp 0      TMA producer: per k-block A [128 x 128 B], two boxes of B [64 x 128 B] and the 128 activation scales into a 5-stage
@@ -105,9 +105,9 @@ __device__ __forceinline__ uint32_t pack16(float a, float b, int out_dtype) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-__device__ __forceinline__ void fma32(float2* acc, const uint32_t (&v)[32], float2 scale2) {
+__device__ __forceinline__ void fma64(float2* acc, const uint32_t (&v)[64], float2 scale2) {
 #pragma unroll
-  for (int j = 0; j < 16; ++j)
+  for (int j = 0; j < 32; ++j)
     acc[j] = __ffma2_rn(make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), scale2, acc[j]);
 }
 
@@ -192,17 +192,14 @@ fp8_block_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
         }
         ptx::tc_fence_after();
         const uint32_t taddr = tlane + acc_stage * 128;
-        uint32_t va[32], vb[32];
-        ptx::tmem_ld_32x32(taddr, va);
-        ptx::tmem_ld_32x32(taddr + 32, vb);
+        uint32_t v[64];
+        ptx::tmem_ld_32x64(taddr, v);
         const float scale = ptx::ld_shared_f32(sc0 + slot) * b;
         const float2 s2 = make_float2(scale, scale);
-        ptx::tmem_ld_wait2(va, vb);
-        fma32(acc, va, s2);
-        ptx::tmem_ld_32x32_reuse(taddr + 64, va);
-        fma32(acc + 16, vb, s2);
-        ptx::tmem_ld_32x32_reuse(taddr + 96, vb);
-        ptx::tmem_ld_wait2(va, vb);
+        ptx::tmem_ld_wait(v);
+        fma64(acc, v, s2);
+        ptx::tmem_ld_32x64_reuse(taddr + 64, v);
+        ptx::tmem_ld_wait(v);
         ptx::tc_fence_before();
         __syncwarp();
         ptx::mbar_arrive_cluster_if(lead_acc_empty0 + acc_stage * 8, leader);
@@ -214,8 +211,7 @@ fp8_block_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
         if (((kb + 1) & 31) == 0) sb_now = __ldg(sb + (int64_t)min(kb + 1 + lane, p.k_tiles - 1) * p.sb_stride_k);
         b = __shfl_sync(0xffffffffu, sb_now, (kb + 1) & 31);
         slot = slot == (kScaleSlots - 1) * kSlotBytes ? 0 : slot + kSlotBytes;
-        fma32(acc + 32, va, s2);
-        fma32(acc + 48, vb, s2);
+        fma64(acc + 32, v, s2);
       }
       if (!ok || ctl->abort_flag) break;
       // 64 columns per pass: a lane's row of 128 bytes into the warp's swizzled staging, from there one TMA store (which leaves out
