@@ -1306,7 +1306,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
 
   const int splits = !grouped && !push && workspace != nullptr ? dense_splits(total_rows, N, K, di.sm_count) : 1;
   const bool split = splits > 1 && (int64_t)splits * total_rows * N <= workspace_floats;
-  if (!grouped && !push && !split && allow_pairs && pair_takes_scales(sa, sa_stride_m, sa_stride_k) &&
+  if (!grouped && !push && !split && allow_pairs && pair_takes_scales(sa, total_rows, sa_stride_m, sa_stride_k) &&
       pair_preferred(total_rows, N, K, di.sm_count))
     return pair_gemm(a, b, sa, sb, out, total_rows, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k, out_dtype,
                      bias, di.sm_count, stream);

@@ -329,9 +329,10 @@ fp8_block_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
 
 }  // namespace
 
-// Activation scales that the kernel's TMA copies can fetch: M-major, whole 16-byte units.
-bool pair_takes_scales(const float* sa, int64_t sa_stride_m, int64_t sa_stride_k) {
-  return sa_stride_m == 1 && sa_stride_k > 0 && sa_stride_k % 4 == 0 && aligned(sa, 16);
+// Activation scales that the kernel's TMA copies can fetch: M-major, whole 16-byte units, columns that do not overlap (a tensor map's
+// strides are not smaller than its rows).
+bool pair_takes_scales(const float* sa, int64_t M, int64_t sa_stride_m, int64_t sa_stride_k) {
+  return sa_stride_m == 1 && sa_stride_k >= M && sa_stride_k % 4 == 0 && aligned(sa, 16);
 }
 
 // Dense GEMM on CTA pairs; arguments as gemm_common's dense case (checked there), scales as above.
@@ -415,7 +416,7 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm_pair(const void* a, const void* b
   if (int rc = device_info(&di)) return rc;
   SGLB_REQUIRE(di.cc_major == 10, SGLB200_ERR_ARCH, "compute capability %d.%d: this library is built for sm_100a only",
                di.cc_major, di.cc_minor);
-  if (di.sm_count < 2 || !pair_takes_scales(sa, sa_stride_m, sa_stride_k))  // the same bits from the 128 x 128 tiles
+  if (di.sm_count < 2 || !pair_takes_scales(sa, M, sa_stride_m, sa_stride_k))  // the same bits from the 128 x 128 tiles
     return tile_gemm(a, b, sa, sb, out, M, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k, out_dtype, stream);
   return pair_gemm(a, b, sa, sb, out, M, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k,
                    out_dtype, nullptr, di.sm_count, stream);

@@ -67,7 +67,7 @@ constexpr int kGroupM = 16;
 constexpr int kMaxExperts = 1024;
 // Grouped: the rows of a tile that an expert's end cuts are loaded in boxes of so many, those past the end from outside the tensor,
 // as zeros, which cost the tensor core little power: 256 x 7168 x 2048 at 1021 tokens (every tile) 1659 -> 1587 us in boxes of 32 and,
-// on another box, 1820 -> 1725 in boxes of 16, for which two producers have the time.
+// on another GPU, 1820 -> 1725 in boxes of 16, for which two producers have the time.
 constexpr int kRowBox = 16;
 constexpr size_t kSmemBytes = 1024 + (size_t)kStages * kStageBytes + (size_t)kSfBufs * kSfBufBytes + 256 +
                               (kMaxExperts + 1) * sizeof(int32_t);

@@ -103,6 +103,21 @@ def test_pair_gemm_edges_of_tiles_bit_for_bit(M, N, K, out_dtype):
     assert torch.equal(bits(out), bits(plain))  # the three rows behind the output included
 
 
+@pytest.mark.parametrize("step", [4, 8, 128])
+def test_scales_whose_columns_overlap_stay_on_the_tiles(step):
+    # M-major scales with a column stride below M, which a tensor map's strides do not describe: the same bits as from a copy of them
+    M, N, K = 132, 256, 1024
+    aq, _ = oracle.per_token_group_quant_fp8(make_activations(M, K, seed=1), 128)
+    wq, ws = make_weight(N, K, seed=2)
+    buf = torch.rand(M + 7 * step, generator=torch.Generator().manual_seed(3)).cuda() * 0.1
+    s = buf.as_strided((M, 8), (1, step))
+    aq_d, wq_d, ws_d = aq.cuda(), wq.cuda(), ws.cuda()
+    out, want = _pair(aq_d, s, wq_d, ws_d, 256), _pair(aq_d, s.contiguous(), wq_d, ws_d, 256)
+    torch.cuda.synchronize()
+    assert torch.equal(bits(out), bits(want))
+    assert_gemm_close(out, oracle.w8a8_block_fp8_matmul(aq, wq, s.cpu().contiguous(), ws), f"step={step}")
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_linear_layer_on_pairs_adds_its_bias(dtype):
     # 3072 x 4096 x 4096 is a size the plain entry gives to the pairs; through row-major scales it stays on the 128 x 128 tiles
