@@ -1200,20 +1200,21 @@ int dense_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
 }
 
 // Whether CTA pairs (gemm_pair.cu, 256 x 256 tiles) take a dense call that leaves K whole, or the 128 x 128 tiles here.  Cost model
-// in nanoseconds (runs of one call at a time, 11 layers of N = 576 to 36864, K = 1024 to 16384, 160 to 4096 rows): a k-block
-// takes a pair 505 and a CTA of the tile kernel 295, the end of a tile 2000 and 1000; the pair kernel starts 2500 later.  Mostly
-// it decides by waves: N=4096 K=4096 M=3072 48.5 against 53.7 us (pair / tile), M=1536 34.1 against 28.2; N=24576 K=1536 M=4096 165
-// against 188, M=640 31.6 against 29.8; N=1536 K=7168 M=1536 28 against 17.  Under sustained load at the power cap the pairs gain
-// 12 % more, because they move half of the operand bytes (figures in gemm_pair.cu): calls of more than 2e11 operations, which take
-// 100 us and more, go to them while the model has them up to 6 % behind, smaller ones where it has them 2 % ahead.
+// in nanoseconds (runs of one call at a time, 11 layers of N = 576 to 36864, K = 1024 to 16384, 160 to 4096 rows; the choice is
+// within 0.1 % of the better kernel on average, 5 % at most): a k-block takes a pair 510 and a CTA of the tile kernel 295, the
+// end of a tile 1500 and 1000; the pair kernel starts 1500 later.  Mostly it decides by waves: N=4096 K=4096 M=4096 62.5 against
+// 66.8 us (pair / tile), M=1024 18.8 against 19.6, M=1536 32.5 against 27.5; N=7168 K=2048 M=4096 60.8 against 66.2; N=24576 K=1536
+// M=4096 154 against 170, M=640 30.2 against 28.2; N=1536 K=7168 M=1536 27 against 17.  Under sustained load at the power cap the
+// pairs gain more, because they move half of the operand bytes (figures in gemm_pair.cu): calls of more than 2e11 operations,
+// which take 100 us and more, go to them while the model has them up to 4 % behind.
 bool pair_preferred(int64_t M, int64_t N, int64_t K, int sm_count) {
   if (sm_count < 2) return false;
   const int64_t kb = (K + BK - 1) / BK, pairs = sm_count / 2;
   const int64_t waves2 = (((M + 255) / 256) * ((N + 255) / 256) + pairs - 1) / pairs;
   const int64_t waves1 = (((M + BM - 1) / BM) * ((N + BN - 1) / BN) + sm_count - 1) / sm_count;
-  const int64_t cost2 = 2500 + waves2 * (kb * 505 + 2000), cost1 = waves1 * (kb * 295 + 1000);
+  const int64_t cost2 = 1500 + waves2 * (kb * 510 + 1500), cost1 = waves1 * (kb * 295 + 1000);
   const bool sustained = 2.0 * (double)M * (double)N * (double)K > 2e11;
-  return cost2 * 100 < cost1 * (sustained ? 106 : 98);
+  return cost2 * 100 < cost1 * (sustained ? 104 : 100);
 }
 
 template <bool GROUPED, bool PUSH>

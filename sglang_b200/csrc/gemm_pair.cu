@@ -21,8 +21,8 @@
 //               columns each.  acc += partial * scale in fp32 registers (packed FMAs); the TMEM stage is handed back by an arrival
 //               on the even CTA's `acc_empty` barrier; results leave through swizzled shared memory and TMA stores.
 // What bounds it: the two TMEM stages a half has, times the time a stage is away (about 1100 cycles from the issue of its MMAs
-// to the promotion warps' seeing them, the other half's MMAs among them, 450 of reading, 150 of hand-back): 900 to 950 cycles
-// per k-block against 512 of MMA.  Sixteen promotion warps of 64 columns, one 256-column stage for both halves, and 256 x 128
+// to the promotion warps' seeing them, the other half's MMAs among them, then reading and 150 of hand-back): 767 cycles per
+// k-block against 512 of MMA at 2048 x 36864 x 7168 (70 % tensor pipe; 900 to 950 with loads of 32 columns in turn).  Sixteen promotion warps of 64 columns, one 256-column stage for both halves, and 256 x 128
 // tiles with four stages are level or slower (549, 542 and 587 ns per 256 x 256 x 128 against 535 at the time).
 // Scales: a warp that wrote the products sa * sb into a ring of its own, with two more barriers, cost 150 ns of 620 per k-block in
 // shared-memory and barrier latency of the promotion warps; the TMA copy shares the operands' barrier, and sb (one value per

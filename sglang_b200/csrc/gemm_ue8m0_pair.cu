@@ -8,6 +8,8 @@
 // Why pairs: the single-CTA kernel moves 45 KB of operands per SM and k-block, 14.4 TB/s out of L2 at the rate it reaches, and has
 // shared memory for four stages of that; here it is 30 KB and six stages.  Measured in bursts, single-CTA kernel / this: 4096 x
 // 7168 x 18432 426 / 368 us (2942 TFLOP/s), 8192 x 24576 x 1536 421 / 237 (that one's epilogue stores 32 rows an instruction).
+// What bounds it: the tensor pipe, 484 cycles per k-block of which 448 are MMA at 2048 x 36864 x 7168 (97 % of active cycles; the
+// single-CTA kernel 634), and the power cap.
 //
 // Per CTA, 384 threads: warp 0 TMA producer; warps 1 and 3 scale loaders (per group of four k-blocks the packed exponent words of 128 A rows
 // and 224 B rows, in the arrangement of tcgen05.cp.32x128b.warpx4); warp 2 MMA issuer (even CTA only; one thread issues copies,
