@@ -154,10 +154,11 @@ int sglb200_group_quant_fp8_batched(const void* input, int in_dtype, void* out_q
  * K need not be a multiple of 128 (the tail block is zero-filled), but K % 16 == 0.
  * fp32 accumulation; each 128-deep partial product is scaled and added in registers.
  * Any M >= 0 is accepted with no padding copy (the reference pads M to a multiple of 4).
- * Up to 128 rows the weight-streaming kernel with swapped operands runs (128 weight rows x up to 16 / 32 / 64 / 128
- * activation rows per MMA), above that the 128 x 128 kernel.  The weight-streaming kernel may be launched beside the end of
- * the kernel before it and then reads the first tiles of `b` at once: b must not be written by a kernel that releases its
- * dependents early (griddepcontrol.launch_dependents).  All other work of the stream is ordered as usual.
+ * Up to 64 rows, and up to 128 where the CTAs of a cluster share K, the weight-streaming kernel with swapped operands runs (128
+ * weight rows x up to 16 / 32 / 64 / 128 activation rows per MMA), above that the kernel on 128 x 128 tiles, or on CTA pairs (256 x
+ * 256) where those are faster and sa is as sglb200_fp8_blockwise_scaled_mm_pair asks.  Up to 128 rows either kernel may be launched
+ * beside the end of the kernel before it and then reads the first tiles of `b` at once: b must not be written by a kernel that
+ * releases its dependents early (griddepcontrol.launch_dependents).  All other work of the stream is ordered as usual.
  */
 int sglb200_fp8_blockwise_scaled_mm(const void* a, const void* b, const float* sa, const float* sb, void* out,
                                     int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc,
@@ -229,9 +230,10 @@ int sglb200_fp8_blockwise_scaled_mm_noalloc(const void* a, const void* b, const 
  * two CTAs that share tcgen05.mma.cta_group::2 over a 256 x 256 output tile.  Each CTA loads its own 128 rows of A and half of the B
  * rows with its own TMA copies (nothing is broadcast): half of the L2 -> shared-memory bytes per flop of the 128 x 128 tiles.
  * sglb200_fp8_blockwise_scaled_mm and its forms choose this kernel themselves where it is the faster one (gemm.cu,
- * pair_preferred); the entry takes it always.  tile_n, 128 or 256, no longer changes anything.  The kernel fetches the
- * activation scales by TMA: where they are not M-major (sa_stride_m == 1) with sa 16-byte aligned and sa_stride_k a multiple
- * of 4, the call runs on the 128 x 128 tiles, with the same bits.  No split-K, no scratch.
+ * pair_preferred).  The kernel fetches the activation scales by TMA, so this entry takes it for every size whose scales are
+ * M-major (sa_stride_m == 1) with sa 16-byte aligned, sa_stride_k a multiple of 4 and sa_stride_k >= M; with scales in any other
+ * layout, the row-major default of the quantiser among them, the call runs on the 128 x 128 tiles, at every size, with the same
+ * bits.  tile_n must be 128 or 256 and changes nothing else.  No split-K, no scratch.
  * Replaces: the 2-SM configuration of the reference's sm_100 kernels
  *           (KernelPtrArrayTmaWarpSpecializedBlockwise2SmSm100, sgl-kernel/csrc/moe/fp8_blockwise_moe_kernel.cu:300-310;
  *           dense launch sgl-kernel/csrc/gemm/fp8_blockwise_gemm_kernel.cu:39-196).

@@ -85,7 +85,7 @@ int pair_gemm(const void* a, const void* b, const float* sa, const float* sb, vo
               int64_t sb_stride_k, int out_dtype, const void* bias, int sm_count, void* stream);
 
 bool pair_takes_scales(const float* sa, int64_t M, int64_t sa_stride_m, int64_t sa_stride_k);
-// The dense GEMM on 128 x 128 tiles (few-rows kernel for few rows), gemm.cu: the pair entry's way out for other scale layouts
+// The dense GEMM on 128 x 128 tiles at any size, K uncut, gemm.cu: the pair entry's way out for other scale layouts
 int tile_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K, int64_t lda,
               int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n, int64_t sb_stride_k,
               int out_dtype, void* stream);

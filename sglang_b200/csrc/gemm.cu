@@ -1237,7 +1237,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
                 int64_t sb_stride_e, int64_t sb_stride_n, int64_t sb_stride_k, int out_dtype, void* stream,
                 float* workspace = nullptr, int64_t workspace_floats = 0, const PushParams* push = nullptr,
                 int64_t rows_per_expert = 0, int64_t sa_stride_e = 0, int64_t expected_rows = 0, const void* bias = nullptr,
-                bool allow_pairs = true) {
+                bool tiles_only = false) {
   const bool grouped = expert_offsets != nullptr || rows_per_expert > 0;
   SGLB_REQUIRE(total_rows >= 0 && N >= 0 && K >= 0, SGLB200_ERR_SHAPE, "M=%lld N=%lld K=%lld: negative size",
                (long long)total_rows, (long long)N, (long long)K);
@@ -1290,7 +1290,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
     SGLB_CHECK_LAUNCH("splitk_reduce_push_kernel");
     return SGLB200_OK;
   }
-  if (!grouped && !push && takes_few_rows(total_rows, N, K, di.sm_count)) {
+  if (!grouped && !push && !tiles_only && takes_few_rows(total_rows, N, K, di.sm_count)) {
     // few rows: the weight-streaming kernel with swapped operands (gemm_smallm.cu)
     return smallm_gemm(a, b, sa, sb, out, total_rows, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k,
                        out_dtype, bias, nullptr, 0, di.sm_count, stream, nullptr, false);
@@ -1307,7 +1307,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
 
   const int splits = !grouped && !push && workspace != nullptr ? dense_splits(total_rows, N, K, di.sm_count) : 1;
   const bool split = splits > 1 && (int64_t)splits * total_rows * N <= workspace_floats;
-  if (!grouped && !push && !split && allow_pairs && pair_takes_scales(sa, total_rows, sa_stride_m, sa_stride_k) &&
+  if (!grouped && !push && !split && !tiles_only && pair_takes_scales(sa, total_rows, sa_stride_m, sa_stride_k) &&
       pair_preferred(total_rows, N, K, di.sm_count))
     return pair_gemm(a, b, sa, sb, out, total_rows, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k, out_dtype,
                      bias, di.sm_count, stream);
@@ -1387,7 +1387,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
     if (int rc = set_smem_attr_once<false, false>()) return rc;
     // Up to smallm_max_rows() rows, one or two waves that wait for weights, the kernel starts beside the quantiser and requests
     // its first weights meanwhile, as the few-rows kernel does.  Above, that gained 1 % at 777 rows and cost 3 to 7 % at 8192.
-    p.early_next = total_rows <= smallm_max_rows();
+    p.early_next = total_rows <= smallm_max_rows() && !tiles_only;
     if (p.early_next) {
       const cudaError_t e = launch_pdl(fp8_block_gemm_kernel<false, false>, dim3(grid), dim3(kThreads), kSmemBytes, st, map_a, map_b, map_out, map_rows,
                                        static_cast<const GemmParams&>(p));
@@ -1409,12 +1409,12 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
 
 }  // namespace
 
-// The dense GEMM without the CTA pairs
+// The dense GEMM on the 128 x 128 tiles whatever its size, K uncut, started after the kernel before it has ended
 int tile_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K, int64_t lda,
               int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n, int64_t sb_stride_k,
               int out_dtype, void* stream) {
   return gemm_common(a, b, sa, sb, out, nullptr, nullptr, M, 1, N, K, lda, ldb, 0, ldc, sa_stride_m, sa_stride_k, 0, sb_stride_n, sb_stride_k,
-                     out_dtype, stream, nullptr, 0, nullptr, 0, 0, 0, nullptr, false);
+                     out_dtype, stream, nullptr, 0, nullptr, 0, 0, 0, nullptr, true);
 }
 }  // namespace sglb
 

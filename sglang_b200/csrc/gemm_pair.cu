@@ -416,7 +416,9 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm_pair(const void* a, const void* b
   if (int rc = device_info(&di)) return rc;
   SGLB_REQUIRE(di.cc_major == 10, SGLB200_ERR_ARCH, "compute capability %d.%d: this library is built for sm_100a only",
                di.cc_major, di.cc_minor);
-  if (di.sm_count < 2 || !pair_takes_scales(sa, M, sa_stride_m, sa_stride_k))  // the same bits from the 128 x 128 tiles
+  // The same bits from the 128 x 128 tiles, which add K in the same order at every size.  Not the plain entry's choice: for few rows
+  // that is the few-rows kernel, whose clusters add ranges of K (16 x 7168 x 16384: 14 of 114688 results one rounding apart).
+  if (di.sm_count < 2 || !pair_takes_scales(sa, M, sa_stride_m, sa_stride_k))
     return tile_gemm(a, b, sa, sb, out, M, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k, out_dtype, stream);
   return pair_gemm(a, b, sa, sb, out, M, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k,
                    out_dtype, nullptr, di.sm_count, stream);

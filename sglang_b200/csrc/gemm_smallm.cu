@@ -825,7 +825,8 @@ int smallm_quant_rows() { return kQuantRows; }
 // the call (GEMM alone in a replayed graph, this / the tile kernel, us: 113 x 10240 x 8192 27.5/20.3, 65 x 36864 x 7168 48.6/46.6,
 // 128 x 57344 x 8192 108/94, 128 x 24576 x 1536 16.9/12.3, 100 x 5120 x 2560 11.6/9.8).  Where clusters share K most SMs
 // would be idle without them, and a split through memory is no faster (M = 96, weights from HBM: N=4096 K=4096 11.6/12.7, N=7168
-// K=16384 32.7/30.3) and needs scratch.  Both add k-blocks in the same order, so that the bits do not depend on the choice.
+// K=16384 32.7/30.3) and needs scratch.  Where no cluster shares K both add k-blocks in the same order, so that the bits are the
+// few-rows kernel's either way.
 bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count) {
   return M <= 64 || (M <= smallm_max_rows() && smallm_cluster(M, N, K, sm_count) > 1);
 }

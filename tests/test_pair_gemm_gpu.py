@@ -103,6 +103,33 @@ def test_pair_gemm_edges_of_tiles_bit_for_bit(M, N, K, out_dtype):
     assert torch.equal(bits(out), bits(plain))  # the three rows behind the output included
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 576, 7168), (16, 7168, 16384), (64, 1024, 8192), (100, 2112, 7168), (128, 5120, 2560)])
+def test_other_scale_layouts_give_the_pairs_bits_at_few_rows(M, N, K):
+    # sizes at which the plain entry adds K in ranges (clusters of the few-rows kernel): scales that the pairs do not take, and a limit
+    # of one SM, send the call to the 128 x 128 tiles, which add it in the pairs' order
+    from sglang_b200._lib import check, lib
+    from sglang_b200.layers.quantization import block_quant_weight_fp8, sglang_per_token_group_quant_fp8
+    g = torch.Generator(device="cuda").manual_seed(M)
+    q, s = sglang_per_token_group_quant_fp8(torch.randn(M, K, generator=g, device="cuda").bfloat16(), 128, column_major_scales=True,
+                                            scale_tma_aligned=True)
+    wq, ws = block_quant_weight_fp8(torch.randn(N, K, generator=g, device="cuda") * 0.02)
+    want = _pair(q, s, wq, ws, 256)
+    ld = (M + 3) // 4 * 4
+    odd = torch.empty(1 + K // 128 * ld, device="cuda").as_strided((M, K // 128), (1, ld), 1)
+    odd.copy_(s)  # M-major, off the 16-byte boundary
+    got = [_pair(q, scales, wq, ws, 256) for scales in (s.contiguous(), odd)]
+    check(lib().sglb200_set_num_sms(1), "set_num_sms")
+    try:
+        got.append(_pair(q, s, wq, ws, 256))
+    finally:
+        lib().sglb200_set_num_sms(0)
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    ref = oracle.w8a8_block_fp8_matmul(q.cpu(), wq[:256].cpu(), s.cpu().contiguous(), ws[:2].cpu())
+    assert_gemm_close(want[:, :256], ref, f"pair M={M} N={N} K={K}")
+    assert all(torch.equal(bits(o), bits(want)) for o in got)
+
+
 @pytest.mark.parametrize("step", [4, 8, 128])
 def test_scales_whose_columns_overlap_stay_on_the_tiles(step):
     # M-major scales with a column stride below M, which a tensor map's strides do not describe: the same bits as from a copy of them
