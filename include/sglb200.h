@@ -45,6 +45,11 @@ extern "C" {
 
 const char* sglb200_status_string(int status);
 const char* sglb200_last_error_detail(void);
+/*
+ * Name of the GEMM kernel that the calling thread launched last through this library ("" before the first): which kernel a size
+ * was given to is decided inside the calls.  Host state, no synchronisation; a replayed CUDA graph launches without it.
+ */
+const char* sglb200_last_gemm_kernel(void);
 /* Library version, "major.minor". */
 const char* sglb200_version(void);
 
@@ -490,8 +495,8 @@ int sglb200_moe_sum_reduce(const void* input, void* output, int64_t num_tokens, 
  * 1024 output tiles of 128 x 128; world <= 8.
  * workspace / workspace_bytes: scratch for M <= 128 (size from sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes; 0 for
  * larger M).  With it the few-rows weight-streaming kernel computes fp32 sums (K in the ranges of the plain entry) and
- * a second small kernel adds the ranges, casts and does the pushing and flagging; without it (NULL) the 128-row kernel
- * with the push epilogue runs.  Both produce the bits of the corresponding plain entry point.
+ * a second small kernel adds the ranges, casts and does the pushing and flagging, with the bits of the plain entry; without it
+ * (NULL) the 128-row kernel with the push epilogue runs, which adds K uncut: the plain entry's bits where that does not cut K either.
  * A wait that runs out (a rank that never pushed) leaves its tile unwritten, sets device status 5
  * (sglb200_read_device_status) and does not advance the epoch, so the same exchange can be reduced again once the
  * missing rank has pushed; if only some ranks timed out the group is out of step and the buffers must be set up

@@ -79,6 +79,7 @@ SIGNATURES = {
     "sglb200_read_device_status": [],
     "sglb200_status_string": [_I],
     "sglb200_last_error_detail": [],
+    "sglb200_last_gemm_kernel": [],
     "sglb200_version": [],
     "sglb200_set_num_sms": [_I],
     "sglb200_get_num_sms": [],
@@ -94,7 +95,7 @@ _RESTYPES = {"sglb200_fp8_blockwise_scaled_mm_workspace_bytes": c_int64,
              "sglb200_fp8_blockwise_scaled_mm_noalloc_max_bytes": c_int64,
              "sglb200_fp8_block_linear_scratch_bytes": c_int64,
              "sglb200_fp8_ue8m0_scaled_mm_scratch_bytes": c_int64,
-             "sglb200_fused_experts_scratch_bytes": c_int64, "sglb200_ep_buffer_bytes": c_int64, "sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes": c_int64, "sglb200_peer_flag_bytes": c_int64, "sglb200_nvls_flag_bytes": c_int64, "sglb200_peer_recv_bytes": c_int64, "sglb200_status_string": c_char_p, "sglb200_last_error_detail": c_char_p, "sglb200_version": c_char_p}
+             "sglb200_fused_experts_scratch_bytes": c_int64, "sglb200_ep_buffer_bytes": c_int64, "sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes": c_int64, "sglb200_peer_flag_bytes": c_int64, "sglb200_nvls_flag_bytes": c_int64, "sglb200_peer_recv_bytes": c_int64, "sglb200_status_string": c_char_p, "sglb200_last_error_detail": c_char_p, "sglb200_last_gemm_kernel": c_char_p, "sglb200_version": c_char_p}
 
 _lib = None
 

@@ -17,6 +17,9 @@ int fail(int code, const char* fmt, ...) {
   return code;
 }
 
+static thread_local const char* t_last_gemm = "";
+void note_gemm(const char* kernel) { t_last_gemm = kernel; }
+
 static int g_num_sms_limit = 0;  // 0: no limit
 int g_grouped_few_rows_max = kGroupedFewRowsDefault;  // sglb200_set_grouped_few_rows
 
@@ -64,6 +67,8 @@ const char* sglb200_status_string(int status) {
 }
 
 const char* sglb200_last_error_detail(void) { return sglb::error_buffer(); }
+
+const char* sglb200_last_gemm_kernel(void) { return sglb::t_last_gemm; }
 
 const char* sglb200_version(void) { return "0.2"; }
 

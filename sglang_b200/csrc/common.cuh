@@ -13,6 +13,8 @@ namespace sglb {
 // Thread-local text of the last failed host-side check.
 char* error_buffer();
 int fail(int code, const char* fmt, ...);
+// Name of the GEMM kernel that this thread launched last (sglb200_last_gemm_kernel); a string literal.
+void note_gemm(const char* kernel);
 
 // Number of SMs and compute capability of the current device, cached per device.
 struct DeviceInfo {

@@ -1404,6 +1404,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
     }
   }
   SGLB_CHECK_LAUNCH("fp8_block_gemm_kernel");
+  note_gemm("fp8_block_gemm_kernel");
   return SGLB200_OK;
 }
 
@@ -1967,6 +1968,7 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm_allreduce(const void* a, const vo
     cudaGetLastError();
     return fail(SGLB200_ERR_LAUNCH, "fp8_block_gemm_kernel (fused all-reduce): %s", cudaGetErrorString(e));
   }
+  note_gemm("fp8_block_gemm_kernel");
   return SGLB200_OK;
 }
 

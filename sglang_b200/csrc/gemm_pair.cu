@@ -386,6 +386,7 @@ int pair_gemm(const void* a, const void* b, const float* sa, const float* sb, vo
   if (tiles < pairs) pairs = tiles;
   fp8_block_gemm_pair_kernel<<<(unsigned)(2 * pairs), kThreads, kSmem, static_cast<cudaStream_t>(stream)>>>(map_a, map_b, map_sa, map_out, p);
   SGLB_CHECK_LAUNCH("fp8_block_gemm_pair_kernel");
+  note_gemm("fp8_block_gemm_pair_kernel");
   return SGLB200_OK;
 }
 

@@ -798,6 +798,7 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams
     cudaGetLastError();
     return fail(SGLB200_ERR_LAUNCH, "fp8_block_gemm_smallm_kernel: %s", cudaGetErrorString(le));
   }
+  note_gemm("fp8_block_gemm_smallm_kernel");
   return SGLB200_OK;
 }
 

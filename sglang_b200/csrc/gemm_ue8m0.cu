@@ -664,6 +664,7 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
     }
   }
   SGLB_CHECK_LAUNCH("fp8_ue8m0_gemm_kernel");
+  note_gemm("fp8_ue8m0_gemm_kernel");
   return SGLB200_OK;
 }
 }  // namespace

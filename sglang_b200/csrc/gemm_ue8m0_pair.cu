@@ -420,6 +420,7 @@ int ue8m0_pair_gemm(const void* a, const void* b, const int32_t* sfa, const int3
   if (tiles < pairs) pairs = tiles;
   fp8_ue8m0_gemm_pair_kernel<<<(unsigned)(2 * pairs), kThreads, kSmem, static_cast<cudaStream_t>(stream)>>>(map_a, map_b, map_out, p);
   SGLB_CHECK_LAUNCH("fp8_ue8m0_gemm_pair_kernel");
+  note_gemm("fp8_ue8m0_gemm_pair_kernel");
   return SGLB200_OK;
 }
 

@@ -52,6 +52,12 @@ def max_abs_over_rms(x, ref):
     return float((x - ref).abs().max() / rms)
 
 
+def last_gemm():
+    """Name of the GEMM kernel that this thread launched last."""
+    from sglang_b200._lib import lib
+    return lib().sglb200_last_gemm_kernel().decode()
+
+
 # ----------------------------------------------------------------------------- workloads
 def make_activations(M, K, seed=0, outliers=True, dtype=torch.bfloat16, row_scale=False):
     """Seeded activations ~N(0,1) on the CPU; 1% of entries x50 (the sweep's outliers) and

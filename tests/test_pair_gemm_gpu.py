@@ -5,9 +5,10 @@ import pytest
 import torch
 
 import oracle
-from helpers import assert_gemm_close, bits, make_activations, make_weight
+from helpers import assert_gemm_close, bits, last_gemm, make_activations, make_weight
 
 pytestmark = pytest.mark.gpu
+PAIRS, TILES, FEW_ROWS = "fp8_block_gemm_pair_kernel", "fp8_block_gemm_kernel", "fp8_block_gemm_smallm_kernel"
 
 
 def _pair(aq, a_s, wq, ws, tile_n, out_dtype=torch.bfloat16):
@@ -22,28 +23,27 @@ def _pair(aq, a_s, wq, ws, tile_n, out_dtype=torch.bfloat16):
     return out
 
 
-@pytest.mark.parametrize("tile_n", [128, 256])
 @pytest.mark.parametrize("M,N,K", [(1, 128, 128), (129, 576, 1024), (300, 1536, 384), (2100, 2368, 512),
                                    (512, 4096, 4096)])
-def test_pair_gemm_matches_oracle_and_single_cta_kernel(M, N, K, tile_n):
+def test_pair_gemm_matches_oracle_and_single_cta_kernel(M, N, K):
     from sglang_b200._lib import check, lib
     a = make_activations(M, K, seed=M + N)
     aq, a_s = oracle.per_token_group_quant_fp8(a, 128)
     wq, ws = make_weight(N, K, seed=K + N)
     ref = oracle.w8a8_block_fp8_matmul(aq, wq, a_s, ws)
     aq_d, as_d, wq_d, ws_d = aq.cuda(), a_s.cuda(), wq.cuda(), ws.cuda()
-    if M % 2:
-        as_d = as_d.t().contiguous().t()  # M-major scales
-    out = _pair(aq_d, as_d, wq_d, ws_d, tile_n)
+    out = _pair(aq_d, _m_major(a_s), wq_d, ws_d, 256)
+    assert last_gemm() == PAIRS
     torch.cuda.synchronize()
     assert lib().sglb200_read_device_status() == 0
-    assert_gemm_close(out, ref, f"pair tile_n={tile_n} M={M} N={N} K={K}")
-    if M > 64:  # the plain entry runs the 128 x 128 kernel without a K-split here
+    assert_gemm_close(out, ref, f"pair M={M} N={N} K={K}")
+    if M > 64:  # with row-major scales the plain entry runs the 128 x 128 kernel, and without scratch it leaves K whole
         plain = torch.empty_like(out)
         check(lib().sglb200_fp8_blockwise_scaled_mm(
             aq_d.data_ptr(), wq_d.data_ptr(), as_d.data_ptr(), ws_d.data_ptr(), plain.data_ptr(), M, N, K, K, K, N,
             as_d.stride(0), as_d.stride(1), ws_d.stride(0), ws_d.stride(1), 0, torch.cuda.current_stream().cuda_stream),
             "mm")
+        assert last_gemm() == TILES
         torch.cuda.synchronize()
         assert torch.equal(bits(out), bits(plain))
 
@@ -60,6 +60,7 @@ def test_pair_gemm_full_size_rows_sample_and_f16():
                                        output_dtype=torch.float16)
     for tile_n in (128, 256):
         out = _pair(q, s, wq, ws, tile_n, out_dtype=torch.float16)
+        assert last_gemm() == PAIRS
         torch.cuda.synchronize()
         assert_gemm_close(out[rows], ref, f"pair tile_n={tile_n} full size")
 
@@ -77,7 +78,8 @@ def _m_major(scales):
                                    (2500, 5120, 384), (2304, 12288, 128)])
 def test_pair_gemm_edges_of_tiles_bit_for_bit(M, N, K, out_dtype):
     # tiles cut off in either direction, one to 33 k-blocks (the shuffle of the weight scales wraps at 32), a K tail, more tiles than
-    # pairs, and a dozen tiles of one k-block for every CTA of the other kernel (its ring of tile notes has eight); rows behind the output stay untouched.  Row-major scales send the plain entry to the kernels that the pairs are compared with.
+    # pairs, and a dozen tiles of one k-block for every CTA of the other kernel (its ring of tile notes has eight); rows behind the
+    # output stay untouched.  Row-major scales send the plain entry to the kernels that the pairs are compared with.
     from sglang_b200._lib import check, dtype_code, lib
     kg = (K + 127) // 128
     a = make_activations(M, kg * 128, seed=M + N)
@@ -92,9 +94,11 @@ def test_pair_gemm_edges_of_tiles_bit_for_bit(M, N, K, out_dtype):
     check(lib().sglb200_fp8_blockwise_scaled_mm_pair(
         aq_d.data_ptr(), wq_d.data_ptr(), sm.data_ptr(), ws_d.data_ptr(), out.data_ptr(), M, N, K, kg * 128, kg * 128, N, sm.stride(0),
         sm.stride(1), ws_d.stride(0), ws_d.stride(1), dtype_code(out_dtype), 256, st), "pair")
+    assert last_gemm() == PAIRS
     check(lib().sglb200_fp8_blockwise_scaled_mm(
         aq_d.data_ptr(), wq_d.data_ptr(), sr.data_ptr(), ws_d.data_ptr(), plain.data_ptr(), M, N, K, kg * 128, kg * 128, N, sr.stride(0),
         sr.stride(1), ws_d.stride(0), ws_d.stride(1), dtype_code(out_dtype), st), "mm")
+    assert last_gemm() == (FEW_ROWS if M <= 64 else TILES)
     torch.cuda.synchronize()
     assert lib().sglb200_read_device_status() == 0
     # one unit in the last place: the tensor core sums a k-block in another order than the oracle, and among 28 million results
@@ -114,10 +118,12 @@ def test_other_scale_layouts_give_the_pairs_bits_at_few_rows(M, N, K):
                                             scale_tma_aligned=True)
     wq, ws = block_quant_weight_fp8(torch.randn(N, K, generator=g, device="cuda") * 0.02)
     want = _pair(q, s, wq, ws, 256)
+    assert last_gemm() == PAIRS
     ld = (M + 3) // 4 * 4
     odd = torch.empty(1 + K // 128 * ld, device="cuda").as_strided((M, K // 128), (1, ld), 1)
     odd.copy_(s)  # M-major, off the 16-byte boundary
     got = [_pair(q, scales, wq, ws, 256) for scales in (s.contiguous(), odd)]
+    assert last_gemm() == TILES
     check(lib().sglb200_set_num_sms(1), "set_num_sms")
     try:
         got.append(_pair(q, s, wq, ws, 256))
@@ -139,7 +145,9 @@ def test_scales_whose_columns_overlap_stay_on_the_tiles(step):
     buf = torch.rand(M + 7 * step, generator=torch.Generator().manual_seed(3)).cuda() * 0.1
     s = buf.as_strided((M, 8), (1, step))
     aq_d, wq_d, ws_d = aq.cuda(), wq.cuda(), ws.cuda()
-    out, want = _pair(aq_d, s, wq_d, ws_d, 256), _pair(aq_d, s.contiguous(), wq_d, ws_d, 256)
+    out = _pair(aq_d, s, wq_d, ws_d, 256)
+    assert last_gemm() == TILES
+    want = _pair(aq_d, s.contiguous(), wq_d, ws_d, 256)
     torch.cuda.synchronize()
     assert torch.equal(bits(out), bits(want))
     assert_gemm_close(out, oracle.w8a8_block_fp8_matmul(aq, wq, s.cpu().contiguous(), ws), f"step={step}")
@@ -161,8 +169,10 @@ def test_linear_layer_on_pairs_adds_its_bias(dtype):
     method.process_weights_after_loading(layer)
     bias = torch.randn(N, generator=g, device="cuda").to(dtype)
     out = method.apply(layer, x, bias)
+    assert last_gemm() == PAIRS
     q, s = sglang_per_token_group_quant_fp8(x, 128)
     want = w8a8_block_fp8_matmul(q, codes, s, scales, [128, 128], dtype) + bias
+    assert last_gemm() == TILES
     torch.cuda.synchronize()
     assert torch.equal(bits(out), bits(want))
 

@@ -8,7 +8,7 @@ import pytest
 import torch
 
 import oracle
-from helpers import FP8, assert_gemm_close, make_activations, rel_l2
+from helpers import FP8, assert_gemm_close, last_gemm, make_activations, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -209,9 +209,11 @@ def test_dense_pairs_edges_of_tiles(M, N, K, out_dtype):
     offsets, st = torch.tensor([0, M], dtype=torch.int32, device="cuda"), torch.cuda.current_stream().cuda_stream
     check(L.sglb200_fp8_ue8m0_scaled_mm(a.data_ptr(), w.data_ptr(), sa.data_ptr(), sw.data_ptr(), out.data_ptr(), M, N, K, K, K, N,
                                         sa.stride(1), sw.stride(0), sw.stride(1), dtype_code(out_dtype), st), "mm")
+    assert last_gemm() == "fp8_ue8m0_gemm_pair_kernel"  # by the cost model: sizes move with it
     check(L.sglb200_fp8_ue8m0_scaled_grouped_mm(a.data_ptr(), w.data_ptr(), sa.data_ptr(), sw.data_ptr(), single.data_ptr(),
                                                 offsets.data_ptr(), M, 1, N, K, K, K, N * K, N, sa.stride(0), sa.stride(1), 0,
                                                 sw.stride(0), sw.stride(1), dtype_code(out_dtype), st), "grouped mm")
+    assert last_gemm() == "fp8_ue8m0_gemm_kernel"
     torch.cuda.synchronize()
     assert L.sglb200_read_device_status() == 0
     ref = oracle.w8a8_block_fp8_matmul(aq, wq, a_s, ws, output_dtype=out_dtype)
@@ -235,6 +237,7 @@ def test_dense_pairs_add_the_bias_and_survive_repeated_launches():
     x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
     bias = torch.randn(N, generator=g, device="cuda").bfloat16()
     outs = [method.apply(layer, x, bias) for _ in range(20)]
+    assert last_gemm() == "fp8_ue8m0_gemm_pair_kernel"
     want = method.apply(layer, x, None) + bias
     torch.cuda.synchronize()
     assert lib().sglb200_read_device_status() == 0
