@@ -58,6 +58,8 @@ const char* sglb200_version(void);
  * grid-sized helpers): their grids are sized from min(num_sms, SMs of the device).  0 lifts the bound.  Process-wide,
  * read at every launch; set it from the thread that launches.  Use: leave SMs free for a communication kernel that runs
  * beside a GEMM (a persistent GEMM that fills every SM makes a concurrent kernel wait for one of its CTAs to finish).
+ * GEMMs on CTA pairs take num_sms / 2 pairs of SMs, each the two of one TPC.  The block scheduler fills whole TPCs, so they fit
+ * beside a kernel of the remaining number of CTAs; a kernel that held ONE SM of many TPCs would make some pairs wait.
  * Replaces: deep_gemm.set_num_sms / get_num_sms as used by configure_deep_gemm_num_sms,
  *           python/sglang/srt/layers/deep_gemm_wrapper/entrypoint.py:94-104.
  * sglb200_get_num_sms returns the bound in force (the device's SM count when none is set).

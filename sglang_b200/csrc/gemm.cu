@@ -1207,6 +1207,12 @@ int dense_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
 // M=4096 154 against 170, M=640 30.2 against 28.2; N=1536 K=7168 M=1536 27 against 17.  Under sustained load at the power cap the
 // pairs gain more, because they move half of the operand bytes (figures in gemm_pair.cu): calls of more than 2e11 operations,
 // which take 100 us and more, go to them while the model has them up to 4 % behind.
+// Under a limit on SMs (sglb200_set_num_sms: the rest is for a kernel that runs beside) the rule is the same with that many.  A pair
+// needs both SMs of a TPC, and the block scheduler hands out whole TPCs first, to the CTAs of the kernel beside as well: with one
+// kernel of 4, 5, 8, 16 or 32 CTAs resident, or two to eight kernels of one CTA, all pairs of the limit fit (4096 x 7168 x 2304 beside
+// 16 CTAs, pairs / tiles 79.4 / 84.8 us, UE8M0 57.8 / 70.4; 2048 x 36864 x 7168 480 / 537, UE8M0 378 / 436).
+// Were the CTAs beside spread over twice the TPCs, the pairs that do not fit would take a second turn (127 and 805 us
+// for the sizes above, tiles unchanged); none of the launches above came to lie so, it took CTAs that leave at once on every other SM.
 bool pair_preferred(int64_t M, int64_t N, int64_t K, int sm_count) {
   if (sm_count < 2) return false;
   const int64_t kb = (K + BK - 1) / BK, pairs = sm_count / 2;

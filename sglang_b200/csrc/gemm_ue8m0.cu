@@ -492,7 +492,7 @@ namespace {
 // (whole groups of four k-blocks, for callers with scratch; 1 = not cut).  Cost models in nanoseconds at 1.9 GHz: for the choice
 // among ranges a k-block takes a CTA 380 and a work item 800 more, splitting costs the reduce kernel (3500) and the partial
 // sums' way to memory and back (8 bytes each at about 5 TB/s); against the pairs a k-block of an uncut call counts 340 and a
-// tile's store, which the pairs do not pay, 1700.
+// tile's store, which the pairs do not pay, 1700.  Under a limit on SMs: see pair_preferred in gemm.cu.
 struct Plan {
   int splits;
   bool pair;

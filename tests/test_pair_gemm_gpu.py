@@ -177,6 +177,40 @@ def test_linear_layer_on_pairs_adds_its_bias(dtype):
     assert torch.equal(bits(out), bits(want))
 
 
+@pytest.mark.parametrize("limit", [1, 2, 3, 17, 132, 147])
+def test_pairs_under_an_sm_limit(limit):
+    # even and odd limits, from one tile after the other on a single pair to all but one SM; under 1 no pair is left and under 3 the
+    # 128 x 128 tiles are the better choice.  Plain entries and the pair entry, fp32 and UE8M0 scales: the bits of an unlimited call
+    from sglang_b200._lib import check, lib
+    from sglang_b200.layers.quantization import (block_quant_weight_fp8, pack_ue8m0_scales, per_block_cast_to_fp8,
+                                                 sglang_per_token_group_quant_fp8, w8a8_block_fp8_matmul, w8a8_block_fp8_matmul_ue8m0)
+    M, N, K = 1024, 2368, 2048
+    g = torch.Generator(device="cuda").manual_seed(limit)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w = torch.randn(N, K, generator=g, device="cuda") * 0.02
+    (wq, ws), (uq, us) = block_quant_weight_fp8(w), per_block_cast_to_fp8(w)
+    up = pack_ue8m0_scales(us)
+    q, s = sglang_per_token_group_quant_fp8(x, 128, column_major_scales=True, scale_tma_aligned=True)
+    uxq, uxs = sglang_per_token_group_quant_fp8(x, 128, column_major_scales=True, scale_tma_aligned=True, scale_ue8m0=True)
+    calls = [lambda: w8a8_block_fp8_matmul(q, wq, s, ws, [128, 128], torch.bfloat16), lambda: _pair(q, s, wq, ws, 256),
+             lambda: w8a8_block_fp8_matmul_ue8m0(uxq, uq, uxs, up, torch.bfloat16)]
+    want = [f() for f in calls]
+    check(lib().sglb200_set_num_sms(limit), "set_num_sms")
+    try:
+        got, ran = [], []
+        for f in calls:
+            got.append(f())
+            ran.append(last_gemm())
+    finally:
+        lib().sglb200_set_num_sms(0)
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    pairs = limit not in (1, 3)
+    assert ran == [PAIRS if pairs else TILES, PAIRS if limit > 1 else TILES,
+                   "fp8_ue8m0_gemm_pair_kernel" if pairs else "fp8_ue8m0_gemm_kernel"]
+    assert all(torch.equal(bits(a), bits(b)) for a, b in zip(got, want))
+
+
 def test_pair_gemm_refuses_bad_arguments():
     from sglang_b200._lib import lib
     L = lib()
