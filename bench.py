@@ -78,7 +78,14 @@ class ClockSampler:
     """Samples SM clock and throttle reasons of one GPU while timed regions run.  The NVML polling (read-only queries,
     every 4 ms) runs in ONE CHILD PROCESS for the whole run, writing to a scratch file: a polling thread inside the
     benchmark process takes the interpreter lock away from the thread that launches the kernels, which showed as idle GPU
-    time in steps of one or two milliseconds.  start() / stop() mark the wall-clock window whose samples count."""
+    time in steps of one or two milliseconds.  start() / stop() mark the wall-clock window whose samples count.
+
+    NVML refreshes its reading about every 100 ms and shows a load 100 to 150 ms late (measured from an idle board under the
+    gate_up GEMM: 1965 MHz and no reason for 0.1 to 0.15 s, then 1360 to 1380, while a step took 1.82 ms at first and 2.08 from 0.08 s on).
+    A shorter region is read by keeping its load on after the timing (``hold_ms`` of the same step, untimed) and
+    leaving the first ``LAG`` of the window out."""
+
+    LAG = 0.15
 
     REASONS = (("hw_slowdown", 0x8), ("hw_thermal_slowdown", 0x40), ("sw_thermal_slowdown", 0x20),
                ("sw_power_cap", 0x4))
@@ -112,12 +119,20 @@ class ClockSampler:
     def start(self):
         self.t0 = time.time()
 
+    @staticmethod
+    def hold(step, step_ms: float, hold_ms: float = 300.0) -> None:
+        """The load of a timed region for another ``hold_ms``; ``step_ms`` is the same on every rank, and so is the count."""
+        for _ in range(max(1, min(2000, int(hold_ms / max(step_ms, 1e-3)) + 1))):
+            step()
+
     def stop(self):
         self.t1 = time.time()
         if ClockSampler._child is None or not ClockSampler._path:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["clock sampler unavailable"]}
         time.sleep(0.01)
         clk, near, mx, reasons, err = [], [], None, set(), None
+        late = self.t1 - self.t0 > 1.5 * self.LAG
+        first = self.t0 + self.LAG if late else self.t0
         with open(ClockSampler._path) as f:
             for line in f:
                 fld = line.split()
@@ -127,7 +142,7 @@ class ClockSampler:
                     err = line.strip()
                 elif len(fld) == 3:
                     t, c, r = float(fld[0]), int(fld[1]), int(fld[2])
-                    if self.t0 <= t <= self.t1:
+                    if first <= t <= self.t1:
                         clk.append(c)
                         for name, bit in self.REASONS:
                             if r & bit:
@@ -138,7 +153,9 @@ class ClockSampler:
             return {"sm_mhz": None, "sm_max_mhz": mx, "reasons": [err]}
         use = clk or near  # a region shorter than the polling period: the samples right beside it
         return {"sm_mhz": statistics.median(use) if use else None, "sm_max_mhz": mx, "reasons": sorted(reasons),
-                "samples": len(clk), "source": "nvml (child process)"}
+                "samples": len(clk), "source": "nvml (child process)",
+                "window": f"{self.t1 - first:.2f} s of the timed step, from {self.LAG} s after its start (NVML lags)" if late else
+                          "shorter than NVML's refresh of about 0.1 s: the reading is from before or from the region's start"}
 
 
 # --------------------------------------------------------------------------- CPU arm
@@ -899,6 +916,8 @@ def main():
     ar_blocks = [args.ar_blocks if args.ar_blocks > 0 else 16]
     fused_ctas = [0]  # > 0: GEMM and multicast all-reduce in one launch, this many communication CTAs
 
+    from sglang_b200._lib import lib
+
     def step(record=False):
         for L in layers:
             if multicast and fused_ctas[0] > 0 and L["mode"] == "row":
@@ -925,6 +944,8 @@ def main():
                 e0.record()
             y = w8a8_block_fp8_matmul(q, L["layer"].weight, s, L["layer"].weight_scale_inv, [128, 128], torch.bfloat16,
                                       out=mc.view((M, L["n_loc"])) if use_mc else None)
+            if not record:  # untimed: the kernel that the layer's GEMM was given to
+                L["kernel"] = lib().sglb200_last_gemm_kernel().decode()
             if record:
                 e1.record()
                 L["ev"].append((e0, e1))
@@ -1075,11 +1096,14 @@ def main():
     t1.record()
     timed_launches = own_launches[0]
     fence()
-    clocks = sampler.stop()
     ms = torch.tensor([t0.elapsed_time(t1)], device=dev)
     if world > 1:
         dist.all_reduce(ms, op=dist.ReduceOp.MAX)
     ms_per_step = float(ms) / main_steps
+    if args.only not in ("quant", "ue8m0"):
+        sampler.hold(step, ms_per_step)
+        fence()
+    clocks = sampler.stop()
     value = total_flops / (ms_per_step * 1e-3) / 1e12
 
     breakdown = None
@@ -1129,13 +1153,20 @@ def main():
                                 "gemm_tflops": f / (statistics.median(t) * 1e-3) / 1e12}
     fp8_peak = 2.0 * peaks["bf16_tflops_sustained"]
     achieved = gemm_flops / (gemm_ms * 1e-3) / 1e12
-    # DRAM traffic per launch: algorithmic operand + output bytes x 1.08, the read + write / algorithmic ratio of one ncu
-    # capture of the tile kernel at M = 2048, N = 7168, K = 16384 (194.1 MB measured, 180.4 MB algorithmic), scaled up
-    alg_bytes = sum(L["n_loc"] * L["k_loc"] + M * L["k_loc"] + 2.0 * M * L["n_loc"] for L in layers) / len(layers)
+    # DRAM traffic per launch: algorithmic operand + output bytes x the read + write / algorithmic ratio of one ncu capture of
+    # the layer's kernel: on CTA pairs 0.96 (M = 2048, N = 36864, K = 7168: 413.3 MB of 430; part of the output is still in L2 at the
+    # kernel's end), on 128 x 128 tiles 1.08 (M = 2048, N = 7168, K = 16384: 194.1 MB of 180.4), scaled up
+    def by_kernel(key):
+        names = [L.get(key, "not noted") for L in layers]
+        return ", ".join(f"{k} ({'/'.join(L['name'] for n, L in zip(names, layers) if n == k)})" for k in sorted(set(names)))
+
+    traffic = sum((0.96 if L.get("kernel") == "fp8_block_gemm_pair_kernel" else 1.08) *
+                  (L["n_loc"] * L["k_loc"] + M * L["k_loc"] + 2.0 * M * L["n_loc"]) for L in layers) / len(layers)
     roofline = {"bound": "tensor", "achieved": achieved, "peak": fp8_peak, "unit": "TFLOP/s",
-                "frac": achieved / fp8_peak, "traffic": 1.08 * alg_bytes,
-                "traffic_note": "bytes per launch averaged over the layers; ncu ratio 1.08 of the tile kernel on a smaller M scaled up",
-                "kernel": "fp8_block_gemm_pair_kernel (N = 576: fp8_block_gemm_kernel)",
+                "frac": achieved / fp8_peak, "traffic": traffic,
+                "traffic_note": "bytes per launch averaged over the layers; ncu ratio of the layer's kernel on a smaller M scaled "
+                                "up (CTA pairs 0.96, 128 x 128 tiles 1.08)",
+                "kernel": by_kernel("kernel"),
                 "peak_source": f"2 x bf16_tflops_sustained ({peaks['source']}); nominal dense FP8 is 4500",
                 "frac_of_nominal_fp8": achieved / 4500.0, "launches": sum(len(L["ev"]) for L in layers),
                 "avg_launch_ms": gemm_ms / max(1, sum(len(L["ev"]) for L in layers)), "others": []}
@@ -1153,6 +1184,8 @@ def main():
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 e0.record()
             y = w8a8_block_fp8_matmul_ue8m0(q, L["wq_u"], s, L["ws_u"], torch.bfloat16)
+            if not record:
+                L["kernel_u"] = lib().sglb200_last_gemm_kernel().decode()
             if record:
                 e1.record()
                 L["ev_u"].append((e0, e1))
@@ -1173,11 +1206,13 @@ def main():
             step_u(record=True)
         u1.record()
         fence()
-        clocks_u = sampler_u.stop()
         ms_u = torch.tensor([u0.elapsed_time(u1)], device=dev)
         if world > 1:
             dist.all_reduce(ms_u, op=dist.ReduceOp.MAX)
         ms_u_step = float(ms_u) / args.steps
+        sampler_u.hold(step_u, ms_u_step)
+        fence()
+        clocks_u = sampler_u.stop()
         g_ms, g_fl, shp = 0.0, 0.0, {}
         for L in layers:
             tt = [a.elapsed_time(b) for a, b in L["ev_u"]]
@@ -1191,7 +1226,7 @@ def main():
                  "value": total_flops / (ms_u_step * 1e-3) / 1e12, "unit": "TFLOP/s", "ms_per_step": ms_u_step,
                  "roofline": {"bound": "tensor", "achieved": ach_u, "peak": 2.0 * peaks["bf16_tflops_sustained"],
                               "unit": "TFLOP/s", "frac": ach_u / (2.0 * peaks["bf16_tflops_sustained"]),
-                              "frac_of_nominal_fp8": ach_u / 4500.0, "kernel": "fp8_ue8m0_gemm_pair_kernel"},
+                              "frac_of_nominal_fp8": ach_u / 4500.0, "kernel": by_kernel("kernel_u")},
                  "per_shape": shp, "clocks": clocks_u, "gpu_launches": args.steps * len(layers) * 2}
 
     quant_after = None
