@@ -92,7 +92,7 @@ constexpr size_t kScaleOffset = (kCtlOffset + 256 /*barriers*/ + (kMaxExperts + 
 // Grouped: the rows of a tile that an expert's end cuts are loaded in boxes of so many, those past the end from
 // outside the tensor, as zeros.  The tensor core multiplies them all the same, but products of zeros cost it little power, and
 // power is what bounds an expert layer: with the next experts' rows in their place 256 x 7168 x 2048 at 4096 tokens (half of
-// the tiles such ends) took 3750 us, now 3540,.  Boxes of 16 keep the one producer too long (3610).  Running those
+// the tiles such ends) took 3750 us, now 3540.  Boxes of 16 keep the one producer too long (3610).  Running those
 // tiles on swapped operands instead, 128 weight rows by 32 or 64 tokens, was level with the former: the chain of a k-block is
 // as long, and the ordinary tiles' loop compiled worse beside it.
 constexpr int kRowBox = 32;
@@ -161,8 +161,8 @@ struct Tile {
 
 // Where a tile's results go.  The scale loader, which walks the tiles ahead of the promotion warps, writes it for them: eight
 // warps that took the tile number apart themselves (integer divisions, a search through the experts) stood still for 900 cycles
-// between two tiles (expert layer of 256 x 7168 x 2048 at 4096 tokens 3740 -> 3510 us, dense N=24576 K=1536 M=777 40.2 -> 38.8 with
-// store_rows).  Only the coordinates come from here: loop bounds read from memory make the compiler treat the loop as divergent
+// between two tiles (expert layer of 256 x 7168 x 2048 at 4096 tokens 3740 -> 3510 us, dense N=24576 K=1536 M=777 40.2 -> 38.8, in
+// both with store_rows, whose part of it is noted there).  Only the coordinates come from here: loop bounds read from memory make the compiler treat the loop as divergent
 // (38.8 -> 51 us).
 struct TileNote {
   int32_t row0, row_end, n0, split;
@@ -285,8 +285,9 @@ __device__ __forceinline__ void warp_rows_via_smem(uint32_t* stg, const uint32_t
 
 // A promotion warp's 32 rows x 64 columns, rounded, to rows [row0, row_end) of the output: 32 columns per pass into the warp's box
 // (a lane's row of 64 bytes, 16-byte pieces swizzled), then one TMA store.  Only where an expert's rows end inside the 32 do
-// the lanes store what is theirs: the store would reach into the next expert's rows.  N=24576 K=1536 M=777: 39.7 -> 38.8 us against
-// 64-byte pieces stored by the lanes (the epilogue as a whole, 1000 to 1700 cycles a tile, is 13 of 45 us there).
+// the lanes store what is theirs: the store would reach into the next expert's rows.  Against 64-byte pieces stored by the lanes:
+// N=24576 K=1536 M=777 39.7 -> 38.8 us (52.3 -> 51.2 with its quantiser; the epilogue as a whole, 1000 to 1700 cycles a tile, was 13 of
+// 45 us there), expert layer of 256 x 7168 x 2048 at 4096 tokens 3443 -> 3411.
 template <typename OutT, bool GROUPED>
 __device__ __forceinline__ void store_rows(const GemmParams& p, const CUtensorMap& map_out, const float2* acc, uint32_t box, int32_t n0,
                                            int32_t row0, int32_t row_end, int lane, bool leader) {
@@ -1392,7 +1393,8 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
     const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
     if (int rc = set_smem_attr_once<false, false>()) return rc;
     // Up to smallm_max_rows() rows, one or two waves that wait for weights, the kernel starts beside the quantiser and requests
-    // its first weights meanwhile, as the few-rows kernel does.  Above, that gained 1 % at 777 rows and cost 3 to 7 % at 8192.
+    // its first weights meanwhile, as the few-rows kernel does: 113 x 10240 x 8192 with its quantiser 28.4 -> 26.3 us (31.2 on the
+    // few-rows kernel, see takes_few_rows).  Above, that gained 1 % at 777 rows and cost 3 to 7 % at 8192.
     p.early_next = total_rows <= smallm_max_rows() && !tiles_only;
     if (p.early_next) {
       const cudaError_t e = launch_pdl(fp8_block_gemm_kernel<false, false>, dim3(grid), dim3(kThreads), kSmemBytes, st, map_a, map_b, map_out, map_rows,
