@@ -8,7 +8,16 @@
 // N / 128 tiles alone cannot occupy the SMs, the CTAs of a cluster cut a tile's K among themselves and rank 0 adds their sums up
 // out of their shared memory (smallm_cluster): against fp32 partial sums in memory and a kernel that adds them, quantiser
 // included, N=576 K=7168 M=1 / 48: 9.6 / 14.1 -> 6.8 / 11.1 us, N=7168 K=16384 M=48 32.3 -> 27.1, N=10240 K=8192 M=48 27.0 -> 22.1.
-// From 65 to 128 rows eight or sixteen promotion warps share every accumulator stage.
+// From 65 to 128 rows eight or sixteen promotion warps share every accumulator stage, from 33 rows eight where clusters share K.
+//
+// One barrier each way per k-block.  `full` counts the producer's bytes, the scale loader and the promotion warps, who arrive for the
+// k-block that gets the TMEM stage they have just read; `done` is one commit, on which the producer, the scale loader and the
+// promotion warps wait.  A wait on a barrier that is ready costs its warp about 120 cycles and a commit 60: with a barrier per ring
+// (two waits, two commits) a k-block took the one issuing warp 500 cycles with everything ready, so 337, and issued under a
+// predicate instead of a branch 256 at 128 columns, which is what the MMAs take.  The promotion warps are what is left: they ask
+// for the next k-block before they add, step through the rings by offsets and take four k-blocks a turn (a turn each: 4 to 10 % slower).  Two
+// waits and two commits -> this, GEMM alone, weights from HBM, us: 48 x 10240 x 8192 21.8 -> 18.6, 64 x 7168 x 16384 27.5 -> 24.6, 32 x
+// 10240 x 8192 18.0 -> 16.7, 48 x 24576 x 1536 13.2 -> 11.4, 96 x 7168 x 16384 31.4 -> 30.5, 16 x 7168 x 16384 22.2 -> 21.5.
 // Measured against scales that every promotion warp fetched and spread by shuffles, weights from HBM (B200):
 // N=36864 K=7168 M=32 / 64 / 128: 46.6 / 54.8 / 75.0 -> 41.8 / 43.3 / 55.1 us (6.1 TB/s at 64 rows);
 // N=24576 K=1536 M=16 / 64 / 128: 8.4 / 15.4 / 21.8 -> 7.7 / 9.8 / 13.9 us.
@@ -18,7 +27,7 @@
 // tables as in the 128 x 128 grouped kernel; an expert with more than MT rows gets several chunks (its weight tile is
 // then re-read, from L2), an expert without rows gets no item, so only the weights of routed experts are streamed.
 //
-// warp 0: TMA producer; warp 1: TMEM owner + MMA issuer; warp 2: scale loader (sa[token] * sb into shared memory), or
+// warp 0: TMA producer; warp 1: TMEM owner + MMA issuer; warp 2: scale loader (sa[token] * sb into a slot per k-block), or
 // at one or two rows warps 2 and 3: quantisers (QUANT); warps 4..7
 // (..11): promotion (tcgen05.ld, acc += p * scale) and the transposed store.  All waits are bounded.
 //
@@ -63,9 +72,8 @@ namespace {
 constexpr int BN = 128, BK = 128;  // weight rows per tile, K per block
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kWBytes = BN * BK;
-constexpr int kScaleGroup = 4;   // k-blocks per stage of the scale ring
-constexpr int kScaleStages = 4;
-constexpr uint32_t kCtlBytes = 640;
+constexpr int kScaleGroup = 4;   // k-blocks whose scales the loader fetches at once
+constexpr uint32_t kCtlBytes = 256;
 constexpr uint32_t kPatchRow = 80, kPatchBytes = 16 * kPatchRow;  // epilogue patch of a warp: 16 tokens x 64 bytes, padded
 
 constexpr int kAuxRegs = 96, kPromoRegs = 200;  // register split of the NSUB = 2 form (four and eight warps)
@@ -80,12 +88,15 @@ constexpr int kMaxExperts = 1024;
 template <int MT, int NSUB = 1>
 struct Cfg {
   static constexpr int kTile = MT * NSUB;  // most activation rows per work item = TMEM columns per stage
-  static constexpr int kStages = kTile == 128 ? 6 : (kTile == 64 ? 8 : (kTile == 32 ? 10 : 11));
-  static constexpr int kAcc = (512 / kTile) < 16 ? (512 / kTile) : 16;
+  static constexpr int kStages = kTile == 160 ? 5 : (kTile == 128 ? 6 : (kTile == 64 ? 8 : (kTile == 32 ? 10 : 11)));
+  static constexpr int kAcc = (512 / kTile) < kStages ? (512 / kTile) : kStages;
   static constexpr int kThreads = 128 + 128 * NSUB;
   static constexpr uint32_t kABytes = kTile * BK;
   static constexpr uint32_t kStageBytes = kWBytes + kABytes;
-  static constexpr uint32_t kScaleBytes = kScaleStages * kScaleGroup * kTile * sizeof(float);
+  // Slots of kTile scale products, one per k-block.  Slot j + kStages is written when the MMAs of j are done; those were issued
+  // after every promotion warp had read the sums of j - kAcc, and its scales before them.
+  static constexpr int kScaleSlots = 2 * kStages;
+  static constexpr uint32_t kSlotBytes = kTile * sizeof(float), kScaleBytes = kScaleSlots * kSlotBytes;
   static constexpr size_t kPatchOffset = (size_t)kStages * kStageBytes + kScaleBytes;
   static constexpr size_t kSmem = 1024 + kPatchOffset + 4 * NSUB * kPatchBytes + kCtlBytes;
   // grouped: the table of first work items per expert follows the control block
@@ -171,12 +182,8 @@ __device__ __forceinline__ Item get_item(const SmallParams& p, const int32_t* it
 }
 
 struct Ctl {
-  uint64_t full[12];
-  uint64_t empty[12];
-  uint64_t acc_full[16];
-  uint64_t acc_empty[16];
-  uint64_t sc_full[kScaleStages];
-  uint64_t sc_empty[kScaleStages];
+  uint64_t full[12];  // k-block g may be multiplied: operands and scales have arrived, its TMEM stage has been read out
+  uint64_t done[12];  // k-block g has been multiplied: its operands may be overwritten, its sums be read
   uint32_t tmem_base;
   volatile int32_t abort_flag;
   int32_t total;
@@ -273,8 +280,7 @@ template <typename T, int MT, bool UE, bool CLUSTER>
 __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, uint8_t* smem, float* scale_ring, uint32_t me, int lane,
                                               int32_t total) {
   using C = Cfg<MT>;
-  const uint32_t full0 = ptx::smem_u32(&ctl->full[0]), empty0 = ptx::smem_u32(&ctl->empty[0]);
-  const uint32_t sc_full0 = ptx::smem_u32(&ctl->sc_full[0]), sc_empty0 = ptx::smem_u32(&ctl->sc_empty[0]);
+  const uint32_t full0 = ptx::smem_u32(&ctl->full[0]), done0 = ptx::smem_u32(&ctl->done[0]);
   // eight lanes (sixteen elements each) take a row of a k-block; a pass of the warp covers the rows of `per_pass` k-blocks
   static_assert(kScaleGroup == 4 && kQuantRows == 2, "four rows of k-blocks per pass");
   const int rows = p.M, per_pass = kScaleGroup / rows;
@@ -282,7 +288,7 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
   const uint4* row = reinterpret_cast<const uint4*>(static_cast<const T*>(p.x) + (int64_t)r * p.K) + 2 * sub;
   const uint32_t piece = kWBytes + (uint32_t)(r * 128 + ((sub ^ r) << 4));  // 128-byte swizzle
   const float inv_max = __frcp_rn(448.0f);
-  uint32_t stage = 0, phase = 0, sc_stage = 0, sc_phase = 0, turn = 0;
+  uint32_t stage = 0, phase = 0, slot = 0, turn = 0;
   for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
     const Item it = get_item<C::kTile, false, CLUSTER>(p, nullptr, t);
     const float* sb_blk = p.sb + (int64_t)it.nt * p.sb_stride_n;
@@ -298,8 +304,6 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
           v[u][1] = __ldg(row + (int64_t)kb * (BK / 8) + 1);
           b[u] = load_scale<UE>(sb_blk, kb, p.sb_stride_k);
         }
-        if (!ptx::mbar_wait_inl_a(sc_empty0 + sc_stage * 8, sc_phase ^ 1)) { timeout(ctl, 16); return; }
-        float* dst = scale_ring + (size_t)sc_stage * kScaleGroup * C::kTile + r;
 #pragma unroll
         for (int u = 0; u < kQuantRows; ++u) {
           if (u >= rows || kb0 + u * per_pass >= it.kb1) break;
@@ -308,26 +312,30 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
           for (int m = 4; m >= 1; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
           const float s = group_scale_fast(amax, 448.0f, inv_max, UE);
           const uint4 codes = encode16_e4m3<T>(v[u][0], v[u][1], s);
-          if (sub == 0) dst[(u * per_pass + ko) * C::kTile] = s * b[u];
           const int n = min(per_pass, it.kb1 - kb0 - u * per_pass);  // k-blocks of this pass
-          uint32_t mine = stage;
+          uint32_t mine = stage, mine_slot = slot;
           for (int i = 0; i < n; ++i) {
-            if (!ptx::mbar_wait_inl_a(empty0 + stage * 8, phase ^ 1)) { timeout(ctl, 11); return; }
-            if (i == ko) mine = stage;
+            if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 11); return; }
+            if (i == ko) { mine = stage; mine_slot = slot; }
             if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+            if (++slot == C::kScaleSlots) slot = 0;
           }
-          if (ko < n) *reinterpret_cast<uint4*>(smem + (size_t)mine * C::kStageBytes + piece) = codes;
+          if (ko < n) {
+            *reinterpret_cast<uint4*>(smem + (size_t)mine * C::kStageBytes + piece) = codes;
+            if (sub == 0) scale_ring[mine_slot * C::kTile + r] = s * b[u];
+          }
           ptx::fence_proxy_async();  // the MMA reads shared memory through the asynchronous proxy
           __syncwarp();
           if (ko < n && (lane & (8 * rows - 1)) == 0) ptx::mbar_arrive_a(full0 + mine * 8);
         }
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_a(sc_full0 + sc_stage * 8);
       } else {
-        stage += min(kScaleGroup, it.kb1 - kb0);
+        const uint32_t n = min(kScaleGroup, it.kb1 - kb0);
+        stage += n;
         if (stage >= (uint32_t)C::kStages) { stage -= C::kStages; phase ^= 1; }
+        slot += n;
+        if (slot >= (uint32_t)C::kScaleSlots) slot -= C::kScaleSlots;
       }
-      if (++sc_stage == kScaleStages) { sc_stage = 0; sc_phase ^= 1; }
     }
     if (ctl->abort_flag) return;
   }
@@ -345,23 +353,16 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
   using C = Cfg<MT, NSUB>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* scale_ring = reinterpret_cast<float*>(smem + (size_t)C::kStages * C::kStageBytes);  // [stage][k-block][token]
+  float* scale_ring = reinterpret_cast<float*>(smem + (size_t)C::kStages * C::kStageBytes);  // [slot][token]
   Ctl* ctl = reinterpret_cast<Ctl*>(smem + C::kPatchOffset + 4 * NSUB * kPatchBytes);
   int32_t* item_start = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(ctl) + kCtlBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::kStages; ++i) {
-      ptx::mbar_init(&ctl->full[i], QUANT ? 2 : 1);  // the weights' bytes; QUANT: and the warp that wrote the codes
-      ptx::mbar_init(&ctl->empty[i], 1);
-    }
-    for (int i = 0; i < C::kAcc; ++i) {
-      ptx::mbar_init(&ctl->acc_full[i], 1);
-      ptx::mbar_init(&ctl->acc_empty[i], 4 * NSUB);  // one arrival per promotion warp
-    }
-    for (int i = 0; i < kScaleStages; ++i) {
-      ptx::mbar_init(&ctl->sc_full[i], 1);
-      ptx::mbar_init(&ctl->sc_empty[i], 4 * NSUB);
+      // the producer (and its bytes), the scale loader or (QUANT) the warp that wrote codes and scales, every promotion warp
+      ptx::mbar_init(&ctl->full[i], 2 + 4 * NSUB);
+      ptx::mbar_init(&ctl->done[i], 1);
     }
     ctl->abort_flag = 0;
     ptx::fence_barrier_init();
@@ -408,9 +409,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
   ptx::tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
   const int32_t total = ctl->total;
-  const uint32_t full0 = ptx::smem_u32(&ctl->full[0]), empty0 = ptx::smem_u32(&ctl->empty[0]);
-  const uint32_t acc_full0 = ptx::smem_u32(&ctl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctl->acc_empty[0]);
-  const uint32_t sc_full0 = ptx::smem_u32(&ctl->sc_full[0]), sc_empty0 = ptx::smem_u32(&ctl->sc_empty[0]);
+  const uint32_t full0 = ptx::smem_u32(&ctl->full[0]), done0 = ptx::smem_u32(&ctl->done[0]);
   const uint32_t stage0 = ptx::smem_u32(smem);
 
   if (threadIdx.x == 0) ptx::grid_dep_launch();  // the next kernel of the stream may begin its own set-up
@@ -432,7 +431,12 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
     const int sub = NSUB == 1 ? 0 : (warp - 4) >> 2;  // which sub-tile of the item this warp promotes
     const int tr = lane >> 2, tc = 2 * (lane & 3);    // this thread's row inside 8 weight rows / column inside 8 tokens
     uint8_t* patch = reinterpret_cast<uint8_t*>(smem) + C::kPatchOffset + (size_t)(warp - 4) * kPatchBytes;
-    uint32_t acc_stage = 0, acc_phase = 0, sc_stage = 0, sc_phase = 0;
+    const uint32_t sc_row = ptx::smem_u32(scale_ring + sub * MT + tc), tlane = tmem_base + ((uint32_t)(q * 32) << 16);
+    // The next k-block's place in the rings, as offsets that are added to: `done` barrier, the `full` barrier kAcc k-blocks on, TMEM
+    // columns, scales.
+    uint32_t done_at = 0, phase = 0, full_at = C::kAcc % C::kStages * 8, column = sub * MT, slot = 0;
+    bool ready = false;  // the next k-block's sums are known to be there
+    for (uint32_t i = 0; i < C::kAcc; ++i) ptx::mbar_arrive_if(full0 + i * 8, leader);  // every TMEM stage is free
     [[maybe_unused]] bool met = false;  // this warp has passed the cluster's first barrier
     float2 acc[2][G][2];  // [lanes 0-15 / 16-31][token group][rows tr / tr + 8]: two neighbouring tokens
     for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
@@ -444,51 +448,46 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
 #pragma unroll
         for (int g = 0; g < G; ++g) acc[h][g][0] = acc[h][g][1] = make_float2(0.f, 0.f);
       bool ok = true;
-      for (int32_t kbb = kb0; kbb < kb1 && ok; kbb += kScaleGroup) {
-        if (!ptx::mbar_wait_inl_a(sc_full0 + sc_stage * 8, sc_phase)) {
-          timeout(ctl, 17);
+#pragma unroll 4
+      for (int32_t kb = kb0; kb < kb1; ++kb) {
+        if (!ready && !ptx::mbar_wait_inl_a(done0 + done_at, phase)) {
+          timeout(ctl, 14);
           ok = false;
           break;
         }
-        const float* sc_row = scale_ring + (size_t)sc_stage * kScaleGroup * C::kTile + sub * MT + tc;
+        ptx::tc_fence_after();
+        const uint32_t taddr = tlane + column;
+        const bool mine = NSUB == 1 || rows > 0;  // uniform over the warp
+        uint32_t v[2 * 4 * G];
+        float2 s[G];
+        if (mine) {
+          tmem_ld_16x256<G>(taddr, v);
+          tmem_ld_16x256<G>(taddr + (16u << 16), v + 4 * G);
 #pragma unroll
-        for (int u = 0; u < kScaleGroup; ++u) {
-          if (kbb + u >= kb1) break;
-          float2 s[G];
-#pragma unroll
-          for (int g = 0; g < G; ++g) s[g] = *reinterpret_cast<const float2*>(sc_row + u * C::kTile + 8 * g);
-          if (!ptx::mbar_wait_inl_a(acc_full0 + acc_stage * 8, acc_phase)) {
-            timeout(ctl, 14);
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc_stage * C::kTile + sub * MT;
-          uint32_t v[2 * 4 * G];
-          if (NSUB == 1 || rows > 0) {  // uniform over the warp
-            tmem_ld_16x256<G>(taddr, v);
-            tmem_ld_16x256<G>(taddr + (16u << 16), v + 4 * G);
-            tmem_ld_fence<8 * G>(v);
-          }
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_a(acc_empty0 + acc_stage * 8);
-          if (NSUB == 1 || rows > 0) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-              for (int g = 0; g < G; ++g)
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                  const int i = (h * G + g) * 4 + 2 * r;
-                  acc[h][g][r] = __ffma2_rn(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), s[g], acc[h][g][r]);
-                }
-          }
-          if (++acc_stage == C::kAcc) { acc_stage = 0; acc_phase ^= 1; }
+          for (int g = 0; g < G; ++g) s[g] = ptx::ld_shared_f32x2(sc_row + slot + 32 * g);
         }
-        __syncwarp();  // every lane has read this group's scales
-        if (lane == 0) ptx::mbar_arrive_a(sc_empty0 + sc_stage * 8);
-        if (++sc_stage == kScaleStages) { sc_stage = 0; sc_phase ^= 1; }
+        column = column >= (C::kAcc - 1) * C::kTile ? sub * MT : column + C::kTile;
+        phase ^= done_at == (C::kStages - 1) * 8;
+        done_at = done_at == (C::kStages - 1) * 8 ? 0 : done_at + 8;
+        slot = slot == (C::kScaleSlots - 1) * C::kSlotBytes ? 0 : slot + C::kSlotBytes;
+        if (mine) tmem_ld_fence<8 * G>(v);
+        // this TMEM stage and these scales have been read: the k-block kAcc further on may have the stage
+        ptx::tc_fence_before();
+        __syncwarp();
+        ptx::mbar_arrive_if(full0 + full_at, leader);
+        full_at = full_at == (C::kStages - 1) * 8 ? 0 : full_at + 8;
+        ready = ptx::mbar_test_wait_a(done0 + done_at, phase);  // answered while the sums are added
+        if (mine) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                const int i = (h * G + g) * 4 + 2 * r;
+                acc[h][g][r] = __ffma2_rn(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), s[g], acc[h][g][r]);
+              }
+        }
       }
       if (!ok || ctl->abort_flag) break;
       const int32_t n_warp = it.nt * BN + q * 32;  // first of the warp's 32 output columns
@@ -619,7 +618,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
               if constexpr (!QUANT)
                 if (leader) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, 0);
             } else {
-              if (!ptx::mbar_wait_inl_a(empty0 + stage * 8, phase ^ 1)) {
+              if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) {
                 timeout(ctl, 11);
                 ok = false;
                 break;
@@ -639,13 +638,14 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         if (pass == 0) {
           ptx::grid_dep_wait();  // the activations are written by the kernel before this one
         } else if (ctl->abort_flag) {
-          // bulk copies must not be in flight when the CTA exits: wait (bounded) for every stage that may still be armed
+          // bulk copies must not be in flight when the CTA exits: wait for every stage that may still be armed (20 ms, in which the
+          // copies land; the stage's other arrivals may never come)
           for (int i = 0; i < C::kStages; ++i)
             if (armed & (1u << i)) ptx::mbar_wait_inl_a(full0 + i * 8, (armed_phase >> i) & 1u, 20000000ull);
         } else {
           // the last tcgen05.commit arrivals on `empty` must have landed before the CTA's shared memory is reused
           for (int i = 0; i < C::kStages; ++i) {
-            if (!ptx::mbar_wait_inl_a(empty0 + stage * 8, phase ^ 1)) { timeout(ctl, 15); break; }
+            if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 15); break; }
             if (++stage == C::kStages) { stage = 0; phase ^= 1; }
           }
         }
@@ -654,41 +654,20 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       // ===== MMA issuer: D[128 weight rows][tokens] (+)= W_tile * A_tile^T, one TMEM stage per k-block; the instruction is
       // as wide as the item's rows (in steps of 16), so a ragged chunk costs neither time nor power for its padding
       const uint64_t desc0 = ptx::make_kmajor_sw128_desc(stage0);
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+      uint32_t stage = 0, phase = 0, acc = 0;
       for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
         const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
         const int32_t kb0 = it.kb0, kb1 = it.kb1;
         const uint32_t idesc = ptx::make_idesc_e4m3_f32(BN, (uint32_t)(it.rows + 15) / 16 * 16);
         bool ok = true;
         for (int32_t kb = kb0; kb < kb1; ++kb) {
-          if constexpr (MT == 16 && NSUB == 1) {
-            // Both waits at once, one half of the warp each: with 16 columns a k-block costs this warp little else (N=10240 K=8192
-            // M=1 18.1 -> 16.1 us a call, N=24576 K=1536 M=16 10.2 -> 9.8); with more it gained nothing.  The vote does not order
-            // memory, and the issuing lane has seen only one of the two barriers: the warp barrier passes on what the others saw.
-            const bool op = (lane & 1) != 0;
-            if (!__all_sync(0xffffffffu, ptx::mbar_wait_inl_a(op ? full0 + stage * 8 : acc_empty0 + acc * 8, op ? phase : acc_phase ^ 1))) {
-              timeout(ctl, 12);
-              ok = false;
-              break;
-            }
-            __syncwarp();
-          } else {
-            if (!ptx::mbar_wait_inl_a(acc_empty0 + acc * 8, acc_phase ^ 1)) { timeout(ctl, 12); ok = false; break; }
-            if (!ptx::mbar_wait_inl_a(full0 + stage * 8, phase)) { timeout(ctl, 13); ok = false; break; }
-          }
+          if (!ptx::mbar_wait_inl_a(full0 + stage * 8, phase)) { timeout(ctl, 13); ok = false; break; }
           ptx::tc_fence_after();
-          if (leader) {
-            const uint64_t w_desc = desc0 + (uint64_t)(stage * (C::kStageBytes >> 4));
-            const uint64_t a_desc = w_desc + (kWBytes >> 4);
-            const uint32_t d_tmem = tmem_base + acc * C::kTile;
-            ptx::mma_f8f6f4(d_tmem, w_desc, a_desc, idesc, 0);
-#pragma unroll
-            for (uint32_t k = 1; k < BK / 32; ++k) ptx::mma_f8f6f4(d_tmem, w_desc + 2 * k, a_desc + 2 * k, idesc, 1);
-            ptx::mma_commit_a(empty0 + stage * 8);
-            ptx::mma_commit_a(acc_full0 + acc * 8);
-          }
+          const uint64_t w_desc = desc0 + (uint64_t)(stage * (C::kStageBytes >> 4));
+          ptx::mma_f8f6f4_x4_if(tmem_base + acc * C::kTile, w_desc, w_desc + (kWBytes >> 4), idesc, leader);
+          ptx::mma_commit_if(done0 + stage * 8, leader);
           if (++stage == C::kStages) { stage = 0; phase ^= 1; }
-          if (++acc == C::kAcc) { acc = 0; acc_phase ^= 1; }
+          if (++acc == C::kAcc) acc = 0;
         }
         if (!ok || ctl->abort_flag) break;
       }
@@ -703,7 +682,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       // while this group waits for its place in the ring.
       if constexpr (!GROUPED) ptx::grid_dep_wait();  // the activation scales come from the kernel before this one
       constexpr int kPerLane = C::kTile / 32 > 0 ? C::kTile / 32 : 1;
-      uint32_t stage = 0, phase = 0;
+      uint32_t stage = 0, phase = 0, slot = 0;
       for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
         const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
         const float* sb_blk = p.sb + (int64_t)it.nt * p.sb_stride_n;
@@ -728,24 +707,25 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         };
         fetch(it.kb0);
         bool ok = true;
-        for (int32_t kb0 = it.kb0; kb0 < it.kb1; kb0 += kScaleGroup) {
+        for (int32_t kb0 = it.kb0; kb0 < it.kb1 && ok; kb0 += kScaleGroup) {
           float v[kPerLane][kScaleGroup];
 #pragma unroll
           for (int h = 0; h < kPerLane; ++h)
 #pragma unroll
             for (int u = 0; u < kScaleGroup; ++u) v[h][u] = a[h][u] * b[u];
           if (kb0 + kScaleGroup < it.kb1) fetch(kb0 + kScaleGroup);
-          if (!ptx::mbar_wait_inl_a(sc_empty0 + stage * 8, phase ^ 1)) { timeout(ctl, 16); ok = false; break; }
-          float* dst = scale_ring + (size_t)stage * kScaleGroup * C::kTile;
 #pragma unroll
-          for (int h = 0; h < kPerLane; ++h)
-            if (C::kTile >= 32 || lane < C::kTile) {
+          for (int u = 0; u < kScaleGroup; ++u) {
+            if (kb0 + u >= it.kb1) break;
+            if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 16); ok = false; break; }
 #pragma unroll
-              for (int u = 0; u < kScaleGroup; ++u) dst[u * C::kTile + lane + 32 * h] = v[h][u];
-            }
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_a(sc_full0 + stage * 8);
-          if (++stage == kScaleStages) { stage = 0; phase ^= 1; }
+            for (int h = 0; h < kPerLane; ++h)
+              if (C::kTile >= 32 || lane < C::kTile) scale_ring[slot * C::kTile + lane + 32 * h] = v[h][u];
+            __syncwarp();
+            ptx::mbar_arrive_if(full0 + stage * 8, leader);
+            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+            if (++slot == C::kScaleSlots) slot = 0;
+          }
         }
         if (!ok || ctl->abort_flag) break;
       }
@@ -811,7 +791,7 @@ int launch_cluster(int MT, bool two, const CUtensorMap& map_w, const CUtensorMap
   switch (MT) {
     case 16: return launch<16, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
     case 32: return launch<32, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
-    default: return launch<64, UE, false, 1, true>(map_w, map_a, p, grid, st, items, c);
+    default: return launch<32, UE, false, 2, true>(map_w, map_a, p, grid, st, items, c);  // two sets: 64 x 7168 x 16384 24.9 -> 24.6 us, 40 x 2112 x 7168 9.4 -> 8.9
   }
 }
 

@@ -112,6 +112,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
 __device__ __forceinline__ void mbar_arrive_a(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// The same where `pred` holds, without a branch around it
+__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool pred) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %1, 0;\n"
+      "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n"
+      "}\n" ::"r"(bar),
+      "r"((uint32_t)pred)
+      : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_expect_tx_a(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -198,6 +209,11 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu_u32(const uint32_t* p) {
   return v;
 }
 
+__device__ __forceinline__ float2 ld_shared_f32x2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
@@ -286,6 +302,41 @@ __device__ __forceinline__ void mma_f8f6f4(uint32_t d_tmem, uint64_t a_desc, uin
 // The mbarrier gets one arrival when all tcgen05 operations issued so far by this thread are done.
 __device__ __forceinline__ void mma_commit_a(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// One k-block: four MMAs 32 bytes of K apart (+2 in the descriptors' address fields, inside the 128-byte swizzle atom), the first of
+// which overwrites D, then the commit, issued by the lane whose `pred` holds.  The whole warp runs through them with a predicate
+// instead of one lane through a branch.
+__device__ __forceinline__ void mma_f8f6f4_x4_if(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool pred) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e, first, more;\n"
+      ".reg .b64 a, b;\n"
+      "setp.ne.b32 e, %4, 0;\n"
+      "setp.ne.b32 first, 0, 0;\n"
+      "setp.eq.b32 more, 0, 0;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, first;\n"
+      "add.s64 a, %1, 2;\n"
+      "add.s64 b, %2, 2;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, more;\n"
+      "add.s64 a, %1, 4;\n"
+      "add.s64 b, %2, 4;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, more;\n"
+      "add.s64 a, %1, 6;\n"
+      "add.s64 b, %2, 6;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, more;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)pred)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit_if(uint32_t bar, bool pred) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "setp.ne.b32 e, %1, 0;\n"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(bar),
+      "r"((uint32_t)pred)
+      : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))

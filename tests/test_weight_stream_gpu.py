@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import oracle
-from helpers import assert_gemm_close, make_activations, make_weight
+from helpers import assert_gemm_close, last_gemm, make_activations, make_weight
 
 pytestmark = pytest.mark.gpu
 
@@ -128,3 +128,47 @@ def test_weights_written_by_the_kernel_before(M):
     torch.cuda.synchronize()
     for i, out in enumerate(got):
         assert torch.equal(out, want[i % 3]), f"call {i} saw other weights"
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64])
+@pytest.mark.parametrize("k_blocks", [1, 2, 5, 11, 12, 23])
+def test_rings_over_several_tiles(M, k_blocks):
+    """Barriers, tensor-memory stages and scale slots go round in rings of different lengths, over the end of a tile too: up to
+    three tiles on a CTA, K from one k-block to more than twice the longest ring, an odd end of K.  No cluster shares K here, so
+    the bits are those of the 128 x 128 tiles (row-major scales keep the explicit entry on them)."""
+    from sglang_b200._lib import check, lib
+    from sglang_b200.layers.quantization import w8a8_block_fp8_matmul
+    N, K = 128 * 300 + 8, 128 * k_blocks - (96 if k_blocks > 1 else 0)
+    g = torch.Generator(device="cuda").manual_seed(M * 100 + k_blocks)
+    a = (torch.randn(M, K, generator=g, device="cuda") * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    w = (torch.randn(N, K, generator=g, device="cuda") * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    a_s = torch.rand(M, k_blocks, generator=g, device="cuda") + 0.5
+    w_s = torch.rand(-(-N // 128), k_blocks, generator=g, device="cuda") + 0.5
+    got = w8a8_block_fp8_matmul(a, w, a_s, w_s, [128, 128], torch.bfloat16)
+    assert last_gemm() == "fp8_block_gemm_smallm_kernel"
+    want = torch.empty_like(got)
+    check(lib().sglb200_fp8_blockwise_scaled_mm_pair(
+        a.data_ptr(), w.data_ptr(), a_s.data_ptr(), w_s.data_ptr(), want.data_ptr(), M, N, K, K, K, N, a_s.stride(0), a_s.stride(1),
+        w_s.stride(0), w_s.stride(1), 0, 256, torch.cuda.current_stream().cuda_stream), "fp8_blockwise_scaled_mm_pair")
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    if M > 1:  # a single row's scales pass for M-major ones, which the pair kernel takes (the same bits again)
+        assert last_gemm() == "fp8_block_gemm_kernel"
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("ue8m0", [False, True])
+@pytest.mark.parametrize("M", [33, 47, 48, 49, 64])
+@pytest.mark.parametrize("N,K", [(576, 7168), (2112, 1536), (1000, 1024)])
+def test_two_promotion_sets_in_clusters(M, N, K, ue8m0):
+    """33 to 64 rows where clusters share K: two sets of 32 columns, the second one full, ragged and down to a single column."""
+    from sglang_b200._lib import lib
+    from sglang_b200.layers.quantization import w8a8_block_fp8_matmul
+    x = make_activations(M, K, seed=M)
+    w, w_s = oracle.block_quant_weight(torch.randn(N, K, generator=torch.Generator().manual_seed(N)) * 0.02, scale_ue8m0=ue8m0)
+    a, a_s = oracle.per_token_group_quant_fp8(x, 128, scale_ue8m0=ue8m0)
+    got = w8a8_block_fp8_matmul(a.cuda(), w.cuda(), a_s.cuda(), w_s.cuda(), [128, 128], torch.bfloat16)
+    assert last_gemm() == "fp8_block_gemm_smallm_kernel"
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    assert_gemm_close(got, oracle.w8a8_block_fp8_matmul(a, w, a_s, w_s), f"{M}x{N}x{K}")
