@@ -1568,6 +1568,16 @@ extern "C" int sglb200_fp8_block_linear(const void* x, const void* w, const void
   const sglb::LinearScratch l = sglb::linear_scratch(M, N, K, ue, di.sm_count);
   SGLB_REQUIRE(scratch_bytes >= l.bytes, SGLB200_ERR_WORKSPACE, "scratch_bytes=%lld: %lld needed", (long long)scratch_bytes,
                (long long)l.bytes);
+  // The GEMM quantises the rows itself and leaves the scratch alone.  It reads x while other CTAs store already, so an output on top of
+  // x takes the general way, as does what that way refuses or has another path for.
+  const char *x0 = static_cast<const char*>(x), *out0 = static_cast<const char*>(out);
+  if (M <= 16 && N % 8 == 0 && N < ((int64_t)1 << 31) - 256 && K < ((int64_t)1 << 31) - 256 && x && w && w_scale && out &&
+      sglb::aligned(x, 16) && sglb::aligned(w, 16) && sglb::aligned(out, 16) && sglb::aligned(w_scale, 4) && eps >= 0.f &&
+      di.cc_major == 10 && (out0 + M * N * 2 <= x0 || x0 + M * K * 2 <= out0) && sglb::smallm_quantises(M, N, K, di.sm_count)) {
+    const sglb::RawRows raw = {eps};
+    return sglb::smallm_gemm(x, w, nullptr, static_cast<const float*>(w_scale), out, M, N, K, K, K, N, 0, 0, w_scale_stride_n,
+                             w_scale_stride_k, dtype, bias, nullptr, 0, di.sm_count, stream, nullptr, ue, &raw);
+  }
   char* base = static_cast<char*>(scratch);
   void *scales = base + l.scales_at, *codes = base + l.codes_at;
   if (int rc = sglb::quant_rows(x, dtype, codes, scales, M, K, eps, ue, 1, l.ld, stream)) return rc;

@@ -28,8 +28,8 @@
 // then re-read, from L2), an expert without rows gets no item, so only the weights of routed experts are streamed.
 //
 // warp 0: TMA producer; warp 1: TMEM owner + MMA issuer; warp 2: scale loader (sa[token] * sb into a slot per k-block), or
-// at one or two rows warps 2 and 3: quantisers (QUANT); warps 4..7
-// (..11): promotion (tcgen05.ld, acc += p * scale) and the transposed store.  All waits are bounded.
+// up to sixteen rows warps 2, 3 and 8..15: quantisers (QUANT); warps 4..7
+// (..11, ..19): promotion (tcgen05.ld, acc += p * scale) and the transposed store.  All waits are bounded.
 //
 // The kernel is launched with programmatic stream serialization: it may start while the kernel before it (the
 // activation quantiser, or the previous layer's reduce kernel) is still running.  Its set-up and the WEIGHT tiles of the
@@ -88,7 +88,7 @@ constexpr int kMaxExperts = 1024;
 template <int MT, int NSUB = 1>
 struct Cfg {
   static constexpr int kTile = MT * NSUB;  // most activation rows per work item = TMEM columns per stage
-  static constexpr int kStages = kTile == 160 ? 5 : (kTile == 128 ? 6 : (kTile == 64 ? 8 : (kTile == 32 ? 10 : 11)));
+  static constexpr int kStages = kTile == 128 ? 6 : (kTile == 64 ? 8 : (kTile == 32 ? 10 : 11));
   static constexpr int kAcc = (512 / kTile) < kStages ? (512 / kTile) : kStages;
   static constexpr int kThreads = 128 + 128 * NSUB;
   static constexpr uint32_t kABytes = kTile * BK;
@@ -267,78 +267,109 @@ __device__ __forceinline__ uint32_t pack16(float a, float b, int out_dtype) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// Warps 2 and 3 of the QUANT form (one or two rows): the activations come as they are, and these two warps quantise them on their
-// way into the ring, four k-blocks each in turn, with the arithmetic of the separate quantiser.  Every CTA does so for all k-blocks
-// it multiplies; at one or two rows a group of four k-blocks is one or two passes of a warp, less than the weights take to
-// arrive, and it saves a launch and the hand-over between two kernels.  With four passes it no longer hides.  Replayed graph of
-// calls over rotating weights, quantiser kernel -> this, N x K: M=1 576 x 7168 6.6 -> 6.1 us, 24576 x 1536 9.6 -> 9.05, 7168 x
-// 16384 23.4 -> 21.9, 36864 x 7168 43.0 -> 40.4; M=2 6.95 -> 6.3, 9.7 -> 9.3, 23.7 -> 23.0, 42.2 -> 41.5; M=4 7.0 -> 7.4, 10.5 ->
-// 12.9, 23.9 -> 31.2, 42.6 -> 53.
-constexpr int kQuantRows = 2;
+// Ten warps (2, 3 and 8 to 15) of the QUANT form, up to sixteen rows: the activations come as they are, and these warps quantise them
+// on their way into the ring, with the arithmetic of the separate quantiser.  Each takes every tenth k-block whole, four rows a pass,
+// with the rows of its next k-block in flight while it converts.  Every CTA does so for all k-blocks it multiplies, which is less
+// work than the weights take to arrive, and saves a kernel and the hand-over from it.  Bound by instructions issued: a k-block of 16
+// rows takes the ten warps about 220 ns (16 KB of weights for each of 112 CTAs: 280 ns of HBM).  Replayed graph of calls over
+// rotating weights, quantiser kernel -> this, N x K at M = 4 / 8 / 16, us: 576 x 7168 6.8 / 6.8 / 7.2 -> 5.5 / 5.9 / 7.1, 24576 x 1536
+// 10.2 / 10.2 / 10.4 -> 8.6 / 9.0 / 9.6, 7168 x 16384 23.2 / 23.8 / 24.3 -> 21.5 / 22.0 / 23.2, 36864 x 7168 42.2 / 42.6 / 43.5 -> 40.0 /
+// 41.1 / 42.5.  Two warps with four k-blocks each in turn, at one or two rows (more were slower than the kernel): 576 x 7168 5.66 / 5.96
+// -> 5.48 / 5.50, 10240 x 8192 17.2 / 19.7 -> 16.7 / 16.6.  Each pass with its own maxima, scale and branch on it: 16 x 7168 x 16384 27.0.
+//
+// A warp's wait for a stage looks at one parity, which is right only if the stage's k-block before last is known to be done; the
+// warp's wait for its own k-block before this one says so if that one is at most a ring back (commits arrive in order).
+constexpr int kQuantRows = 2;  // rows that a call may pass without scratch
+constexpr int kMaxQuantRows = 16, kQuantWarps = 10;
+static_assert(kQuantWarps <= Cfg<16>::kStages, "see above");
 
-template <typename T, int MT, bool UE, bool CLUSTER>
+template <typename T, int PASSES, bool UE, bool CLUSTER>
 __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, uint8_t* smem, float* scale_ring, uint32_t me, int lane,
-                                              int32_t total) {
-  using C = Cfg<MT>;
+                                                   int32_t total) {
+  using C = Cfg<16>;
+  static_assert(kMaxQuantRows == C::kTile && PASSES <= 4, "four rows a pass");
   const uint32_t full0 = ptx::smem_u32(&ctl->full[0]), done0 = ptx::smem_u32(&ctl->done[0]);
-  // eight lanes (sixteen elements each) take a row of a k-block; a pass of the warp covers the rows of `per_pass` k-blocks
-  static_assert(kScaleGroup == 4 && kQuantRows == 2, "four rows of k-blocks per pass");
-  const int rows = p.M, per_pass = kScaleGroup / rows;
-  const int sub = lane & 7, r = (lane >> 3) & (rows - 1), ko = (lane >> 3) / rows;
-  const uint4* row = reinterpret_cast<const uint4*>(static_cast<const T*>(p.x) + (int64_t)r * p.K) + 2 * sub;
-  const uint32_t piece = kWBytes + (uint32_t)(r * 128 + ((sub ^ r) << 4));  // 128-byte swizzle
+  const int rows = p.M, sub = lane & 7, r0 = lane >> 3;  // eight lanes, sixteen elements each, take a row of a pass
+  const uint4* row[PASSES];
+#pragma unroll
+  for (int u = 0; u < PASSES; ++u)  // rows past the last one are read as the last one, and not stored
+    row[u] = reinterpret_cast<const uint4*>(static_cast<const T*>(p.x) + (int64_t)min(4 * u + r0, rows - 1) * p.K) + 2 * sub;
   const float inv_max = __frcp_rn(448.0f);
-  uint32_t stage = 0, phase = 0, slot = 0, turn = 0;
+  const int scale_row = 4 * (sub >> 1) + r0;  // the row whose scale this lane computes
+  const bool has_scale = (sub & 1) == 0 && scale_row < rows;
+  uint32_t stage = me, phase = 0, slot = me;
+  int32_t i = (int32_t)me;  // this warp's next k-block, counted from the item's first
   for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
     const Item it = get_item<C::kTile, false, CLUSTER>(p, nullptr, t);
     const float* sb_blk = p.sb + (int64_t)it.nt * p.sb_stride_n;
-    for (int32_t kb0 = it.kb0; kb0 < it.kb1; kb0 += kScaleGroup, turn ^= 1) {
-      if (turn == me) {
-        uint4 v[kQuantRows][2];
-        float b[kQuantRows];
+    uint4 v[PASSES][2];
+    float b = 0.f;
+    auto fetch = [&](int32_t kb) {
+      b = load_scale<UE>(sb_blk, kb, p.sb_stride_k);
 #pragma unroll
-        for (int u = 0; u < kQuantRows; ++u) {
-          if (u >= rows) break;
-          const int32_t kb = min(kb0 + u * per_pass + ko, it.kb1 - 1);
-          v[u][0] = __ldg(row + (int64_t)kb * (BK / 8));
-          v[u][1] = __ldg(row + (int64_t)kb * (BK / 8) + 1);
-          b[u] = load_scale<UE>(sb_blk, kb, p.sb_stride_k);
-        }
-#pragma unroll
-        for (int u = 0; u < kQuantRows; ++u) {
-          if (u >= rows || kb0 + u * per_pass >= it.kb1) break;
-          float amax = fmaxf(p.eps, fmaxf(Elem<T>::vec_absmax(v[u][0]), Elem<T>::vec_absmax(v[u][1])));
-#pragma unroll
-          for (int m = 4; m >= 1; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
-          const float s = group_scale_fast(amax, 448.0f, inv_max, UE);
-          const uint4 codes = encode16_e4m3<T>(v[u][0], v[u][1], s);
-          const int n = min(per_pass, it.kb1 - kb0 - u * per_pass);  // k-blocks of this pass
-          uint32_t mine = stage, mine_slot = slot;
-          for (int i = 0; i < n; ++i) {
-            if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 11); return; }
-            if (i == ko) { mine = stage; mine_slot = slot; }
-            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
-            if (++slot == C::kScaleSlots) slot = 0;
-          }
-          if (ko < n) {
-            *reinterpret_cast<uint4*>(smem + (size_t)mine * C::kStageBytes + piece) = codes;
-            if (sub == 0) scale_ring[mine_slot * C::kTile + r] = s * b[u];
-          }
-          ptx::fence_proxy_async();  // the MMA reads shared memory through the asynchronous proxy
-          __syncwarp();
-          if (ko < n && (lane & (8 * rows - 1)) == 0) ptx::mbar_arrive_a(full0 + mine * 8);
-        }
-        __syncwarp();
-      } else {
-        const uint32_t n = min(kScaleGroup, it.kb1 - kb0);
-        stage += n;
-        if (stage >= (uint32_t)C::kStages) { stage -= C::kStages; phase ^= 1; }
-        slot += n;
-        if (slot >= (uint32_t)C::kScaleSlots) slot -= C::kScaleSlots;
+      for (int u = 0; u < PASSES; ++u) {
+        v[u][0] = __ldg(row[u] + (int64_t)kb * (BK / 8));
+        v[u][1] = __ldg(row[u] + (int64_t)kb * (BK / 8) + 1);
       }
+    };
+    const int32_t n = it.kb1 - it.kb0;
+    if (i < n) fetch(it.kb0 + i);
+    for (; i < n; i += kQuantWarps) {
+      // Maxima of all passes at once: two lanes end up with the maximum of each pass's row, and with one scale and one
+      // reciprocal to compute for it.
+      float m[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        m[u] = u < PASSES ? fmaxf(Elem<T>::vec_absmax(v[u < PASSES ? u : 0][0]), Elem<T>::vec_absmax(v[u < PASSES ? u : 0][1])) : 1.f;
+      const bool up = (sub & 4) != 0, odd = (sub & 2) != 0;
+      const float x0 = fmaxf(up ? m[2] : m[0], __shfl_xor_sync(0xffffffffu, up ? m[0] : m[2], 4));
+      const float x1 = fmaxf(up ? m[3] : m[1], __shfl_xor_sync(0xffffffffu, up ? m[1] : m[3], 4));
+      float amax = fmaxf(odd ? x1 : x0, __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 2));
+      amax = fmaxf(p.eps, fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1)));
+      uint4 codes[PASSES];
+      float s;
+      // no branch inside the passes where every scale is an ordinary number, so that they run side by side
+      if (__all_sync(0xffffffffu, amax >= 1e-27f && amax <= 1e30f)) {
+        s = group_scale_fast(amax, 448.0f, inv_max, UE, true);
+        const float r = __frcp_rn(s);
+#pragma unroll
+        for (int u = 0; u < PASSES; ++u)
+          codes[u] = encode16_e4m3<T, true>(v[u][0], v[u][1], __shfl_sync(0xffffffffu, s, 2 * u, 8), __shfl_sync(0xffffffffu, r, 2 * u, 8));
+      } else {
+        s = group_scale_fast(amax, 448.0f, inv_max, UE);
+#pragma unroll
+        for (int u = 0; u < PASSES; ++u) codes[u] = encode16_e4m3<T>(v[u][0], v[u][1], __shfl_sync(0xffffffffu, s, 2 * u, 8));
+      }
+      const float prod = s * b;
+      if (i + kQuantWarps < n) fetch(it.kb0 + i + kQuantWarps);
+      if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 11); return; }
+      uint8_t* dst = smem + (size_t)stage * C::kStageBytes + kWBytes;
+#pragma unroll
+      for (int u = 0; u < PASSES; ++u) {
+        const int r = 4 * u + r0;
+        if (r < rows) *reinterpret_cast<uint4*>(dst + r * 128 + ((sub ^ (r & 7)) << 4)) = codes[u];  // 128-byte swizzle
+      }
+      if (has_scale) scale_ring[slot * C::kTile + scale_row] = prod;
+      ptx::fence_proxy_async();  // the MMA reads shared memory through the asynchronous proxy
+      __syncwarp();
+      ptx::mbar_arrive_if(full0 + stage * 8, lane == 0);
+      stage += kQuantWarps;
+      if (stage >= (uint32_t)C::kStages) { stage -= C::kStages; phase ^= 1; }
+      slot += kQuantWarps;
+      if (slot >= (uint32_t)C::kScaleSlots) slot -= C::kScaleSlots;
     }
+    i -= n;
     if (ctl->abort_flag) return;
   }
+}
+
+template <typename T, bool UE, bool CLUSTER>
+__device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, uint8_t* smem, float* scale_ring, uint32_t me, int lane,
+                                                   int32_t total) {
+  if (p.M <= 4) quantise_rows<T, 1, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
+  else if (p.M <= 8) quantise_rows<T, 2, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
+  else if (p.M <= 12) quantise_rows<T, 3, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
+  else quantise_rows<T, 4, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
 }
 
 // CLUSTER is a template parameter because the mere presence of the adding-up code cost the main loop of the other form up to
@@ -347,7 +378,7 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
 template <int MT, bool UE, bool GROUPED, int NSUB, bool CLUSTER, bool QUANT>
 // NSUB = 1 has 256 threads; the bound of 320 keeps it at 200 registers, so that a block of the quantiser or of another small
 // kernel (256 threads of 48) fits beside it and programmatic dependent launch really overlaps the two.
-__global__ void __launch_bounds__(NSUB == 1 ? 320 : 128 + 128 * NSUB, 1)
+__global__ void __launch_bounds__(QUANT ? 192 + 32 * kQuantWarps : (NSUB == 1 ? 320 : 128 + 128 * NSUB), 1)
 fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                              const SmallParams p) {
   using C = Cfg<MT, NSUB>;
@@ -418,7 +449,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
   // Register split (NSUB = 2): eight promotion warps with 64 accumulators, 64 loaded sums and the scales in flight want more
   // than the 168 registers that 384 threads start with; the other four warps need few: 128 * 96 + 256 * 200 = 63488 <=
   // 384 * 168.  No call may sit in a region with a changed limit, hence the inlined waits.
-  if (warp >= 4) {
+  if (warp >= 4 && (!QUANT || warp < 8)) {
     if constexpr (NSUB == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPromoRegs));
     // ===== promotion + transposed store; TMEM lane quarter = warp % 4.  A warp owns 32 weight rows (columns of the output)
     // and MT tokens.  The sums are loaded in fragment arrangement (tmem_ld_16x256), in which a thread meets only MT / 4
@@ -671,11 +702,12 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         }
         if (!ok || ctl->abort_flag) break;
       }
-    } else if (QUANT) {
-      // ===== quantisers (warps 2 and 3)
+    } else if constexpr (QUANT) {
+      // ===== quantisers (warps 2, 3 and 8 to 15)
       ptx::grid_dep_wait();  // the rows come from the kernel before this one
-      if (p.out_dtype == SGLB200_BF16) quantise_rows<__nv_bfloat16, MT, UE, CLUSTER>(p, ctl, smem, scale_ring, warp - 2, lane, total);
-      else quantise_rows<__half, MT, UE, CLUSTER>(p, ctl, smem, scale_ring, warp - 2, lane, total);
+      const uint32_t me = warp < 4 ? warp - 2 : warp - 6;
+      if (p.out_dtype == SGLB200_BF16) quantise_rows<__nv_bfloat16, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
+      else quantise_rows<__half, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
     } else if (warp == 2) {
       // ===== scale loader: per group of four k-blocks the products sa[token, kb] * sb[nt, kb], 0 for tokens past the item's
       // rows (the accumulator columns there hold leftovers and are not stored).  The loads of the next group are in flight
@@ -752,7 +784,7 @@ template <int MT, bool UE, bool GROUPED, int NSUB = 1, bool CLUSTER = false, boo
 int launch(const CUtensorMap& map_w, const CUtensorMap& map_a, const SmallParams& p, int sm_count, cudaStream_t st,
            int64_t max_items, int cluster = 1) {
   constexpr size_t smem = GROUPED ? Cfg<MT, NSUB>::kSmemGrouped : Cfg<MT, NSUB>::kSmem;
-  constexpr int kThreads = Cfg<MT, NSUB>::kThreads;
+  constexpr int kThreads = QUANT ? 192 + 32 * kQuantWarps : Cfg<MT, NSUB>::kThreads;
   static bool done[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -795,12 +827,32 @@ int launch_cluster(int MT, bool two, const CUtensorMap& map_w, const CUtensorMap
   }
 }
 
+// rows that the GEMM itself quantises
+int launch_quant(const CUtensorMap& map_w, const SmallParams& p, bool ue8m0, int sm_count, cudaStream_t st, int64_t items) {
+  if (p.cluster > 1)
+    return ue8m0 ? launch<16, true, false, 1, true, true>(map_w, map_w, p, (int)items, st, items, p.cluster)
+                 : launch<16, false, false, 1, true, true>(map_w, map_w, p, (int)items, st, items, p.cluster);
+  return ue8m0 ? launch<16, true, false, 1, false, true>(map_w, map_w, p, sm_count, st, items)
+               : launch<16, false, false, 1, false, true>(map_w, map_w, p, sm_count, st, items);
+}
+
 }  // namespace
 
 // Row limit of this kernel, and of the scratch sizes that callers know (smallm_splits)
 int smallm_max_rows() { return 128; }
 
 int smallm_quant_rows() { return kQuantRows; }
+
+// Whether the GEMM quantises M rows itself rather than after the quantiser kernel.  Above eight rows the ten warps' instructions begin to
+// show; graph of calls, quantiser kernel / this, us.  More than two tiles a CTA, each with all of its k-blocks again: 12 x 57344 x 8192
+// 75.5 / 77.1.  Above twelve rows also: long ranges of K on too few CTAs for HBM to be the limit, 16 x 10240 x 8192 18.1 / 18.6, and
+// clusters of eight on most of the SMs, 16 x 2112 x 7168 8.4 / 8.8 (16 x 1536 x 7168, 96 CTAs, 7.8 / 7.8).
+bool smallm_quantises(int64_t M, int64_t N, int64_t K, int sm_count) {
+  if (M <= 8) return true;
+  const int64_t n_tiles = (N + BN - 1) / BN, c = smallm_cluster(M, N, K, sm_count), ctas = n_tiles * c, kb = K / BK / c;
+  if (M > kMaxQuantRows || n_tiles > 2 * sm_count) return false;
+  return M <= 12 || ((ctas >= 88 || kb <= 24) && (c < kMaxCluster || ctas <= 96));
+}
 
 // From 65 rows up a k-block takes this kernel 780 cycles and the 128 x 128 kernel 425: where every CTA works alone, that one takes
 // the call (GEMM alone in a replayed graph, this / the tile kernel, us: 113 x 10240 x 8192 27.5/20.3, 65 x 36864 x 7168 48.6/46.6,
@@ -917,11 +969,7 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
   if (raw != nullptr) {
     p.x = a;
     p.eps = raw->eps;
-    if (p.cluster > 1)
-      return ue8m0 ? launch<16, true, false, 1, true, true>(map_w, map_w, p, (int)items, st, items, p.cluster)
-                   : launch<16, false, false, 1, true, true>(map_w, map_w, p, (int)items, st, items, p.cluster);
-    return ue8m0 ? launch<16, true, false, 1, false, true>(map_w, map_w, p, sm_count, st, items)
-                 : launch<16, false, false, 1, false, true>(map_w, map_w, p, sm_count, st, items);
+    return launch_quant(map_w, p, ue8m0, sm_count, st, items);
   }
   if (p.cluster > 1)
     return ue8m0 ? launch_cluster<true>(MT, two, map_w, map_a, p, st, items) : launch_cluster<false>(MT, two, map_w, map_a, p, st, items);

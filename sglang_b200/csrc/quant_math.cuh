@@ -84,9 +84,10 @@ SGLB_HD float mul_rn(float a, float b) {
 // rem = amax - q0*fp8_max (exact, one FMA), s = q0 + rem*c is the correctly rounded quotient
 // whenever it is a normal number (checked on the host for fp8_max = 448 over every 16-bit-float
 // amax and a long run of random fp32 ones); tiny maxima, which need eps < 2^-100, take the division.
-SGLB_HD float group_scale_fast(float amax, float fp8_max, float inv_max, bool ue8m0) {
+// `normal`: the caller knows that amax is not one of them.
+SGLB_HD float group_scale_fast(float amax, float fp8_max, float inv_max, bool ue8m0, bool normal = false) {
   float s;
-  if (amax >= 7.888609e-31f) {
+  if (normal || amax >= 7.888609e-31f) {
     const float q0 = mul_rn(amax, inv_max);
     const float rem = fma_rn(-q0, fp8_max, amax);
     s = fma_rn(rem, inv_max, q0);

@@ -135,10 +135,10 @@ __device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
 
 // Sixteen consecutive 16-bit inputs (two 16-byte vectors) divided by the group's scale and converted to e4m3 with the
 // e4m3 limits (the saturating conversion clamps): the same operations, in the same order, as group_quant16_kernel.
-template <typename T>
-__device__ __forceinline__ uint4 encode16_e4m3(const uint4& v0, const uint4& v1, float s) {
-  const bool fast = (s >= 7.888609e-31f) && (s <= 1.2676506e30f);
-  const float r = __frcp_rn(s);
+// r = RN(1 / s); kNormal: the caller knows that the scale lies between the limits below.
+template <typename T, bool kNormal = false>
+__device__ __forceinline__ uint4 encode16_e4m3(const uint4& v0, const uint4& v1, float s, float r) {
+  const bool fast = kNormal || (s >= 7.888609e-31f) && (s <= 1.2676506e30f);
   const float2 rr = make_float2(r, r), nss = make_float2(-s, -s);
   uint32_t packed[4];
 #pragma unroll
@@ -161,6 +161,10 @@ __device__ __forceinline__ uint4 encode16_e4m3(const uint4& v0, const uint4& v1,
     }
   }
   return make_uint4(packed[0], packed[1], packed[2], packed[3]);
+}
+template <typename T>
+__device__ __forceinline__ uint4 encode16_e4m3(const uint4& v0, const uint4& v1, float s) {
+  return encode16_e4m3<T>(v0, v1, s, __frcp_rn(s));
 }
 
 }  // namespace sglb

@@ -104,6 +104,64 @@ def test_rows_quantised_by_the_gemm_itself(M, N, K, dtype, ue8m0):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("ue8m0", [False, True])
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 9, 12, 13, 16])
+@pytest.mark.parametrize("N,K,dtype", [(576, 7168, torch.bfloat16), (136, 640, torch.float16), (20000, 1408, torch.bfloat16),
+                                       (3072, 1536, torch.float16), (1000, 128, torch.bfloat16)])
+def test_up_to_sixteen_rows_quantised_by_the_gemm(N, K, dtype, M, ue8m0):
+    """Every number of passes of four rows, full and ragged, from one k-block to several rings on a CTA: the bits of the quantiser
+    kernel and the same GEMM.  A group of zeros, and a row beyond the range of the branch-free division (scale above 2^100)."""
+    from sglang_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(M * 1000 + K)
+    x = torch.randn(M, K, generator=g, device="cuda")
+    x = (x * torch.pow(10.0, torch.rand(M, 1, generator=g, device="cuda") * 4 - 2)).to(dtype)
+    x[M // 2, :128] = 0
+    if dtype == torch.bfloat16:
+        x[M - 1, -128:] *= 1e35
+    w = (torch.randn(N, K, generator=g, device="cuda") * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    words = (K // 128 + 3) // 4
+    if ue8m0:
+        ws = torch.randint(120, 130, (-(-N // 128), words * 4), generator=g, device="cuda", dtype=torch.uint8).view(torch.int32)
+    else:
+        ws = torch.rand(-(-N // 128), K // 128, generator=g, device="cuda") + 0.5
+    kind = 0 if dtype == torch.bfloat16 else 1
+    L, stream = lib(), torch.cuda.current_stream().cuda_stream
+    bytes_ = L.sglb200_fp8_block_linear_scratch_bytes(M, N, K, int(ue8m0))
+    scratch = torch.full((max(bytes_, 1),), 0x5a, dtype=torch.uint8, device="cuda")
+    got = torch.full((M, N), 7.0, dtype=dtype, device="cuda")
+
+    def linear(rows, out):
+        check(L.sglb200_fp8_block_linear(rows.data_ptr(), w.data_ptr(), ws.data_ptr(), None, out.data_ptr(), M, N, K, ws.stride(0),
+                                         ws.stride(1), int(ue8m0), 1e-10, kind, scratch.data_ptr(), bytes_, stream), "fp8_block_linear")
+
+    linear(x, got)
+    torch.cuda.synchronize()
+    assert last_gemm() == "fp8_block_gemm_smallm_kernel"
+    assert (scratch == 0x5a).all(), "a separate quantiser ran"
+    # the quantiser kernel, then the same GEMM on its codes
+    q = torch.empty(M, K, dtype=torch.float8_e4m3fn, device="cuda")
+    ld = (M + 3) // 4 * 4
+    s = torch.zeros(words if ue8m0 else K // 128, ld, dtype=torch.int32 if ue8m0 else torch.float32, device="cuda")
+    check(L.sglb200_per_token_group_quant_fp8(x.data_ptr(), kind, q.data_ptr(), s.data_ptr(), M, K, 128, 1e-10, -448.0, 448.0,
+                                              int(ue8m0), 1, ld, stream), "per_token_group_quant_fp8")
+    want = torch.empty_like(got)
+    if ue8m0:
+        check(L.sglb200_fp8_ue8m0_scaled_mm(q.data_ptr(), w.data_ptr(), s.data_ptr(), ws.data_ptr(), want.data_ptr(), M, N, K, K, K, N,
+                                            ld, ws.stride(0), ws.stride(1), kind, stream), "fp8_ue8m0_scaled_mm")
+    else:
+        check(L.sglb200_fp8_blockwise_scaled_mm(q.data_ptr(), w.data_ptr(), s.data_ptr(), ws.data_ptr(), want.data_ptr(), M, N, K, K, K,
+                                                N, 1, ld, ws.stride(0), ws.stride(1), kind, stream), "fp8_blockwise_scaled_mm")
+    torch.cuda.synchronize()
+    assert L.sglb200_read_device_status() == 0
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    if N <= K:  # an output on top of the input: quantised before anything is stored, as ever
+        both = x.clone()
+        linear(both, both.view(-1)[:M * N].view(M, N))
+        torch.cuda.synchronize()
+        if M > 2:
+            assert torch.equal(both.view(-1)[:M * N].view(M, N).view(torch.int16), want.view(torch.int16))
+
+
 @pytest.mark.parametrize("M", [1, 16, 128])
 def test_weights_written_by_the_kernel_before(M):
     """The quantiser writes the codes that the next call takes as weights, into the same memory every time: the
