@@ -258,6 +258,10 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uin
                "r"(d)
                : "memory");
 }
+// two of them: lanes 0 to 15 pass the addresses
+__device__ __forceinline__ void stmatrix_x2_trans(uint32_t addr, uint32_t a, uint32_t b) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x2.trans.shared.b16 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
 __device__ __forceinline__ uint32_t pack16(float a, float b, int out_dtype) {
   if (out_dtype == SGLB200_BF16) {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -370,6 +374,58 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
   else if (p.M <= 8) quantise_rows<T, 2, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
   else if (p.M <= 12) quantise_rows<T, 3, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
   else quantise_rows<T, 4, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
+}
+
+// One CTA's share of a tile whose K a cluster of RANKS cuts.  A piece is 16 weight rows x 8 tokens of a warp's 32 x MT sums, 16 bytes a
+// lane, piece 2g + h for token group g and half h of the rows; the CTAs take equal runs of the pieces that have rows, and add them in
+// the order of K.  All loads of a turn (eight) are in flight at once: a round trip through another CTA's shared memory is what
+// bounds this.  Rank 0 adding up everything, rank after rank, took 7 round trips in clusters of eight, and 32 KB of the
+// other CTAs' memory for each 32 tokens of it; call, N x K, us, that -> this: @@S3
+template <int RANKS>
+__device__ __forceinline__ void add_up_share(const SmallParams& p, uint32_t local, uint8_t* patch, int32_t rank, int32_t row0, int32_t rows,
+                                             int32_t n_warp, int lane) {
+  constexpr int kTurn = RANKS == 2 ? 4 : (RANKS == 4 ? 2 : 1);  // pieces a turn
+  const int32_t pieces = 2 * ((rows + 7) >> 3), per = (pieces + RANKS - 1) / RANKS;
+  const int32_t first = rank * per, last = min(first + per, pieces);
+  char* out = static_cast<char*>(p.out) + ((int64_t)row0 * p.ldc + n_warp) * 2;
+  const char* bias = static_cast<const char*>(p.bias);
+  const uint32_t st_addr = ptx::smem_u32(patch) + (uint32_t)(lane & 7) * kPatchRow + (uint32_t)((lane >> 3) & 1) * 16;
+#pragma unroll 1
+  for (int32_t e0 = first; e0 < last; e0 += kTurn) {
+    float4 v[kTurn][RANKS];
+#pragma unroll
+    for (int k = 0; k < kTurn; ++k)
+#pragma unroll
+      for (int r = 0; r < RANKS; ++r)  // past the last piece: that one again, not stored
+        v[k][r] = ptx::ld_cluster_f4(ptx::mapa_shared(local + (uint32_t)min(e0 + k, last - 1) * 32 * (uint32_t)sizeof(float4), (uint32_t)r));
+    __syncwarp();  // the patch has been read out
+#pragma unroll
+    for (int k = 0; k < kTurn; ++k) {
+      float4 sum = v[k][0];
+#pragma unroll
+      for (int r = 1; r < RANKS; ++r) {
+        sum.x += v[k][r].x;
+        sum.y += v[k][r].y;
+        sum.z += v[k][r].z;
+        sum.w += v[k][r].w;
+      }
+      stmatrix_x2_trans(st_addr + (k >> 1) * 8 * kPatchRow + (k & 1) * 32, pack16(sum.x, sum.y, p.out_dtype),
+                        pack16(sum.z, sum.w, p.out_dtype));
+    }
+    __syncwarp();
+    // 16 bytes a lane: eight tokens x two halves of a piece's 16 columns, as many pieces as the warp has lanes for
+#pragma unroll
+    for (int i = 0; i < (kTurn + 1) / 2; ++i) {
+      const int32_t k = 2 * i + (lane >> 4), e = e0 + k, tok = 8 * (e >> 1) + (lane & 7), part = (lane >> 3) & 1;
+      const int32_t c = (e & 1) * 16 + part * 8;
+      if (k < kTurn && e < last && tok < rows && n_warp + c < p.N) {  // N % 8 == 0
+        uint4 val = *reinterpret_cast<const uint4*>(patch + (i * 8 + (lane & 7)) * kPatchRow + (lane >> 4) * 32 + part * 16);
+        if (bias != nullptr)
+          val = ptx::add_bias8(val, __ldg(reinterpret_cast<const uint4*>(bias + (int64_t)(n_warp + c) * 2)), p.out_dtype);
+        *reinterpret_cast<uint4*>(out + ((int64_t)tok * p.ldc + c) * 2) = val;
+      }
+    }
+  }
 }
 
 // CLUSTER is a template parameter because the mere presence of the adding-up code cost the main loop of the other form up to
@@ -523,43 +579,26 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       if (!ok || ctl->abort_flag) break;
       const int32_t n_warp = it.nt * BN + q * 32;  // first of the warp's 32 output columns
       if constexpr (CLUSTER) {
-        {
-          // One tile per cluster, K cut into as many ranges.  The others leave their sums, fragment order, in their own shared
-          // memory (the ring of stages: all of its loads and MMAs are done) and rank 0 adds them in the order of K.
-          constexpr int kWarps = 4 * NSUB;
-          float4* mine = reinterpret_cast<float4*>(smem) + (size_t)(warp - 4) * 2 * G * 32 + lane;
-          if (it.split != 0) {
+        // One tile per cluster, K cut into as many ranges.  Every CTA leaves its sums, fragment order, in its own shared memory (the
+        // ring of stages: all of its loads and MMAs are done), and adds up and stores its share of the tile.
+        constexpr int kWarps = 4 * NSUB;
+        static_assert((size_t)kWarps * 2 * G * 32 * sizeof(float4) <= (size_t)C::kStages * C::kStageBytes, "sums of a tile");
+        float4* mine = reinterpret_cast<float4*>(smem) + (size_t)(warp - 4) * 2 * G * 32 + lane;
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+        for (int g = 0; g < G; ++g)
 #pragma unroll
-              for (int g = 0; g < G; ++g)
-                if (8 * g < rows)
-                  mine[(h * G + g) * 32] = make_float4(acc[h][g][0].x, acc[h][g][0].y, acc[h][g][1].x, acc[h][g][1].y);
-          }
-          met = true;
-          ptx::cluster_arrive_release();
-          ptx::cluster_wait_acquire();
-          static_assert((size_t)kWarps * 2 * G * 32 * sizeof(float4) <= (size_t)C::kStages * C::kStageBytes, "sums of a tile");
-          if (it.split == 0) {
-            const uint32_t local = ptx::smem_u32(mine);
-            for (int32_t r = 1; r < p.cluster; ++r) {
-              const uint32_t src = ptx::mapa_shared(local, (uint32_t)r);
-#pragma unroll
-              for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int g = 0; g < G; ++g)
-                  if (8 * g < rows) {
-                    const float4 v = ptx::ld_cluster_f4(src + (h * G + g) * 32 * (uint32_t)sizeof(float4));
-                    acc[h][g][0].x += v.x;
-                    acc[h][g][0].y += v.y;
-                    acc[h][g][1].x += v.z;
-                    acc[h][g][1].y += v.w;
-                  }
-            }
-          } else {
-            continue;
-          }
+          for (int h = 0; h < 2; ++h)
+            if (8 * g < rows) mine[(2 * g + h) * 32] = make_float4(acc[h][g][0].x, acc[h][g][0].y, acc[h][g][1].x, acc[h][g][1].y);
+        met = true;
+        ptx::cluster_arrive_release();
+        ptx::cluster_wait_acquire();
+        const uint32_t local = ptx::smem_u32(mine);
+        switch (p.cluster) {
+          case 2: add_up_share<2>(p, local, patch, it.split, row0, rows, n_warp, lane); break;
+          case 4: add_up_share<4>(p, local, patch, it.split, row0, rows, n_warp, lane); break;
+          default: add_up_share<8>(p, local, patch, it.split, row0, rows, n_warp, lane); break;
         }
+        continue;
       }
       if (p.partial != nullptr) {
         float* dst = p.partial + ((int64_t)it.split * p.M + row0) * p.N + n_warp;
