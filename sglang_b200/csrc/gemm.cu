@@ -1274,8 +1274,8 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
   SGLB_REQUIRE(di.cc_major == 10, SGLB200_ERR_ARCH, "compute capability %d.%d: this library is built for sm_100a only",
                di.cc_major, di.cc_minor);
 
-  if (!grouped && push && total_rows <= smallm_max_rows() && workspace != nullptr &&
-      (int64_t)smallm_cluster(total_rows, N, K, di.sm_count) * total_rows * N <= workspace_floats) {
+  if (!grouped && push && takes_few_rows(total_rows, N, K, di.sm_count, false) && workspace != nullptr &&
+      (int64_t)smallm_cluster(total_rows, N, K, di.sm_count, false) * total_rows * N <= workspace_floats) {
     // few rows, exchanged: the weight-streaming kernel leaves fp32 sums, a second kernel casts and pushes them.  K is cut as
     // for the plain entry (smallm_cluster), which makes the bits the same.  Both kernels against the ranges that a split through
     // memory would choose by itself (smallm_splits), one rank, M = 16 / 64 / 128: N=7168 K=16384 30.1 / 36.6 / 45.2 against 30.5 /
@@ -1297,7 +1297,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
     SGLB_CHECK_LAUNCH("splitk_reduce_push_kernel");
     return SGLB200_OK;
   }
-  if (!grouped && !push && !tiles_only && takes_few_rows(total_rows, N, K, di.sm_count)) {
+  if (!grouped && !push && !tiles_only && takes_few_rows(total_rows, N, K, di.sm_count, false)) {
     // few rows: the weight-streaming kernel with swapped operands (gemm_smallm.cu)
     return smallm_gemm(a, b, sa, sb, out, total_rows, N, K, lda, ldb, ldc, sa_stride_m, sa_stride_k, sb_stride_n, sb_stride_k,
                        out_dtype, bias, nullptr, 0, di.sm_count, stream, nullptr, false);
@@ -1682,7 +1682,7 @@ extern "C" int64_t sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes(int64_t 
   sglb::DeviceInfo di;
   int sms = 148;
   if (sglb::device_info(&di) == SGLB200_OK) sms = di.sm_count;
-  return (int64_t)sglb::smallm_cluster(M, N, K, sms) * M * N * (int64_t)sizeof(float);
+  return (int64_t)sglb::smallm_cluster(M, N, K, sms, false) * M * N * (int64_t)sizeof(float);
 }
 
 extern "C" int64_t sglb200_peer_recv_bytes(int64_t slot_elems) {

@@ -5,8 +5,8 @@
 // stage is then only MT TMEM columns wide, so 4 to 16 k-blocks are in flight between the MMA warp and the promotion warps, and
 // a shared-memory stage is 16 KB of weights plus MT x 128 bytes of activations, 6 to 11 of them: 64 KB of weights in flight
 // per SM already bring a plain stream of such tiles to 90 % of the HBM rate, 128 KB to all of it.  When
-// N / 128 tiles alone cannot occupy the SMs, the CTAs of a cluster cut a tile's K among themselves and rank 0 adds their sums up
-// out of their shared memory (smallm_cluster): against fp32 partial sums in memory and a kernel that adds them, quantiser
+// N / 128 tiles alone cannot occupy the SMs, the CTAs of a cluster cut a tile's K among themselves and add their sums up
+// out of each other's shared memory, each a share of the tile (smallm_cluster, add_up_share), measured with all of it on rank 0: against fp32 partial sums in memory and a kernel that adds them, quantiser
 // included, N=576 K=7168 M=1 / 48: 9.6 / 14.1 -> 6.8 / 11.1 us, N=7168 K=16384 M=48 32.3 -> 27.1, N=10240 K=8192 M=48 27.0 -> 22.1.
 // From 65 to 128 rows eight or sixteen promotion warps share every accumulator stage, from 33 rows eight where clusters share K.
 //
@@ -110,7 +110,7 @@ struct SmallParams {
   void* out;
   const void* bias;  // [N] of the output type, or NULL: added to the rounded result
   float* partial;    // fp32 sums [splits][M][N] instead of `out`
-  int32_t cluster;   // > 1: the CTAs of a cluster share one tile's K, rank 0 adds their sums up (k_splits == cluster)
+  int32_t cluster;   // > 1: the CTAs of a cluster share one tile's K and add their sums up (k_splits == cluster)
   int32_t M, N, K;
   int32_t n_tiles, k_tiles, k_splits, kb_per_split;
   int64_t ldc;
@@ -379,8 +379,11 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
 // One CTA's share of a tile whose K a cluster of RANKS cuts.  A piece is 16 weight rows x 8 tokens of a warp's 32 x MT sums, 16 bytes a
 // lane, piece 2g + h for token group g and half h of the rows; the CTAs take equal runs of the pieces that have rows, and add them in
 // the order of K.  All loads of a turn (eight) are in flight at once: a round trip through another CTA's shared memory is what
-// bounds this.  Rank 0 adding up everything, rank after rank, took 7 round trips in clusters of eight, and 32 KB of the
-// other CTAs' memory for each 32 tokens of it; call, N x K, us, that -> this: @@S3
+// bounds this.  Rank 0 adding up everything, rank after rank, took
+// seven round trips in clusters of eight, each over the whole tile.  Calls, weights from HBM, us, that -> this, M = 1 / 16 / 64 / 128: 576 x 7168
+// 5.6 / 7.1 / 11.3 / 18.7 -> 4.8 / 5.9 / 7.9 / 10.8, 1536 x 7168 6.2 / 7.8 / 12.3 / 20.3 -> 5.5 / 6.6 / 8.8 / 11.8, 4096 x 4096 (four) 6.6 / 8.1 /
+// 11.4 / 16.8 -> 6.3 / 7.7 / 9.4 / 12.6, 7168 x 16384 (two) 26.7 -> 26.4 at 64.  With 16 loads a turn the kernel spilled in its main loop and
+// took twice as long.
 template <int RANKS>
 __device__ __forceinline__ void add_up_share(const SmallParams& p, uint32_t local, uint8_t* patch, int32_t rank, int32_t row0, int32_t rows,
                                              int32_t n_warp, int lane) {
@@ -809,7 +812,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
 
   ptx::tc_fence_before();
   __syncthreads();
-  if constexpr (CLUSTER) {  // no CTA leaves, and no shared memory goes, before rank 0 has read the sums
+  if constexpr (CLUSTER) {  // no CTA leaves, and no shared memory goes, before all have read the sums
     ptx::cluster_arrive_release();
     ptx::cluster_wait_acquire();
   }
@@ -888,28 +891,31 @@ int smallm_quant_rows() { return kQuantRows; }
 // clusters of eight on most of the SMs, 16 x 2112 x 7168 8.4 / 8.8 (16 x 1536 x 7168, 96 CTAs, 7.8 / 7.8).
 bool smallm_quantises(int64_t M, int64_t N, int64_t K, int sm_count) {
   if (M <= 8) return true;
-  const int64_t n_tiles = (N + BN - 1) / BN, c = smallm_cluster(M, N, K, sm_count), ctas = n_tiles * c, kb = K / BK / c;
+  const int64_t n_tiles = (N + BN - 1) / BN, c = smallm_cluster(M, N, K, sm_count, false), ctas = n_tiles * c, kb = K / BK / c;
   if (M > kMaxQuantRows || n_tiles > 2 * sm_count) return false;
   return M <= 12 || ((ctas >= 88 || kb <= 24) && (c < kMaxCluster || ctas <= 96));
 }
 
-// From 65 rows up a k-block takes this kernel 780 cycles and the 128 x 128 kernel 425: where every CTA works alone, that one takes
-// the call (GEMM alone in a replayed graph, this / the tile kernel, us: 113 x 10240 x 8192 27.5/20.3, 65 x 36864 x 7168 48.6/46.6,
-// 128 x 57344 x 8192 108/94, 128 x 24576 x 1536 16.9/12.3, 100 x 5120 x 2560 11.6/9.8).  Where clusters share K most SMs
-// would be idle without them, and a split through memory is no faster (M = 96, weights from HBM: N=4096 K=4096 11.6/12.7, N=7168
-// K=16384 32.7/30.3) and needs scratch.  Where no cluster shares K both add k-blocks in the same order, so that the bits are the
-// few-rows kernel's either way.
-bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count) {
-  return M <= 64 || (M <= smallm_max_rows() && smallm_cluster(M, N, K, sm_count) > 1);
+// From 65 rows up a k-block takes this kernel 390 ns where clusters share K, 360 alone, and the 128 x 128 kernel 250: where every CTA works alone,
+// that one takes the call (GEMM alone in a replayed graph, this / the tile kernel, us: 113 x 10240 x 8192 27.5/20.3, 65 x 36864 x 7168
+// 48.6/46.6, 128 x 57344 x 8192 108/94, 128 x 24576 x 1536 16.9/12.3), and so it does where the cost model has a cluster behind it.  Where
+// no cluster shares K both add k-blocks in the same order, so that the bits are the few-rows kernel's either way.
+bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count, bool ue8m0) {
+  return M <= 64 || (M <= smallm_max_rows() && smallm_cluster(M, N, K, sm_count, ue8m0) > 1);
 }
 
-// CTAs per cluster that share one tile's K (1, 2, 4 or 8) for a dense problem.  Cost model in nanoseconds, from runs with one
-// tile per CTA at 1.9 GHz: a k-block takes one CTA `step` (the MMA issuer at 16 columns, the promotion above), or longer once
-// the CTAs together ask for more than HBM delivers (16 KB of weights each at 6.5 TB/s); adding up over the cluster costs a
-// barrier and one pass over the sums.  Larger clusters leave SMs of a GPC unused.
-int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count) {
+// CTAs per cluster that share one tile's K (1, 2, 4 or 8) for a dense problem.  Cost model in nanoseconds: a k-block takes one CTA
+// `step` (the MMA issuer at 16 columns, the promotion above), or longer once the CTAs together ask for more than HBM delivers (16 KB
+// of weights each at 6.5 TB/s); adding up over the cluster costs a barrier and a round trip or two (add_up_share).  From 65 rows a CTA
+// that works alone is the tile kernel's (takes_few_rows).  Fitted to calls of thirteen layers, K = 512 to 16384, at every cluster
+// size, 2 to 128 rows; the choice is the best one or within 3 % of it, where the constants of rank 0 adding up alone were up to 19 % off: 24 x
+// 3072 x 1536 6.6 -> 6.0 us, 32 x 7168 x 2048 7.85 -> 7.3, 16 x 6144 x 1536 6.3 -> 5.8, 128 x 6144 x 1536 10.2 -> 8.5, 128 x 7168 x 2048 11.3 ->
+// 9.8, 128 x 9216 x 4096 16.2 -> 14.1, 128 x 1000 x 1024 (UE8M0) 9.4 -> 7.7.  Larger clusters leave SMs of a GPC unused.
+int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count, bool ue8m0) {
   const int64_t n_tiles = (N + BN - 1) / BN, k_tiles = (K + BK - 1) / BK;
-  const int64_t step = M <= 16 ? 195 : (M <= 32 ? 215 : (M <= 64 ? 240 : 360));
+  const int64_t step = M <= 16 ? 195 : (M <= 32 ? 215 : (M <= 64 ? 240 : 390));
+  const int64_t base = M <= 16 ? 800 : (M <= 64 ? 1000 : 2400);
+  const int64_t rank = M <= 16 ? 60 : (M <= 32 ? 100 : (M <= 64 ? 130 : 150));
   int best = 1;
   int64_t best_cost = INT64_MAX;
   for (int c = 1; c <= kMaxCluster; c *= 2) {
@@ -921,7 +927,8 @@ int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count) {
     if (c > 1 && ctas > fit) break;
     const int64_t waves = (ctas + fit - 1) / fit, hbm = (ctas < fit ? ctas : fit) * 16384 * 10 / 65000;
     int64_t cost = waves * kb * (step > hbm ? step : hbm);
-    if (c > 1) cost += (M <= 16 ? 900 : 1500) + (int64_t)(c - 1) * (M <= 16 ? 60 : (M <= 64 ? 200 : 500));
+    if (c == 1 && M > 64) cost = waves * (ue8m0 ? kb * 340 + 1700 : kb * 250 + 500);
+    if (c > 1) cost += base + (int64_t)(c - 1) * rank;
     if (cost < best_cost) {
       best_cost = cost;
       best = c;
@@ -995,10 +1002,10 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
   int splits = 1;
   if (partial != nullptr) {
     p.partial = partial;
-    splits = smallm_cluster(M, N, K, sm_count);  // the same ranges, added in the same order: the same bits as `out`
+    splits = smallm_cluster(M, N, K, sm_count, ue8m0);  // the same ranges, added in the same order: the same bits as `out`
     if ((int64_t)splits * M * N > partial_floats) splits = 1;
   } else {
-    splits = p.cluster = smallm_cluster(M, N, K, sm_count);
+    splits = p.cluster = smallm_cluster(M, N, K, sm_count, ue8m0);
   }
   p.kb_per_split = (p.k_tiles + splits - 1) / splits;
   p.k_splits = (p.k_tiles + p.kb_per_split - 1) / p.kb_per_split;

@@ -518,7 +518,7 @@ Plan dense_plan(int64_t M, int64_t N, int64_t K, int sm_count, bool scratch) {
 }  // namespace
 
 int ue8m0_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
-  return takes_few_rows(M, N, K, sm_count) ? 1 : dense_plan(M, N, K, sm_count, true).splits;
+  return takes_few_rows(M, N, K, sm_count, true) ? 1 : dense_plan(M, N, K, sm_count, true).splits;
 }
 
 namespace {
@@ -558,7 +558,7 @@ int ue8m0_common(const void* a, const void* b, const int32_t* sfa, const int32_t
   SGLB_REQUIRE(di.cc_major == 10, SGLB200_ERR_ARCH, "compute capability %d.%d: this library is built for sm_100a only",
                di.cc_major, di.cc_minor);
 
-  if (!grouped && takes_few_rows(M, N, K, di.sm_count)) {
+  if (!grouped && takes_few_rows(M, N, K, di.sm_count, true)) {
     // few rows: the weight-streaming kernel with swapped operands decodes the exponent bytes itself (gemm_smallm.cu);
     // from 65 rows up the block-scaled tile kernel below, which has no promotion, is level or faster (N=24576 K=1536 M=100 15.9
     // against 17.9 us), except where it would leave most SMs idle and the other shares K inside clusters (N=2112 K=7168 M=100

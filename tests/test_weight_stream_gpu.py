@@ -162,6 +162,43 @@ def test_up_to_sixteen_rows_quantised_by_the_gemm(N, K, dtype, M, ue8m0):
             assert torch.equal(both.view(-1)[:M * N].view(M, N).view(torch.int16), want.view(torch.int16))
 
 
+@pytest.mark.parametrize("ue8m0", [False, True])
+@pytest.mark.parametrize("M", [1, 7, 9, 16, 17, 31, 33, 64, 65, 100, 121, 128])
+@pytest.mark.parametrize("N,K,dtype", [(1000, 7168, torch.bfloat16), (4072, 4096, torch.float16), (7112, 7168, torch.bfloat16)])
+def test_shares_of_a_tile_in_clusters(N, K, dtype, M, ue8m0):
+    """Clusters of eight, four and two add up a tile's sums, a share each: rows that give every CTA a full share, an uneven one or
+    none, a ragged last tile, a bias, and nothing written past the last row."""
+    from sglang_b200._lib import check, lib
+    w, w_s = make_weight(N, K, seed=N) if not ue8m0 else oracle.block_quant_weight(
+        torch.randn(N, K, generator=torch.Generator().manual_seed(N)) * 0.02, scale_ue8m0=True)
+    x = make_activations(M, K, seed=M).to(dtype)
+    a, a_s = oracle.per_token_group_quant_fp8(x, 128, scale_ue8m0=ue8m0)
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(3)).to(dtype).cuda()
+    ref = oracle.w8a8_block_fp8_matmul(a, w, a_s, w_s, output_dtype=dtype)
+    L, kind = lib(), 0 if dtype == torch.bfloat16 else 1
+    xd, wd = x.cuda(), w.cuda()
+    if ue8m0:
+        from sglang_b200.layers.quantization.fp8_kernel import pack_ue8m0_scales
+        ws = pack_ue8m0_scales(w_s.cuda())
+    else:
+        ws = w_s.cuda()
+    bytes_ = L.sglb200_fp8_block_linear_scratch_bytes(M, N, K, int(ue8m0))
+    scratch = torch.empty(max(bytes_, 1), dtype=torch.uint8, device="cuda")
+    outs = []
+    for b in (None, bias):
+        out = torch.full((M + 1, N), 7.0, dtype=dtype, device="cuda")
+        check(L.sglb200_fp8_block_linear(xd.data_ptr(), wd.data_ptr(), ws.data_ptr(), None if b is None else b.data_ptr(), out.data_ptr(),
+                                         M, N, K, ws.stride(0), ws.stride(1), int(ue8m0), 1e-10, kind, scratch.data_ptr(), bytes_,
+                                         torch.cuda.current_stream().cuda_stream), "fp8_block_linear")
+        assert last_gemm() == "fp8_block_gemm_smallm_kernel"
+        outs.append(out)
+    torch.cuda.synchronize()
+    assert L.sglb200_read_device_status() == 0
+    assert (outs[0][M] == 7.0).all() and (outs[1][M] == 7.0).all(), "a row past the last one was written"
+    assert torch.equal(outs[1][:M], outs[0][:M] + bias)
+    assert_gemm_close(outs[0][:M], ref, f"{M}x{N}x{K}", allow_one_ulp=True)
+
+
 @pytest.mark.parametrize("M", [1, 16, 128])
 def test_weights_written_by_the_kernel_before(M):
     """The quantiser writes the codes that the next call takes as weights, into the same memory every time: the
