@@ -40,6 +40,7 @@ int make_map_out16(CUtensorMap* map, void* base, uint64_t cols, uint64_t rows, u
 int smallm_max_rows();
 constexpr int kMaxCluster = 8;
 int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count, bool ue8m0);  // CTAs that share a tile's K, 1..kMaxCluster
+int64_t tile_cost(int64_t M, int64_t N, int64_t K, int sm_count);  // what the tile kernel is expected to take, ns, K cut or not
 bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count, bool ue8m0);  // a dense call of either scale kind runs on it
 int smallm_splits(int64_t N, int64_t K, int sm_count);  // K ranges of a split through memory: sizes scratch, see there
 // Rows that are not quantised yet: `a` of smallm_gemm is [M, K] of the output type, contiguous, K in whole groups of 128, and the

@@ -1177,7 +1177,7 @@ namespace {
 // at 1.9 GHz: a k-block takes a CTA 230 and a work item 500 more; splitting costs the reduce kernel (3500) and the partial sums'
 // way to memory and back (8 bytes each at about 5 TB/s).  The rule before aimed at two items per SM whatever the sums cost, and
 // often hit three waves: N=4096 K=4096 M=256 27.9 us (now 17), N=1536 K=7168 M=512 30.0 (22), N=3072 K=1536 M=256 13.4 (10).
-int splitk_choice(int64_t M, int64_t N, int64_t K, int sm_count) {
+int splitk_choice(int64_t M, int64_t N, int64_t K, int sm_count, int64_t* ns = nullptr) {
   const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int64_t k_tiles = (K + BK - 1) / BK;
   int best = 1;
@@ -1192,13 +1192,23 @@ int splitk_choice(int64_t M, int64_t N, int64_t K, int sm_count) {
       best = (int)c;
     }
   }
+  if (ns) *ns = best_cost;
   return best;
 }
 
-// K ranges whose sums a dense call puts into its scratch; up to smallm_max_rows() K is added up on the chip
+// K ranges whose sums a dense call puts into its scratch; up to smallm_max_rows() K is added up on the chip.  Above, a call that
+// takes_few_rows has with clusters leaves the scratch alone; its size stays what callers know.
 int dense_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
   return M > smallm_max_rows() ? splitk_choice(M, N, K, sm_count) : 1;
 }
+
+}  // namespace
+int64_t tile_cost(int64_t M, int64_t N, int64_t K, int sm_count) {
+  int64_t ns = 0;
+  splitk_choice(M, N, K, sm_count, &ns);
+  return ns;
+}
+namespace {
 
 // Whether CTA pairs (gemm_pair.cu, 256 x 256 tiles) take a dense call that leaves K whole, or the 128 x 128 tiles here.  Cost model
 // in nanoseconds (runs of one call at a time, 11 layers of N = 576 to 36864, K = 1024 to 16384, 160 to 4096 rows; the choice is
@@ -1274,7 +1284,7 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
   SGLB_REQUIRE(di.cc_major == 10, SGLB200_ERR_ARCH, "compute capability %d.%d: this library is built for sm_100a only",
                di.cc_major, di.cc_minor);
 
-  if (!grouped && push && takes_few_rows(total_rows, N, K, di.sm_count, false) && workspace != nullptr &&
+  if (!grouped && push && total_rows <= smallm_max_rows() && takes_few_rows(total_rows, N, K, di.sm_count, false) && workspace != nullptr &&
       (int64_t)smallm_cluster(total_rows, N, K, di.sm_count, false) * total_rows * N <= workspace_floats) {
     // few rows, exchanged: the weight-streaming kernel leaves fp32 sums, a second kernel casts and pushes them.  K is cut as
     // for the plain entry (smallm_cluster), which makes the bits the same.  Both kernels against the ranges that a split through

@@ -111,6 +111,7 @@ struct SmallParams {
   const void* bias;  // [N] of the output type, or NULL: added to the rounded result
   float* partial;    // fp32 sums [splits][M][N] instead of `out`
   int32_t cluster;   // > 1: the CTAs of a cluster share one tile's K and add their sums up (k_splits == cluster)
+  int32_t chunks, chunk_rows;  // cluster form: M rows in `chunks` of chunk_rows, one work item each
   int32_t M, N, K;
   int32_t n_tiles, k_tiles, k_splits, kb_per_split;
   int64_t ldc;
@@ -146,9 +147,17 @@ template <int TILE, bool GROUPED, bool CLUSTER>
 __device__ __forceinline__ Item get_item(const SmallParams& p, const int32_t* item_start, int32_t t) {
   Item it;
   if constexpr (!GROUPED) {
+    it.row0 = 0;
+    it.rows = p.M;
     if constexpr (CLUSTER) {
       it.nt = t / p.cluster;
       it.split = t - it.nt * p.cluster;
+      if (p.chunks > 1) {  // chunks of one weight tile side by side: it comes from HBM once
+        const int32_t tile = it.nt;
+        it.nt = tile / p.chunks;
+        it.row0 = (tile - it.nt * p.chunks) * p.chunk_rows;
+        it.rows = min(p.chunk_rows, p.M - it.row0);
+      }
     } else {
       it.split = t / p.n_tiles;
       it.nt = t - it.split * p.n_tiles;
@@ -156,8 +165,6 @@ __device__ __forceinline__ Item get_item(const SmallParams& p, const int32_t* it
     it.kb0 = it.split * p.kb_per_split;
     it.kb1 = min(it.kb0 + p.kb_per_split, p.k_tiles);
     it.e = 0;
-    it.row0 = 0;
-    it.rows = p.M;
   } else {
     int32_t lo = 0, hi = p.num_experts;  // last e with item_start[e] <= t
     while (hi - lo > 1) {
@@ -492,7 +499,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       }
     }
   } else {
-    if (threadIdx.x == 0) ctl->total = p.n_tiles * p.k_splits;
+    if (threadIdx.x == 0) ctl->total = p.n_tiles * p.chunks * p.k_splits;
   }
   ptx::tc_fence_before();
   __syncthreads();
@@ -689,7 +696,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
               pre = idx + 1;
             } else if (idx < pre) {
               if constexpr (!QUANT)
-                if (leader) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, 0);
+                if (leader) ptx::tma_load_2d_a(dst + kWBytes, &map_a, full0 + stage * 8, kb * BK, it.row0);
             } else {
               if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) {
                 timeout(ctl, 11);
@@ -882,6 +889,7 @@ int launch_quant(const CUtensorMap& map_w, const SmallParams& p, bool ue8m0, int
 
 // Row limit of this kernel, and of the scratch sizes that callers know (smallm_splits)
 int smallm_max_rows() { return 128; }
+constexpr int kMaxChunkedRows = 256;  // two chunks, fp32 scales: see takes_few_rows
 
 int smallm_quant_rows() { return kQuantRows; }
 
@@ -898,10 +906,14 @@ bool smallm_quantises(int64_t M, int64_t N, int64_t K, int sm_count) {
 
 // From 65 rows up a k-block takes this kernel 390 ns where clusters share K, 360 alone, and the 128 x 128 kernel 250: where every CTA works alone,
 // that one takes the call (GEMM alone in a replayed graph, this / the tile kernel, us: 113 x 10240 x 8192 27.5/20.3, 65 x 36864 x 7168
-// 48.6/46.6, 128 x 57344 x 8192 108/94, 128 x 24576 x 1536 16.9/12.3), and so it does where the cost model has a cluster behind it.  Where
-// no cluster shares K both add k-blocks in the same order, so that the bits are the few-rows kernel's either way.
+// 48.6/46.6, 128 x 57344 x 8192 108/94, 128 x 24576 x 1536 16.9/12.3), and so it does where the cost model has a cluster behind it.  Up to 128
+// rows, where no cluster shares K, both add k-blocks in the same order, so that the bits are the few-rows kernel's either way.
+// From 129 to 256 rows (fp32 scales) clusters work on two even chunks, as long as all of them fit the chip at once, where the tile kernel, which
+// would cut K through memory and add the sums up in a kernel of its own, is expected to be slower.  Calls, tile kernel / this, us, 129 / 192 / 256 rows:
+// 576 x 7168 14.0 / 14.0 / 14.2 -> 10.2 / 11.0 / 12.3, 1536 x 7168 16.1 / 16.1 / 16.4 -> 16.1 (not taken) / 14.4 / 14.9; three and more chunks
+// are level.  UE8M0 calls there keep the block-scaled kernels, whose sums the entry with a workspace shares.
 bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count, bool ue8m0) {
-  return M <= 64 || (M <= smallm_max_rows() && smallm_cluster(M, N, K, sm_count, ue8m0) > 1);
+  return M <= 64 || smallm_cluster(M, N, K, sm_count, ue8m0) > 1;
 }
 
 // CTAs per cluster that share one tile's K (1, 2, 4 or 8) for a dense problem.  Cost model in nanoseconds: a k-block takes one CTA
@@ -912,7 +924,9 @@ bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count, bool ue8m0) {
 // 3072 x 1536 6.6 -> 6.0 us, 32 x 7168 x 2048 7.85 -> 7.3, 16 x 6144 x 1536 6.3 -> 5.8, 128 x 6144 x 1536 10.2 -> 8.5, 128 x 7168 x 2048 11.3 ->
 // 9.8, 128 x 9216 x 4096 16.2 -> 14.1, 128 x 1000 x 1024 (UE8M0) 9.4 -> 7.7.  Larger clusters leave SMs of a GPC unused.
 int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count, bool ue8m0) {
-  const int64_t n_tiles = (N + BN - 1) / BN, k_tiles = (K + BK - 1) / BK;
+  const int64_t k_tiles = (K + BK - 1) / BK, chunks = M <= smallm_max_rows() ? 1 : (M + 127) / 128;
+  const int64_t n_tiles = (N + BN - 1) / BN * chunks;
+  if (M > kMaxChunkedRows || (ue8m0 && chunks > 1) || (M > 64 && n_tiles > sm_count)) return 1;
   const int64_t step = M <= 16 ? 195 : (M <= 32 ? 215 : (M <= 64 ? 240 : 390));
   const int64_t base = M <= 16 ? 800 : (M <= 64 ? 1000 : 2400);
   const int64_t rank = M <= 16 ? 60 : (M <= 32 ? 100 : (M <= 64 ? 130 : 150));
@@ -928,6 +942,7 @@ int smallm_cluster(int64_t M, int64_t N, int64_t K, int sm_count, bool ue8m0) {
     const int64_t waves = (ctas + fit - 1) / fit, hbm = (ctas < fit ? ctas : fit) * 16384 * 10 / 65000;
     int64_t cost = waves * kb * (step > hbm ? step : hbm);
     if (c == 1 && M > 64) cost = waves * (ue8m0 ? kb * 340 + 1700 : kb * 250 + 500);
+    if (c == 1 && chunks > 1) cost = tile_cost(M, N, K, sm_count);
     if (c > 1) cost += base + (int64_t)(c - 1) * rank;
     if (cost < best_cost) {
       best_cost = cost;
@@ -1011,7 +1026,10 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
   p.k_splits = (p.k_tiles + p.kb_per_split - 1) / p.kb_per_split;
   if (splits_used) *splits_used = p.k_splits;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t items = (int64_t)p.n_tiles * p.k_splits;
+  p.chunks = M <= 128 ? 1 : (int32_t)((M + 127) / 128);
+  p.chunk_rows = (int32_t)((M + p.chunks - 1) / p.chunks);
+  p.chunks = (int32_t)((M + p.chunk_rows - 1) / p.chunk_rows);
+  const int64_t items = (int64_t)p.n_tiles * p.chunks * p.k_splits;
   if (raw != nullptr) {
     p.x = a;
     p.eps = raw->eps;
@@ -1019,6 +1037,7 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
   }
   if (p.cluster > 1)
     return ue8m0 ? launch_cluster<true>(MT, two, map_w, map_a, p, st, items) : launch_cluster<false>(MT, two, map_w, map_a, p, st, items);
+  if (M > smallm_max_rows()) return fail(SGLB200_ERR_SHAPE, "%lld rows: at most %d unless K is shared", (long long)M, smallm_max_rows());
   if (two) {
     if (ue8m0) return fail(SGLB200_ERR_SHAPE, "UE8M0 scales: at most 64 rows unless K is shared, not %lld", (long long)M);
     return launch<32, false, false, 4>(map_w, map_a, p, sm_count, st, items);

@@ -199,6 +199,35 @@ def test_shares_of_a_tile_in_clusters(N, K, dtype, M, ue8m0):
     assert_gemm_close(outs[0][:M], ref, f"{M}x{N}x{K}", allow_one_ulp=True)
 
 
+@pytest.mark.parametrize("M,N,K,kernel", [(129, 576, 7168, "fp8_block_gemm_smallm_kernel"), (177, 1000, 4096, "fp8_block_gemm_smallm_kernel"),
+                                          (255, 520, 7168, "fp8_block_gemm_smallm_kernel"), (256, 576, 7168, "fp8_block_gemm_smallm_kernel"),
+                                          (257, 576, 7168, "fp8_block_gemm_kernel"), (200, 4096, 4096, "fp8_block_gemm_kernel")])
+def test_two_chunks_of_rows_in_clusters(M, N, K, kernel):
+    """129 to 256 rows where clusters share K: two chunks of rows, even and uneven, and the sizes beyond, which keep the 128 x 128
+    tiles with K cut through scratch.  A bias, nothing written past the last row, the same result twice."""
+    from sglang_b200._lib import check, lib
+    w, w_s = make_weight(N, K, seed=N)
+    x = make_activations(M, K, seed=M)
+    a, a_s = oracle.per_token_group_quant_fp8(x, 128)
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(3)).bfloat16().cuda()
+    L, xd, wd, ws = lib(), x.cuda(), w.cuda(), w_s.cuda()
+    bytes_ = L.sglb200_fp8_block_linear_scratch_bytes(M, N, K, 0)
+    scratch = torch.empty(bytes_, dtype=torch.uint8, device="cuda")
+    outs = []
+    for b in (None, bias, None):
+        out = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device="cuda")
+        check(L.sglb200_fp8_block_linear(xd.data_ptr(), wd.data_ptr(), ws.data_ptr(), None if b is None else b.data_ptr(), out.data_ptr(),
+                                         M, N, K, ws.stride(0), ws.stride(1), 0, 1e-10, 0, scratch.data_ptr(), bytes_,
+                                         torch.cuda.current_stream().cuda_stream), "fp8_block_linear")
+        assert last_gemm() == kernel
+        outs.append(out)
+    torch.cuda.synchronize()
+    assert L.sglb200_read_device_status() == 0
+    assert all((out[M] == 7.0).all() for out in outs), "a row past the last one was written"
+    assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1][:M], outs[0][:M] + bias)
+    assert_gemm_close(outs[0][:M], oracle.w8a8_block_fp8_matmul(a, w, a_s, w_s), f"{M}x{N}x{K}")
+
+
 @pytest.mark.parametrize("M", [1, 16, 128])
 def test_weights_written_by_the_kernel_before(M):
     """The quantiser writes the codes that the next call takes as weights, into the same memory every time: the
