@@ -99,9 +99,9 @@ struct Cfg {
   static constexpr uint32_t kSlotBytes = kTile * sizeof(float), kScaleBytes = kScaleSlots * kSlotBytes;
   static constexpr size_t kPatchOffset = (size_t)kStages * kStageBytes + kScaleBytes;
   static constexpr size_t kSmem = 1024 + kPatchOffset + 4 * NSUB * kPatchBytes + kCtlBytes;
-  // grouped: the table of first work items per expert follows the control block
-  static constexpr size_t kSmemGrouped = kSmem + (kMaxExperts + 1) * sizeof(int32_t) + 12;
-  static_assert(kSmemGrouped <= 227 * 1024, "shared memory of one CTA");
+  // grouped: the tables of rows and of first work items per expert follow the control block
+  static constexpr size_t kSmemGrouped = kSmem + kMaxExperts * sizeof(int2) + (kMaxExperts + 1) * sizeof(int32_t) + 12;
+  static_assert((kTile > 64 ? kSmem : kSmemGrouped) <= 227 * 1024, "shared memory of one CTA");  // grouped: chunks of up to 64 rows
 };
 
 struct SmallParams {
@@ -143,8 +143,10 @@ __device__ __forceinline__ void expert_rows(const SmallParams& p, int32_t e, int
   }
 }
 
+// Work item t.  Grouped: `e` is the expert of an earlier item of this warp (0 at first), from which its 32 lanes look for that of t side
+// by side; the rows come from shared memory.
 template <int TILE, bool GROUPED, bool CLUSTER>
-__device__ __forceinline__ Item get_item(const SmallParams& p, const int32_t* item_start, int32_t t) {
+__device__ __forceinline__ Item get_item(const SmallParams& p, const int2* expert, const int32_t* item_start, int32_t t, int32_t& e) {
   Item it;
   if constexpr (!GROUPED) {
     it.row0 = 0;
@@ -166,16 +168,17 @@ __device__ __forceinline__ Item get_item(const SmallParams& p, const int32_t* it
     it.kb1 = min(it.kb0 + p.kb_per_split, p.k_tiles);
     it.e = 0;
   } else {
-    int32_t lo = 0, hi = p.num_experts;  // last e with item_start[e] <= t
-    while (hi - lo > 1) {
-      const int32_t mid = (lo + hi) >> 1;
-      if (item_start[mid] <= t) lo = mid; else hi = mid;
+    const int32_t lane = threadIdx.x & 31;
+    for (;;) {  // last e with item_start[e] <= t
+      const int32_t n = e + 1 + lane;
+      const int32_t k = __popc(__ballot_sync(0xffffffffu, n < p.num_experts && item_start[n] <= t));
+      e += k;
+      if (k < 32) break;
     }
-    int32_t r0, cnt;
-    expert_rows(p, lo, &r0, &cnt);
+    const int32_t r0 = expert[e].x, cnt = expert[e].y;
     const int32_t chunks = (cnt + TILE - 1) / TILE;
-    const int32_t local = t - item_start[lo];
-    it.e = lo;
+    const int32_t local = t - item_start[e];
+    it.e = e;
     it.nt = local / chunks;
     const int32_t ch = local - it.nt * chunks;
     const int32_t per = (cnt + chunks - 1) / chunks;  // chunks of even size: the MMA is as wide as the chunk
@@ -311,7 +314,8 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
   uint32_t stage = me, phase = 0, slot = me;
   int32_t i = (int32_t)me;  // this warp's next k-block, counted from the item's first
   for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
-    const Item it = get_item<C::kTile, false, CLUSTER>(p, nullptr, t);
+    int32_t none = 0;
+    const Item it = get_item<C::kTile, false, CLUSTER>(p, nullptr, nullptr, t, none);
     const float* sb_blk = p.sb + (int64_t)it.nt * p.sb_stride_n;
     uint4 v[PASSES][2];
     float b = 0.f;
@@ -452,7 +456,8 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   float* scale_ring = reinterpret_cast<float*>(smem + (size_t)C::kStages * C::kStageBytes);  // [slot][token]
   Ctl* ctl = reinterpret_cast<Ctl*>(smem + C::kPatchOffset + 4 * NSUB * kPatchBytes);
-  int32_t* item_start = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(ctl) + kCtlBytes);
+  int2* expert = reinterpret_cast<int2*>(reinterpret_cast<uint8_t*>(ctl) + kCtlBytes);  // grouped: first row and rows
+  int32_t* item_start = reinterpret_cast<int32_t*>(expert + kMaxExperts);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -482,6 +487,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         if (e < p.num_experts) {
           int32_t r0, cnt;
           expert_rows(p, e, &r0, &cnt);
+          expert[e] = make_int2(r0, cnt);
           v = ((cnt + C::kTile - 1) / C::kTile) * p.n_tiles;
         }
         int32_t incl = v;
@@ -535,9 +541,10 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
     bool ready = false;  // the next k-block's sums are known to be there
     for (uint32_t i = 0; i < C::kAcc; ++i) ptx::mbar_arrive_if(full0 + i * 8, leader);  // every TMEM stage is free
     [[maybe_unused]] bool met = false;  // this warp has passed the cluster's first barrier
+    int32_t e_last = 0;
     float2 acc[2][G][2];  // [lanes 0-15 / 16-31][token group][rows tr / tr + 8]: two neighbouring tokens
     for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
-      const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
+      const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, expert, item_start, t, e_last);
       const int32_t kb0 = it.kb0, kb1 = it.kb1;
       const int32_t row0 = it.row0 + sub * MT, rows = max(0, min(MT, it.rows - sub * MT));
 #pragma unroll
@@ -679,9 +686,10 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       uint32_t armed = 0, armed_phase = 0;  // bit i: stage i was armed / the phase bit of its last arming
       for (int pass = GROUPED ? 1 : 0; pass < 2; ++pass) {
         uint32_t stage = 0, phase = 0, idx = 0;
+        int32_t e_last = 0;
         bool ok = true;
         for (int32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
-          const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
+          const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, expert, item_start, t, e_last);
           const int32_t nt = it.nt;
           for (int32_t kb = it.kb0; kb < it.kb1; ++kb, ++idx) {
             const uint32_t dst = stage0 + stage * C::kStageBytes;
@@ -735,8 +743,9 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       // as wide as the item's rows (in steps of 16), so a ragged chunk costs neither time nor power for its padding
       const uint64_t desc0 = ptx::make_kmajor_sw128_desc(stage0);
       uint32_t stage = 0, phase = 0, acc = 0;
+      int32_t e_last = 0;
       for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
-        const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
+        const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, expert, item_start, t, e_last);
         const int32_t kb0 = it.kb0, kb1 = it.kb1;
         const uint32_t idesc = ptx::make_idesc_e4m3_f32(BN, (uint32_t)(it.rows + 15) / 16 * 16);
         bool ok = true;
@@ -757,58 +766,87 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       const uint32_t me = warp < 4 ? warp - 2 : warp - 6;
       if (p.out_dtype == SGLB200_BF16) quantise_rows<__nv_bfloat16, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
       else quantise_rows<__half, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
-    } else if (warp == 2) {
+    } else if (warp == 2 || (GROUPED && p.k_tiles < C::kStages)) {
       // ===== scale loader: per group of four k-blocks the products sa[token, kb] * sb[nt, kb], 0 for tokens past the item's
-      // rows (the accumulator columns there hold leftovers and are not stored).  The loads of the next group are in flight
-      // while this group waits for its place in the ring.
+      // rows (the accumulator columns there hold leftovers and are not stored).  The loads of the next group, the next item's
+      // too, are in flight while this group waits for its place in the ring.  Grouped items of fewer k-blocks than the ring has
+      // stages (quantise_rows says why not more) come to warps 2 and 3 in turn: a short item is mostly these loads' way to
+      // memory and back.  One loader, which looked for its item and its rows in global memory before each fetch -> this, expert layer
+      // of 256 x (7168, 256), eight a token, at 4 / 16 / 64 / 128 / 512 tokens: 67 / 146 / 272 / 306 / 347 us -> 62 / 123 / 224 / 252 / 292
       if constexpr (!GROUPED) ptx::grid_dep_wait();  // the activation scales come from the kernel before this one
       constexpr int kPerLane = C::kTile / 32 > 0 ? C::kTile / 32 : 1;
+      const uint32_t loaders = GROUPED && p.k_tiles < C::kStages ? 2 : 1, skip = loaders == 2 ? p.k_tiles : 0;
       uint32_t stage = 0, phase = 0, slot = 0;
-      for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
-        const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, item_start, t);
-        const float* sb_blk = p.sb + (int64_t)it.nt * p.sb_stride_n;
-        const float* sa_base = p.sa + (int64_t)it.row0 * p.sa_stride_m;
+      auto pass_over = [&](uint32_t n) {  // n k-blocks, fewer than the ring has stages
+        stage += n;
+        if (stage >= (uint32_t)C::kStages) { stage -= C::kStages; phase ^= 1; }
+        slot += n;
+        if (slot >= (uint32_t)C::kScaleSlots) slot -= C::kScaleSlots;
+      };
+      if (warp == 3) pass_over(skip);
+      int32_t e_last = 0, t = blockIdx.x + (warp - 2) * gridDim.x;
+      const int32_t step = loaders * gridDim.x;
+      float a[kPerLane][kScaleGroup], b[kScaleGroup];
+      const float *sb_blk = nullptr, *sa_base = nullptr;
+      int32_t rows = 0, kb = 0, kb1 = 0;  // of the group to be fetched
+      auto next_item = [&] {
+        const Item it = get_item<C::kTile, GROUPED, CLUSTER>(p, expert, item_start, t, e_last);
+        sb_blk = p.sb + (int64_t)it.nt * p.sb_stride_n;
+        sa_base = p.sa + (int64_t)it.row0 * p.sa_stride_m;
         if constexpr (GROUPED) {
           sb_blk += (int64_t)it.e * p.sb_stride_e;
           if (p.rows_per_expert > 0)
             sa_base = p.sa + (int64_t)it.e * p.sa_stride_e + (int64_t)(it.row0 - it.e * p.rows_per_expert) * p.sa_stride_m;
         }
-        float a[kPerLane][kScaleGroup], b[kScaleGroup];
-        auto fetch = [&](int32_t first) {
+        rows = it.rows;
+        kb = it.kb0;
+        kb1 = it.kb1;
+      };
+      auto fetch = [&] {
 #pragma unroll
-          for (int u = 0; u < kScaleGroup; ++u) {
-            const int32_t kb = min(first + u, it.kb1 - 1);
-            b[u] = load_scale<UE>(sb_blk, kb, p.sb_stride_k);
+        for (int u = 0; u < kScaleGroup; ++u) {
+          const int32_t k = min(kb + u, kb1 - 1);
+          b[u] = load_scale<UE>(sb_blk, k, p.sb_stride_k);
 #pragma unroll
-            for (int h = 0; h < kPerLane; ++h) {
-              const int32_t tok = lane + 32 * h;
-              a[h][u] = tok < it.rows ? load_scale<UE>(sa_base + (int64_t)tok * p.sa_stride_m, kb, p.sa_stride_k) : 0.f;
-            }
-          }
-        };
-        fetch(it.kb0);
-        bool ok = true;
-        for (int32_t kb0 = it.kb0; kb0 < it.kb1 && ok; kb0 += kScaleGroup) {
-          float v[kPerLane][kScaleGroup];
-#pragma unroll
-          for (int h = 0; h < kPerLane; ++h)
-#pragma unroll
-            for (int u = 0; u < kScaleGroup; ++u) v[h][u] = a[h][u] * b[u];
-          if (kb0 + kScaleGroup < it.kb1) fetch(kb0 + kScaleGroup);
-#pragma unroll
-          for (int u = 0; u < kScaleGroup; ++u) {
-            if (kb0 + u >= it.kb1) break;
-            if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 16); ok = false; break; }
-#pragma unroll
-            for (int h = 0; h < kPerLane; ++h)
-              if (C::kTile >= 32 || lane < C::kTile) scale_ring[slot * C::kTile + lane + 32 * h] = v[h][u];
-            __syncwarp();
-            ptx::mbar_arrive_if(full0 + stage * 8, leader);
-            if (++stage == C::kStages) { stage = 0; phase ^= 1; }
-            if (++slot == C::kScaleSlots) slot = 0;
+          for (int h = 0; h < kPerLane; ++h) {
+            const int32_t tok = lane + 32 * h;
+            a[h][u] = tok < rows ? load_scale<UE>(sa_base + (int64_t)tok * p.sa_stride_m, k, p.sa_stride_k) : 0.f;
           }
         }
-        if (!ok || ctl->abort_flag) break;
+      };
+      bool ok = true;
+      if (t < total) {
+        next_item();
+        fetch();
+      }
+      while (t < total && ok) {
+        float v[kPerLane][kScaleGroup];
+#pragma unroll
+        for (int h = 0; h < kPerLane; ++h)
+#pragma unroll
+          for (int u = 0; u < kScaleGroup; ++u) v[h][u] = a[h][u] * b[u];
+        const int32_t n = min(kScaleGroup, kb1 - kb);
+        kb += kScaleGroup;
+        const bool last = kb >= kb1;
+        if (last) {
+          t += step;
+          if (t < total) next_item();
+        }
+        if (t < total) fetch();
+#pragma unroll
+        for (int u = 0; u < kScaleGroup; ++u) {
+          if (u >= n) break;
+          if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 16); ok = false; break; }
+#pragma unroll
+          for (int h = 0; h < kPerLane; ++h)
+            if (C::kTile >= 32 || lane < C::kTile) scale_ring[slot * C::kTile + lane + 32 * h] = v[h][u];
+          __syncwarp();
+          ptx::mbar_arrive_if(full0 + stage * 8, leader);
+          if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+          if (++slot == C::kScaleSlots) slot = 0;
+        }
+        if (last) pass_over(skip);
+        if (ctl->abort_flag) break;
       }
     }
     if constexpr (CLUSTER) {  // the barrier at which the promotion warps meet those of the other CTAs counts every thread

@@ -230,3 +230,61 @@ def test_ue8m0_tile_kernel_at_the_ends_of_experts():
     ref = torch.cat([oracle.w8a8_block_fp8_matmul(aq[offs[e]:offs[e + 1]], wq[e], a_s[offs[e]:offs[e + 1]], wsc[e])
                      for e in range(E) if ROW_ENDS[e]])
     assert_gemm_close(out[:rows], ref, "ends of experts, UE8M0", allow_one_ulp=True)
+
+
+@pytest.mark.parametrize("ue8m0", [False, True])
+@pytest.mark.parametrize("rows", [5, 20, 60])
+@pytest.mark.parametrize("K", [128, 256, 896, 1024, 1280, 1408])
+def test_few_rows_many_short_items(K, rows, ue8m0):
+    """Several items on every CTA, K from one k-block to past the ring: below its length two warps load the scales in turn, from there
+    one.  Experts without rows in between (runs of more than a warp's 32 too) and the masked layout; the bits of the tile kernel."""
+    from sglang_b200.layers.deep_gemm_wrapper import grouped_gemm_nt_f8f8bf16_masked
+    from sglang_b200.layers.moe import _grouped_mm
+    from sglang_b200._lib import lib
+    E, N = 120, 1160
+    g = torch.Generator(device="cuda").manual_seed(K + rows)
+    counts = torch.randint(0, 2 * rows + 1, (E,), generator=g, device="cuda").clamp(max=64)
+    counts[3:40] = 0
+    counts[E - 1] = 0
+    w = (torch.randn(E, N, K, generator=g, device="cuda") * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    ws = torch.rand(E, -(-N // 128), K // 128, generator=g, device="cuda") + 0.5
+    total = int(counts.sum())
+    a = (torch.randn(total, K, generator=g, device="cuda") * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    a_s = torch.rand(total, K // 128, generator=g, device="cuda") + 0.5
+    offs = torch.cat([torch.zeros(1, dtype=torch.long, device="cuda"), counts.cumsum(0)]).int()
+    if ue8m0:  # the masked layout has fp32 scales only: powers of two in both forms of the sorted one
+        from sglang_b200.layers.quantization import pack_ue8m0_scales
+        a_s, ws = torch.exp2(torch.floor(torch.log2(a_s))), torch.exp2(torch.floor(torch.log2(ws)))
+        pa, pw = pack_ue8m0_scales(a_s), pack_ue8m0_scales(ws.view(-1, K // 128)).view(E, -(-N // 128), -1)
+        outs = []
+        for limit in (64, 0):
+            out = torch.full((total + 1, N), 7.0, dtype=torch.bfloat16, device="cuda")
+            with few_rows_limit(limit):
+                from sglang_b200._lib import check
+                check(lib().sglb200_fp8_ue8m0_scaled_grouped_mm(
+                    a.data_ptr(), w.data_ptr(), pa.data_ptr(), pw.data_ptr(), out.data_ptr(), offs.data_ptr(), total, E, N, K, K, K, N * K, N,
+                    pa.stride(0), pa.stride(1), pw.stride(0), pw.stride(1), pw.stride(2), 0, torch.cuda.current_stream().cuda_stream), "mm")
+            outs.append(out)
+        torch.cuda.synchronize()
+        assert lib().sglb200_read_device_status() == 0 and (outs[0][total] == 7.0).all()
+        err = (outs[0][:total].float() - outs[1][:total].float()).norm() / outs[1][:total].float().norm()
+        assert err < 2e-3, "another order of the same fp32 sums: a bf16 rounding apart at most"
+        return
+    outs, masked = [], []
+    for limit in (64, 0):
+        out = torch.full((total + 1, N), 7.0, dtype=torch.bfloat16, device="cuda")
+        rows_out = torch.full((E, 64, N), 7.0, dtype=torch.bfloat16, device="cuda")
+        am, sm = torch.zeros(E, 64, K, device="cuda").to(a.dtype), torch.ones(E, 64, K // 128, device="cuda")
+        for e in range(E):
+            n, o = int(counts[e]), int(offs[e])
+            am[e, :n], sm[e, :n] = a[o:o + n], a_s[o:o + n]
+        with few_rows_limit(limit):
+            _grouped_mm(a, a_s, w, ws, out[:total], offs)
+            grouped_gemm_nt_f8f8bf16_masked((am, sm), (w, ws), rows_out, counts.int(), rows)
+        outs.append(out)
+        masked.append(rows_out)
+    torch.cuda.synchronize()
+    assert lib().sglb200_read_device_status() == 0
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
+    assert torch.equal(masked[0].view(torch.int16), masked[1].view(torch.int16))
+    assert (outs[0][total] == 7.0).all()
