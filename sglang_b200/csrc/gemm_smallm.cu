@@ -8,7 +8,7 @@
 // N / 128 tiles alone cannot occupy the SMs, the CTAs of a cluster cut a tile's K among themselves and add their sums up
 // out of each other's shared memory, each a share of the tile (smallm_cluster, add_up_share), measured with all of it on rank 0: against fp32 partial sums in memory and a kernel that adds them, quantiser
 // included, N=576 K=7168 M=1 / 48: 9.6 / 14.1 -> 6.8 / 11.1 us, N=7168 K=16384 M=48 32.3 -> 27.1, N=10240 K=8192 M=48 27.0 -> 22.1.
-// From 65 to 128 rows eight or sixteen promotion warps share every accumulator stage, from 33 rows eight where clusters share K.
+// From 65 to 128 rows sixteen promotion warps share every accumulator stage, eight where clusters share K, there from 33 rows on.
 //
 // One barrier each way per k-block.  `full` counts the producer's bytes, the scale loader and the promotion warps, who arrive for the
 // k-block that gets the TMEM stage they have just read; `done` is one commit, on which the producer, the scale loader and the
@@ -83,8 +83,8 @@ constexpr int kMaxExperts = 1024;
 // NSUB > 1 (65 to 128 rows per item): the MMA covers up to MT * NSUB = 128 activation rows and every set of four promotion warps
 // takes its MT of every accumulator stage's columns.  Alone on a tile, four sets of 32 columns are the better split: 16 warps hide
 // each other's chain of wait, load, hand-back and FMA (N=10240 K=8192 M=113 31.3 -> 30.1 us, N=24576 K=1536 18.7 -> 17.6, N=36864
-// K=7168 65 -> 59 against two sets of 64).  In a cluster two sets of 64 are: with the code that adds the sums up, 96 registers do
-// not hold four sets' (N=7168 K=16384 M=113 36.7 against 40.1 us).
+// K=7168 65 -> 59 against two sets of 64).  In a cluster two sets of 64 are (call, two sets / four, us: 113 x
+// 7168 x 16384 35.1 / 36.0, 128 x 576 x 7168 10.8 / 11.7, 113 x 2048 x 2048 8.8 / 9.4).
 template <int MT, int NSUB = 1>
 struct Cfg {
   static constexpr int kTile = MT * NSUB;  // most activation rows per work item = TMEM columns per stage
