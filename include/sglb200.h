@@ -161,8 +161,8 @@ int sglb200_group_quant_fp8_batched(const void* input, int in_dtype, void* out_q
  * K need not be a multiple of 128 (the tail block is zero-filled), but K % 16 == 0.
  * fp32 accumulation; each 128-deep partial product is scaled and added in registers.
  * Any M >= 0 is accepted with no padding copy (the reference pads M to a multiple of 4).
- * Up to 64 rows, and up to 128 where the CTAs of a cluster share K, the weight-streaming kernel with swapped operands runs (128
- * weight rows x up to 16 / 32 / 64 / 128 activation rows per MMA), above that the kernel on 128 x 128 tiles, or on CTA pairs (256 x
+ * Up to 64 rows, and up to 256 where the CTAs of a cluster share K, the weight-streaming kernel with swapped operands runs (128
+ * weight rows x up to 16 / 32 / 64 / 128 activation rows per MMA), else the kernel on 128 x 128 tiles, or on CTA pairs (256 x
  * 256) where those are faster and sa is as sglb200_fp8_blockwise_scaled_mm_pair asks.  Up to 128 rows either kernel may be launched
  * beside the end of the kernel before it and then reads the first tiles of `b` at once: b must not be written by a kernel that
  * releases its dependents early (griddepcontrol.launch_dependents).  All other work of the stream is ordered as usual.

@@ -33,8 +33,8 @@
 //
 // The kernel is launched with programmatic stream serialization: it may start while the kernel before it (the
 // activation quantiser, or the previous layer's reduce kernel) is still running.  Its set-up and the WEIGHT tiles of the
-// first ring of stages are issued at once, ahead of griddepcontrol.wait; the activation tiles, all scales and every store
-// come after it.  The kernel starts when all blocks of the one before have ended, or have released it early: no kernel of this
+// first ring of stages are issued at once (up to 128 rows), ahead of griddepcontrol.wait; the activation tiles, all scales and
+// every store come after it.  The kernel starts when all blocks of the one before have ended, or have released it early: no kernel of this
 // library that could have written the weights does that (quant.cu), and callers' own kernels must not.  At decode sizes the fixed cost of a call (launch,
 // set-up, first TMA round trip) is of the order of the streaming time itself, and this hides most of it.
 #include <cuda.h>
@@ -688,7 +688,9 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
     if (warp == 0) {
       // ===== TMA producer.  Pass 0 runs before griddepcontrol.wait: the weight tiles of the first k-blocks (at most one
       // ring of stages, whose barriers are fresh) are requested; pass 1 adds their activation tiles and then continues
-      // with whole stages.
+      // with whole stages.  Above 128 rows (two chunks) nothing is requested early: a caller may have those weights written by a
+      // kernel that releases its dependents before it has ended.
+      const uint32_t early = CLUSTER && p.chunks > 1 ? 0 : C::kStages;
       uint32_t pre = 0;
       uint32_t armed = 0, armed_phase = 0;  // bit i: stage i was armed / the phase bit of its last arming
       for (int pass = GROUPED ? 1 : 0; pass < 2; ++pass) {
@@ -701,7 +703,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
           for (int32_t kb = it.kb0; kb < it.kb1; ++kb, ++idx) {
             const uint32_t dst = stage0 + stage * C::kStageBytes;
             if (pass == 0) {
-              if (idx >= (uint32_t)C::kStages) { ok = false; break; }
+              if (idx >= early) { ok = false; break; }
               if (leader) {
                 ptx::mbar_arrive_expect_tx_a(full0 + stage * 8, QUANT ? kWBytes : C::kStageBytes);
                 ptx::tma_load_3d_a(dst, &map_w, full0 + stage * 8, kb * BK, nt * BN, 0);

@@ -254,6 +254,36 @@ def test_weights_written_by_the_kernel_before(M):
         assert torch.equal(out, want[i % 3]), f"call {i} saw other weights"
 
 
+@pytest.mark.parametrize("M", [129, 200, 256])
+def test_weights_written_by_a_kernel_that_releases_early(M):
+    """Above 128 rows the weights may come from a kernel that releases its dependents before it has ended, as the SiLU quantiser
+    does: the few-rows kernel, which takes these sizes too, must not read them ahead of it."""
+    from sglang_b200._lib import check, lib
+    from sglang_b200.layers.quantization import w8a8_block_fp8_matmul
+    N, K = 576, 7168
+    a, a_s = oracle.per_token_group_quant_fp8(make_activations(M, K, seed=M), 128)
+    a, a_s = a.cuda(), a_s.cuda()
+    y = [torch.randn(N, 2 * K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(i)).bfloat16() for i in range(3)]
+    w, w_s = torch.empty(N, K, dtype=torch.float8_e4m3fn, device="cuda"), torch.empty(N, K // 128, device="cuda")
+    blocks = torch.ones(-(-N // 128), K // 128, device="cuda")
+
+    def product(i, wait):
+        check(lib().sglb200_silu_mul_group_quant_fp8(y[i].data_ptr(), 0, w.data_ptr(), w_s.data_ptr(), None, N, K, 128, 1e-10, -448.0, 448.0,
+                                                     0, K // 128, 1, torch.cuda.current_stream().cuda_stream), "silu_mul_group_quant_fp8")
+        if wait:
+            torch.cuda.synchronize()
+        out = w8a8_block_fp8_matmul(a, w, a_s, blocks, [128, 128], torch.bfloat16)
+        assert last_gemm() == "fp8_block_gemm_smallm_kernel"
+        return out
+
+    want = [product(i, True) for i in range(3)]
+    assert not torch.equal(want[0], want[1])
+    got = [product(i % 3, False) for i in range(9)]
+    torch.cuda.synchronize()
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 3]), f"call {i} saw other weights"
+
+
 @pytest.mark.parametrize("M", [1, 16, 17, 33, 64])
 @pytest.mark.parametrize("k_blocks", [1, 2, 5, 11, 12, 23])
 def test_rings_over_several_tiles(M, k_blocks):
