@@ -201,7 +201,8 @@ int sglb200_fp8_blockwise_scaled_mm_ws(const void* a, const void* b, const float
  *   bias [N] of dtype or NULL: added to the rounded product, one more rounding, as `output += bias` does
  *   out [M, N] of dtype, contiguous;  eps as in sglb200_per_token_group_quant_fp8 (already rounded to dtype)
  *   scratch: sglb200_fp8_block_linear_scratch_bytes(M, N, K, scale_ue8m0) bytes, 256-byte aligned, contents arbitrary.
- *   At 0 bytes (one or two rows, which the GEMM quantises itself) it may be NULL.
+ *   At 0 bytes (one or two rows, which the GEMM quantises itself) it may be NULL.  out may lie on top of x; at one or two rows the
+ *   call then needs the scratch of three (M = 3) and is refused without any.
  * Replaces: w8a8_block_fp8_linear  python/sglang/srt/layers/quantization/fp8_utils.py:184-301.
  */
 int sglb200_fp8_block_linear(const void* x, const void* w, const void* w_scale, const void* bias, void* out, int64_t M,

@@ -1558,10 +1558,17 @@ extern "C" int sglb200_fp8_block_linear(const void* x, const void* w, const void
   if (M == 0 || N == 0) return SGLB200_OK;
   SGLB_REQUIRE(K > 0, SGLB200_ERR_SHAPE, "K must be positive");
   SGLB_REQUIRE(bias == nullptr || sglb::aligned(bias, 16), SGLB200_ERR_ALIGN, "bias must be 16-byte aligned");
+  // Where the GEMM quantises the rows itself it reads x while other CTAs store already.  An output on top of x takes the general way,
+  // which has read all of x before anything is stored; at one or two rows that needs scratch which other calls do without.
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), out0 = reinterpret_cast<uintptr_t>(out);
+  const bool sizes = N < ((int64_t)1 << 31) - 256 && K < ((int64_t)1 << 31) - 256;
+  const bool on_top = M <= 16 && sizes && x && out && out0 < x0 + M * K * 2 && x0 < out0 + M * N * 2;
+  SGLB_REQUIRE(!on_top || M > sglb::smallm_quant_rows() || scratch != nullptr, SGLB200_ERR_WORKSPACE,
+               "out overlaps x: scratch as for three rows needed");
   sglb::DeviceInfo di;
   if (int rc = sglb::device_info(&di)) return rc;
   const bool ue = scale_ue8m0 != 0;
-  if (M <= sglb::smallm_quant_rows()) {  // no quantiser kernel, no scratch
+  if (M <= sglb::smallm_quant_rows() && !on_top) {  // no quantiser kernel, no scratch
     SGLB_REQUIRE(N % 8 == 0, SGLB200_ERR_SHAPE, "N=%lld must be a multiple of 8 (16-byte output rows)", (long long)N);
     SGLB_REQUIRE(N < ((int64_t)1 << 31) - 256 && K < ((int64_t)1 << 31) - 256, SGLB200_ERR_SHAPE, "a dimension exceeds 2^31");
     SGLB_REQUIRE(x && w && w_scale && out, SGLB200_ERR_NULL, "x, w, w_scale and out must not be NULL");
@@ -1578,12 +1585,10 @@ extern "C" int sglb200_fp8_block_linear(const void* x, const void* w, const void
   const sglb::LinearScratch l = sglb::linear_scratch(M, N, K, ue, di.sm_count);
   SGLB_REQUIRE(scratch_bytes >= l.bytes, SGLB200_ERR_WORKSPACE, "scratch_bytes=%lld: %lld needed", (long long)scratch_bytes,
                (long long)l.bytes);
-  // The GEMM quantises the rows itself and leaves the scratch alone.  It reads x while other CTAs store already, so an output on top of
-  // x takes the general way, as does what that way refuses or has another path for.
-  const char *x0 = static_cast<const char*>(x), *out0 = static_cast<const char*>(out);
-  if (M <= 16 && N % 8 == 0 && N < ((int64_t)1 << 31) - 256 && K < ((int64_t)1 << 31) - 256 && x && w && w_scale && out &&
-      sglb::aligned(x, 16) && sglb::aligned(w, 16) && sglb::aligned(out, 16) && sglb::aligned(w_scale, 4) && eps >= 0.f &&
-      di.cc_major == 10 && (out0 + M * N * 2 <= x0 || x0 + M * K * 2 <= out0) && sglb::smallm_quantises(M, N, K, di.sm_count)) {
+  // The GEMM quantises the rows itself and leaves the scratch alone; what the general way refuses goes there.
+  if (M <= 16 && N % 8 == 0 && sizes && !on_top && x && w && w_scale && out && sglb::aligned(x, 16) && sglb::aligned(w, 16) &&
+      sglb::aligned(out, 16) && sglb::aligned(w_scale, 4) && eps >= 0.f && di.cc_major == 10 &&
+      sglb::smallm_quantises(M, N, K, di.sm_count)) {
     const sglb::RawRows raw = {eps};
     return sglb::smallm_gemm(x, w, nullptr, static_cast<const float*>(w_scale), out, M, N, K, K, K, N, 0, 0, w_scale_stride_n,
                              w_scale_stride_k, dtype, bias, nullptr, 0, di.sm_count, stream, nullptr, ue, &raw);

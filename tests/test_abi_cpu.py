@@ -307,6 +307,19 @@ def test_scratch_that_a_dense_call_uses(built_lib, M, N, K, ranges):
         assert used + rest <= L.sglb200_fp8_block_linear_scratch_bytes(M, N, K, 0) <= used + rest + 1024
 
 
+@pytest.mark.parametrize("M", [1, 2])
+def test_one_or_two_rows_under_their_own_output_are_refused_without_scratch(built_lib, M):
+    """At one or two rows the GEMM reads x while it stores: an output that overlaps x is refused before anything else happens, one
+    that only touches it is not (the pointers are never read here)."""
+    from sglang_b200._lib import lib
+    L, N, K, x = lib(), 512, 1024, 1 << 20
+    call = lambda out: L.sglb200_fp8_block_linear(x, 1 << 24, 1 << 25, None, out, M, N, K, 8, 1, 0, 1e-10, 0, None, 0, None)
+    assert [call(out) for out in (x, x + 16, x + M * K * 2 - 16, x - M * N * 2 + 16)] == [-7] * 4
+    assert "overlaps" in L.sglb200_last_error_detail().decode()
+    if not torch.cuda.is_available():
+        assert all(call(out) not in (0, -7) for out in (x + M * K * 2, x - M * N * 2))  # no device here
+
+
 def test_host_path_reports_integers_out_of_range(built_lib):
     """An integer argument that does not fit is an OverflowError, raised before anything is launched, and leaves no pending
     exception behind."""

@@ -154,12 +154,20 @@ def test_up_to_sixteen_rows_quantised_by_the_gemm(N, K, dtype, M, ue8m0):
     torch.cuda.synchronize()
     assert L.sglb200_read_device_status() == 0
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
-    if N <= K:  # an output on top of the input: quantised before anything is stored, as ever
+    if N <= K:  # an output on top of the input: quantised before anything is stored; one or two rows need scratch for it
+        three = L.sglb200_fp8_block_linear_scratch_bytes(max(M, 3), N, K, int(ue8m0))
+        more = torch.empty(three, dtype=torch.uint8, device="cuda")
         both = x.clone()
-        linear(both, both.view(-1)[:M * N].view(M, N))
+        on_top = both.view(-1)[:M * N].view(M, N)
+
+        def in_place(room, size):
+            return L.sglb200_fp8_block_linear(both.data_ptr(), w.data_ptr(), ws.data_ptr(), None, on_top.data_ptr(), M, N, K, ws.stride(0),
+                                              ws.stride(1), int(ue8m0), 1e-10, kind, room, size, stream)
+
+        assert in_place(None, 0) != 0 and torch.equal(both, x)
+        check(in_place(more.data_ptr(), three), "fp8_block_linear")
         torch.cuda.synchronize()
-        if M > 2:
-            assert torch.equal(both.view(-1)[:M * N].view(M, N).view(torch.int16), want.view(torch.int16))
+        assert torch.equal(on_top.view(torch.int16), want.view(torch.int16))
 
 
 @pytest.mark.parametrize("ue8m0", [False, True])
