@@ -44,12 +44,13 @@ int64_t tile_cost(int64_t M, int64_t N, int64_t K, int sm_count);  // what the t
 bool takes_few_rows(int64_t M, int64_t N, int64_t K, int sm_count, bool ue8m0);  // a dense call of either scale kind runs on it
 int smallm_splits(int64_t N, int64_t K, int sm_count);  // K ranges of a split through memory: sizes scratch, see there
 // Rows that are not quantised yet: `a` of smallm_gemm is [M, K] of the output type, contiguous, K in whole groups of 128, and the
-// kernel quantises them itself with this floor; M <= 16, `sa` and `partial` unused
+// kernel quantises them itself with this floor; M <= kMaxQuantRows, `sa` and `partial` unused
 struct RawRows {
   float eps;
 };
 int smallm_quant_rows();
-bool smallm_quantises(int64_t M, int64_t N, int64_t K, int sm_count);
+constexpr int kMaxQuantRows = 8;
+bool smallm_quantises(int64_t M, int64_t N, int sm_count);
 int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t M, int64_t N, int64_t K,
                 int64_t lda, int64_t ldb, int64_t ldc, int64_t sa_stride_m, int64_t sa_stride_k, int64_t sb_stride_n,
                 int64_t sb_stride_k, int out_dtype, const void* bias, float* partial, int64_t partial_floats, int sm_count,

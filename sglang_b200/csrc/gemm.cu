@@ -1562,7 +1562,7 @@ extern "C" int sglb200_fp8_block_linear(const void* x, const void* w, const void
   // which has read all of x before anything is stored; at one or two rows that needs scratch which other calls do without.
   const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), out0 = reinterpret_cast<uintptr_t>(out);
   const bool sizes = N < ((int64_t)1 << 31) - 256 && K < ((int64_t)1 << 31) - 256;
-  const bool on_top = M <= 16 && sizes && x && out && out0 < x0 + M * K * 2 && x0 < out0 + M * N * 2;
+  const bool on_top = M <= sglb::kMaxQuantRows && sizes && x && out && out0 < x0 + M * K * 2 && x0 < out0 + M * N * 2;
   SGLB_REQUIRE(!on_top || M > sglb::smallm_quant_rows() || scratch != nullptr, SGLB200_ERR_WORKSPACE,
                "out overlaps x: scratch as for three rows needed");
   sglb::DeviceInfo di;
@@ -1586,9 +1586,8 @@ extern "C" int sglb200_fp8_block_linear(const void* x, const void* w, const void
   SGLB_REQUIRE(scratch_bytes >= l.bytes, SGLB200_ERR_WORKSPACE, "scratch_bytes=%lld: %lld needed", (long long)scratch_bytes,
                (long long)l.bytes);
   // The GEMM quantises the rows itself and leaves the scratch alone; what the general way refuses goes there.
-  if (M <= 16 && N % 8 == 0 && sizes && !on_top && x && w && w_scale && out && sglb::aligned(x, 16) && sglb::aligned(w, 16) &&
-      sglb::aligned(out, 16) && sglb::aligned(w_scale, 4) && eps >= 0.f && di.cc_major == 10 &&
-      sglb::smallm_quantises(M, N, K, di.sm_count)) {
+  if (sizes && sglb::smallm_quantises(M, N, di.sm_count) && N % 8 == 0 && !on_top && x && w && w_scale && out && sglb::aligned(x, 16) &&
+      sglb::aligned(w, 16) && sglb::aligned(out, 16) && sglb::aligned(w_scale, 4) && eps >= 0.f && di.cc_major == 10) {
     const sglb::RawRows raw = {eps};
     return sglb::smallm_gemm(x, w, nullptr, static_cast<const float*>(w_scale), out, M, N, K, K, K, N, 0, 0, w_scale_stride_n,
                              w_scale_stride_k, dtype, bias, nullptr, 0, di.sm_count, stream, nullptr, ue, &raw);

@@ -28,7 +28,7 @@
 // then re-read, from L2), an expert without rows gets no item, so only the weights of routed experts are streamed.
 //
 // warp 0: TMA producer; warp 1: TMEM owner + MMA issuer; warp 2: scale loader (sa[token] * sb into a slot per k-block), or
-// up to sixteen rows warps 2, 3 and 8..15: quantisers (QUANT); warps 4..7
+// up to eight rows warps 2, 3 and 8..15: quantisers (QUANT); warps 4..7
 // (..11, ..19): promotion (tcgen05.ld, acc += p * scale) and the transposed store.  All waits are bounded.
 //
 // The kernel is launched with programmatic stream serialization: it may start while the kernel before it (the
@@ -281,43 +281,42 @@ __device__ __forceinline__ uint32_t pack16(float a, float b, int out_dtype) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// Ten warps (2, 3 and 8 to 15) of the QUANT form, up to sixteen rows: the activations come as they are, and these warps quantise them
+// Ten warps (2, 3 and 8 to 15) of the QUANT form, up to eight rows: the activations come as they are, and these warps quantise them
 // on their way into the ring, with the arithmetic of the separate quantiser.  Each takes every tenth k-block whole, four rows a pass,
-// with the rows of its next k-block in flight while it converts.  Every CTA does so for all k-blocks it multiplies, which is less
-// work than the weights take to arrive, and saves a kernel and the hand-over from it.  Bound by instructions issued: a k-block of 16
-// rows takes the ten warps about 220 ns (16 KB of weights for each of 112 CTAs: 280 ns of HBM).  Replayed graph of calls over
-// rotating weights, quantiser kernel -> this, N x K at M = 4 / 8 / 16, us: 576 x 7168 6.8 / 6.8 / 7.2 -> 5.5 / 5.9 / 7.1, 24576 x 1536
-// 10.2 / 10.2 / 10.4 -> 8.6 / 9.0 / 9.6, 7168 x 16384 23.2 / 23.8 / 24.3 -> 21.5 / 22.0 / 23.2, 36864 x 7168 42.2 / 42.6 / 43.5 -> 40.0 /
-// 41.1 / 42.5.  Two warps with four k-blocks each in turn, at one or two rows (more were slower than the kernel): 576 x 7168 5.66 / 5.96
-// -> 5.48 / 5.50, 10240 x 8192 17.2 / 19.7 -> 16.7 / 16.6.  Each pass with its own maxima, scale and branch on it: 16 x 7168 x 16384 27.0.
+// with the rows of its next k-block in flight while it waits for its stage.  Every CTA does so for all k-blocks it multiplies, which
+// is less work than the weights take to arrive, and saves a kernel and the hand-over from it.
+//
+// Eight rows are the limit (smallm_quantises) because of what these loads take where the rows have just been written by another kernel:
+// by the times of calls about 2 us beside the weight stream, against the 2.8 us in which 112 CTAs go through ten k-blocks.  With one or two passes of
+// conversion that fits in, with three or four it does not, and every k-block waits.  With registers for four passes the block also left
+// no room on its SM for another kernel's (94 a thread now, 127 then).  Graph of calls, quantiser kernel / this, us, at 4 / 8 rows:
+// 576 x 7168 6.2 / 6.4 -> 4.8 / 5.1, 24576 x 1536 10.4 / 10.3 -> 8.6 / 8.7, 7168 x 16384 23.6 / 24.1 -> 21.7 / 21.9, 36864 x 7168 42.3 / 42.2 ->
+// 40.5 / 40.6.  The same with rms_norm before each call and a bf16 matmul, softmax and top-k behind it, this less the kernel, at 4 / 8 rows:
+// -0.7 / -1.0, 0.0 / -0.2, -0.9 / -1.0, -0.6 / -0.2; with three and four passes, at 9 / 16 rows: +0.3 / +0.8, +1.1 / +2.5, +3.2 / +5.1, +3.1 /
+// +4.7, which a graph of nothing but such calls did not show (24.7 -> 23.1 at 16 x 7168 x 16384).  Five projections of a layer in
+// turn: 140 -> 138 / 139, and 153 / 161 at 9 / 16 rows.  Rows asked for into the L2 ahead: level where they were not there, 1 us
+// slower where they were.
 //
 // A warp's wait for a stage looks at one parity, which is right only if the stage's k-block before last is known to be done; the
 // warp's wait for its own k-block before this one says so if that one is at most a ring back (commits arrive in order).
 constexpr int kQuantRows = 2;  // rows that a call may pass without scratch
-constexpr int kMaxQuantRows = 16, kQuantWarps = 10;
+constexpr int kQuantWarps = 10;
 static_assert(kQuantWarps <= Cfg<16>::kStages, "see above");
 
 template <typename T, int PASSES, bool UE, bool CLUSTER>
 __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, uint8_t* smem, float* scale_ring, uint32_t me, int lane,
-                                                   int32_t total) {
+                                              int32_t total) {
   using C = Cfg<16>;
-  static_assert(kMaxQuantRows == C::kTile && PASSES <= 4, "four rows a pass");
+  static_assert(kMaxQuantRows == 8 && (PASSES == 1 || PASSES == 2), "four rows a pass");
   const uint32_t full0 = ptx::smem_u32(&ctl->full[0]), done0 = ptx::smem_u32(&ctl->done[0]);
   const int rows = p.M, sub = lane & 7, r0 = lane >> 3;  // eight lanes, sixteen elements each, take a row of a pass
   const uint4* row[PASSES];
 #pragma unroll
   for (int u = 0; u < PASSES; ++u)  // rows past the last one are read as the last one, and not stored
     row[u] = reinterpret_cast<const uint4*>(static_cast<const T*>(p.x) + (int64_t)min(4 * u + r0, rows - 1) * p.K) + 2 * sub;
-  // Rows that are not in the L2 yet: every CTA asks for a share of them at once, or each k-block would wait for HBM in its turn:
-  // 16 x 7168 x 16384 over two sets of rows and weights, called from Python, 25.0 -> 23.6 us.
-  if (me == 0) {
-    const char* x = static_cast<const char*>(p.x);
-    for (int64_t at = ((int64_t)blockIdx.x * 32 + lane) * 128; at < (int64_t)rows * p.K * 2; at += (int64_t)gridDim.x * 32 * 128)
-      ptx::prefetch_l2(x + at);
-  }
   const float inv_max = __frcp_rn(448.0f);
-  const int scale_row = 4 * (sub >> 1) + r0;  // the row whose scale this lane computes
-  const bool has_scale = (sub & 1) == 0 && scale_row < rows;
+  const int scale_row = sub + r0;  // the row whose scale this lane has, if it is lane 0 or 4 of the eight
+  const bool has_scale = (sub & 3) == 0 && scale_row < rows;
   uint32_t stage = me, phase = 0, slot = me;
   int32_t i = (int32_t)me;  // this warp's next k-block, counted from the item's first
   for (int32_t t = blockIdx.x; t < total; t += gridDim.x) {
@@ -337,16 +336,16 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
     const int32_t n = it.kb1 - it.kb0;
     if (i < n) fetch(it.kb0 + i);
     for (; i < n; i += kQuantWarps) {
-      // Maxima of all passes at once: two lanes end up with the maximum of each pass's row, and with one scale and one
-      // reciprocal to compute for it.
-      float m[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        m[u] = u < PASSES ? fmaxf(Elem<T>::vec_absmax(v[u < PASSES ? u : 0][0]), Elem<T>::vec_absmax(v[u < PASSES ? u : 0][1])) : 1.f;
-      const bool up = (sub & 4) != 0, odd = (sub & 2) != 0;
-      const float x0 = fmaxf(up ? m[2] : m[0], __shfl_xor_sync(0xffffffffu, up ? m[0] : m[2], 4));
-      const float x1 = fmaxf(up ? m[3] : m[1], __shfl_xor_sync(0xffffffffu, up ? m[1] : m[3], 4));
-      float amax = fmaxf(odd ? x1 : x0, __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 2));
+      // Maxima of both passes at once: lanes 0 to 3 of a row's eight end up with that of the first pass, 4 to 7 with the second's
+      float amax = fmaxf(Elem<T>::vec_absmax(v[0][0]), Elem<T>::vec_absmax(v[0][1]));
+      float other = amax;  // what the lane four away is to have
+      if constexpr (PASSES == 2) {
+        const float second = fmaxf(Elem<T>::vec_absmax(v[1][0]), Elem<T>::vec_absmax(v[1][1]));
+        if (sub & 4) amax = second;
+        else other = second;
+      }
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, other, 4));
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
       amax = fmaxf(p.eps, fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1)));
       uint4 codes[PASSES];
       float s;
@@ -356,11 +355,11 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
         const float r = __frcp_rn(s);
 #pragma unroll
         for (int u = 0; u < PASSES; ++u)
-          codes[u] = encode16_e4m3<T, true>(v[u][0], v[u][1], __shfl_sync(0xffffffffu, s, 2 * u, 8), __shfl_sync(0xffffffffu, r, 2 * u, 8));
+          codes[u] = encode16_e4m3<T, true>(v[u][0], v[u][1], __shfl_sync(0xffffffffu, s, 4 * u, 8), __shfl_sync(0xffffffffu, r, 4 * u, 8));
       } else {
         s = group_scale_fast(amax, 448.0f, inv_max, UE);
 #pragma unroll
-        for (int u = 0; u < PASSES; ++u) codes[u] = encode16_e4m3<T>(v[u][0], v[u][1], __shfl_sync(0xffffffffu, s, 2 * u, 8));
+        for (int u = 0; u < PASSES; ++u) codes[u] = encode16_e4m3<T>(v[u][0], v[u][1], __shfl_sync(0xffffffffu, s, 4 * u, 8));
       }
       const float prod = s * b;
       if (i + kQuantWarps < n) fetch(it.kb0 + i + kQuantWarps);
@@ -369,7 +368,7 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
 #pragma unroll
       for (int u = 0; u < PASSES; ++u) {
         const int r = 4 * u + r0;
-        if (r < rows) *reinterpret_cast<uint4*>(dst + r * 128 + ((sub ^ (r & 7)) << 4)) = codes[u];  // 128-byte swizzle
+        if (r < rows) *reinterpret_cast<uint4*>(dst + r * 128 + ((sub ^ r) << 4)) = codes[u];  // 128-byte swizzle
       }
       if (has_scale) scale_ring[slot * C::kTile + scale_row] = prod;
       ptx::fence_proxy_async();  // the MMA reads shared memory through the asynchronous proxy
@@ -387,11 +386,9 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
 
 template <typename T, bool UE, bool CLUSTER>
 __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, uint8_t* smem, float* scale_ring, uint32_t me, int lane,
-                                                   int32_t total) {
+                                              int32_t total) {
   if (p.M <= 4) quantise_rows<T, 1, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
-  else if (p.M <= 8) quantise_rows<T, 2, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
-  else if (p.M <= 12) quantise_rows<T, 3, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
-  else quantise_rows<T, 4, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
+  else quantise_rows<T, 2, UE, CLUSTER>(p, ctl, smem, scale_ring, me, lane, total);
 }
 
 // One CTA's share of a tile whose K a cluster of RANKS cuts.  A piece is 16 weight rows x 8 tokens of a warp's 32 x MT sums, 16 bytes a
@@ -942,15 +939,11 @@ constexpr int kMaxChunkedRows = 256;  // two chunks, fp32 scales: see takes_few_
 
 int smallm_quant_rows() { return kQuantRows; }
 
-// Whether the GEMM quantises M rows itself rather than after the quantiser kernel.  Above eight rows the ten warps' instructions begin to
-// show; graph of calls, quantiser kernel / this, us.  More than two tiles a CTA, each with all of its k-blocks again: 12 x 57344 x 8192
-// 75.5 / 77.1.  Above twelve rows also: long ranges of K on too few CTAs for HBM to be the limit, 16 x 10240 x 8192 18.1 / 18.6, and
-// clusters of eight on most of the SMs, 16 x 2112 x 7168 8.4 / 8.8 (16 x 1536 x 7168, 96 CTAs, 7.8 / 7.8).
-bool smallm_quantises(int64_t M, int64_t N, int64_t K, int sm_count) {
-  if (M <= 8) return true;
-  const int64_t n_tiles = (N + BN - 1) / BN, c = smallm_cluster(M, N, K, sm_count, false), ctas = n_tiles * c, kb = K / BK / c;
-  if (M > kMaxQuantRows || n_tiles > 2 * sm_count) return false;
-  return M <= 12 || ((ctas >= 88 || kb <= 24) && (c < kMaxCluster || ctas <= 96));
+// Whether the GEMM quantises M rows itself rather than after the quantiser kernel: up to eight (see quantise_rows), and where no CTA has
+// more than two tiles, each with all of its k-blocks to convert again: 4 / 8 x 57344 x 8192 among other kernels 99.5 / 100.5 -> 101.3 /
+// 102.1 us, 36864 x 7168 (two tiles) 67.5 / 67.6 -> 67.0 / 67.4.  One and two rows have no scratch for the kernel.
+bool smallm_quantises(int64_t M, int64_t N, int sm_count) {
+  return M <= kQuantRows || (M <= kMaxQuantRows && (N + BN - 1) / BN <= 2 * (int64_t)sm_count);
 }
 
 // From 65 rows up a k-block takes this kernel 390 ns where clusters share K, 360 alone, and the 128 x 128 kernel 250: where every CTA works alone,

@@ -303,7 +303,6 @@ __device__ __forceinline__ void mma_f8f6f4(uint32_t d_tmem, uint64_t a_desc, uin
 __device__ __forceinline__ void mma_commit_a(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // One k-block: four MMAs 32 bytes of K apart (+2 in the descriptors' address fields, inside the 128-byte swizzle atom), the first of
 // which overwrites D, then the commit, issued by the lane whose `pred` holds.  The whole warp runs through them with a predicate
 // instead of one lane through a branch.
