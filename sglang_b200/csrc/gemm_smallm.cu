@@ -568,17 +568,19 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         const bool mine = NSUB == 1 || rows > 0;  // uniform over the warp
         uint32_t v[2 * 4 * G];
         float2 s[G];
+        // The loads and the wait for them stand in one block: with a wait in a block of its own, behind the same condition, the
+        // registers pass the point where the two join before they have been filled, where nothing keeps the compiler from copying them.
         if (mine) {
           tmem_ld_16x256<G>(taddr, v);
           tmem_ld_16x256<G>(taddr + (16u << 16), v + 4 * G);
 #pragma unroll
           for (int g = 0; g < G; ++g) s[g] = ptx::ld_shared_f32x2(sc_row + slot + 32 * g);
+          tmem_ld_fence<8 * G>(v);
         }
         column = column >= (C::kAcc - 1) * C::kTile ? sub * MT : column + C::kTile;
         phase ^= done_at == (C::kStages - 1) * 8;
         done_at = done_at == (C::kStages - 1) * 8 ? 0 : done_at + 8;
         slot = slot == (C::kScaleSlots - 1) * C::kSlotBytes ? 0 : slot + C::kSlotBytes;
-        if (mine) tmem_ld_fence<8 * G>(v);
         // this TMEM stage and these scales have been read: the k-block kAcc further on may have the stage
         ptx::tc_fence_before();
         __syncwarp();
