@@ -364,6 +364,7 @@ __device__ __forceinline__ void quantise_rows(const SmallParams& p, Ctl* ctl, ui
       const float prod = s * b;
       if (i + kQuantWarps < n) fetch(it.kb0 + i + kQuantWarps);
       if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 11); return; }
+      (void)ptx::mbar_test_wait_a(full0 + stage * 8, phase ^ 1);  // the promotion warps have read this slot: see there
       uint8_t* dst = smem + (size_t)stage * C::kStageBytes + kWBytes;
 #pragma unroll
       for (int u = 0; u < PASSES; ++u) {
@@ -563,6 +564,11 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
           ok = false;
           break;
         }
+        // The scales come from another warp's ordinary stores, released through `full`; the commit on `done` says nothing of them, nor,
+        // to the warp that writes the slot again, of these reads.  `full` of a k-block is complete when `done` is (the MMAs were issued
+        // after) and cannot go on before this warp has read the sums, nor before the scales of the stage's next k-block are there.  So
+        // the answer needs no look: it is asked for its acquire, and nothing waits for it (0 to 1.6 % of a call).
+        (void)ptx::mbar_test_wait_a(full0 + done_at, phase);
         ptx::tc_fence_after();
         const uint32_t taddr = tlane + column;
         const bool mine = NSUB == 1 || rows > 0;  // uniform over the warp
@@ -845,6 +851,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
         for (int u = 0; u < kScaleGroup; ++u) {
           if (u >= n) break;
           if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 16); ok = false; break; }
+          (void)ptx::mbar_test_wait_a(full0 + stage * 8, phase ^ 1);  // the promotion warps have read this slot: see there
 #pragma unroll
           for (int h = 0; h < kPerLane; ++h)
             if (C::kTile >= 32 || lane < C::kTile) scale_ring[slot * C::kTile + lane + 32 * h] = v[h][u];
