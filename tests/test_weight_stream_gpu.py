@@ -173,6 +173,84 @@ def test_up_to_eight_rows_quantised_by_the_gemm(N, K, dtype, M, ue8m0):
         assert torch.equal(on_top.view(torch.int16), want.view(torch.int16))
 
 
+def _linear(x, w, ws, ue8m0, eps, in_parts):
+    """The C linear layer, or the quantiser kernel followed by the GEMM entry."""
+    from sglang_b200._lib import check, lib
+    L, (M, K), N, kind = lib(), x.shape, w.shape[0], 0 if x.dtype == torch.bfloat16 else 1
+    stream = torch.cuda.current_stream().cuda_stream
+    out = torch.full((M, N), 7.0, dtype=x.dtype, device="cuda")
+    if not in_parts:
+        scratch = torch.empty(L.sglb200_fp8_block_linear_scratch_bytes(M, N, K, int(ue8m0)) + 256, dtype=torch.uint8, device="cuda")
+        check(L.sglb200_fp8_block_linear(x.data_ptr(), w.data_ptr(), ws.data_ptr(), None, out.data_ptr(), M, N, K, ws.stride(0), ws.stride(1),
+                                         int(ue8m0), eps, kind, scratch.data_ptr(), scratch.numel(), stream), "fp8_block_linear")
+        return out
+    ld = (M + 3) // 4 * 4
+    q = torch.empty(M, K, dtype=torch.float8_e4m3fn, device="cuda")
+    s = torch.zeros(-(-K // 512) if ue8m0 else K // 128, ld, dtype=torch.int32 if ue8m0 else torch.float32, device="cuda")
+    check(L.sglb200_per_token_group_quant_fp8(x.data_ptr(), kind, q.data_ptr(), s.data_ptr(), M, K, 128, eps, -448.0, 448.0, int(ue8m0), 1,
+                                              ld, stream), "per_token_group_quant_fp8")
+    if ue8m0:
+        check(L.sglb200_fp8_ue8m0_scaled_mm(q.data_ptr(), w.data_ptr(), s.data_ptr(), ws.data_ptr(), out.data_ptr(), M, N, K, K, K, N, ld,
+                                            ws.stride(0), ws.stride(1), kind, stream), "fp8_ue8m0_scaled_mm")
+    else:
+        check(L.sglb200_fp8_blockwise_scaled_mm(q.data_ptr(), w.data_ptr(), s.data_ptr(), ws.data_ptr(), out.data_ptr(), M, N, K, K, K, N, 1,
+                                                ld, ws.stride(0), ws.stride(1), kind, stream), "fp8_blockwise_scaled_mm")
+    return out
+
+
+@pytest.mark.parametrize("ue8m0", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M", [1, 2, 4, 7, 8])
+def test_odd_values_quantised_by_the_gemm(M, dtype, ue8m0):
+    """NaN, infinities, denormals and groups of zeros with no floor, rows that begin on 16 bytes and no more, a limit on the SMs and
+    a captured graph: what the quantiser kernel and the GEMM give, bit for bit (a NaN for a NaN)."""
+    from sglang_b200._lib import lib
+    N, K, L = 1160, 1408, lib()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    room = torch.randn(M * K + 8, generator=g, device="cuda").to(dtype)
+    x = room[8:].view(M, K)  # 16 bytes past the allocation's alignment
+    assert x.data_ptr() % 32 == 16
+    w = (torch.randn(N, K, generator=g, device="cuda") * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    if ue8m0:
+        ws = torch.randint(120, 130, (-(-N // 128), 12), generator=g, device="cuda", dtype=torch.uint8).view(torch.int32)
+    else:
+        ws = torch.rand(-(-N // 128), K // 128, generator=g, device="cuda") + 0.5
+    tiny = torch.finfo(dtype).smallest_normal
+
+    def same(got, want):
+        nan = want.isnan()
+        return torch.equal(got.isnan(), nan) and torch.equal(got[~nan].view(torch.int16), want[~nan].view(torch.int16))
+
+    odd = {"plain": lambda: None, "nan": lambda: x[M // 2, 130:133].fill_(float("nan")),
+           "nan group": lambda: x[M - 1, 256:384].fill_(float("nan")), "inf": lambda: x[0, 5].fill_(float("-inf")),
+           "zeros": lambda: x[M // 2, 512:640].zero_(), "denormals": lambda: x[M - 1, 640:768].fill_(tiny / 4),
+           "minus zero": lambda: x[0, 768:800].fill_(-0.0)}
+    for name, put in odd.items():
+        x.copy_(torch.randn(M, K, generator=g, device="cuda"))
+        put()
+        for eps in (1e-10, 0.0):
+            got, want = _linear(x, w, ws, ue8m0, eps, False), _linear(x, w, ws, ue8m0, eps, True)
+            assert same(got, want), f"{name}, eps {eps}"
+    x.copy_(torch.randn(M, K, generator=g, device="cuda"))
+    want = _linear(x, w, ws, ue8m0, 1e-10, True)
+    try:
+        assert L.sglb200_set_num_sms(5) == 0  # ten tiles at most: two each
+        assert same(_linear(x, w, ws, ue8m0, 1e-10, False), _linear(x, w, ws, ue8m0, 1e-10, True))
+    finally:
+        assert L.sglb200_set_num_sms(0) == 0
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = _linear(x, w, ws, ue8m0, 1e-10, False)
+    keep = x.clone()
+    x.zero_()
+    graph.replay()
+    assert (out == 0).all()
+    x.copy_(keep)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert same(out, want) and L.sglb200_read_device_status() == 0
+
+
 @pytest.mark.parametrize("ue8m0", [False, True])
 @pytest.mark.parametrize("M", [1, 7, 9, 16, 17, 31, 33, 64, 65, 100, 121, 128])
 @pytest.mark.parametrize("N,K,dtype", [(1000, 7168, torch.bfloat16), (4072, 4096, torch.float16), (7112, 7168, torch.bfloat16)])
