@@ -176,10 +176,13 @@ int sglb200_fp8_blockwise_scaled_mm(const void* a, const void* b, const float* s
  * G with scratch for split-K.  When the output tiles alone cannot occupy the SMs the kernel is bound by streaming the
  * weights; cutting K into ranges that run on different SMs restores the bandwidth.  Above 128 rows the ranges write fp32
  * partial sums to `workspace` ([splits, M, N] floats) and a second small kernel adds them in ascending split order and
- * casts; up to 128 rows the CTAs of a cluster share a tile's K and add up on the chip, with or without `workspace`.
+ * casts; up to 128 rows, and in narrow layers up to 256, the CTAs of a cluster share a tile's K and add up on the chip, with or
+ * without `workspace`.
  * sglb200_fp8_blockwise_scaled_mm_workspace_bytes() returns a sufficient size for a shape on the current device (0 = K is
  * not cut; up to 128 rows the size of a split through memory, which this kernel does without).
- * sglb200_fp8_blockwise_scaled_mm_scratch_bytes() returns what the call really makes use of (0 = a workspace changes nothing).  With workspace == NULL or a workspace that is too small the call is exactly sglb200_fp8_blockwise_scaled_mm.
+ * sglb200_fp8_blockwise_scaled_mm_scratch_bytes() returns what the call can make use of (0 = a workspace changes nothing; from 129 to
+ * 256 rows the size of the split that clusters stand in for, which then stays untouched).
+ * With workspace == NULL or a workspace that is too small the call is exactly sglb200_fp8_blockwise_scaled_mm.
  * The workspace is scratch: contents on entry are ignored, calls on the same stream may share it.  Replaces the per-call
  * cudaMalloc'ed CUTLASS workspace of the reference (sgl-kernel/csrc/gemm/fp8_blockwise_gemm_kernel.cu:162-163) and its
  * stream-K path (sgl-kernel/csrc/cutlass_extensions/gemm/fp8_blockwise_gemm_sm90_dispatch.cuh:179-197).
@@ -201,8 +204,9 @@ int sglb200_fp8_blockwise_scaled_mm_ws(const void* a, const void* b, const float
  *   bias [N] of dtype or NULL: added to the rounded product, one more rounding, as `output += bias` does
  *   out [M, N] of dtype, contiguous;  eps as in sglb200_per_token_group_quant_fp8 (already rounded to dtype)
  *   scratch: sglb200_fp8_block_linear_scratch_bytes(M, N, K, scale_ue8m0) bytes, 256-byte aligned, contents arbitrary.
- *   At 0 bytes (one or two rows, which the GEMM quantises itself) it may be NULL.  out may lie on top of x; at one or two rows the
- *   call then needs the scratch of three (M = 3) and is refused without any.
+ *   At 0 bytes (one or two rows) it may be NULL.  Up to eight rows the GEMM quantises x itself, in layers of up to 256 output columns
+ *   per SM, and leaves the scratch alone.  out may lie on top of x; at one or two rows the call then needs the scratch of three
+ *   (M = 3) and is refused without any.
  * Replaces: w8a8_block_fp8_linear  python/sglang/srt/layers/quantization/fp8_utils.py:184-301.
  */
 int sglb200_fp8_block_linear(const void* x, const void* w, const void* w_scale, const void* bias, void* out, int64_t M,
@@ -499,7 +503,8 @@ int sglb200_moe_sum_reduce(const void* input, void* output, int64_t num_tokens, 
  * workspace / workspace_bytes: scratch for M <= 128 (size from sglb200_fp8_blockwise_scaled_mm_push_workspace_bytes; 0 for
  * larger M).  With it the few-rows weight-streaming kernel computes fp32 sums (K in the ranges of the plain entry) and
  * a second small kernel adds the ranges, casts and does the pushing and flagging, with the bits of the plain entry; without it
- * (NULL) the 128-row kernel with the push epilogue runs, which adds K uncut: the plain entry's bits where that does not cut K either.
+ * (NULL), and with it from 65 rows up where the plain entry does not cut K, the 128-row kernel with the push epilogue runs, which adds
+ * K uncut: the plain entry's bits where that does not cut K either.
  * A wait that runs out (a rank that never pushed) leaves its tile unwritten, sets device status 5
  * (sglb200_read_device_status) and does not advance the epoch, so the same exchange can be reduced again once the
  * missing rank has pushed; if only some ranks timed out the group is out of step and the buffers must be set up

@@ -1197,7 +1197,8 @@ int splitk_choice(int64_t M, int64_t N, int64_t K, int sm_count, int64_t* ns = n
 }
 
 // K ranges whose sums a dense call puts into its scratch; up to smallm_max_rows() K is added up on the chip.  Above, a call that
-// takes_few_rows has with clusters leaves the scratch alone; its size stays what callers know.
+// takes_few_rows gives to clusters is answered with the ranges that the tile kernel would cut, and leaves that scratch alone: the
+// size stays what callers know.
 int dense_splits(int64_t M, int64_t N, int64_t K, int sm_count) {
   return M > smallm_max_rows() ? splitk_choice(M, N, K, sm_count) : 1;
 }
@@ -1287,7 +1288,8 @@ int gemm_common(const void* a, const void* b, const float* sa, const float* sb, 
   if (!grouped && push && total_rows <= smallm_max_rows() && takes_few_rows(total_rows, N, K, di.sm_count, false) && workspace != nullptr &&
       (int64_t)smallm_cluster(total_rows, N, K, di.sm_count, false) * total_rows * N <= workspace_floats) {
     // few rows, exchanged: the weight-streaming kernel leaves fp32 sums, a second kernel casts and pushes them.  K is cut as
-    // for the plain entry (smallm_cluster), which makes the bits the same.  Both kernels against the ranges that a split through
+    // for the plain entry (smallm_cluster), which makes the bits the same.  From 65 rows up only where clusters share K: alone, the
+    // 128-row kernel below pushes its tiles itself, K uncut as in the plain entry, and leaves the workspace alone.  Both kernels against the ranges that a split through
     // memory would choose by itself (smallm_splits), one rank, M = 16 / 64 / 128: N=7168 K=16384 30.1 / 36.6 / 45.2 against 30.5 /
     // 38.8 / 50.9 us, N=576 K=7168 10.8 / 18.1 / 26.7 against 13.6 / 33.0 / 57.8, N=8192 K=4096 level; behind only at 128 rows and
     // K = 2048 (N=7168 21.9 against 20.4).

@@ -1,20 +1,24 @@
-// Block-scaled FP8 GEMM for few rows of activations (M <= 128: the decode case), weight-streaming bound.
+// Block-scaled FP8 GEMM for few rows of activations (up to 64, or 256 where clusters share K: the decode case), weight-streaming bound.
 //
 // The roles of the operands are swapped: the tensor core computes C^T = W * A^T, a tile being 128 WEIGHT rows (the MMA's
 // M) by MT token columns (the MMA's N, MT = 16 / 32 / 64 / 128, and as few of them as the item has rows).  An accumulator
-// stage is then only MT TMEM columns wide, so 4 to 16 k-blocks are in flight between the MMA warp and the promotion warps, and
+// stage is then only MT TMEM columns wide, so 4 to 11 k-blocks are in flight between the MMA warp and the promotion warps, and
 // a shared-memory stage is 16 KB of weights plus MT x 128 bytes of activations, 6 to 11 of them: 64 KB of weights in flight
-// per SM already bring a plain stream of such tiles to 90 % of the HBM rate, 128 KB to all of it.  When
-// N / 128 tiles alone cannot occupy the SMs, the CTAs of a cluster cut a tile's K among themselves and add their sums up
-// out of each other's shared memory, each a share of the tile (smallm_cluster, add_up_share), measured with all of it on rank 0: against fp32 partial sums in memory and a kernel that adds them, quantiser
-// included, N=576 K=7168 M=1 / 48: 9.6 / 14.1 -> 6.8 / 11.1 us, N=7168 K=16384 M=48 32.3 -> 27.1, N=10240 K=8192 M=48 27.0 -> 22.1.
-// From 65 to 128 rows sixteen promotion warps share every accumulator stage, eight where clusters share K, there from 33 rows on.
+// per SM already bring a plain stream of such tiles to 90 % of the HBM rate, 128 KB to all of it.  When N / 128 tiles alone cannot
+// occupy the SMs, the CTAs of a cluster cut a tile's K among themselves and add their sums up out of each other's shared memory, each
+// a share of the tile (smallm_cluster, add_up_share).  Against fp32 partial sums in memory and a kernel that adds them, quantiser
+// included, N=576 K=7168 M=1 / 48 went 9.6 / 14.1 -> 6.8 / 11.1 us, N=7168 K=16384 M=48 32.3 -> 27.1, N=10240 K=8192 M=48 27.0 -> 22.1
+// with rank 0 adding everything; 4.7 / 7.8, 26.6 and 20.9 are calls of the present kernel.
+// Where clusters share K eight promotion warps share every accumulator stage from 33 rows on; from 65 to 128 rows without (partial
+// sums for the peer exchange, the only such calls left) sixteen do.
 //
 // One barrier each way per k-block.  `full` counts the producer's bytes, the scale loader and the promotion warps, who arrive for the
 // k-block that gets the TMEM stage they have just read; `done` is one commit, on which the producer, the scale loader and the
 // promotion warps wait.  A wait on a barrier that is ready costs its warp about 120 cycles and a commit 60: with a barrier per ring
 // (two waits, two commits) a k-block took the one issuing warp 500 cycles with everything ready, so 337, and issued under a
-// predicate instead of a branch 256 at 128 columns, which is what the MMAs take.  The promotion warps are what is left: they ask
+// predicate instead of a branch 256 at 128 columns, which is what the MMAs take.  The scales have no barrier of their own: the
+// promotion warps, who wait for `done` alone, ask `full` too, which is complete by then, so that they acquire what the loader
+// released there.  These warps are what is left: they ask
 // for the next k-block before they add, step through the rings by offsets and take four k-blocks a turn (a turn each: 4 to 10 % slower).  Two
 // waits and two commits -> this, GEMM alone, weights from HBM, us: 48 x 10240 x 8192 21.8 -> 18.6, 64 x 7168 x 16384 27.5 -> 24.6, 32 x
 // 10240 x 8192 18.0 -> 16.7, 48 x 24576 x 1536 13.2 -> 11.4, 96 x 7168 x 16384 31.4 -> 30.5, 16 x 7168 x 16384 22.2 -> 21.5.
@@ -34,9 +38,10 @@
 // The kernel is launched with programmatic stream serialization: it may start while the kernel before it (the
 // activation quantiser, or the previous layer's reduce kernel) is still running.  Its set-up and the WEIGHT tiles of the
 // first ring of stages are issued at once (up to 128 rows), ahead of griddepcontrol.wait; the activation tiles, all scales and
-// every store come after it.  The kernel starts when all blocks of the one before have ended, or have released it early: no kernel of this
-// library that could have written the weights does that (quant.cu), and callers' own kernels must not.  At decode sizes the fixed cost of a call (launch,
-// set-up, first TMA round trip) is of the order of the streaming time itself, and this hides most of it.
+// every store come after it.  The kernel starts when all blocks of the one before have ended, or have released it early: of this
+// library's kernels that write e4m3 codes only those for activations do that (quant.cu), and callers' own kernels that write weights
+// must not.  At decode sizes the fixed cost of a call (launch, set-up, first TMA round trip) is of the order of the streaming time
+// itself, and this hides most of it.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -80,11 +85,11 @@ constexpr int kAuxRegs = 96, kPromoRegs = 200;  // register split of the NSUB = 
 
 constexpr int kMaxExperts = 1024;
 
-// NSUB > 1 (65 to 128 rows per item): the MMA covers up to MT * NSUB = 128 activation rows and every set of four promotion warps
-// takes its MT of every accumulator stage's columns.  Alone on a tile, four sets of 32 columns are the better split: 16 warps hide
-// each other's chain of wait, load, hand-back and FMA (N=10240 K=8192 M=113 31.3 -> 30.1 us, N=24576 K=1536 18.7 -> 17.6, N=36864
-// K=7168 65 -> 59 against two sets of 64).  In a cluster two sets of 64 are (call, two sets / four, us: 113 x
-// 7168 x 16384 35.1 / 36.0, 128 x 576 x 7168 10.8 / 11.7, 113 x 2048 x 2048 8.8 / 9.4).
+// NSUB > 1: the MMA covers up to MT * NSUB activation rows and every set of four promotion warps takes its MT of every accumulator
+// stage's columns.  Two sets of 32 from 33 to 64 rows in a cluster (launch_cluster); at 65 to 128 rows two sets of 64 there (call, two
+// sets / four, us: 113 x 7168 x 16384 35.1 / 36.0, 128 x 576 x 7168 10.8 / 11.7, 113 x 2048 x 2048 8.8 / 9.4), and four of 32 alone on a
+// tile, where 16 warps hide each other's chain of wait, load, hand-back and FMA (measured when such calls came here: N=10240 K=8192 M=113
+// 31.3 -> 30.1 us, N=24576 K=1536 18.7 -> 17.6, N=36864 K=7168 65 -> 59 against two sets of 64).
 template <int MT, int NSUB = 1>
 struct Cfg {
   static constexpr int kTile = MT * NSUB;  // most activation rows per work item = TMEM columns per stage
@@ -451,8 +456,8 @@ __device__ __forceinline__ void add_up_share(const SmallParams& p, uint32_t loca
 // 18 % (N=36864 K=7168 M=113: 57 -> 68 us) through its register allocation.
 // QUANT: see quantise_rows.
 template <int MT, bool UE, bool GROUPED, int NSUB, bool CLUSTER, bool QUANT>
-// NSUB = 1 has 256 threads; the bound of 320 keeps it at 200 registers, so that a block of the quantiser or of another small
-// kernel (256 threads of 48) fits beside it and programmatic dependent launch really overlaps the two.
+// NSUB = 1 has 256 threads of at most 166 registers (QUANT: 512 of 94), so that a block of the quantiser or of another small kernel
+// (256 threads of 48) fits beside it and programmatic dependent launch really overlaps the two.
 __global__ void __launch_bounds__(QUANT ? 192 + 32 * kQuantWarps : (NSUB == 1 ? 320 : 128 + 128 * NSUB), 1)
 fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                              const SmallParams p) {
@@ -745,7 +750,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
           for (int i = 0; i < C::kStages; ++i)
             if (armed & (1u << i)) ptx::mbar_wait_inl_a(full0 + i * 8, (armed_phase >> i) & 1u, 20000000ull);
         } else {
-          // the last tcgen05.commit arrivals on `empty` must have landed before the CTA's shared memory is reused
+          // the last tcgen05.commit arrivals on `done` must have landed before the CTA's shared memory is reused
           for (int i = 0; i < C::kStages; ++i) {
             if (!ptx::mbar_wait_inl_a(done0 + stage * 8, phase ^ 1)) { timeout(ctl, 15); break; }
             if (++stage == C::kStages) { stage = 0; phase ^= 1; }
@@ -1112,11 +1117,13 @@ int smallm_gemm(const void* a, const void* b, const float* sa, const float* sb, 
 // kernel has no promotion to pay for and draws level much earlier (whole layer at 32 rows: 1940 us it, 1990 the chunks).
 // With a K of a few k-blocks an item is mostly start and store, of which the UE8M0 tile kernel has less (its epilogue overlaps the
 // next tile), once there are enough items for that to outweigh its later start (it is launched without programmatic overlap).
-// Measured on 11 layers of 8 to 256 experts and 2048 to 7168 columns, K = 128 to 512, 0.5 to 20 rows per expert: with up to 1400
-// items (128 weight rows of an expert that has rows) the chunks take 0.67 to 1.05 of the tile kernel's time (64 x 2048 x 256 at 4
-// rows: 12.3 against 14.4 us), with more 0.95 to 1.48 (256 x 7168 x 256 at 1 / 16 rows: 94 / 164 against 74 / 114 us).  K = 1024
-// still gives 1.0 to 1.12 there and K = 2048 0.94 to 1.02.  The fp32 tile kernel gains nothing from a short K (layer of 256 x 7168 x 256 at
-// 256 tokens: 325 against 376 us).
+// Measured when the line was drawn, on 11 layers of 8 to 256 experts and 2048 to 7168 columns, K = 128 to 512, 0.5 to 20 rows per
+// expert: with up to 1400 items (128 weight rows of an expert that has rows) the chunks took 0.67 to 1.05 of the tile kernel's time
+// (64 x 2048 x 256 at 4 rows: 12.3 against 14.4 us), with more 0.95 to 1.48; K = 1024 gave 1.0 to 1.12 there and K = 2048 0.94 to 1.02.
+// Since short items look for their scales ahead, with two loaders, the line is behind the kernel: with more than 1400 items the chunks
+// take 0.62 to 0.98 of the tile kernel's time up to K = 384 and 24 rows per expert (256 x 7168 x 256 at 1 / 4 / 16 rows: 57 / 82 / 97 against
+// 79 / 113 / 117 us), and 0.90 to 1.05 at K = 512.  It stays where it is until it is fitted again.
+// The fp32 tile kernel gains nothing from a short K (256 x 7168 x 256 at 4 rows: 151 against 82 us).
 constexpr int64_t kWideRowsMax = 48, kWideRowsMaxUe8m0 = 20, kShortKUe8m0 = 512;
 constexpr double kShortKItems = 1400.;
 
