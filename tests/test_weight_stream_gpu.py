@@ -105,7 +105,7 @@ def test_rows_quantised_by_the_gemm_itself(M, N, K, dtype, ue8m0):
 
 
 @pytest.mark.parametrize("ue8m0", [False, True])
-@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 7, 8, 9, 16])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 7, 8, 9, 12, 13, 16])
 @pytest.mark.parametrize("N,K,dtype", [(576, 7168, torch.bfloat16), (136, 640, torch.float16), (20000, 1408, torch.bfloat16),
                                        (3072, 1536, torch.float16), (1000, 128, torch.bfloat16), (37888, 256, torch.bfloat16),
                                        (37896, 256, torch.bfloat16)])
