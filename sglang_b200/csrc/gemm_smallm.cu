@@ -255,15 +255,19 @@ __device__ __forceinline__ void tmem_ld_fence(uint32_t* r) {
   for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i])::"memory");
 }
 
-// scale of k-block kc: fp32 at base[kc * stride_k], or 2^(byte - 127) of the packed word at base[(kc / 4) * stride_k]
+// The 32 bits that hold the scale of k-block kc: fp32 at base[kc * stride_k], or the packed word at base[(kc / 4) * stride_k], whose
+// byte kc % 4 stands for 2^(byte - 127).  Loads that are to stay in flight are decoded where they are used, not here.
+template <bool UE>
+__device__ __forceinline__ float load_scale_bits(const float* base, int32_t kc, int64_t stride_k) {
+  return __ldg(base + (int64_t)(UE ? kc >> 2 : kc) * stride_k);
+}
+template <bool UE>
+__device__ __forceinline__ float scale_of(float bits, int32_t kc) {
+  return UE ? __uint_as_float(((__float_as_uint(bits) >> (8 * (kc & 3))) & 0xffu) << 23) : bits;
+}
 template <bool UE>
 __device__ __forceinline__ float load_scale(const float* base, int32_t kc, int64_t stride_k) {
-  if constexpr (UE) {
-    const uint32_t w = (uint32_t)__ldg(reinterpret_cast<const int32_t*>(base) + (int64_t)(kc >> 2) * stride_k);
-    return __uint_as_float(((w >> (8 * (kc & 3))) & 0xffu) << 23);
-  } else {
-    return __ldg(base + (int64_t)kc * stride_k);
-  }
+  return scale_of<UE>(load_scale_bits<UE>(base, kc, stride_k), kc);
 }
 
 // Four 8 x 8 matrices of 16-bit values in fragment arrangement, stored transposed: lane l passes the address of row l % 8 of
@@ -792,6 +796,9 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
       // stages (quantise_rows says why not more) come to warps 2 and 3 in turn: a short item is mostly these loads' way to
       // memory and back.  One loader, which looked for its item and its rows in global memory before each fetch -> this, expert layer
       // of 256 x (7168, 256), eight a token, at 4 / 16 / 64 / 128 / 512 tokens: 67 / 146 / 272 / 306 / 347 us -> 62 / 123 / 224 / 252 / 292
+      // Exponent words are decoded where the products are formed.  Decoded at the load they had to arrive before the group ahead of them
+      // was handed over, a way to memory and back in every call and, at K = 2560, 7 % of it: UE8M0, 24 / 64 x 5120 x 2560 7.5 / 8.85 ->
+      // 7.05 / 8.4 us, 32 x 1000 x 1024 5.9 -> 5.6, 24 x 576 x 7168 6.8 -> 6.5, 48 x 10240 x 8192 21.6 -> 20.7, 48 x 36864 x 7168 level.
       if constexpr (!GROUPED) ptx::grid_dep_wait();  // the activation scales come from the kernel before this one
       constexpr int kPerLane = C::kTile / 32 > 0 ? C::kTile / 32 : 1;
       const uint32_t loaders = GROUPED && p.k_tiles < C::kStages ? 2 : 1, skip = loaders == 2 ? p.k_tiles : 0;
@@ -825,11 +832,11 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
 #pragma unroll
         for (int u = 0; u < kScaleGroup; ++u) {
           const int32_t k = min(kb + u, kb1 - 1);
-          b[u] = load_scale<UE>(sb_blk, k, p.sb_stride_k);
+          b[u] = load_scale_bits<UE>(sb_blk, k, p.sb_stride_k);
 #pragma unroll
           for (int h = 0; h < kPerLane; ++h) {
             const int32_t tok = lane + 32 * h;
-            a[h][u] = tok < rows ? load_scale<UE>(sa_base + (int64_t)tok * p.sa_stride_m, k, p.sa_stride_k) : 0.f;
+            a[h][u] = tok < rows ? load_scale_bits<UE>(sa_base + (int64_t)tok * p.sa_stride_m, k, p.sa_stride_k) : 0.f;
           }
         }
       };
@@ -843,7 +850,7 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
 #pragma unroll
         for (int h = 0; h < kPerLane; ++h)
 #pragma unroll
-          for (int u = 0; u < kScaleGroup; ++u) v[h][u] = a[h][u] * b[u];
+          for (int u = 0; u < kScaleGroup; ++u) v[h][u] = scale_of<UE>(a[h][u], kb + u) * scale_of<UE>(b[u], kb + u);
         const int32_t n = min(kScaleGroup, kb1 - kb);
         kb += kScaleGroup;
         const bool last = kb >= kb1;
