@@ -542,6 +542,9 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
     // tokens: with one weight row per thread (32x32b loads) every thread needs every token's scale, and the 64 KB of
     // broadcast scale reads per k-block of 128 tokens kept the shared memory busier than the loads and the MMAs.
     // (16x256b loads are slower, 125 against 74 cycles per k-block of 128 x 128, and still far from the bound.)
+    // Every TMEM stage is free, which waits for no other kernel: after the wait below it held the first MMA up (512 x 256 at one to
+    // nine rows 0.04 us of 2.6 to 4)
+    for (uint32_t i = 0; i < C::kAcc; ++i) ptx::mbar_arrive_if(full0 + i * 8, leader);
     if constexpr (!GROUPED) ptx::grid_dep_wait();  // the kernel before this one may still read `out` / `partial`
     constexpr int G = MT / 8;  // groups of eight tokens
     const int q = warp & 3;
@@ -553,7 +556,6 @@ fp8_block_gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __
     // columns, scales.
     uint32_t done_at = 0, phase = 0, full_at = C::kAcc % C::kStages * 8, column = sub * MT, slot = 0;
     bool ready = false;  // the next k-block's sums are known to be there
-    for (uint32_t i = 0; i < C::kAcc; ++i) ptx::mbar_arrive_if(full0 + i * 8, leader);  // every TMEM stage is free
     [[maybe_unused]] bool met = false;  // this warp has passed the cluster's first barrier
     int32_t e_last = 0;
     float2 acc[2][G][2];  // [lanes 0-15 / 16-31][token group][rows tr / tr + 8]: two neighbouring tokens
